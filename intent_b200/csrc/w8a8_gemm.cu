@@ -10,11 +10,17 @@
 // both go to shared memory unchanged through 128B-swizzled TMA boxes (A: 128 rows x 128 k,
 // B: two boxes of 128 k rows x 128 columns) and the B operand is described to the tensor core
 // as MN-major, so no transposition pass exists anywhere.  One persistent CTA per SM walks
-// 128 x 256 tiles: warp 0 issues TMA (4 stages of 48 KiB), one thread of warp 1 issues four
-// M128 N256 K32 MMAs per stage, warps 2..5 drain the two TMEM accumulators.
+// 128 x 256 tiles, or a pair of CTAs on neighbouring SMs 256 x 256 tiles (cta_group::2): warp 0
+// issues TMA (4 stages of 48 KiB; pair: 6 of 32 KiB per CTA), one thread of warp 1 issues four
+// K32 MMAs per stage, warps 2..5 drain the two TMEM accumulators.  What bounds it is the rate at
+// which operands get into and out of shared memory; the pair reads two thirds of the bytes per
+// operation.  4096 x 8192 x 8192 scaled, calls back to back: 214.7 -> 200.5 us (2.56 -> 2.74 POP/s).
 // With B_K_MAJOR the second operand is given as [N,K] (K contiguous, e.g. decoded packed weights)
 // and is loaded as one 256-row K-major box.
 // Every wait is bounded (see tma.cuh); a wait that gives up records a timeout status.
+#include <algorithm>
+
+#include "cluster.cuh"
 #include "common.cuh"
 #include "dense.cuh"
 #include "tma.cuh"
@@ -27,12 +33,18 @@ __device__ int g_w8a8_gemm_status = 0;
 namespace {
 
 constexpr int BM = 128, BN = 256, BK = 128;
-constexpr int STAGES = 4;
 constexpr int A_BYTES = BM * BK;       // 16 KiB
 constexpr int B_BOX_BYTES = BK * 128;  // one 128-column box, 16 KiB
-constexpr int B_BYTES = 2 * B_BOX_BYTES;
 constexpr int THREADS = 6 * 32;
-constexpr int SMEM_BYTES = 1024 + STAGES * (A_BYTES + B_BYTES) + 256;
+
+// CG = CTAs that share a tile: 1 = 128 x 256, 2 = a pair on neighbouring SMs computes 256 x 256, each CTA holding its
+// own 128 rows of A and half of the tile's B columns (32 KiB per k block and CTA instead of 48).
+template <int CG>
+struct Ring {
+  static constexpr int STAGES = CG == 1 ? 4 : 6;
+  static constexpr int B_BYTES = 2 * B_BOX_BYTES / CG;
+  static constexpr int SMEM_BYTES = 1024 + STAGES * (A_BYTES + B_BYTES) + 256;
+};
 
 struct I8Params {
   void* out;
@@ -43,11 +55,24 @@ struct I8Params {
   int k_blocks, m_tiles, n_tiles;
 };
 
+// Tile walk: bands of rows, the row tile varying fastest, so that the band of A and the columns of B in flight stay in L2.
+template <int CG>
+__device__ __forceinline__ void tile_coords(int tile, int m_tiles, int n_tiles, int& m_tile, int& n_tile) {
+  constexpr int BAND = 32 / CG;   // 4096 rows
+  const int band_size = BAND * n_tiles;
+  const int band = tile / band_size;
+  const int in_band = tile - band * band_size;
+  const int rows_in_band = min(BAND, m_tiles - band * BAND);
+  n_tile = in_band / rows_in_band;
+  m_tile = band * BAND + (in_band - n_tile * rows_in_band);
+}
+
 // EPILOGUE 0: bf16(acc * sa[m] * sb[n]);  1: int32 acc + bias[n]
-template <int EPILOGUE, bool B_K_MAJOR>
+template <int EPILOGUE, bool B_K_MAJOR, int CG>
 __global__ void __launch_bounds__(THREADS, 1)
 i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const I8Params p) {
+  constexpr int STAGES = Ring<CG>::STAGES, B_BYTES = Ring<CG>::B_BYTES;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -65,6 +90,8 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const int tiles = p.m_tiles * p.n_tiles;
+  const int rank = CG == 2 ? int(cluster_rank()) : 0;
+  const int first_tile = int(blockIdx.x) / CG, tile_step = int(gridDim.x) / CG;
 
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -73,13 +100,17 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(tmem_full + 8 * s, 1);
-      mbar_init(tmem_empty + 8 * s, 4);
+      mbar_init(tmem_empty + 8 * s, 4 * CG);
     }
     fence_mbar_init();
   }
-  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  if (warp == 1) {
+    if (CG == 2) tmem_alloc_pair(tmem_slot, 512);
+    else tmem_alloc(tmem_slot, 512);
+  }
   tcgen05_fence_before();
   __syncthreads();
+  if (CG == 2) cluster_sync();   // barriers of both CTAs are initialised before anything arrives remotely
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 
@@ -87,31 +118,41 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const int m_tile = tile % p.m_tiles, n_tile = tile / p.m_tiles;
+      for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
+        int m_tile, n_tile;
+        tile_coords<CG>(tile, p.m_tiles, p.n_tiles, m_tile, n_tile);
         for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           if (!mbar_wait(empty + 8 * s, ((it / STAGES) & 1) ^ 1)) { ok = false; break; }
+          const int row0 = (m_tile * CG + rank) * BM, col0 = n_tile * BN + rank * (BN / CG);
+          if (CG == 2) {   // the bytes of both CTAs complete on the leader's barrier
+            if (rank == 0) mbar_expect_tx(full + 8 * s, 2 * (A_BYTES + B_BYTES));
+            const uint32_t bar = map_to_rank(full + 8 * s, 0);
+            tma_load_2d_pair(smem_a + s * A_BYTES, &map_a, kb * BK, row0, bar);
+            if (B_K_MAJOR) tma_load_2d_pair(smem_b + s * B_BYTES, &map_b, kb * BK, col0, bar);
+            else tma_load_2d_pair(smem_b + s * B_BYTES, &map_b, col0, kb * BK, bar);
+            continue;
+          }
           const uint32_t bar = full + 8 * s;
           mbar_expect_tx(bar, A_BYTES + B_BYTES);
-          tma_load_2d(smem_a + s * A_BYTES, &map_a, kb * BK, m_tile * BM, bar);
+          tma_load_2d(smem_a + s * A_BYTES, &map_a, kb * BK, row0, bar);
           if (B_K_MAJOR) {
-            tma_load_2d(smem_b + s * B_BYTES, &map_b, kb * BK, n_tile * BN, bar);
+            tma_load_2d(smem_b + s * B_BYTES, &map_b, kb * BK, col0, bar);
           } else {
-            tma_load_2d(smem_b + s * B_BYTES, &map_b, n_tile * BN, kb * BK, bar);
-            tma_load_2d(smem_b + s * B_BYTES + B_BOX_BYTES, &map_b, n_tile * BN + 128, kb * BK, bar);
+            tma_load_2d(smem_b + s * B_BYTES, &map_b, col0, kb * BK, bar);
+            tma_load_2d(smem_b + s * B_BYTES + B_BOX_BYTES, &map_b, col0 + 128, kb * BK, bar);
           }
         }
       }
       if (!ok) atomicExch(&g_w8a8_gemm_status, INTENT_B200_ERR_TIMEOUT);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (lane == 0 && rank == 0) {   // the leader issues for the pair
       // s32 accumulator, signed 8-bit operands, A K-major, B MN-major (N contiguous)
-      constexpr uint32_t idesc = umma_idesc(2, 1, 1, 0, B_K_MAJOR ? 0 : 1, BM, BN);
+      constexpr uint32_t idesc = umma_idesc(2, 1, 1, 0, B_K_MAJOR ? 0 : 1, CG * BM, BN);
       uint32_t it = 0, local = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++local) {
+      for (int tile = first_tile; tile < tiles && ok; tile += tile_step, ++local) {
         const uint32_t acc = local & 1;
         if (!mbar_wait(tmem_empty + 8 * acc, ((local >> 1) & 1) ^ 1)) { ok = false; break; }
         tcgen05_fence_after();
@@ -125,28 +166,35 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const uint64_t desc_b = B_K_MAJOR ? umma_desc_k_major_sw128(smem_b + s * B_BYTES)
                                             : umma_desc_mn_major_sw128(smem_b + s * B_BYTES, B_BOX_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < BK / 32; ++kk)
+          for (int kk = 0; kk < BK / 32; ++kk) {
             // A: 32 k = 32 bytes along its 128-byte row (2 units); B: 32 k rows of 128 bytes (256 units)
-            umma_i8(tmem_d, desc_a + uint64_t(2 * kk), desc_b + uint64_t((B_K_MAJOR ? 2 : 256) * kk), idesc,
-                    (kb | kk) != 0);
-          umma_commit(empty + 8 * s);
+            const uint64_t a = desc_a + uint64_t(2 * kk), b = desc_b + uint64_t((B_K_MAJOR ? 2 : 256) * kk);
+            if (CG == 2) umma_i8_pair(tmem_d, a, b, idesc, (kb | kk) != 0);
+            else umma_i8(tmem_d, a, b, idesc, (kb | kk) != 0);
+          }
+          if (CG == 2) umma_commit_pair(empty + 8 * s);
+          else umma_commit(empty + 8 * s);
         }
-        if (ok) umma_commit(tmem_full + 8 * acc);
+        if (ok) {
+          if (CG == 2) umma_commit_pair(tmem_full + 8 * acc);
+          else umma_commit(tmem_full + 8 * acc);
+        }
       }
       if (!ok) atomicExch(&g_w8a8_gemm_status, INTENT_B200_ERR_TIMEOUT);
     }
   } else {
     const int quadrant = warp & 3;
     uint32_t local = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
-      const int m_tile = tile % p.m_tiles, n_tile = tile / p.m_tiles;
+    for (int tile = first_tile; tile < tiles; tile += tile_step, ++local) {
+      int m_tile, n_tile;
+        tile_coords<CG>(tile, p.m_tiles, p.n_tiles, m_tile, n_tile);
       const uint32_t acc = local & 1;
       if (!__all_sync(0xffffffffu, mbar_wait(tmem_full + 8 * acc, (local >> 1) & 1))) {
         if (lane == 0) atomicExch(&g_w8a8_gemm_status, INTENT_B200_ERR_TIMEOUT);
         break;
       }
       tcgen05_fence_after();
-      const int row = m_tile * BM + quadrant * 32 + lane;
+      const int row = (m_tile * CG + rank) * BM + quadrant * 32 + lane;
       const uint32_t taddr = tmem_base + acc * BN + (uint32_t(quadrant * 32) << 16);
       float row_scale = 0.f;
       if (EPILOGUE == 0 && row < p.M) row_scale = p.a_scales[row];
@@ -196,15 +244,20 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(tmem_empty + 8 * acc);
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_remote(map_to_rank(tmem_empty + 8 * acc, 0));
+        else mbar_arrive(tmem_empty + 8 * acc);
+      }
     }
   }
 
   tcgen05_fence_before();
   __syncthreads();
+  if (CG == 2) cluster_sync();   // the peer's shared memory and TMEM stay alive until both CTAs are done
   if (warp == 1) {
     tcgen05_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    if (CG == 2) tmem_dealloc_pair(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -216,6 +269,51 @@ int device_sms() {
     return value;
   }();
   return sms;
+}
+
+struct I8Operands {
+  View2 a, b;
+  int64_t M, N, K;
+};
+
+template <int EPILOGUE, bool B_K_MAJOR, int CG>
+int launch(const I8Operands& q, I8Params& p, int sms, cudaStream_t stream) {
+  p.m_tiles = int((q.M + CG * BM - 1) / (CG * BM));
+  p.n_tiles = int((q.N + BN - 1) / BN);
+  CUtensorMap map_a, map_b;
+  if (!make_tensor_map_2d(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, q.a.p, uint64_t(q.M), uint64_t(q.K), uint64_t(q.K), BM,
+                          BK, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !(B_K_MAJOR ? make_tensor_map_2d(&map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, q.b.p, uint64_t(q.N), uint64_t(q.K),
+                                       uint64_t(q.K), BN / CG, BK, CU_TENSOR_MAP_SWIZZLE_128B)
+                  : make_tensor_map_2d(&map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, q.b.p, uint64_t(q.K), uint64_t(q.N),
+                                       uint64_t(q.N), BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)))
+    return INTENT_B200_ERR_UNSUPPORTED;
+  auto kernel = i8_gemm_kernel<EPILOGUE, B_K_MAJOR, CG>;
+  constexpr int smem = Ring<CG>::SMEM_BYTES;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return cuda_status(e);
+  const int tiles = p.m_tiles * p.n_tiles;
+  const int grid = CG * std::min(tiles, sms / CG);
+  if (LaunchFacts* sink = observe_sink())
+    return record_launch(sink, reinterpret_cast<const void*>(kernel),
+                         CG == 2 ? "i8_gemm_kernel CTA pairs, 256x256 tiles" : "i8_gemm_kernel 128x256 tiles, two accumulators",
+                         grid, THREADS, smem, CG);
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(unsigned(grid), 1, 1);
+  config.blockDim = dim3(THREADS, 1, 1);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = CG;
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = CG > 1 ? 1 : 0;
+  e = cudaLaunchKernelEx(&config, kernel, map_a, map_b, p);
+  if (e != cudaSuccess) return cuda_status(e);
+  note_launch();
+  return launch_status();
 }
 
 // b is [K,N] (N contiguous), or [N,K] (K contiguous) with B_K_MAJOR
@@ -240,26 +338,14 @@ int run(View2 a, View2 b, void* out, const int32_t* bias, const float* sa, const
   p.N = int(N);
   p.K = int(K);
   p.k_blocks = int((K + BK - 1) / BK);
-  p.m_tiles = int((M + BM - 1) / BM);
-  p.n_tiles = int((N + BN - 1) / BN);
-  CUtensorMap map_a, map_b;
-  if (!make_tensor_map_2d(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, a.p, uint64_t(M), uint64_t(K), uint64_t(K), BM, BK,
-                          CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !(B_K_MAJOR ? make_tensor_map_2d(&map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, b.p, uint64_t(N), uint64_t(K), uint64_t(K),
-                                       BN, BK, CU_TENSOR_MAP_SWIZZLE_128B)
-                  : make_tensor_map_2d(&map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, b.p, uint64_t(K), uint64_t(N), uint64_t(N),
-                                       BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)))
-    return INTENT_B200_ERR_UNSUPPORTED;
-  auto kernel = i8_gemm_kernel<EPILOGUE, B_K_MAJOR>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-  if (e != cudaSuccess) return cuda_status(e);
-  const int tiles = p.m_tiles * p.n_tiles;
-  if (LaunchFacts* sink = observe_sink())
-    return record_launch(sink, reinterpret_cast<const void*>(kernel), "i8_gemm_kernel 128x256 tiles, two accumulators",
-                         tiles < sms ? tiles : sms, THREADS, SMEM_BYTES, 1);
-  kernel<<<tiles < sms ? tiles : sms, THREADS, SMEM_BYTES, stream>>>(map_a, map_b, p);
-  note_launch();
-  return launch_status();
+  const I8Operands q{a, b, M, N, K};
+  // A pair tile reads two thirds of the operand bytes per operation but covers 256 rows: it is taken unless the 128-row
+  // tiles fill clearly fewer waves of the chip.
+  const int64_t n_tiles = (N + BN - 1) / BN;
+  const int64_t single_waves = ((M + BM - 1) / BM * n_tiles + sms - 1) / sms;
+  const int64_t paired_waves = ((M + 2 * BM - 1) / (2 * BM) * n_tiles + sms / 2 - 1) / std::max(1, sms / 2);
+  if (sms >= 2 && M > BM && paired_waves * 9 <= single_waves * 10) return launch<EPILOGUE, B_K_MAJOR, 2>(q, p, sms, stream);
+  return launch<EPILOGUE, B_K_MAJOR, 1>(q, p, sms, stream);
 }
 
 }  // namespace
