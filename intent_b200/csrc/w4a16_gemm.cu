@@ -9,10 +9,11 @@
 // One persistent CTA per SM walks output tiles of (MT * 128) rows x 256 columns; 22 warps in
 // four roles:
 //   warp 0        TMA producer: per 64-wide k block MT 128B-swizzled boxes of X (128 rows x 64 k).
-//   warps 6..21   dequantisers: two threads per weight column of the tile, each expanding half of
-//                 the k block (four packed words).  A thread reads its packed words straight from
-//                 global memory (a warp reads 128 contiguous bytes per packed row; three k blocks
-//                 are kept in flight in registers), expands them to values of T with the
+//   warps 6..21   dequantisers: sets of BN / 32 warps (one thread per weight column of the tile)
+//                 take turns at the k blocks (eight packed words per thread and block).  A thread
+//                 reads its packed words straight from global memory (a warp reads 128 contiguous
+//                 bytes per packed row; three blocks are kept in flight in registers), expands
+//                 them to values of T with the
 //                 magic-number trick (prmt + lop3, exact subtract, one rounding multiply by the
 //                 scale) and writes them into the 128-byte row n of the K-major, 128B-swizzled B
 //                 operand tile.  Shared memory therefore carries each weight once (the operand
@@ -24,8 +25,13 @@
 //   warps 2..5    epilogue: tcgen05.ld the accumulators (each warp its 32-lane TMEM quadrant),
 //                 convert, store.  With MT = 1 two accumulators alternate so the epilogue of a
 //                 tile overlaps the next tile's MMAs; with MT = 2 the two row blocks fill TMEM.
-// Shared-memory bandwidth is what bounds this kernel (operand reads by the tensor core, operand
-// tile writes, TMA writes); MT = 2 halves the B traffic per flop.  Tiles are walked in bands of
+// What bounds it is the dequantiser warps: about 18 instructions per packed word and a hundred per
+// k block and warp whatever the block holds (the wait, the loads' addresses, the proxy fence, the
+// arrival).  With two threads on a column, all sixteen warps paid the hundred on every k block; in
+// sets they pay it on every second one, and the loads have twice as long to arrive.  Measured
+// (bf16, group 128, graph replay): M77 K14336 N4096 223 -> 156 us, M256 K4096 N14336 75 -> 60;
+// the MoE prefill contractions (16384 tokens, 64 experts, 4096 x 1408) 1077 + 590 -> 848 + 504.
+// MT = 2 halves the B traffic per flop.  Tiles are walked in bands of
 // rows so that the band of X and all of W stay in L2.
 // Every wait is bounded; a wait that gives up records INTENT_B200_ERR_TIMEOUT and the CTA drains
 // and frees its TMEM.
@@ -61,24 +67,29 @@ int64_t w4a16_prelayout_words(int64_t K, int64_t N);
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64;
+constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;  // one 128-row box of X, 16 KiB
-constexpr int B_BYTES = BN * BK * 2;  // dequantised operand tile, 32 KiB
-constexpr int DEQUANT_WARPS = 16;          // two threads per weight column, each expands half a k block
-constexpr int DQ_PARTS = DEQUANT_WARPS / 8;  // threads per column
-constexpr int DQ_ROWS = (BK / 8) / DQ_PARTS; // packed words per thread and k block
+constexpr int DEQUANT_WARPS = 16;
+constexpr int DQ_ROWS = BK / 8;       // packed words per thread and k block
 constexpr int THREADS = (6 + DEQUANT_WARPS) * 32;
 constexpr int BAND_TILES = 8;         // row tiles per band of the tile walk
 
 constexpr int PAIR_LIST_BLOCKS = 8192;  // most 128-row blocks the in-kernel block pairing handles
 
-template <int MT>
+template <int MT, int BN>
 struct Stages {
-  static constexpr int A = MT == 1 ? 5 : 3;   // stages of X
-  static constexpr int B = 3;                 // stages of the dequantised tile
-  static constexpr int SMEM = 1024 + A * MT * A_BYTES + B * B_BYTES + 256;
+  static constexpr int B_BYTES = BN * BK * 2;         // dequantised operand tile
+  // Sets of BN / 32 dequantiser warps (one thread per weight column) take turns at the k blocks; every set has a
+  // stage of its own to write, and the tensor core is given at least one more.
+  static constexpr int SETS = DEQUANT_WARPS * 32 / BN;
+  static constexpr int B = BN == 256 ? (MT == 1 ? 5 : 3) : SETS + 2;   // stages of the dequantised tile
+  static constexpr int A = MT == 2 ? 3 : BN == 256 ? 4 : 7;            // stages of X
+  static constexpr int BARS = (16 * (A + B) + 8 * 4 + 16 + 255) / 256 * 256;
+  static constexpr int SMEM = 1024 + A * MT * A_BYTES + B * B_BYTES + BARS;
   // grouped modes with two row blocks per tile keep the list of block pairs behind the barriers
   static constexpr int SMEM_PAIRED = SMEM + PAIR_LIST_BLOCKS * 2 + 16;
+  static_assert(SMEM_PAIRED <= 227 * 1024 || MT == 1, "shared memory of one CTA");
+  static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
 };
 
 struct GemmParams {
@@ -122,10 +133,11 @@ __device__ __forceinline__ void tile_coords(int tile, int m_tiles, int n_tiles, 
   m_tile = band * BAND_TILES + (in_band - n_tile * rows_in_band);
 }
 
-template <typename T, int MODE, int MT>
+template <typename T, int MODE, int MT, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
-  constexpr int A_STAGES = Stages<MT>::A, B_STAGES = Stages<MT>::B;
+  using Plan = Stages<MT, BN>;
+  constexpr int A_STAGES = Plan::A, B_STAGES = Plan::B, B_BYTES = Plan::B_BYTES, DQ_SETS = Plan::SETS;
   constexpr int ACC_BUFFERS = 2 / MT;       // accumulator sets that alternate between tiles
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -157,7 +169,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
       mbar_init(empty_a + 8 * s, 1);
     }
     for (int s = 0; s < B_STAGES; ++s) {
-      mbar_init(full_b + 8 * s, DEQUANT_WARPS);
+      mbar_init(full_b + 8 * s, DEQUANT_WARPS / DQ_SETS);
       mbar_init(empty_b + 8 * s, 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -394,8 +406,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
     }
   } else {
     // ------------------------------ dequantisers --------------------------------
-    const int n = (tid - 6 * 32) & 255;   // accumulator column of the tile owned by this thread, 0..255
-    const int part = (tid - 6 * 32) >> 8; // which DQ_ROWS packed rows of every k block it expands
+    const int n = (tid - 6 * 32) & (BN - 1);   // accumulator column of the tile owned by this thread
+    const int set = (tid - 6 * 32) / BN;       // this thread expands k blocks set, set + DQ_SETS, ... of the CTA's sequence
     const uint32_t magic = Elem<T>::kMagic2 ^ (p.twos_complement ? 0x00080008u : 0u);
     const uint32_t row_off = uint32_t(n) * 128u;
     const uint32_t swz = uint32_t(n & 7);
@@ -407,17 +419,24 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
       uint32_t w[DQ_ROWS];
       uint32_t s_lo, s_hi;  // scale of k 0..31 and of k 32..63 of the block, duplicated into both halves
     };
-    // Fetch state: walks this CTA's (tile, k block) sequence in order, three blocks ahead of the
-    // consumer; everything that depends only on the tile is recomputed when the tile changes.
+    // Fetch state: walks this set's share of the CTA's (tile, k block) sequence in order, three blocks ahead of
+    // the consumer; everything that depends only on the tile is recomputed when the tile changes.
     const int group_shift = 31 - __clz(p.group_size);  // the group size is a power of two
-    int f_tile = int(blockIdx.x), f_kb = 0, f_left = total;
+    int f_tile = int(blockIdx.x), f_kb = set, f_left = (total - set + DQ_SETS - 1) / DQ_SETS;
+    bool f_new = true;   // the tile has changed
     bool f_col_ok = false;
     const uint32_t* f_w = p.packed;
     const uint16_t* f_s = p.scales;
     auto fetch = [&](Block& b) {
       if (f_left <= 0) return;
       --f_left;
-      if (f_kb == 0) {
+      while (f_kb >= p.k_blocks) {
+        f_kb -= p.k_blocks;
+        f_tile += int(gridDim.x);
+        f_new = true;
+      }
+      if (f_new) {
+        f_new = false;
         int m_tile, n_tile;
         tile_coords(f_tile, m_tiles, p.n_tiles, m_tile, n_tile);
         int first_block, halves;
@@ -434,29 +453,30 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
         }
         f_w = p.packed + size_t(expert) * packed_rows * p.WN + (f_col_ok ? col : 0);
         f_s = p.scales + size_t(expert) * scale_rows * p.WN + (f_col_ok ? col : 0);
-        if (p.prelaid) {   // per expert: [column block of 128][k block][part][column][4 words]
+        if (p.prelaid) {   // per expert: [column block of 128][k block][half of the k block][column][4 words]
           const size_t column_blocks = size_t(p.WN + 127) >> 7;
-          const size_t expert_words = column_blocks * p.k_blocks * DQ_PARTS * 128 * 4;
-          f_w = p.packed + size_t(expert) * expert_words +
-                ((size_t(col >> 7) * p.k_blocks * DQ_PARTS + part) * 128 + (col & 127)) * 4;
+          const size_t expert_words = column_blocks * p.k_blocks * 2 * 128 * 4;
+          f_w = p.packed + size_t(expert) * expert_words + (size_t(col >> 7) * p.k_blocks * 2 * 128 + (col & 127)) * 4;
           if (!f_col_ok) f_w = p.packed;   // a column past WN: any valid address, the words are not used
         }
+        f_w += size_t(f_kb) * (p.prelaid ? (f_col_ok ? size_t(2) * 128 * 4 : 0) : size_t(BK / 8) * p.WN);
       }
-      const int rows_left = packed_rows - f_kb * (BK / 8) - part * DQ_ROWS;
+      const int rows_left = packed_rows - f_kb * (BK / 8);
       if (p.prelaid) {
-        // tiled copy: this thread's four words of the k block are one 16-byte load (rows past K are zeros)
-        static_assert(DQ_ROWS == 4 && DQ_PARTS == 2, "the tiled layout is two halves of four words per column");
+        // tiled copy: this thread's words of the k block are two 16-byte loads (rows past K are zeros)
+        static_assert(DQ_ROWS == 8, "the tiled layout is two halves of four words per column");
         const uint4 v = __ldg(reinterpret_cast<const uint4*>(f_w));
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(f_w + (f_col_ok ? 128 * 4 : 0)));
         const bool use = f_col_ok;
         b.w[0] = use ? v.x : 0u; b.w[1] = use ? v.y : 0u; b.w[2] = use ? v.z : 0u; b.w[3] = use ? v.w : 0u;
+        b.w[4] = use ? u.x : 0u; b.w[5] = use ? u.y : 0u; b.w[6] = use ? u.z : 0u; b.w[7] = use ? u.w : 0u;
       } else if (f_col_ok && rows_left >= DQ_ROWS) {
-        const uint32_t* q = f_w + size_t(part * DQ_ROWS) * p.WN;
+        const uint32_t* q = f_w;
 #pragma unroll
         for (int r = 0; r < DQ_ROWS; ++r, q += p.WN) b.w[r] = __ldg(q);
       } else {
 #pragma unroll
-        for (int r = 0; r < DQ_ROWS; ++r)
-          b.w[r] = (f_col_ok && r < rows_left) ? __ldg(f_w + size_t(part * DQ_ROWS + r) * p.WN) : 0u;
+        for (int r = 0; r < DQ_ROWS; ++r) b.w[r] = (f_col_ok && r < rows_left) ? __ldg(f_w + size_t(r) * p.WN) : 0u;
       }
       const int g0 = (f_kb * BK) >> group_shift;
       const int g1 = p.group_size < BK ? g0 + 1 : g0;
@@ -464,11 +484,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
       const uint32_t c = g1 == g0 ? a : ((f_col_ok && g1 < scale_rows) ? __ldg(f_s + size_t(g1) * p.WN) : 0u);
       b.s_lo = a | (a << 16);
       b.s_hi = c | (c << 16);
-      f_w += p.prelaid ? (f_col_ok ? size_t(DQ_PARTS) * 128 * 4 : 0) : size_t(BK / 8) * p.WN;
-      if (++f_kb == p.k_blocks) {
-        f_kb = 0;
-        f_tile += int(gridDim.x);
-      }
+      f_w += DQ_SETS * (p.prelaid ? (f_col_ok ? size_t(2) * 128 * 4 : 0) : size_t(BK / 8) * p.WN);
+      f_kb += DQ_SETS;
     };
     bool ok = true;
     auto consume = [&](int i, const Block& b) {
@@ -479,7 +496,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
       const uint32_t dst = smem_b + t * B_BYTES + row_off;
 #pragma unroll
       for (int j = 0; j < DQ_ROWS; ++j) {
-        const int r = part * DQ_ROWS + j;   // packed row (16-byte chunk) of the k block
+        const int r = j;   // packed row (16-byte chunk) of the k block
         const uint32_t w = b.w[j], w4 = w >> 4;
         const uint32_t scale2 = r < 4 ? b.s_lo : b.s_hi;
         uint4 o;
@@ -503,12 +520,12 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
     fetch(b0);
     fetch(b1);
     fetch(b2);
-    for (int i = 0; i < total && ok; i += 3) {
+    for (int i = set; i < total && ok; i += 3 * DQ_SETS) {
       consume(i, b0);
       fetch(b0);
-      consume(i + 1, b1);
+      consume(i + DQ_SETS, b1);
       fetch(b1);
-      consume(i + 2, b2);
+      consume(i + 2 * DQ_SETS, b2);
       fetch(b2);
     }
     if (!ok && lane == 0) atomicExch(&g_w4a16_gemm_status, INTENT_B200_ERR_TIMEOUT);
@@ -533,7 +550,7 @@ int device_sms() {
 }
 
 // x: [rows, K] activations; w: [E, K/8, WN] packed; s: [E, K/G, WN] scales; out: [rows, out_cols].
-template <typename T, int MODE, int MT>
+template <typename T, int MODE, int MT, int BN = 256>
 int launch_gemm(const void* x, int64_t rows, int64_t K, const void* w, const void* s, int64_t WN, void* out,
                 int64_t out_cols, int group_size, int zero_point, const int* total_rows, const int* tile_expert,
                 cudaStream_t stream, bool pair_blocks = false, int64_t experts = 1, const int* row_route = nullptr,
@@ -571,8 +588,8 @@ int launch_gemm(const void* x, int64_t rows, int64_t K, const void* w, const voi
                           CU_TENSOR_MAP_SWIZZLE_128B))
     return INTENT_B200_ERR_UNSUPPORTED;
 
-  auto kernel = w4a16_gemm_kernel<T, MODE, MT>;
-  constexpr int smem = (MODE != MODE_DENSE && MT == 2) ? Stages<MT>::SMEM_PAIRED : Stages<MT>::SMEM;
+  auto kernel = w4a16_gemm_kernel<T, MODE, MT, BN>;
+  constexpr int smem = (MODE != MODE_DENSE && MT == 2) ? Stages<MT, BN>::SMEM_PAIRED : Stages<MT, BN>::SMEM;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_status(e);
   const int tiles = p.m_tiles * p.n_tiles;

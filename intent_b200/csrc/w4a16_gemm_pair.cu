@@ -39,10 +39,11 @@ constexpr int MT = 2;                       // 128-row blocks per CTA
 constexpr int PAIR_ROWS = 2 * MT * BM;      // 512
 constexpr int A_BYTES = BM * BK * 2;        // one 128-row box of X
 constexpr int B_HALF_BYTES = (BN / 2) * BK * 2;  // this CTA's half of the operand tile, 16 KiB
-constexpr int A_STAGES = 3, B_STAGES = 4;
+constexpr int A_STAGES = 3, B_STAGES = 6;
 constexpr int DEQUANT_WARPS = 16;
-constexpr int DQ_PARTS = DEQUANT_WARPS * 32 / (BN / 2);  // threads per weight column (4)
-constexpr int DQ_ROWS = (BK / 8) / DQ_PARTS;             // packed words per thread and k block (2)
+constexpr int DQ_SETS = DEQUANT_WARPS * 32 / (BN / 2);   // sets of four warps (a thread per weight column) that
+                                                         // take turns at the k blocks
+constexpr int DQ_ROWS = BK / 8;                          // packed words per thread and k block
 constexpr int THREADS = (6 + DEQUANT_WARPS) * 32;
 constexpr int SMEM_BYTES = 1024 + A_STAGES * MT * A_BYTES + B_STAGES * B_HALF_BYTES + 256;
 constexpr int BAND_TILES = 4;               // 512-row tiles per band of the tile walk
@@ -97,8 +98,8 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairPara
       mbar_init(empty_a + 8 * s, 1);
     }
     for (int s = 0; s < B_STAGES; ++s) {
-      // leader: its own dequantiser warps + one relayed arrival for the peer's; peer: its own warps
-      mbar_init(full_b + 8 * s, rank == 0 ? DEQUANT_WARPS + 1 : DEQUANT_WARPS);
+      // the set of dequantiser warps that writes the stage; leader: + one relayed arrival for the peer's set
+      mbar_init(full_b + 8 * s, DEQUANT_WARPS / DQ_SETS + (rank == 0 ? 1 : 0));
       mbar_init(empty_b + 8 * s, 1);
     }
     mbar_init(tmem_full, 1);
@@ -230,7 +231,7 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairPara
     // ------------------------------ dequantisers (both CTAs, own half of the columns) -------
     const int dq = tid - 6 * 32;
     const int n = dq & (BN / 2 - 1);        // row of this CTA's operand tile = weight column of its half
-    const int part = dq / (BN / 2);         // which DQ_ROWS packed rows of every k block
+    const int set = dq / (BN / 2);          // expands k blocks set, set + DQ_SETS, ... of the pair's sequence
     const uint32_t magic = Elem<T>::kMagic2 ^ (p.twos_complement ? 0x00080008u : 0u);
     const uint32_t row_off = uint32_t(n) * 128u;
     const uint32_t swz = uint32_t(n & 7);
@@ -243,43 +244,48 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairPara
       uint32_t w[DQ_ROWS];
       uint32_t s_lo, s_hi;
     };
-    int f_tile = pair, f_kb = 0, f_left = total;
+    int f_tile = pair, f_kb = set, f_left = (total - set + DQ_SETS - 1) / DQ_SETS;
+    bool f_new = true;   // the tile has changed
     bool f_col_ok = false;
     const uint32_t* f_w = p.packed;
     const uint16_t* f_s = p.scales;
     auto fetch = [&](Block& b) {
       if (f_left <= 0) return;
       --f_left;
-      if (f_kb == 0) {
+      while (f_kb >= p.k_blocks) {
+        f_kb -= p.k_blocks;
+        f_tile += pairs;
+        f_new = true;
+      }
+      if (f_new) {
+        f_new = false;
         int m_tile, n_tile;
         pair_tile_coords(f_tile, p.m_tiles, p.n_tiles, m_tile, n_tile);
         const int col = n_tile * BN + int(rank) * (BN / 2) + n;
         f_col_ok = col < p.N;
         f_w = p.packed + (f_col_ok ? col : 0);
         f_s = p.scales + (f_col_ok ? col : 0);
-        // tiled copy: [column block of 128][k block][half of the k block][column][4 words].  This kernel puts four
-        // threads on a column (DQ_ROWS = 2 words each): thread `part` takes words 2 * (part & 1) .. + 1 of half
-        // part >> 1.  A column past N reads word 0 of the buffer, unused.
+        // tiled copy: [column block of 128][k block][half of the k block][column][4 words]; a column past N reads
+        // the first words of the buffer, unused
         if (p.prelaid)
-          f_w = f_col_ok ? p.packed + ((size_t(col >> 7) * p.k_blocks * 2 + (part >> 1)) * 128 + (col & 127)) * 4 +
-                               (part & 1) * 2
-                         : p.packed;
+          f_w = f_col_ok ? p.packed + (size_t(col >> 7) * p.k_blocks * 2 * 128 + (col & 127)) * 4 : p.packed;
+        f_w += size_t(f_kb) * (p.prelaid ? (f_col_ok ? size_t(2) * 128 * 4 : 0) : size_t(BK / 8) * p.N);
       }
-      const int rows_left = packed_rows - f_kb * (BK / 8) - part * DQ_ROWS;
+      const int rows_left = packed_rows - f_kb * (BK / 8);
       if (p.prelaid) {
-        // tiled copy: this thread's words of the k block are adjacent (rows past K are stored as zeros)
-        static_assert(DQ_ROWS == 2, "the tiled fetch below reads this thread's two words as one 8-byte load");
-        const uint2 v = __ldg(reinterpret_cast<const uint2*>(f_w));
-        b.w[0] = f_col_ok ? v.x : 0u;
-        b.w[1] = f_col_ok ? v.y : 0u;
+        // tiled copy: this thread's words of the k block are two 16-byte loads (rows past K are stored as zeros)
+        static_assert(DQ_ROWS == 8, "the tiled layout is two halves of four words per column");
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(f_w));
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(f_w + (f_col_ok ? 128 * 4 : 0)));
+        b.w[0] = f_col_ok ? v.x : 0u; b.w[1] = f_col_ok ? v.y : 0u; b.w[2] = f_col_ok ? v.z : 0u; b.w[3] = f_col_ok ? v.w : 0u;
+        b.w[4] = f_col_ok ? u.x : 0u; b.w[5] = f_col_ok ? u.y : 0u; b.w[6] = f_col_ok ? u.z : 0u; b.w[7] = f_col_ok ? u.w : 0u;
       } else if (f_col_ok && rows_left >= DQ_ROWS) {
-        const uint32_t* q = f_w + size_t(part * DQ_ROWS) * p.N;
+        const uint32_t* q = f_w;
 #pragma unroll
         for (int r = 0; r < DQ_ROWS; ++r, q += p.N) b.w[r] = __ldg(q);
       } else {
 #pragma unroll
-        for (int r = 0; r < DQ_ROWS; ++r)
-          b.w[r] = (f_col_ok && r < rows_left) ? __ldg(f_w + size_t(part * DQ_ROWS + r) * p.N) : 0u;
+        for (int r = 0; r < DQ_ROWS; ++r) b.w[r] = (f_col_ok && r < rows_left) ? __ldg(f_w + size_t(r) * p.N) : 0u;
       }
       const int g0 = (f_kb * BK) >> group_shift;
       const int g1 = p.group_size < BK ? g0 + 1 : g0;
@@ -287,11 +293,8 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairPara
       const uint32_t c = g1 == g0 ? a : ((f_col_ok && g1 < scale_rows) ? __ldg(f_s + size_t(g1) * p.N) : 0u);
       b.s_lo = a | (a << 16);
       b.s_hi = c | (c << 16);
-      f_w += p.prelaid ? (f_col_ok ? size_t(2) * 128 * 4 : 0) : size_t(BK / 8) * p.N;
-      if (++f_kb == p.k_blocks) {
-        f_kb = 0;
-        f_tile += pairs;
-      }
+      f_w += DQ_SETS * (p.prelaid ? (f_col_ok ? size_t(2) * 128 * 4 : 0) : size_t(BK / 8) * p.N);
+      f_kb += DQ_SETS;
     };
     bool ok = true;
     auto consume = [&](int i, const Block& b) {
@@ -302,7 +305,7 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairPara
       const uint32_t dst = smem_b + t * B_HALF_BYTES + row_off;
 #pragma unroll
       for (int j = 0; j < DQ_ROWS; ++j) {
-        const int r = part * DQ_ROWS + j;
+        const int r = j;
         const uint32_t w = b.w[j], w4 = w >> 4;
         const uint32_t scale2 = r < 4 ? b.s_lo : b.s_hi;
         uint4 o;
@@ -322,17 +325,14 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairPara
       __syncwarp();
       if (lane == 0) mbar_arrive(full_b + 8 * t);  // CTA-local; the peer's arrivals are relayed by its warp 1
     };
-    Block b0, b1, b2;
+    Block b0, b1;
     fetch(b0);
     fetch(b1);
-    fetch(b2);
-    for (int i = 0; i < total && ok; i += 3) {
+    for (int i = set; i < total && ok; i += 2 * DQ_SETS) {
       consume(i, b0);
       fetch(b0);
-      consume(i + 1, b1);
+      consume(i + DQ_SETS, b1);
       fetch(b1);
-      consume(i + 2, b2);
-      fetch(b2);
     }
     if (!ok && lane == 0) atomicExch(&g_w4a16_pair_status, INTENT_B200_ERR_TIMEOUT);
   }
