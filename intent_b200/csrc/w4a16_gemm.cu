@@ -62,6 +62,7 @@ __device__ int g_w4a16_gemm_status = 0;
 template <typename T>
 int w4a16_gemm_pair(const void* x, int64_t M, int64_t K, const void* w, const void* s, int64_t N, void* y,
                     int group_size, int zero_point, cudaStream_t stream, bool prelaid);
+bool w4a16_gemm_pairs_enabled();
 int w4a16_gemm_pair_take_status(int* value);
 int64_t w4a16_prelayout_words(int64_t K, int64_t N);
 
@@ -596,11 +597,49 @@ int launch_gemm(const void* x, int64_t rows, int64_t K, const void* w, const voi
   const int grid = tiles < sms ? tiles : sms;
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel),
-                         MT == 2 ? "w4a16_gemm_kernel single CTA, 256x256 tiles" : "w4a16_gemm_kernel single CTA, 128x256 tiles",
+                         MT == 2      ? "w4a16_gemm_kernel single CTA, 256x256 tiles"
+                         : BN == 256 ? "w4a16_gemm_kernel single CTA, 128x256 tiles"
+                         : BN == 128 ? "w4a16_gemm_kernel single CTA, 128x128 tiles"
+                         : BN == 64  ? "w4a16_gemm_kernel single CTA, 128x64 tiles"
+                                     : "w4a16_gemm_kernel single CTA, 128x32 tiles",
                          grid, THREADS, smem, 1);
   kernel<<<grid, THREADS, smem, stream>>>(map_x, p);
   note_launch();
   return launch_status();
+}
+
+// Which tile a dense call runs on: the fewest waves of tiles, weighted by what a k block costs on each form.  The
+// weights are microseconds per k block measured on one tile per SM (bf16, group 128); the k blocks are the same
+// number for all forms.  A wide tile expands the most weights per microsecond, a narrow one spreads a small call over
+// the chip: M77 K14336 N4096 is 16 tiles of 256 columns (156 us), 32 of 128 (94), 64 of 64 (86) or 128 of 32 (81);
+// M512 K2048 N4096 8 pair tiles (33.6 us), 64 of 256 columns (25.6) or 128 of 128 (19.2); M1024 K4096 N4096 32 pair
+// tiles (58.9 us) or 128 of 256 columns (50.3).  Large calls stay on the pairs (M2048 K4096 N4096 59.9 us against
+// 88.2).  All forms add the k blocks in the same order, so the bits of a row do not depend on the form.
+enum class Form { PAIR, TWO_BLOCKS, N256, N128, N64, N32 };
+
+Form choose_form(int64_t M, int64_t N, bool pairs) {
+  const int64_t sms = device_sms() > 0 ? device_sms() : 1;
+  struct Candidate {
+    Form form;
+    int rows, columns, sms_per_tile;
+    double cost;
+  };
+  static const Candidate candidates[] = {
+      {Form::PAIR, 512, 256, 2, 0.86}, {Form::TWO_BLOCKS, 256, 256, 1, 0.86}, {Form::N256, 128, 256, 1, 0.73},
+      {Form::N128, 128, 128, 1, 0.43}, {Form::N64, 128, 64, 1, 0.38},         {Form::N32, 128, 32, 1, 0.36}};
+  Form best = Form::TWO_BLOCKS;
+  double least = 0.0;
+  for (const Candidate& c : candidates) {
+    if (c.form == Form::PAIR && (!pairs || M < c.rows || sms < 2)) continue;
+    const int64_t tiles = ((M + c.rows - 1) / c.rows) * ((N + c.columns - 1) / c.columns);
+    const int64_t at_once = sms / c.sms_per_tile;
+    const double cost = double((tiles + at_once - 1) / at_once) * c.cost;
+    if (least == 0.0 || cost < least) {
+      best = c.form;
+      least = cost;
+    }
+  }
+  return best;
 }
 
 template <typename T>
@@ -616,15 +655,26 @@ int run(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, cuda
   if (!contiguous(x) || !contiguous(w) || !contiguous(s) || !contiguous(y)) return INTENT_B200_ERR_LAYOUT;
   if (!aligned16(x.p) || !aligned16(w.p) || !aligned16(s.p) || !aligned16(y.p)) return INTENT_B200_ERR_LAYOUT;
   if (K == 0 || N % 8 != 0 || M > (1 << 24) || K > (1 << 24) || N > (1 << 24)) return INTENT_B200_ERR_UNSUPPORTED;
-  {  // large M: CTA pairs, each CTA dequantises half of every weight tile
+  const Form form = choose_form(M, N, w4a16_gemm_pairs_enabled());
+  if (form == Form::PAIR) {  // CTA pairs, each CTA dequantises half of every weight tile
     const int status = w4a16_gemm_pair<T>(x.p, M, K, w.p, s.p, N, y.p, group_size, zero_point, stream, prelaid);
     if (status != INTENT_B200_ERR_UNSUPPORTED) return status;
   }
-  if (M > BM)   // two row blocks per tile share every dequantised weight tile
-    return launch_gemm<T, MODE_DENSE, 2>(x.p, M, K, w.p, s.p, N, y.p, N, group_size, zero_point, nullptr, nullptr,
-                                         stream, false, 1, nullptr, nullptr, 0, 1, prelaid);
-  return launch_gemm<T, MODE_DENSE, 1>(x.p, M, K, w.p, s.p, N, y.p, N, group_size, zero_point, nullptr, nullptr,
-                                       stream, false, 1, nullptr, nullptr, 0, 1, prelaid);
+  const auto launch = [&](auto mt, auto columns) {
+    return launch_gemm<T, MODE_DENSE, decltype(mt)::value, decltype(columns)::value>(
+        x.p, M, K, w.p, s.p, N, y.p, N, group_size, zero_point, nullptr, nullptr, stream, false, 1, nullptr, nullptr, 0,
+        1, prelaid);
+  };
+  using std::integral_constant;
+  const integral_constant<int, 1> one{};
+  switch (form) {
+    case Form::N32: return launch(one, integral_constant<int, 32>{});
+    case Form::N64: return launch(one, integral_constant<int, 64>{});
+    case Form::N128: return launch(one, integral_constant<int, 128>{});
+    case Form::N256: return launch(one, integral_constant<int, 256>{});
+    default:   // two row blocks per tile share every dequantised weight tile
+      return launch(integral_constant<int, 2>{}, integral_constant<int, 256>{});
+  }
 }
 
 // Grouped contractions over expert-sorted rows padded to `block_rows` (128 or 256) per expert; with 256
