@@ -67,6 +67,8 @@ INTENT_B200_API int64_t intent_b200_launch_count(void);
  * take part (they launch as usual). */
 INTENT_B200_API int intent_b200_observe_begin(void* facts);
 INTENT_B200_API int intent_b200_observe_end(void);
+/* Turns so far of the process-wide switches that change which kernel an entry selects. */
+INTENT_B200_API extern int32_t intent_b200_selection_epoch;
 
 /* ------------------------------------------------------------------------
  * weight_only_int4_matmul  (W4A16)

@@ -38,6 +38,7 @@ struct LaunchFacts {
   char kernel[64];      // kernel family and the plan's distinguishing choice
 };
 LaunchFacts* observe_sink();
+void note_selection_switch();   // a process-wide switch of the kernel selection was turned
 int record_launch(LaunchFacts* sink, const void* kernel, const char* name, int grid, int threads, int dynamic_smem,
                   int cluster);
 

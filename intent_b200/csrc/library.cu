@@ -60,6 +60,15 @@ extern "C" int intent_b200_observe_end(void) {
   return INTENT_B200_OK;
 }
 
+// Counts the turns of the process-wide switches that change which kernel an entry selects, so that a caller can
+// tell whether a dry run still names the kernel of an earlier launch.
+extern "C" {
+__attribute__((visibility("default"))) int32_t intent_b200_selection_epoch = 0;
+}
+namespace ib200 {
+void note_selection_switch() { ++intent_b200_selection_epoch; }
+}  // namespace ib200
+
 extern "C" const char* intent_b200_version(void) { return "intent_b200 0.1 sm_100a"; }
 
 extern "C" const char* intent_b200_status_string(int status) {

@@ -417,5 +417,6 @@ template int w4a16_gemm_pair<__nv_bfloat16>(const void*, int64_t, int64_t, const
 
 extern "C" int intent_b200_w4a16_gemm_pairs(int32_t enable) {
   ib200::g_pair_enabled = enable ? 1 : 0;
+  ib200::note_selection_switch();
   return INTENT_B200_OK;
 }

@@ -1671,6 +1671,7 @@ extern "C" int intent_b200_w4a16_gemv_table_overlap(int32_t enable) {
 // (the results are WRONG by design for every value but 0: these launches only show where the time goes).
 extern "C" int intent_b200_w4a16_gemv_table_tune(const char* knob, int32_t value) {
   if (!knob) return INTENT_B200_ERR_NULL;
+  ib200::note_selection_switch();
   const auto is = [&](const char* name) {
     int i = 0;
     for (; name[i] && knob[i] == name[i]; ++i) {}
@@ -1701,5 +1702,6 @@ extern "C" int intent_b200_w4a16_gemv_table_tune(const char* knob, int32_t value
 
 extern "C" int intent_b200_w4a16_gemv_table_ride(int32_t enable) {
   ib200::g_table_ride = enable ? 1 : 0;
+  ib200::note_selection_switch();
   return INTENT_B200_OK;
 }

@@ -52,7 +52,13 @@ def dtype(value) -> DType:
     raise ValueError(f"unknown element type {value!r}")
 
 
-def torch_dtype(element: DType):
-    import torch
+_TORCH_DTYPES: dict = {}
 
-    return getattr(torch, _TORCH_NAMES[element.name])
+
+def torch_dtype(element: DType):
+    found = _TORCH_DTYPES.get(element.name)
+    if found is None:
+        import torch
+
+        found = _TORCH_DTYPES[element.name] = getattr(torch, _TORCH_NAMES[element.name])
+    return found

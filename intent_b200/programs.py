@@ -10,6 +10,8 @@ code written against the reference's examples binds the same way:
 """
 from __future__ import annotations
 
+from functools import cache
+
 from . import dtypes
 from .compiler import KernelDefinition
 from .errors import CompilationStageError
@@ -91,7 +93,8 @@ def _lower_w4a16(constants, device):
         _rule(lambda d: d["K"] % group == 0 and d["G"] * group == d["K"],
               lambda d: f"scales.shape[0] must be K/GROUP_SIZE with K a multiple of {group}"),
     ))
-    def workspace_bytes(d):
+    @cache
+    def workspace_query():
         import ctypes
 
         from .runtime import native
@@ -99,8 +102,10 @@ def _lower_w4a16(constants, device):
         query = native.library().intent_b200_weight_only_int4_matmul_workspace_bytes
         query.restype = ctypes.c_int64
         query.argtypes = [ctypes.c_int64] * 3
-        rows = d["M"] if kernel != "gemm" else 1 << 30
-        return int(query(rows, d["K"], d["N"])) if kernel != "gemm" else 0
+        return query
+
+    def workspace_bytes(d):
+        return int(workspace_query()(d["M"], d["K"], d["N"])) if kernel != "gemm" else 0
 
     program = NativeProgram(interface=interface, entry_name=f"intent_b200_{stem}_{act.name}",
                             constants=(group, zp), device=device, workspace=workspace_bytes,

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 from dataclasses import dataclass, field
+from functools import cached_property
 from pathlib import Path
 from typing import Any
 
@@ -60,6 +61,37 @@ _OBSERVABLE = ("intent_b200_weight_only_int4_matmul", "intent_b200_w4a16_gemv", 
                "intent_b200_bf16_gemm", "intent_b200_quantized_gemm", "intent_b200_moe_grouped_w4a16")
 
 
+class _Launched:
+    """What one invocation leaves behind for ``observation``: plain values, so no tensor is kept alive.  The
+    observation is put together when it is asked for, with the resource facts from a dry run of the same slots; on
+    every call the two took about a third of the host time of ``run``.  ``epoch`` counts the process-wide switches
+    of the kernel selection: once one has been turned since the launch, the dry run could name another kernel, and
+    the facts stay None."""
+
+    __slots__ = ("program", "slots", "views", "workspace_bytes", "status", "epoch", "seen")
+
+    def __init__(self, program, slots, views, workspace_bytes, status, epoch):
+        self.program, self.slots, self.views = program, slots, views
+        self.workspace_bytes, self.status, self.epoch = workspace_bytes, status, epoch
+        self.seen: NativeObservation | None = None
+
+    def observation(self) -> NativeObservation:
+        if self.seen is None:
+            program = self.program
+            facts = {}
+            if self.status == 0 and self.epoch == native.selection_epoch():
+                import torch
+
+                with torch.cuda.device(program.device):
+                    facts = program.observe(self.slots)
+            self.seen = NativeObservation(
+                "b200", program.entry_name, "launched" if self.status == 0 else "failed", program.constants,
+                tuple((p.name, f.shape, f.strides) for p, f in zip(program.interface.parameters, self.views)
+                      if f is not None),
+                self.workspace_bytes, self.status, **facts)
+        return self.seen
+
+
 class PreparedCall:
     """Arguments bound to one C entry; ``launch`` replays the same call."""
 
@@ -68,9 +100,8 @@ class PreparedCall:
         self.invocation = bound
         self._workspace = program.allocate_workspace(bound) if workspace is None else workspace
         self._slots = program.marshal(bound, self._workspace)
-        self._observation: NativeObservation | None = None
+        self._launched: _Launched | None = None
         self._skip = program.is_empty(bound)
-        self._facts: dict | None = None     # resource facts of this binding, observed once
 
     @property
     def outputs(self) -> tuple:
@@ -81,7 +112,7 @@ class PreparedCall:
 
     @property
     def observation(self) -> NativeObservation | None:
-        return self._observation
+        return None if self._launched is None else self._launched.observation()
 
     def inspect_configurations(self):
         raise NotImplementedError("this provider does not export structured tuning configurations")
@@ -110,42 +141,18 @@ class PreparedCall:
 
     __call__ = launch
 
-    def _observe(self, stream: int) -> dict:
-        """The same slots once more in the library's dry-run mode: nothing is launched, the entry reports the
-        kernel instance it selects for them and that instance's resource usage."""
-        program = self.program
-        if not program.entry_name.startswith(_OBSERVABLE):
-            return {}
-        library = native.library()
-        facts = _LaunchFacts()
-        if library.intent_b200_observe_begin(ctypes.byref(facts)) != 0:
-            return {}
-        try:
-            status = program.function()(*self._slots, ctypes.c_void_p(stream))
-        finally:
-            library.intent_b200_observe_end()
-        if status != 0 or not facts.valid:
-            return {}
-        return {"kernel": facts.kernel.decode(), "registers": facts.registers, "spill_bytes": facts.local_bytes,
-                "shared_static": facts.static_smem, "shared_dynamic": facts.dynamic_smem, "threads": facts.threads,
-                "grid": facts.grid, "cluster": facts.cluster}
-
     def _invoke(self) -> None:
-        import torch
-
         program = self.program
-        stream = torch.cuda.current_stream(program.device).cuda_stream
-        status = program.function()(*self._slots, ctypes.c_void_p(stream))
-        if self._facts is None:
-            self._facts = self._observe(stream) if status == 0 else {}
-        observation = NativeObservation(
-            "b200", program.entry_name, "launched" if status == 0 else "failed", program.constants,
-            tuple((p.name, f.shape, f.strides) for p, f in zip(program.interface.parameters, self.invocation.views)
-                  if f is not None),
-            sum(w.numel() * w.element_size() for w in self._workspace), int(status), **self._facts)
-        self._observation = observation
-        program._observation = observation
-        native.check(status, program.entry_name, observation)
+        status = program.function()(*self._slots, program.current_stream())
+        launched = self._launched
+        if launched is None or status or launched.status or launched.epoch != native.selection_epoch():
+            # (a repeated launch of the same binding leaves the same record)
+            launched = self._launched = _Launched(
+                program, self._slots, self.invocation.views,
+                sum(w.numel() * w.element_size() for w in self._workspace), int(status), native.selection_epoch())
+        program._launched = launched
+        if status:
+            native.check(status, program.entry_name, launched.observation())
 
 
 # Which process-wide status word the tensor-core kernels behind an entry write when a bounded wait gives up
@@ -184,7 +191,7 @@ class NativeProgram:
         self._workspace_spec = workspace     # callable(dimensions) -> workspace bytes (0 = none)
         self._stream_workspaces: dict = {}   # stream handle -> zero-initialised buffer reused by run()
         self._empty = empty                  # callable(dimensions) -> bool
-        self._observation: NativeObservation | None = None
+        self._launched: _Launched | None = None
         # where this entry's kernels record a bounded wait that gave up: the first word of its workspace
         # (read by the named C function) and / or process-wide status words with a no-argument reader
         self._workspace_status = workspace_status
@@ -213,13 +220,38 @@ class NativeProgram:
 
     @property
     def observation(self):
-        return self._observation
+        return None if self._launched is None else self._launched.observation()
 
-    @property
+    @cached_property
     def _torch_device(self):
         import torch
 
         return torch.device("cuda", self.device)
+
+    def current_stream(self) -> int:
+        """Handle of torch's current stream of this program's device."""
+        import torch
+
+        return torch._C._cuda_getCurrentRawStream(self.device)
+
+    def observe(self, slots: tuple) -> dict:
+        """The slots once more in the library's dry-run mode: nothing is launched and no memory is touched, the
+        entry reports the kernel instance it selects for them and that instance's resource usage."""
+        if not self.entry_name.startswith(_OBSERVABLE):
+            return {}
+        library = native.library()
+        facts = _LaunchFacts()
+        if library.intent_b200_observe_begin(ctypes.byref(facts)) != 0:
+            return {}
+        try:
+            status = self.function()(*slots, self.current_stream())
+        finally:
+            library.intent_b200_observe_end()
+        if status != 0 or not facts.valid:
+            return {}
+        return {"kernel": facts.kernel.decode(), "registers": facts.registers, "spill_bytes": facts.local_bytes,
+                "shared_static": facts.static_smem, "shared_dynamic": facts.dynamic_smem, "threads": facts.threads,
+                "grid": facts.grid, "cluster": facts.cluster}
 
     def check(self, workspace: tuple | None = None) -> None:
         """Read the device-side status of this entry's kernels (synchronises).  ``workspace``: the buffers of
@@ -246,7 +278,7 @@ class NativeProgram:
                 reader.argtypes = []
                 failures.append(int(reader()))
         for status in failures:
-            native.check(status, self.entry_name, self._observation)
+            native.check(status, self.entry_name, self.observation if status else None)
 
     def is_empty(self, bound: BoundArguments) -> bool:
         return bool(self._empty(bound.dimensions)) if self._empty is not None else False
@@ -265,7 +297,7 @@ class NativeProgram:
             return (torch.empty((0,), dtype=torch.uint8, device=self._torch_device),)
         if not per_stream:
             return (torch.zeros((size,), dtype=torch.uint8, device=self._torch_device),)
-        key = torch.cuda.current_stream(self.device).cuda_stream
+        key = self.current_stream()
         cached = self._stream_workspaces.get(key)
         if cached is None or cached.numel() < size:
             cached = torch.zeros((max(size, 1 << 16),), dtype=torch.uint8, device=self._torch_device)
@@ -273,18 +305,19 @@ class NativeProgram:
         return (cached,)
 
     def marshal(self, bound: BoundArguments, workspace: tuple) -> tuple:
-        slots = []
-        for parameter, value, facts in zip(self.interface.parameters, bound.arguments, bound.views):
-            if isinstance(parameter, ViewParameter):
-                slots.append(ctypes.c_void_p(facts.pointer))
-                slots += [ctypes.c_int64(int(e)) for e in facts.shape]
-                slots += [ctypes.c_int64(int(s)) for s in facts.strides]
-            else:
+        slots = []      # plain values: the entry's argument types convert them
+        for facts, value in zip(bound.views, bound.arguments):
+            if facts is None:
                 slots.append(value)
-        slots += [ctypes.c_int32(c) for c in self.constants]
+            else:
+                slots.append(facts.pointer)
+                slots += facts.shape
+                slots += facts.strides
+        slots += self.constants
         for buffer in workspace:
-            slots.append(ctypes.c_void_p(buffer.data_ptr() if buffer.numel() else None))
-            slots.append(ctypes.c_int64(buffer.numel() * buffer.element_size()))
+            size = buffer.numel() * buffer.element_size()
+            slots.append(buffer.data_ptr() if size else None)
+            slots.append(size)
         self.function(len(workspace))
         return tuple(slots)
 

@@ -77,6 +77,7 @@ class ViewFacts:
     begin: int | None
     end: int | None
     dtype: object
+    contiguous: bool = False      # known to be in canonical order and not empty
 
 
 @dataclass(slots=True)
@@ -122,20 +123,15 @@ class PublicInterface:
         # callables(dimensions: dict) -> None raising ValueError; derived relations such
         # as "packed rows * 8 == K" that tie symbolic dimensions together.
         self.dimension_rules = tuple(dimension_rules)
+        # everything below is fixed by the declaration and read on every call
+        self.views = tuple(p for p in self.parameters if isinstance(p, ViewParameter))
+        self.inputs = tuple(p for p in self.parameters if not isinstance(p, ViewParameter) or not p.output)
+        self.outputs = tuple(p for p in self.views if p.output)
+        self._allocation_errors = self.output_allocation_errors()
+        self._writable_pairs = tuple((left, right) for index, left in enumerate(self.views)
+                                     for right in self.views[index + 1:] if left.writable or right.writable)
 
     # -- views of the declaration ------------------------------------------------
-    @property
-    def views(self) -> tuple:
-        return tuple(p for p in self.parameters if isinstance(p, ViewParameter))
-
-    @property
-    def inputs(self) -> tuple:
-        return tuple(p for p in self.parameters if not isinstance(p, ViewParameter) or not p.output)
-
-    @property
-    def outputs(self) -> tuple:
-        return tuple(p for p in self.views if p.output)
-
     @property
     def mutable_inputs(self) -> tuple:
         return tuple(p for p in self.views if p.access is ViewKind.INOUT)
@@ -164,7 +160,7 @@ class PublicInterface:
         return tuple(errors)
 
     def require_output_allocation(self) -> None:
-        errors = self.output_allocation_errors()
+        errors = self._allocation_errors
         if errors:
             raise NotImplementedError(
                 "Cannot allocate the declared outputs: " + "; ".join(errors) +
@@ -187,7 +183,10 @@ class PublicInterface:
         if abstract:
             return ViewFacts(shape, strides, None, None, None, value.dtype)
         pointer = value.data_ptr()
-        begin, end = _byte_span(pointer, shape, strides, value.element_size())
+        size = value.element_size()
+        if value.numel() and value.is_contiguous():
+            return ViewFacts(shape, strides, pointer, pointer, pointer + value.numel() * size, value.dtype, True)
+        begin, end = _byte_span(pointer, shape, strides, size)
         return ViewFacts(shape, strides, pointer, begin, end, value.dtype)
 
     @staticmethod
@@ -201,7 +200,7 @@ class PublicInterface:
 
     def _check_entry_requirements(self, parameter: ViewParameter, facts: ViewFacts, abstract: bool,
                                   allocated: bool) -> None:
-        if parameter.layout == "contiguous":
+        if parameter.layout == "contiguous" and not facts.contiguous:
             expected = 1
             for extent, stride in zip(reversed(facts.shape), reversed(facts.strides)):
                 if extent != 1 and stride != expected and not abstract:
@@ -233,16 +232,22 @@ class PublicInterface:
         deferred: list = []
 
         def relate(parameter: ViewParameter, observed: ViewFacts) -> None:
-            for axis, extent in enumerate(parameter.shape):
-                message = f"{parameter.name}.shape[{axis}] violates the declared interface relation"
+            for axis, (extent, actual) in enumerate(zip(parameter.shape, observed.shape)):
                 if isinstance(extent, Derived):
-                    deferred.append((extent, observed.shape[axis], message))
-                elif isinstance(extent, int):
-                    self._check_relation(observed.shape[axis], extent, message, abstract)
+                    deferred.append((extent, actual, relation_message(parameter, axis)))
+                    continue
+                if isinstance(extent, int):
+                    expected = extent
                 elif extent in dimensions:
-                    self._check_relation(observed.shape[axis], dimensions[extent], message, abstract)
+                    expected = dimensions[extent]
                 else:
-                    dimensions[extent] = observed.shape[axis]
+                    dimensions[extent] = actual
+                    continue
+                if abstract or actual != expected:
+                    self._check_relation(actual, expected, relation_message(parameter, axis), abstract)
+
+        def relation_message(parameter: ViewParameter, axis: int) -> str:
+            return f"{parameter.name}.shape[{axis}] violates the declared interface relation"
 
         for parameter, value in zip(supplied, arguments):
             values[parameter.position] = value
@@ -276,14 +281,10 @@ class PublicInterface:
                 values[parameter.position] = value
                 facts[parameter.position] = observed
         if not abstract:
-            views = self.views
-            for index, left in enumerate(views):
-                for right in views[index + 1:]:
-                    if not (left.writable or right.writable):
-                        continue
-                    a, b = facts[left.position], facts[right.position]
-                    if byte_spans_overlap((a.begin, a.end), (b.begin, b.end)):
-                        raise NotImplementedError(
-                            f"{left.name} and {right.name}: native entry requires nonoverlapping accessed byte spans")
+            for left, right in self._writable_pairs:
+                a, b = facts[left.position], facts[right.position]
+                if byte_spans_overlap((a.begin, a.end), (b.begin, b.end)):
+                    raise NotImplementedError(
+                        f"{left.name} and {right.name}: native entry requires nonoverlapping accessed byte spans")
         outputs = tuple(values[p.position] for p in self.outputs)
         return BoundArguments(tuple(values), outputs, tuple(facts), dimensions)

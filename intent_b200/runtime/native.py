@@ -17,6 +17,7 @@ from ..errors import CompilationStageError
 _LOCK = Lock()
 _LIBRARY: ctypes.CDLL | None = None
 _ENTRIES: dict = {}
+_EPOCH: ctypes.c_int32 | None = None
 
 _CARRIERS = {"ptr": ctypes.c_void_p, "bool": ctypes.c_bool, "i8": ctypes.c_int8, "i16": ctypes.c_int16,
              "i32": ctypes.c_int32, "i64": ctypes.c_int64, "f32": ctypes.c_float, "f64": ctypes.c_double}
@@ -66,6 +67,14 @@ def entry(name: str, carriers: tuple):
             function.argtypes = [_CARRIERS[c] for c in carriers] + [ctypes.c_void_p]
             _ENTRIES[key] = function
         return function
+
+
+def selection_epoch() -> int:
+    """How often a process-wide switch of the kernel selection has been turned."""
+    global _EPOCH
+    if _EPOCH is None:
+        _EPOCH = ctypes.c_int32.in_dll(library(), "intent_b200_selection_epoch")
+    return _EPOCH.value
 
 
 def status_string(status: int) -> str:
