@@ -277,6 +277,11 @@ INTENT_B200_API int intent_b200_moe_scatter_routes(INTENT_B200_VIEW2(a0), INTENT
 /* moe_align.py:76-86: a0 offsets [E+1] -> a1 expert_blocks [B] (blocks past the padded total are not written) */
 INTENT_B200_API int intent_b200_moe_mark_expert_blocks(INTENT_B200_VIEW1(a0), INTENT_B200_VIEW1(a1),
                                                        int32_t block_size, void* stream);
+/* The four alignment programs in one launch (composition.py:98-174): a0 topk_ids [T,K] -> a1 sorted_route_ids
+ * [capacity] (span padding = T*K, past the padded total = fill), a2 expert_blocks [B], a3 total_padded [1] */
+INTENT_B200_API int intent_b200_moe_align_routes(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2),
+                                                 INTENT_B200_VIEW1(a3), int32_t experts, int32_t block_size,
+                                                 int32_t fill, void* stream);
 /* Inverse of the alignment: a0 sorted_route_ids [capacity], a1 total_padded [1] -> a2 route_positions [R] */
 INTENT_B200_API int intent_b200_moe_route_positions(INTENT_B200_VIEW1(a0), INTENT_B200_VIEW1(a1),
                                                     INTENT_B200_VIEW1(a2), void* stream);

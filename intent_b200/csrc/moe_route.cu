@@ -147,6 +147,72 @@ __global__ void moe_mark_kernel(const int* __restrict__ offsets, int experts, in
   for (int b = first + threadIdx.x; b < last && b < blocks_capacity; b += blockDim.x) blocks[b] = e;
 }
 
+// ---- align: count, prefix, scatter and mark in one launch ----
+// The four stages read 128 KiB of ids and write as little: what they cost is six launches (two of them fills) and
+// the gaps between them.  Here CTA e counts the routes of every expert in shared memory (the ids come from L2), so
+// that it knows the start of its own span without waiting for another CTA, and then partitions as above.
+__global__ void __launch_bounds__(1024)
+moe_align_kernel(const int* __restrict__ ids, int routes, int experts, int block, int* __restrict__ sorted,
+                 int sorted_capacity, int fill, int* __restrict__ blocks, int blocks_capacity,
+                 int* __restrict__ total_padded) {
+  extern __shared__ int counts[];      // [experts]
+  __shared__ int warp_count[32];
+  __shared__ int bounds[2];            // padded start of this CTA's span, padded total
+  const int e = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < experts; i += 1024) counts[i] = 0;
+  __syncthreads();
+  const int slice = ((routes + 31) / 32 + 31) / 32 * 32;          // per warp, a multiple of the warp size
+  const int first = min(routes, warp * slice), last = min(routes, first + slice);
+  int mine = 0;
+  for (int r = first + lane; r < last; r += 32) {
+    const int id = ids[r];
+    if (id >= 0 && id < experts) atomicAdd(&counts[id], 1);       // an id that names no expert is skipped
+    mine += id == e ? 1 : 0;
+  }
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, d);
+  if (lane == 0) warp_count[warp] = mine;
+  __syncthreads();
+  if (warp == 0) {
+    int before = 0, all = 0;
+    for (int i = lane; i < experts; i += 32) {
+      const int padded = (counts[i] + block - 1) / block * block;
+      all += padded;
+      if (i < e) before += padded;
+    }
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) {
+      before += __shfl_xor_sync(0xffffffffu, before, d);
+      all += __shfl_xor_sync(0xffffffffu, all, d);
+    }
+    if (lane == 0) {
+      bounds[0] = before;
+      bounds[1] = all;
+    }
+  }
+  __syncthreads();
+  const int begin = bounds[0], total = bounds[1], count = counts[e];
+  const int end = begin + (count + block - 1) / block * block;
+  int position = begin;
+  for (int w = 0; w < warp; ++w) position += warp_count[w];
+  for (int base = first; base < last; base += 32) {
+    const int r = base + lane;
+    const bool match = r < last && ids[r] == e;
+    const unsigned ballot = __ballot_sync(0xffffffffu, match);
+    if (match) {
+      const int at = position + __popc(ballot & ((1u << lane) - 1u));
+      if (at < sorted_capacity) sorted[at] = r;
+    }
+    position += __popc(ballot);
+  }
+  // the padding of the span holds the sentinel `routes`, what lies past the padded total holds `fill`
+  for (int at = begin + count + threadIdx.x; at < end && at < sorted_capacity; at += 1024) sorted[at] = routes;
+  for (int at = total + e * 1024 + threadIdx.x; at < sorted_capacity; at += experts * 1024) sorted[at] = fill;
+  for (int b = begin / block + threadIdx.x; b < end / block && b < blocks_capacity; b += 1024) blocks[b] = e;
+  if (e == 0 && threadIdx.x == 0) total_padded[0] = total;
+}
+
 // ---- positions: inverse of the alignment, position[route] = slot in the sorted layout ----
 __global__ void moe_positions_kernel(const int* __restrict__ sorted, const int* __restrict__ total, int capacity,
                                      int routes, int* __restrict__ position) {
@@ -265,6 +331,22 @@ extern "C" int intent_b200_moe_mark_expert_blocks(INTENT_B200_VIEW1(a0), INTENT_
   if (!a0 || !a1) return INTENT_B200_ERR_NULL;
   moe_mark_kernel<<<int(a0_d0 - 1), 64, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const int*>(a0), int(a0_d0 - 1), block_size, static_cast<int*>(a1), int(a1_d0));
+  note_launch();
+  return launch_status();
+}
+
+// topk_ids [T,K] -> sorted_route_ids [capacity], expert_blocks [B], total_padded [1]
+extern "C" int intent_b200_moe_align_routes(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2),
+                                            INTENT_B200_VIEW1(a3), int32_t experts, int32_t block_size,
+                                            int32_t fill, void* stream) {
+  if (a3_d0 != 1 || experts <= 0 || block_size <= 0) return INTENT_B200_ERR_SHAPE;
+  if (!a0 || !a1 || !a2 || !a3) return INTENT_B200_ERR_NULL;
+  if (!contiguous(IB200_VIEW2_ARG(a0)) || !contiguous(IB200_VIEW1_ARG(a1)) || !contiguous(IB200_VIEW1_ARG(a2)))
+    return INTENT_B200_ERR_LAYOUT;
+  if (experts > 8192) return INTENT_B200_ERR_UNSUPPORTED;
+  moe_align_kernel<<<experts, 1024, size_t(experts) * 4, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const int*>(a0), int(a0_d0 * a0_d1), experts, block_size, static_cast<int*>(a1), int(a1_d0),
+      fill, static_cast<int*>(a2), int(a2_d0), static_cast<int*>(a3));
   note_launch();
   return launch_status();
 }

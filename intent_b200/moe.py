@@ -57,8 +57,9 @@ class MoEAlignment:
     are the four alignment programs compiled with this object's token / top-k / expert / block constants
     (the reference fixes them at module level; here they are constructor arguments)."""
 
-    def __init__(self, count, prefix, scatter, mark, tokens=4096, top_k=2, experts=64, block_size=128):
+    def __init__(self, count, prefix, scatter, mark, tokens=4096, top_k=2, experts=64, block_size=128, align=None):
         self.count, self.prefix, self.scatter, self.mark = count, prefix, scatter, mark
+        self.align = align          # the four stages in one launch, for results without counters
         self.tokens, self.top_k, self.experts, self.block_size = tokens, top_k, experts, block_size
 
     @classmethod
@@ -66,7 +67,8 @@ class MoEAlignment:
         constants = {"TOKENS": tokens, "TOP_K": top_k, "EXPERTS": experts, "BLOCK_SIZE": block_size}
         stages = [_compile(getattr(programs, name), target=target, constexprs=constants,
                            resolve_target=resolve_target) for name in _ALIGN_STAGES]
-        return cls(*stages, tokens=tokens, top_k=top_k, experts=experts, block_size=block_size)
+        align = _compile(programs.moe_align_routes, target=target, constexprs=constants, resolve_target=resolve_target)
+        return cls(*stages, tokens=tokens, top_k=top_k, experts=experts, block_size=block_size, align=align)
 
     @property
     def routes(self) -> int:
@@ -99,6 +101,9 @@ class MoEAlignment:
         return sorted_routes, self.mark.run(offsets), total_padded
 
     def run(self, ids):
+        if self.align is not None:
+            self._check(ids)
+            return self.align.run(ids)
         counters, sorted_routes = self._buffers(ids.device)
         return self.run_into(ids, counters[:self.experts], counters[self.experts:], sorted_routes)
 

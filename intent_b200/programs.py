@@ -304,6 +304,18 @@ def _lower_mark(c, device):
                          device=device)
 
 
+def _lower_align(c, device):
+    tokens, top_k, experts, block, routes, padded, blocks = _align_sizes(c)
+    interface = PublicInterface((
+        ViewParameter(0, "topk_ids", dtypes.i32, ("T", top_k), IN, alignment=4),
+        ViewParameter(1, "sorted_route_ids", dtypes.i32, (padded,), OUT, alignment=4),
+        ViewParameter(2, "expert_blocks", dtypes.i32, (blocks,), OUT, alignment=4),
+        ViewParameter(3, "total_padded", dtypes.i32, (1,), OUT, alignment=4),
+    ), dimension_rules=(_rule(lambda d: d["T"] <= tokens, f"at most {tokens} tokens (TOKENS constexpr)"),))
+    return NativeProgram(interface=interface, entry_name="intent_b200_moe_align_routes", constants=(experts, block, routes),
+                         device=device)
+
+
 def _lower_positions(c, device):
     _, _, _, _, routes, padded, _ = _align_sizes(c)
     interface = PublicInterface((
@@ -323,6 +335,9 @@ moe_scatter_routes = KernelDefinition("moe_scatter_routes", dict(_ALIGN_CONSTEXP
                                       f"{_MOE_ALIGN_REF}:52-73", "stable partition of route ids by expert")
 moe_mark_expert_blocks = KernelDefinition("moe_mark_expert_blocks", dict(_ALIGN_CONSTEXPRS), _lower_mark,
                                           f"{_MOE_ALIGN_REF}:76-86", "expert of every padded block")
+moe_align_routes = KernelDefinition("moe_align_routes", dict(_ALIGN_CONSTEXPRS), _lower_align,
+                                    "examples/programs/composition.py:98-174",
+                                    "the four alignment programs in one launch")
 moe_route_positions = KernelDefinition("moe_route_positions", dict(_ALIGN_CONSTEXPRS), _lower_positions,
                                        "examples/kernels/ragged/moe.py:24-33 (member_routes indirection, inverted)",
                                        "slot of every route in the sorted layout")
@@ -477,7 +492,7 @@ moe_combine = KernelDefinition("moe_combine", {"ACCUMULATE": True}, _lower_combi
                                "examples/kernels/ragged/moe.py:48-53 (weighted scatter_reduce add)",
                                "y[t] += sum_c weight[t,c] * rows[position[t,c]] in choice order")
 
-ALL.update({d.name: d for d in (moe_count_routes, moe_prefix_routes, moe_scatter_routes, moe_mark_expert_blocks,
+ALL.update({d.name: d for d in (moe_align_routes, moe_count_routes, moe_prefix_routes, moe_scatter_routes, moe_mark_expert_blocks,
                                 moe_route_positions, moe_route_top2, moe_gather_rows, moe_grouped_upgate_silu,
                                 moe_grouped_down, moe_grouped_down_scatter, moe_combine)})
 
