@@ -62,22 +62,22 @@ _OBSERVABLE = ("intent_b200_weight_only_int4_matmul", "intent_b200_w4a16_gemv", 
 
 
 class _Launched:
-    """What one invocation leaves behind for ``observation``: plain values, so no tensor is kept alive.  The
+    """What one invocation leaves behind for ``observation``: plain values, so no tensor is kept alive, and no way
+    back to the program, which keeps the record (a cycle would hold its workspaces until a collection).  The
     observation is put together when it is asked for, with the resource facts from a dry run of the same slots; on
     every call the two took about a third of the host time of ``run``.  ``epoch`` counts the process-wide switches
     of the kernel selection: once one has been turned since the launch, the dry run could name another kernel, and
     the facts stay None."""
 
-    __slots__ = ("program", "slots", "views", "workspace_bytes", "status", "epoch", "seen")
+    __slots__ = ("slots", "views", "workspace_bytes", "status", "epoch", "seen")
 
-    def __init__(self, program, slots, views, workspace_bytes, status, epoch):
-        self.program, self.slots, self.views = program, slots, views
+    def __init__(self, slots, views, workspace_bytes, status, epoch):
+        self.slots, self.views = slots, views
         self.workspace_bytes, self.status, self.epoch = workspace_bytes, status, epoch
         self.seen: NativeObservation | None = None
 
-    def observation(self) -> NativeObservation:
+    def observation(self, program: "NativeProgram") -> NativeObservation:
         if self.seen is None:
-            program = self.program
             facts = {}
             if self.status == 0 and self.epoch == native.selection_epoch():
                 import torch
@@ -112,7 +112,7 @@ class PreparedCall:
 
     @property
     def observation(self) -> NativeObservation | None:
-        return None if self._launched is None else self._launched.observation()
+        return None if self._launched is None else self._launched.observation(self.program)
 
     def inspect_configurations(self):
         raise NotImplementedError("this provider does not export structured tuning configurations")
@@ -148,11 +148,11 @@ class PreparedCall:
         if launched is None or status or launched.status or launched.epoch != native.selection_epoch():
             # (a repeated launch of the same binding leaves the same record)
             launched = self._launched = _Launched(
-                program, self._slots, self.invocation.views,
+                self._slots, self.invocation.views,
                 sum(w.numel() * w.element_size() for w in self._workspace), int(status), native.selection_epoch())
         program._launched = launched
         if status:
-            native.check(status, program.entry_name, launched.observation())
+            native.check(status, program.entry_name, launched.observation(program))
 
 
 # Which process-wide status word the tensor-core kernels behind an entry write when a bounded wait gives up
@@ -220,7 +220,7 @@ class NativeProgram:
 
     @property
     def observation(self):
-        return None if self._launched is None else self._launched.observation()
+        return None if self._launched is None else self._launched.observation(self)
 
     @cached_property
     def _torch_device(self):
