@@ -20,7 +20,8 @@ from .compiler import compile as _compile
 from .targets import B200Target
 
 
-_ALIGN_STAGES = ("moe_count_routes", "moe_prefix_routes", "moe_scatter_routes", "moe_mark_expert_blocks")
+_ALIGN_STAGES = {"count": "moe_count_routes", "prefix": "moe_prefix_routes", "scatter": "moe_scatter_routes",
+                 "mark": "moe_mark_expert_blocks"}
 
 
 class MoEAlignmentCall:
@@ -58,17 +59,30 @@ class MoEAlignment:
     (the reference fixes them at module level; here they are constructor arguments)."""
 
     def __init__(self, count, prefix, scatter, mark, tokens=4096, top_k=2, experts=64, block_size=128, align=None):
-        self.count, self.prefix, self.scatter, self.mark = count, prefix, scatter, mark
+        for name, stage in zip(_ALIGN_STAGES, (count, prefix, scatter, mark)):
+            if stage is not None:
+                setattr(self, name, stage)
         self.align = align          # the four stages in one launch, for results without counters
         self.tokens, self.top_k, self.experts, self.block_size = tokens, top_k, experts, block_size
 
     @classmethod
     def build(cls, *, tokens=4096, top_k=2, experts=64, block_size=128, target=None, resolve_target=True):
         constants = {"TOKENS": tokens, "TOP_K": top_k, "EXPERTS": experts, "BLOCK_SIZE": block_size}
-        stages = [_compile(getattr(programs, name), target=target, constexprs=constants,
-                           resolve_target=resolve_target) for name in _ALIGN_STAGES]
-        align = _compile(programs.moe_align_routes, target=target, constexprs=constants, resolve_target=resolve_target)
-        return cls(*stages, tokens=tokens, top_k=top_k, experts=experts, block_size=block_size, align=align)
+        def bind(name):
+            return _compile(getattr(programs, name), target=target, constexprs=constants,
+                            resolve_target=resolve_target)
+
+        alignment = cls(None, None, None, None, tokens=tokens, top_k=top_k, experts=experts, block_size=block_size,
+                        align=bind("moe_align_routes"))
+        alignment._bind = bind
+        return alignment
+
+    def __getattr__(self, name):
+        """The stages of a built alignment are bound at their first use: ``run`` needs none of them."""
+        if name not in _ALIGN_STAGES or "_bind" not in self.__dict__:
+            raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
+        stage = self.__dict__[name] = self._bind(_ALIGN_STAGES[name])
+        return stage
 
     @property
     def routes(self) -> int:
