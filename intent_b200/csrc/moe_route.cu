@@ -151,6 +151,8 @@ __global__ void moe_mark_kernel(const int* __restrict__ offsets, int experts, in
 // The four stages read 128 KiB of ids and write as little: what they cost is six launches (two of them fills) and
 // the gaps between them.  Here CTA e counts the routes of every expert in shared memory (the ids come from L2), so
 // that it knows the start of its own span without waiting for another CTA, and then partitions as above.
+// Bound by latency (a few dependent passes over the ids).  64 experts, top-2, graph replay: 64 tokens 9.6 -> 3.3 us,
+// 16384 tokens 19.9 -> 9.6 us, besides the host time of five calls.
 __global__ void __launch_bounds__(1024)
 moe_align_kernel(const int* __restrict__ ids, int routes, int experts, int block, int* __restrict__ sorted,
                  int sorted_capacity, int fill, int* __restrict__ blocks, int blocks_capacity,
