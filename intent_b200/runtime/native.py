@@ -60,7 +60,9 @@ def entry(name: str, carriers: tuple):
         function = _ENTRIES.get(key)
         if function is None:
             try:
-                function = getattr(lib, name)
+                # (an index makes a function object of its own; the attribute of that name is one object for all,
+                # whose argument types a second binding of the symbol would change under this one)
+                function = lib[name]
             except AttributeError as error:
                 raise CompilationStageError("native_loading", f"{library_path()} does not export {name}") from error
             function.restype = ctypes.c_int

@@ -89,3 +89,21 @@ def test_programs_marshal_what_the_header_declares():
         assert declared[program.entry_name] == slots, (definition.name, program.entry_name, declared[program.entry_name], slots)
         checked += 1
     assert checked == len(ib.programs.ALL) >= 29
+
+
+def test_a_binding_keeps_its_slot_types():
+    """The slots of a call are plain integers, so the function object of a binding decides their widths: neither a
+    second binding of the symbol nor the library's attribute of that name may change it."""
+    import intent_b200.runtime.native as native
+
+    name = "intent_b200_moe_prefix_routes"
+    first = native.entry(name, ("ptr", "i64", "i64"))
+    types = list(first.argtypes)
+    second = native.entry(name, ("i32",))
+    shared = getattr(native.library(), name)
+    shared.argtypes = [ctypes.c_int32]
+    try:
+        assert list(first.argtypes) == types and list(second.argtypes) == [ctypes.c_int32, ctypes.c_void_p]
+    finally:
+        shared.argtypes = None
+    assert native.entry(name, ("ptr", "i64", "i64")) is first
