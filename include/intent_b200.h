@@ -67,8 +67,11 @@ INTENT_B200_API int64_t intent_b200_launch_count(void);
  * take part (they launch as usual). */
 INTENT_B200_API int intent_b200_observe_begin(void* facts);
 INTENT_B200_API int intent_b200_observe_end(void);
-/* Turns so far of the process-wide switches that change which kernel an entry selects. */
-INTENT_B200_API extern int32_t intent_b200_selection_epoch;
+/* The process-wide switches that change which kernel an entry selects, `*count` int32 that are read in place (turn
+ * them with their own entries); and begin for a dry run that selects by a copy of them taken earlier, so that the
+ * facts of a launch can be read after a switch was turned. */
+INTENT_B200_API const int32_t* intent_b200_selection(int32_t* count);
+INTENT_B200_API int intent_b200_observe_begin_selected(void* facts, const int32_t* selection, int32_t count);
 
 /* ------------------------------------------------------------------------
  * weight_only_int4_matmul  (W4A16)

@@ -38,7 +38,21 @@ struct LaunchFacts {
   char kernel[64];      // kernel family and the plan's distinguishing choice
 };
 LaunchFacts* observe_sink();
-void note_selection_switch();   // a process-wide switch of the kernel selection was turned
+
+// The process-wide switches that change which kernel or which plan an entry selects, in one place: what a launch was
+// selected by can be kept as one copy, and a dry run on behalf of that launch selects by the copy.
+struct Selection {
+  int32_t gemm_pairs = 1;        // dense W4A16: CTA pairs may be chosen
+  int32_t stream_grid = 0;       // bandwidth kernel: CTAs (0 = one per SM)
+  int32_t stream_warps = 0;      // bandwidth kernel: warps (0 = built-in choice)
+  int32_t table_ride = 1;        // 0 forces the staged form (measurement and tests)
+  int32_t table_single = 1;      // a single small problem runs as a table of one (0 = never; for measurement)
+  int32_t table_unit_rows = 0;   // 64 = the ride-along form uses 64-row units for problems of up to four rows; for measurement
+  int32_t table_corr_mma = -1;   // ride-along kernel: correction sums by MMA (1), from the activations (0), built-in choice (-1)
+  int32_t table_slots = 0;       // upper limit on the ring's slots (0 = the built-in choice); for measurement
+};
+Selection& process_selection();      // the switches themselves
+const Selection& selection();        // what the call at hand selects by: the switches, or the copy of the launch observed
 int record_launch(LaunchFacts* sink, const void* kernel, const char* name, int grid, int threads, int dynamic_smem,
                   int cluster);
 

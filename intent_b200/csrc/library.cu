@@ -1,6 +1,7 @@
 // Library identity, status strings, launch counter, and the shape-dispatching
 // entry points that choose between the bandwidth and the tensor-core kernels.
 #include <atomic>
+#include <cstring>
 
 #include "common.cuh"
 
@@ -23,6 +24,11 @@ constexpr int64_t kSkinnyMaxM = 16;
 namespace ib200 {
 static thread_local LaunchFacts* t_sink = nullptr;
 LaunchFacts* observe_sink() { return t_sink; }
+static Selection g_selection;
+static thread_local Selection t_selection;      // valid while t_selected
+static thread_local bool t_selected = false;
+Selection& process_selection() { return g_selection; }
+const Selection& selection() { return t_selected ? t_selection : g_selection; }
 int record_launch(LaunchFacts* sink, const void* kernel, const char* name, int grid, int threads, int dynamic_smem,
                   int cluster) {
   cudaFuncAttributes attributes;
@@ -57,17 +63,25 @@ extern "C" int intent_b200_observe_begin(void* facts) {
 }
 extern "C" int intent_b200_observe_end(void) {
   ib200::t_sink = nullptr;
+  ib200::t_selected = false;
   return INTENT_B200_OK;
 }
 
-// Counts the turns of the process-wide switches that change which kernel an entry selects, so that a caller can
-// tell whether a dry run still names the kernel of an earlier launch.
-extern "C" {
-__attribute__((visibility("default"))) int32_t intent_b200_selection_epoch = 0;
+// The switches as they are now, and a dry run by an earlier copy of them: the facts of a launch do not change when a
+// switch is turned after it.
+extern "C" const int32_t* intent_b200_selection(int32_t* count) {
+  if (count) *count = int32_t(sizeof(ib200::Selection) / sizeof(int32_t));
+  return reinterpret_cast<const int32_t*>(&ib200::g_selection);
 }
-namespace ib200 {
-void note_selection_switch() { ++intent_b200_selection_epoch; }
-}  // namespace ib200
+extern "C" int intent_b200_observe_begin_selected(void* facts, const int32_t* selection, int32_t count) {
+  if (!selection) return INTENT_B200_ERR_NULL;
+  if (count != int32_t(sizeof(ib200::Selection) / sizeof(int32_t))) return INTENT_B200_ERR_SHAPE;
+  const int status = intent_b200_observe_begin(facts);
+  if (status != INTENT_B200_OK) return status;
+  std::memcpy(&ib200::t_selection, selection, sizeof(ib200::Selection));
+  ib200::t_selected = true;
+  return INTENT_B200_OK;
+}
 
 extern "C" const char* intent_b200_version(void) { return "intent_b200 0.1 sm_100a"; }
 

@@ -350,8 +350,6 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairPara
   }
 }
 
-int g_pair_enabled = 1;
-
 }  // namespace
 
 // Dense W4A16 on CTA pairs; returns INTENT_B200_ERR_UNSUPPORTED when the shape should use the
@@ -359,7 +357,7 @@ int g_pair_enabled = 1;
 template <typename T>
 int w4a16_gemm_pair(const void* x, int64_t M, int64_t K, const void* w, const void* s, int64_t N, void* y,
                     int group_size, int zero_point, cudaStream_t stream, bool prelaid) {
-  if (!g_pair_enabled || M < PAIR_ROWS) return INTENT_B200_ERR_UNSUPPORTED;
+  if (!selection().gemm_pairs || M < PAIR_ROWS) return INTENT_B200_ERR_UNSUPPORTED;
   int device = 0, sms = 0;
   if (cudaGetDevice(&device) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 2)
@@ -397,8 +395,6 @@ int w4a16_gemm_pair(const void* x, int64_t M, int64_t K, const void* w, const vo
   return launch_status();
 }
 
-bool w4a16_gemm_pairs_enabled() { return g_pair_enabled != 0; }
-
 // Reads the pair kernel's status word into *value and clears it when it was set (the caller has
 // synchronised the device).
 int w4a16_gemm_pair_take_status(int* value) {
@@ -420,7 +416,6 @@ template int w4a16_gemm_pair<__nv_bfloat16>(const void*, int64_t, int64_t, const
 }  // namespace ib200
 
 extern "C" int intent_b200_w4a16_gemm_pairs(int32_t enable) {
-  ib200::g_pair_enabled = enable ? 1 : 0;
-  ib200::note_selection_switch();
+  ib200::process_selection().gemm_pairs = enable ? 1 : 0;
   return INTENT_B200_OK;
 }

@@ -572,8 +572,6 @@ int device_sms() {
 }
 
 int g_overlap = 0;
-int g_grid_override = 0;
-int g_warps_override = 0;
 
 template <typename T, int MB, int STEPS, int WARPS, bool XSTAGED, int RING>
 int launch_kernel(const CUtensorMap& map_w, const CUtensorMap& map_s, const CUtensorMap& map_x, const StreamParams& p, const Plan& plan,
@@ -638,10 +636,10 @@ int run(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, void
   if (!aligned16(x.p) || !aligned16(w.p) || !aligned16(s.p) || !aligned16(y.p)) return INTENT_B200_ERR_LAYOUT;
   if (K == 0 || N % 8 != 0 || M > 16 || K > (1 << 24) || N > (1 << 24)) return INTENT_B200_ERR_UNSUPPORTED;
   const int mb = M <= 8 ? 1 : 2;
-  const int sms = g_grid_override > 0 ? g_grid_override : device_sms();
+  const int sms = selection().stream_grid > 0 ? selection().stream_grid : device_sms();
   if (sms <= 0) return INTENT_B200_ERR_UNSUPPORTED;
   Plan plan;
-  if (!make_plan(int(M), int(K), int(N), mb, sms, mb == 1 ? g_warps_override : 0, &plan))
+  if (!make_plan(int(M), int(K), int(N), mb, sms, mb == 1 ? selection().stream_warps : 0, &plan))
     return INTENT_B200_ERR_UNSUPPORTED;
   if (!workspace || workspace_bytes < int64_t(plan.workspace_bytes) || !aligned16(workspace))
     return INTENT_B200_ERR_WORKSPACE;
@@ -716,10 +714,10 @@ int w4a16_stream_bf16(View2 x, View2 w, View2 s, View2 y, int g, int zp, void* w
 int64_t w4a16_stream_workspace_bytes(int64_t M, int64_t K, int64_t N) {
   if (M <= 0 || N <= 0 || K <= 0 || M > 16 || K > (1 << 24) || N > (1 << 24)) return 0;
   const int mb = M <= 8 ? 1 : 2;
-  const int sms = g_grid_override > 0 ? g_grid_override : device_sms();
+  const int sms = selection().stream_grid > 0 ? selection().stream_grid : device_sms();
   Plan plan;
   // without a visible device the size is computed for the 148-SM part this library targets
-  if (!make_plan(int(M), int(K), int(N), mb, sms > 0 ? sms : 148, mb == 1 ? g_warps_override : 0, &plan)) return 0;
+  if (!make_plan(int(M), int(K), int(N), mb, sms > 0 ? sms : 148, mb == 1 ? selection().stream_warps : 0, &plan)) return 0;
   return int64_t(plan.workspace_bytes);
 }
 }  // namespace ib200
@@ -735,13 +733,13 @@ extern "C" int intent_b200_w4a16_gemv_overlap(int32_t enable) {
 
 extern "C" int intent_b200_w4a16_gemv_grid(int32_t ctas) {
   if (ctas < 0) return INTENT_B200_ERR_UNSUPPORTED;
-  ib200::g_grid_override = ctas;
+  ib200::process_selection().stream_grid = ctas;
   return INTENT_B200_OK;
 }
 
 extern "C" int intent_b200_w4a16_gemv_warps(int32_t warps) {
   if (warps != 0 && warps != 16 && warps != 32) return INTENT_B200_ERR_UNSUPPORTED;
-  ib200::g_warps_override = warps;
+  ib200::process_selection().stream_warps = warps;
   return INTENT_B200_OK;
 }
 
@@ -823,9 +821,9 @@ extern "C" int intent_b200_w4a16_gemv_f16_builtin_scratch(INTENT_B200_VIEW2(a0),
   const int64_t M = a0_d0, K = a0_d1, N = a1_d1;
   if (M == 0 || N == 0) return INTENT_B200_OK;
   if (M < 0 || M > 16 || K <= 0 || N < 0 || K > (1 << 24) || N > (1 << 24)) return INTENT_B200_ERR_UNSUPPORTED;
-  const int sms = g_grid_override > 0 ? g_grid_override : device_sms();
+  const int sms = selection().stream_grid > 0 ? selection().stream_grid : device_sms();
   Plan plan;
-  if (sms <= 0 || !make_plan(int(M), int(K), int(N), M <= 8 ? 1 : 2, sms, M <= 8 ? g_warps_override : 0, &plan))
+  if (sms <= 0 || !make_plan(int(M), int(K), int(N), M <= 8 ? 1 : 2, sms, M <= 8 ? selection().stream_warps : 0, &plan))
     return INTENT_B200_ERR_UNSUPPORTED;
   if (plan.workspace_bytes > kBuiltinScratchBytes) return INTENT_B200_ERR_SCRATCH_LIMIT;
   void* scratch = nullptr;

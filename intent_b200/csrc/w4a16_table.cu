@@ -1161,7 +1161,6 @@ size_t fixed_bytes(int group_size) {
 }
 // ride-along form: per-warp correction sums of the unit in hand (32 warps x groups of a unit x 8 rows)
 size_t ride_corr_bytes(int group_size, int unit_rows) { return size_t(32) * (unit_rows * 8 / group_size) * 8 * 4; }
-int g_table_unit_rows = 0;   // 64 = the ride-along form uses 64-row units for problems of up to four rows; for measurement
 // the ride-along form is planned only if this many slots fit (about 80 KB of packed weights in flight per SM)
 int min_ride_slots(int unit_rows) { return unit_rows == 64 ? 12 : 20; }
 // ride-along form: what a launch needs in shared memory besides its slots
@@ -1205,7 +1204,7 @@ bool plan_problem(int M, int K, int N, int group_size, int grid, bool allow_ride
   q.ride = false;
   for (int unit_rows : {64, 32}) {
     if (!allow_ride || M > kRideRows || q.ride) break;
-    if (unit_rows == 64 && (M > 4 || g_table_unit_rows != 64)) continue;
+    if (unit_rows == 64 && (M > 4 || selection().table_unit_rows != 64)) continue;
     if (!geometry(unit_rows)) return false;
     int blocks, spans;
     share_bounds(q.tiles, q.chunks, q.chunks, n_max, &blocks, &spans);
@@ -1266,7 +1265,6 @@ int table_sms() {
 }
 
 int g_table_overlap = 0;
-int g_table_ride = 1;     // 0 forces the staged form (measurement and tests)
 
 int validate(const HostProblem& h, int group_size) {
   if (h.M < 0 || h.K < 0 || h.N < 0) return INTENT_B200_ERR_SHAPE;
@@ -1279,8 +1277,6 @@ int validate(const HostProblem& h, int group_size) {
 }
 
 int g_table_probe = 0;
-int g_table_corr_mma = -1;   // ride-along kernel: correction sums by MMA (1), from the activations (0), built-in choice (-1)
-int g_table_slots = 0;     // upper limit on the ring's slots (0 = the built-in choice); for measurement
 
 template <typename T, int MB, int STEPS>
 int launch_table(const TableMaps& maps, const TableParams& p, int grid, size_t smem, cudaStream_t stream) {
@@ -1346,7 +1342,7 @@ int64_t table_workspace(const HostProblem* problems, int count, int group_size, 
         offsets[i] = offset;
         continue;
       }
-      if (!plan_problem(int(h.M), int(h.K), int(h.N), group_size, grid, g_table_ride != 0, &plans[i])) return -1;
+      if (!plan_problem(int(h.M), int(h.K), int(h.N), group_size, grid, selection().table_ride != 0, &plans[i])) return -1;
       offsets[i] = offset;
       offset += plans[i].bytes;
     }
@@ -1500,8 +1496,8 @@ int run_table(const HostProblem* problems, int count, int group_size, int zero_p
       // warp has to check who used a slot before it).  Ride-along form: one slot per ring warp; measured on
       // M = 1, a deeper ring (40 slots) does not stream faster and a shallower one (24) hardly slower.
       const size_t choice = ride ? 31 : size_t(mb == 1 ? 32 : 16);
-      if (g_table_slots > 0) {
-        if (slots > size_t(g_table_slots)) slots = g_table_slots;
+      if (selection().table_slots > 0) {
+        if (slots > size_t(selection().table_slots)) slots = selection().table_slots;
       } else if (slots >= choice) {
         slots = ride ? choice : slots / choice * choice;
       }
@@ -1541,7 +1537,7 @@ int run_table(const HostProblem* problems, int count, int group_size, int zero_p
            : steps == 2 ? launch_table<T, MB_, 2>(maps, p, grid, smem, stream)           \
                         : launch_table<T, MB_, 1>(maps, p, grid, smem, stream);
     if (ride) {
-      const bool corr_mma = g_table_corr_mma < 0 ? rows_max >= 3 : g_table_corr_mma != 0;
+      const bool corr_mma = selection().table_corr_mma < 0 ? rows_max >= 3 : selection().table_corr_mma != 0;
       if (unit_rows == 64)
         status = steps == 4   ? launch_ride<T, 4, 64, false>(maps, p, grid, smem, stream)
                  : steps == 2 ? launch_ride<T, 2, 64, false>(maps, p, grid, smem, stream)
@@ -1564,8 +1560,6 @@ int run_table(const HostProblem* problems, int count, int group_size, int zero_p
   }
   return INTENT_B200_OK;
 }
-
-int g_single_through_table = 1;   // a single small problem runs as a table of one (0 = never; for measurement)
 
 bool plain_matrix(const View2& v) { return v.p != nullptr && v.s1 == 1 && v.s0 == v.d1; }
 
@@ -1593,7 +1587,7 @@ int64_t w4a16_table_single_workspace_bytes(int64_t M, int64_t K, int64_t N) {
 template <typename T>
 int table_single(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, void* workspace,
                  int64_t workspace_bytes, cudaStream_t stream) {
-  if (!g_single_through_table || !g_table_ride) return kTableDeclined;
+  if (!selection().table_single || !selection().table_ride) return kTableDeclined;
   if (!plain_matrix(x) || !plain_matrix(w) || !plain_matrix(s) || !plain_matrix(y)) return kTableDeclined;
   if (group_size != 32 && group_size != 64 && group_size != 128) return kTableDeclined;
   const int64_t M = x.d0, K = x.d1, N = w.d1;
@@ -1671,26 +1665,25 @@ extern "C" int intent_b200_w4a16_gemv_table_overlap(int32_t enable) {
 // (the results are WRONG by design for every value but 0: these launches only show where the time goes).
 extern "C" int intent_b200_w4a16_gemv_table_tune(const char* knob, int32_t value) {
   if (!knob) return INTENT_B200_ERR_NULL;
-  ib200::note_selection_switch();
   const auto is = [&](const char* name) {
     int i = 0;
     for (; name[i] && knob[i] == name[i]; ++i) {}
     return name[i] == 0 && knob[i] == 0;
   };
   if (is("single") && (value == 0 || value == 1)) {
-    ib200::g_single_through_table = value;
+    ib200::process_selection().table_single = value;
     return INTENT_B200_OK;
   }
   if (is("unit_rows") && (value == 0 || value == 64)) {
-    ib200::g_table_unit_rows = value;
+    ib200::process_selection().table_unit_rows = value;
     return INTENT_B200_OK;
   }
   if (is("corr_mma") && value >= -1 && value <= 1) {
-    ib200::g_table_corr_mma = value;
+    ib200::process_selection().table_corr_mma = value;
     return INTENT_B200_OK;
   }
   if (is("slots") && (value == 0 || (value >= 8 && value <= 64))) {
-    ib200::g_table_slots = value;
+    ib200::process_selection().table_slots = value;
     return INTENT_B200_OK;
   }
   if (is("probe") && ((value >= 0 && value <= 5) || value == 7)) {
@@ -1701,7 +1694,6 @@ extern "C" int intent_b200_w4a16_gemv_table_tune(const char* knob, int32_t value
 }
 
 extern "C" int intent_b200_w4a16_gemv_table_ride(int32_t enable) {
-  ib200::g_table_ride = enable ? 1 : 0;
-  ib200::note_selection_switch();
+  ib200::process_selection().table_ride = enable ? 1 : 0;
   return INTENT_B200_OK;
 }

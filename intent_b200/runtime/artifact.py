@@ -65,25 +65,24 @@ class _Launched:
     """What one invocation leaves behind for ``observation``: plain values, so no tensor is kept alive, and no way
     back to the program, which keeps the record (a cycle would hold its workspaces until a collection).  The
     observation is put together when it is asked for, with the resource facts from a dry run of the same slots; on
-    every call the two took about a third of the host time of ``run``.  ``epoch`` counts the process-wide switches
-    of the kernel selection: once one has been turned since the launch, the dry run could name another kernel, and
-    the facts stay None."""
+    every call the two took about a third of the host time of ``run``.  ``selection`` is a copy of the process-wide
+    switches of the kernel selection as the launch found them: the dry run selects by it, whatever was turned since."""
 
-    __slots__ = ("slots", "views", "workspace_bytes", "status", "epoch", "seen")
+    __slots__ = ("slots", "views", "workspace_bytes", "status", "selection", "seen")
 
-    def __init__(self, slots, views, workspace_bytes, status, epoch):
+    def __init__(self, slots, views, workspace_bytes, status, selection):
         self.slots, self.views = slots, views
-        self.workspace_bytes, self.status, self.epoch = workspace_bytes, status, epoch
+        self.workspace_bytes, self.status, self.selection = workspace_bytes, status, selection
         self.seen: NativeObservation | None = None
 
     def observation(self, program: "NativeProgram") -> NativeObservation:
         if self.seen is None:
             facts = {}
-            if self.status == 0 and self.epoch == native.selection_epoch():
+            if self.status == 0:
                 import torch
 
                 with torch.cuda.device(program.device):
-                    facts = program.observe(self.slots)
+                    facts = program.observe(self.slots, self.selection)
             self.seen = NativeObservation(
                 "b200", program.entry_name, "launched" if self.status == 0 else "failed", program.constants,
                 tuple((p.name, f.shape, f.strides) for p, f in zip(program.interface.parameters, self.views)
@@ -143,13 +142,14 @@ class PreparedCall:
 
     def _invoke(self) -> None:
         program = self.program
+        selection = native.selection()
         status = program.function()(*self._slots, program.current_stream())
         launched = self._launched
-        if launched is None or status or launched.status or launched.epoch != native.selection_epoch():
+        if launched is None or status or launched.status or launched.selection != selection:
             # (a repeated launch of the same binding leaves the same record)
             launched = self._launched = _Launched(
                 self._slots, self.invocation.views,
-                sum(w.numel() * w.element_size() for w in self._workspace), int(status), native.selection_epoch())
+                sum(w.numel() * w.element_size() for w in self._workspace), int(status), selection)
         program._launched = launched
         if status:
             native.check(status, program.entry_name, launched.observation(program))
@@ -234,14 +234,14 @@ class NativeProgram:
 
         return torch._C._cuda_getCurrentRawStream(self.device)
 
-    def observe(self, slots: tuple) -> dict:
+    def observe(self, slots: tuple, selection: bytes) -> dict:
         """The slots once more in the library's dry-run mode: nothing is launched and no memory is touched, the
-        entry reports the kernel instance it selects for them and that instance's resource usage."""
+        entry reports the kernel instance it selects for them by these switches and that instance's resource usage."""
         if not self.entry_name.startswith(_OBSERVABLE):
             return {}
         library = native.library()
         facts = _LaunchFacts()
-        if library.intent_b200_observe_begin(ctypes.byref(facts)) != 0:
+        if library.intent_b200_observe_begin_selected(ctypes.byref(facts), selection, len(selection) // 4) != 0:
             return {}
         try:
             status = self.function()(*slots, self.current_stream())

@@ -17,7 +17,7 @@ from ..errors import CompilationStageError
 _LOCK = Lock()
 _LIBRARY: ctypes.CDLL | None = None
 _ENTRIES: dict = {}
-_EPOCH: ctypes.c_int32 | None = None
+_SELECTION: tuple | None = None        # address and bytes of the switches
 
 _CARRIERS = {"ptr": ctypes.c_void_p, "bool": ctypes.c_bool, "i8": ctypes.c_int8, "i16": ctypes.c_int16,
              "i32": ctypes.c_int32, "i64": ctypes.c_int64, "f32": ctypes.c_float, "f64": ctypes.c_double}
@@ -71,12 +71,16 @@ def entry(name: str, carriers: tuple):
         return function
 
 
-def selection_epoch() -> int:
-    """How often a process-wide switch of the kernel selection has been turned."""
-    global _EPOCH
-    if _EPOCH is None:
-        _EPOCH = ctypes.c_int32.in_dll(library(), "intent_b200_selection_epoch")
-    return _EPOCH.value
+def selection() -> bytes:
+    """A copy of the process-wide switches of the kernel selection (int32 each)."""
+    global _SELECTION
+    if _SELECTION is None:
+        where = library()["intent_b200_selection"]
+        where.restype, where.argtypes = ctypes.c_void_p, [ctypes.c_void_p]
+        count = ctypes.c_int32()
+        address = where(ctypes.byref(count))
+        _SELECTION = (address, 4 * count.value)
+    return ctypes.string_at(*_SELECTION)
 
 
 def status_string(status: int) -> str:
