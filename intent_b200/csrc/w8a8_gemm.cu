@@ -187,7 +187,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint32_t local = 0;
     for (int tile = first_tile; tile < tiles; tile += tile_step, ++local) {
       int m_tile, n_tile;
-        tile_coords<CG>(tile, p.m_tiles, p.n_tiles, m_tile, n_tile);
+      tile_coords<CG>(tile, p.m_tiles, p.n_tiles, m_tile, n_tile);
       const uint32_t acc = local & 1;
       if (!__all_sync(0xffffffffu, mbar_wait(tmem_full + 8 * acc, (local >> 1) & 1))) {
         if (lane == 0) atomicExch(&g_w8a8_gemm_status, INTENT_B200_ERR_TIMEOUT);
@@ -316,6 +316,29 @@ int launch(const I8Operands& q, I8Params& p, int sms, cudaStream_t stream) {
   return launch_status();
 }
 
+// Whether a call runs on CTA pairs.  A pair tile reads two thirds of the operand bytes per operation but covers 256
+// rows: not where the 128-row tiles fill clearly fewer waves of the chip.  A pair launch also costs about 0.6 us more
+// than a lone one, which a short walk does not earn back (graph replay, lone against pairs, us):
+//   two tiles   M129 N256:    K1024 15.5 / 16.2, K4096 22.1 / 22.6, K8192 32.4 / 32.2
+//   8 tiles     M129 N1024:   K1024 15.9 / 16.4, K3072 21.1 / 21.2, K4096 23.4 / 23.4, K8192 35.1 / 33.0
+//   32 tiles    M512 N2048:   K1024 18.6 / 19.2, K1536 19.9 / 20.2, K2048 21.2 / 21.2, K4096 26.6 / 25.8
+//   128 tiles   M1024 N4096:  K512 17.7 / 18.0, K1536 20.8 / 20.6, K4096 28.5 / 26.6
+//   136 tiles   M2050 N2048:  K1536 19.4 / 19.7, K2048 21.0 / 21.1, K4096 26.6 / 25.8 (an odd row tile is half padding)
+//   128 tiles   M2048 N2048:  K512 17.6 / 17.3, K1024 19.1 / 18.5, K4096 28.3 / 25.7 (many row tiles share B)
+// so the k blocks that a pair walks, and those of the whole call, have to be enough.
+bool takes_pairs(int64_t M, int64_t N, int64_t k_blocks, int64_t sms) {
+  if (M <= BM) return false;
+  const int64_t row_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
+  const int64_t tiles = row_tiles * n_tiles, pair_tiles = (row_tiles + 1) / 2 * n_tiles;
+  const int64_t waves = (tiles + sms - 1) / sms, pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2);
+  if (pair_waves * 9 > waves * 10) return false;
+  const int64_t walk = pair_waves * k_blocks, all = tiles * k_blocks;
+  if (walk >= 16) return all >= 256;
+  if (row_tiles % 2 != 0) return false;
+  return pair_waves == 1 ? (k_blocks >= 12 && all >= 768) || (row_tiles >= 16 && tiles >= 112)
+                         : pair_waves == 2 && row_tiles >= 16;
+}
+
 // b is [K,N] (N contiguous), or [N,K] (K contiguous) with B_K_MAJOR
 template <int EPILOGUE, bool B_K_MAJOR = false>
 int run(View2 a, View2 b, void* out, const int32_t* bias, const float* sa, const float* sb, cudaStream_t stream) {
@@ -339,12 +362,7 @@ int run(View2 a, View2 b, void* out, const int32_t* bias, const float* sa, const
   p.K = int(K);
   p.k_blocks = int((K + BK - 1) / BK);
   const I8Operands q{a, b, M, N, K};
-  // A pair tile reads two thirds of the operand bytes per operation but covers 256 rows: it is taken unless the 128-row
-  // tiles fill clearly fewer waves of the chip.
-  const int64_t n_tiles = (N + BN - 1) / BN;
-  const int64_t single_waves = ((M + BM - 1) / BM * n_tiles + sms - 1) / sms;
-  const int64_t paired_waves = ((M + 2 * BM - 1) / (2 * BM) * n_tiles + sms / 2 - 1) / std::max(1, sms / 2);
-  if (sms >= 2 && M > BM && paired_waves * 9 <= single_waves * 10) return launch<EPILOGUE, B_K_MAJOR, 2>(q, p, sms, stream);
+  if (sms >= 2 && takes_pairs(M, N, p.k_blocks, sms)) return launch<EPILOGUE, B_K_MAJOR, 2>(q, p, sms, stream);
   return launch<EPILOGUE, B_K_MAJOR, 1>(q, p, sms, stream);
 }
 

@@ -1,23 +1,78 @@
-"""The int8 kernel on CTA pairs (256 x 256 tiles): edges of the pair tile in rows, columns and k, exact integers."""
+"""The int8 kernel on lone CTAs (128 x 256 tiles) and on CTA pairs (256 x 256 tiles): edges of the tiles in rows,
+columns and k, exact integers.  Which of the two a call runs on is read from its observation."""
 import pytest
 import torch
 
 import intent_b200 as ib
+import oracle
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M,K,N", [(129, 16, 16), (256, 128, 256), (257, 144, 272), (385, 1040, 528), (2050, 256, 4112)])
-def test_pair_tiles_are_exact(cuda_device, M, K, N):
+LONE, PAIRS = "i8_gemm_kernel 128x256 tiles", "i8_gemm_kernel CTA pairs"
+
+
+def _operands(M, K, N):
     g = torch.Generator().manual_seed(M)
     a = torch.randint(-128, 128, (M, K), generator=g, dtype=torch.int8)
     b = torch.randint(-128, 128, (K, N), generator=g, dtype=torch.int8)
-    bias = torch.randint(-1000, 1000, (N,), generator=g, dtype=torch.int32)
+    return a, b, torch.randint(-1000, 1000, (N,), generator=g, dtype=torch.int32)
+
+
+def _run(device, a, b, bias):
     artifact = ib.compile(ib.programs.gemm_i8, target=ib.B200Target(0))
-    out = torch.full((M, N), -1, dtype=torch.int32, device=cuda_device)
-    artifact(a.to(cuda_device), b.to(cuda_device), bias.to(cuda_device), out)
+    out = torch.full((a.shape[0], b.shape[1]), -1, dtype=torch.int32, device=device)
+    artifact(a.to(device), b.to(device), bias.to(device), out)
     torch.cuda.synchronize()
     artifact.check()
-    # 16384 * 1040 < 2^24: the products and their sums are exact in f32
-    expected = (a.float() @ b.float()).to(torch.int32) + bias
-    assert torch.equal(out.cpu(), expected)
+    return out.cpu(), artifact.observation.kernel
+
+
+@pytest.mark.parametrize("M,K,N", [(129, 16, 16), (256, 128, 256), (257, 144, 272), (385, 1040, 528), (2050, 256, 4112),
+                                   (4500, 16, 528)])     # (the last: a second band of the tile walk)
+def test_lone_tiles_are_exact(cuda_device, M, K, N):
+    a, b, bias = _operands(M, K, N)
+    out, kernel = _run(cuda_device, a, b, bias)
+    assert kernel.startswith(LONE)
+    assert torch.equal(out, oracle.gemm_i8_exact_f64(a, b, bias))
+
+
+@pytest.mark.parametrize("M,K,N", [
+    (129, 4112, 1040),      # the second CTA of the pair holds one row; 16 k at the end; 16 columns in the last tile
+    (1400, 1040, 4112),     # more tiles than pairs, an odd count of 128-row tiles
+    (4500, 2064, 528),      # a second band of the tile walk
+])
+def test_pair_tiles_are_exact(cuda_device, M, K, N):
+    a, b, bias = _operands(M, K, N)
+    out, kernel = _run(cuda_device, a, b, bias)
+    assert kernel.startswith(PAIRS)
+    assert torch.equal(out, oracle.gemm_i8_exact_f64(a, b, bias))
+
+
+def test_pair_tiles_with_the_second_operand_k_major(cuda_device):
+    """The packed programs hand their decoded weights over as [N, K]; both operands ragged, more tiles than pairs."""
+    M, K, N = 4112, 1056, 1400
+    g = torch.Generator().manual_seed(3)
+    activation = torch.randint(-128, 128, (M, K), generator=g, dtype=torch.int8)
+    packed = torch.randint(0, 256, (N, K // 2), generator=g, dtype=torch.uint8)
+    artifact = ib.compile(ib.programs.w4a8_packed_matmul, target=ib.B200Target(0))
+    out = artifact.run(activation.to(cuda_device), packed.to(cuda_device))        # [N, M]
+    torch.cuda.synchronize()
+    artifact.check()
+    assert torch.equal(out.cpu(), oracle.w4a8_packed_matmul(activation, packed))
+    # (this entry reports no facts; the rule reads the sizes of the product alone)
+    assert _run(cuda_device, *_operands(N, K, M))[1].startswith(PAIRS)
+
+
+@pytest.mark.parametrize("M,K,N,kernel", [
+    (128, 8192, 8192, LONE),                                 # one row tile
+    (512, 1024, 2048, LONE), (512, 4096, 2048, PAIRS),       # too few k blocks to earn the pair launch back, and enough
+    (129, 3072, 1024, LONE), (129, 8192, 1024, PAIRS),       # the same for eight tiles
+    (2050, 1024, 2048, LONE), (2048, 1024, 2048, PAIRS),     # an odd row tile, many row tiles
+])
+def test_short_walks_run_on_lone_tiles(cuda_device, M, K, N, kernel):
+    a, b, bias = (t.to(cuda_device) for t in _operands(M, K, N))
+    artifact = ib.compile(ib.programs.gemm_i8, target=ib.B200Target(0))
+    artifact.run(a, b, bias)
+    torch.cuda.synchronize()
+    assert artifact.observation.kernel.startswith(kernel)
