@@ -39,6 +39,18 @@ def _rule(condition, message):
 # ---------------------------------------------------------------------------------
 # weight_only_int4_matmul (W4A16)
 # ---------------------------------------------------------------------------------
+@cache
+def _w4a16_workspace_query():
+    import ctypes
+
+    from .runtime import native
+
+    query = native.library()["intent_b200_weight_only_int4_matmul_workspace_bytes"]
+    query.restype = ctypes.c_int64
+    query.argtypes = [ctypes.c_int64] * 3
+    return query
+
+
 def _lower_w4a16(constants, device):
     act = _act_dtype(constants)
     group = int(constants["GROUP_SIZE"])
@@ -93,19 +105,9 @@ def _lower_w4a16(constants, device):
         _rule(lambda d: d["K"] % group == 0 and d["G"] * group == d["K"],
               lambda d: f"scales.shape[0] must be K/GROUP_SIZE with K a multiple of {group}"),
     ))
-    @cache
-    def workspace_query():
-        import ctypes
-
-        from .runtime import native
-
-        query = native.library().intent_b200_weight_only_int4_matmul_workspace_bytes
-        query.restype = ctypes.c_int64
-        query.argtypes = [ctypes.c_int64] * 3
-        return query
 
     def workspace_bytes(d):
-        return int(workspace_query()(d["M"], d["K"], d["N"])) if kernel != "gemm" else 0
+        return int(_w4a16_workspace_query()(d["M"], d["K"], d["N"])) if kernel != "gemm" else 0
 
     program = NativeProgram(interface=interface, entry_name=f"intent_b200_{stem}_{act.name}",
                             constants=(group, zp), device=device, workspace=workspace_bytes,

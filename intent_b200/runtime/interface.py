@@ -19,6 +19,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 from enum import IntEnum
+from functools import cached_property
 
 from ..dtypes import DType, torch_dtype
 
@@ -123,15 +124,29 @@ class PublicInterface:
         # callables(dimensions: dict) -> None raising ValueError; derived relations such
         # as "packed rows * 8 == K" that tie symbolic dimensions together.
         self.dimension_rules = tuple(dimension_rules)
-        # everything below is fixed by the declaration and read on every call
-        self.views = tuple(p for p in self.parameters if isinstance(p, ViewParameter))
-        self.inputs = tuple(p for p in self.parameters if not isinstance(p, ViewParameter) or not p.output)
-        self.outputs = tuple(p for p in self.views if p.output)
-        self._allocation_errors = self.output_allocation_errors()
-        self._writable_pairs = tuple((left, right) for index, left in enumerate(self.views)
-                                     for right in self.views[index + 1:] if left.writable or right.writable)
 
-    # -- views of the declaration ------------------------------------------------
+    # -- views of the declaration: fixed by it, read on every call and put together by the first one ------------
+    @cached_property
+    def views(self) -> tuple:
+        return tuple(p for p in self.parameters if isinstance(p, ViewParameter))
+
+    @cached_property
+    def inputs(self) -> tuple:
+        return tuple(p for p in self.parameters if not isinstance(p, ViewParameter) or not p.output)
+
+    @cached_property
+    def outputs(self) -> tuple:
+        return tuple(p for p in self.views if p.output)
+
+    @cached_property
+    def _allocation_errors(self) -> tuple:
+        return self.output_allocation_errors()
+
+    @cached_property
+    def _writable_pairs(self) -> tuple:
+        return tuple((left, right) for index, left in enumerate(self.views)
+                     for right in self.views[index + 1:] if left.writable or right.writable)
+
     @property
     def mutable_inputs(self) -> tuple:
         return tuple(p for p in self.views if p.access is ViewKind.INOUT)

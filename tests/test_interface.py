@@ -30,6 +30,13 @@ def test_interface_declaration(artifact):
     assert artifact.device_type == "cuda" and artifact.entry == artifact.__call__
 
 
+def test_compile_derives_nothing_ahead():
+    """What the declaration implies is put together by the first call: compiling an artifact costs no more for it."""
+    interface = ib.compile(ib.programs.weight_only_int4_matmul, resolve_target=False).runtime.interface
+    assert set(vars(interface)) == {"parameters", "dimension_rules"}
+    assert len(interface.inputs) == 3 and "inputs" in vars(interface)
+
+
 def test_bind_allocates_outputs(artifact):
     x, p, s = _inputs()
     bound = artifact.interface.bind((x, p, s), device=CPU)
