@@ -35,8 +35,9 @@ def test_tiled_layout_is_the_documented_permutation(cuda_device, K, N):
 
 @pytest.mark.parametrize("dtype,M,K,N,group", [
     (torch.bfloat16, 128, 256, 256, 128), (torch.float16, 77, 1024, 520, 64), (torch.bfloat16, 300, 384, 264, 32),
-    (torch.bfloat16, 1100, 1024, 776, 128),        # CTA pairs with ragged tiles
-    (torch.bfloat16, 2048, 2048, 2048, 128)])
+    (torch.bfloat16, 1100, 1024, 776, 128),        # tiles of 64 columns
+    (torch.bfloat16, 2048, 2048, 2048, 128),       # tiles of 256 columns
+    (torch.bfloat16, 1100, 1024, 4104, 128)])      # CTA pairs with ragged tiles
 def test_gemm_on_tiled_weight_equals_reference_layout(cuda_device, dtype, M, K, N, group):
     x, p, s = ib.workloads.w4a16_inputs(M, K, N, dtype=dtype, group_size=group, seed=31)
     xd, pd, sd = x.to(cuda_device), p.to(cuda_device), s.to(cuda_device)

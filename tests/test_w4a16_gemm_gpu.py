@@ -94,10 +94,9 @@ def test_gemm_full_size_prefill_rows(cuda_device):
     assert torch.isfinite(out).all()
 
 
-def test_reference_case_on_cta_pairs(cuda_device):
+def test_reference_case_at_its_own_size(cuda_device):
     """The reference's own W4A16 case at its own size (M512 K2048 N4096, group 64, signed nibbles, f16;
-    experiments/cpu/providers/mojo/contraction.py:190-198): this is the CTA-pair kernel in two's-complement
-    mode.  Checked against stored rows of the reference module's output at the reference's atol = 4e-2,
+    experiments/cpu/providers/mojo/contraction.py:190-198), on tiles of 128 columns.  Checked against stored rows of the reference module's output at the reference's atol = 4e-2,
     against the oracle on every row, and at the benchmark's 2e-2 * max|ref|."""
     import importlib.util
     from pathlib import Path
@@ -122,9 +121,9 @@ def test_reference_case_on_cta_pairs(cuda_device):
         assert max_abs_rel(out, ref) <= 2e-3          # what the kernel really achieves on f16
 
 
-@pytest.mark.parametrize("M,K,N", [(512, 512, 256), (1100, 1024, 776), (2048, 2048, 2048)])
+@pytest.mark.parametrize("M,K,N", [(512, 512, 12296), (1100, 1024, 4104), (2048, 2048, 4096)])
 def test_cta_pair_kernel_equals_single_cta_kernel(cuda_device, M, K, N):
-    """M >= 512 runs on CTA pairs (cta_group::2); the k loop and the rounding are the same as in the
+    """These sizes run on CTA pairs (cta_group::2); the k loop and the rounding are the same as in the
     single-CTA kernel, so the two must agree bit for bit, and with the oracle within tolerance."""
     lib = native.library()
     x, p, s = ib.workloads.w4a16_inputs(M, K, N, dtype=torch.bfloat16, group_size=128, seed=9)
@@ -133,8 +132,10 @@ def test_cta_pair_kernel_equals_single_cta_kernel(cuda_device, M, K, N):
     try:
         lib.intent_b200_w4a16_gemm_pairs(1)
         paired = artifact.run(xd, pd, sd)
+        assert artifact.observation.kernel.startswith("w4a16_gemm_pair_kernel")
         lib.intent_b200_w4a16_gemm_pairs(0)
         single = artifact.run(xd, pd, sd)
+        assert artifact.observation.kernel.startswith("w4a16_gemm_kernel single CTA, 256x256")
         torch.cuda.synchronize()
     finally:
         lib.intent_b200_w4a16_gemm_pairs(1)

@@ -1,5 +1,5 @@
-"""W4A16 calls of few rows on column tiles of 128, 64 and 32 columns: edges of the tile in rows, columns and k, and
-fewer k blocks than there are sets of dequantiser warps."""
+"""W4A16 calls of few rows on column tiles of 64 and 32 columns: edges of the tile in rows, columns and k, and
+fewer k blocks than there are sets of dequantiser warps.  (All forms side by side: test_w4a16_forms_gpu.py.)"""
 import pytest
 import torch
 
@@ -20,7 +20,7 @@ pytestmark = pytest.mark.gpu
 ])
 def test_narrow_tiles_give_the_bits_of_the_wide_ones(cuda_device, dtype, M, K, N, group):
     """Every tile form adds the k blocks in the same order, so a row's bits do not depend on how many rows the call
-    has; the tolerances against the oracle are those of the wide tiles (test_w4a16_gemm_gpu.py)."""
+    has (4096 rows take a wider tile, or the same one where there are only 8 or 40 columns); the tolerances against the oracle are those of the wide tiles (test_w4a16_gemm_gpu.py)."""
     x, p, s = ib.workloads.w4a16_inputs(4096, K, N, dtype=dtype, group_size=group, seed=M)
     artifact = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),
                           constexprs={"GROUP_SIZE": group, "ZERO_POINT": 8,
@@ -28,6 +28,7 @@ def test_narrow_tiles_give_the_bits_of_the_wide_ones(cuda_device, dtype, M, K, N
     xd, pd, sd = x.to(cuda_device), p.to(cuda_device), s.to(cuda_device)
     whole = artifact.run(xd, pd, sd)
     out = artifact.run(xd[:M].contiguous(), pd, sd)
+    assert artifact.observation.kernel.startswith(f"w4a16_gemm_kernel single CTA, 128x{64 if M == 511 else 32} ")
     torch.cuda.synchronize()
     artifact.check()
     assert torch.equal(out, whole[:M])
