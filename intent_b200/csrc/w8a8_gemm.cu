@@ -46,6 +46,8 @@ struct Ring {
   static constexpr int SMEM_BYTES = 1024 + STAGES * (A_BYTES + B_BYTES) + 256;
 };
 
+constexpr int64_t BAND_BYTES = int64_t(64) << 20;   // of A, from which on rows are walked in bands
+
 struct I8Params {
   void* out;
   const int32_t* bias;      // gemm_i8 (may be null)
@@ -53,18 +55,24 @@ struct I8Params {
   const float* b_scales;
   int M, N, K;
   int k_blocks, m_tiles, n_tiles;
+  int band;                 // row tiles of a band of the tile walk
 };
 
-// Tile walk: bands of rows, the row tile varying fastest, so that the band of A and the columns of B in flight stay in L2.
-template <int CG>
-__device__ __forceinline__ void tile_coords(int tile, int m_tiles, int n_tiles, int& m_tile, int& n_tile) {
-  constexpr int BAND = 32 / CG;   // 4096 rows
-  const int band_size = BAND * n_tiles;
-  const int band = tile / band_size;
-  const int in_band = tile - band * band_size;
-  const int rows_in_band = min(BAND, m_tiles - band * BAND);
-  n_tile = in_band / rows_in_band;
-  m_tile = band * BAND + (in_band - n_tile * rows_in_band);
+// Tile walk: the row tile varies fastest, so that the columns of B in flight are few.  Where A is too large to stay in
+// the L2 for a whole column of tiles, rows are walked in bands of 4096.  All rows / bands, us: 20720 x 6272 x 1840
+// (130 MB of A) 240 / 189, 12384 x 7424 x 3664 (92 MB) 313 / 273, 24720 x 2816 x 1744 (70 MB) 181 / 173; but
+// 9584 x 6656 x 2640 (64 MB) 151 / 160, and with two tiles per CTA the bands put full tiles behind full ones where the
+// walk over all rows ends on the narrow last column: 7664 x 2048 x 544 25.2 / 29.9, 7072 x 800 x 1408 39.1 / 45.5.
+__device__ __forceinline__ void tile_coords(int tile, const I8Params& p, int& m_tile, int& n_tile) {
+  int first = 0, rows = p.m_tiles;
+  if (p.band < p.m_tiles) {
+    const int band = tile / (p.band * p.n_tiles);
+    tile -= band * p.band * p.n_tiles;
+    first = band * p.band;
+    rows = min(p.band, p.m_tiles - first);
+  }
+  n_tile = tile / rows;
+  m_tile = first + tile - n_tile * rows;
 }
 
 // EPILOGUE 0: bf16(acc * sa[m] * sb[n]);  1: int32 acc + bias[n]
@@ -120,7 +128,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       bool ok = true;
       for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
         int m_tile, n_tile;
-        tile_coords<CG>(tile, p.m_tiles, p.n_tiles, m_tile, n_tile);
+        tile_coords(tile, p, m_tile, n_tile);
         for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           if (!mbar_wait(empty + 8 * s, ((it / STAGES) & 1) ^ 1)) { ok = false; break; }
@@ -187,7 +195,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint32_t local = 0;
     for (int tile = first_tile; tile < tiles; tile += tile_step, ++local) {
       int m_tile, n_tile;
-      tile_coords<CG>(tile, p.m_tiles, p.n_tiles, m_tile, n_tile);
+      tile_coords(tile, p, m_tile, n_tile);
       const uint32_t acc = local & 1;
       if (!__all_sync(0xffffffffu, mbar_wait(tmem_full + 8 * acc, (local >> 1) & 1))) {
         if (lane == 0) atomicExch(&g_w8a8_gemm_status, INTENT_B200_ERR_TIMEOUT);
@@ -280,6 +288,7 @@ template <int EPILOGUE, bool B_K_MAJOR, int CG>
 int launch(const I8Operands& q, I8Params& p, int sms, cudaStream_t stream) {
   p.m_tiles = int((q.M + CG * BM - 1) / (CG * BM));
   p.n_tiles = int((q.N + BN - 1) / BN);
+  p.band = q.M * q.K >= BAND_BYTES ? 32 / CG : p.m_tiles;   // 4096 rows
   CUtensorMap map_a, map_b;
   if (!make_tensor_map_2d(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, q.a.p, uint64_t(q.M), uint64_t(q.K), uint64_t(q.K), BM,
                           BK, CU_TENSOR_MAP_SWIZZLE_128B) ||

@@ -29,7 +29,7 @@ def _run(device, a, b, bias):
 
 
 @pytest.mark.parametrize("M,K,N", [(129, 16, 16), (256, 128, 256), (257, 144, 272), (385, 1040, 528), (2050, 256, 4112),
-                                   (4500, 16, 528)])     # (the last: a second band of the tile walk)
+                                   (6200, 10832, 528)])     # (the last: two bands of the tile walk)
 def test_lone_tiles_are_exact(cuda_device, M, K, N):
     a, b, bias = _operands(M, K, N)
     out, kernel = _run(cuda_device, a, b, bias)
@@ -40,7 +40,8 @@ def test_lone_tiles_are_exact(cuda_device, M, K, N):
 @pytest.mark.parametrize("M,K,N", [
     (129, 4112, 1040),      # the second CTA of the pair holds one row; 16 k at the end; 16 columns in the last tile
     (1400, 1040, 4112),     # more tiles than pairs, an odd count of 128-row tiles
-    (4500, 2064, 528),      # a second band of the tile walk
+    (4500, 2064, 528),      # more than 4096 rows, all in one band of the tile walk
+    (8200, 8192, 528),      # 64 MB of A: three bands, the last of one row tile
 ])
 def test_pair_tiles_are_exact(cuda_device, M, K, N):
     a, b, bias = _operands(M, K, N)
