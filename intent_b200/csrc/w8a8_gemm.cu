@@ -334,14 +334,44 @@ int launch(const I8Operands& q, I8Params& p, int sms, cudaStream_t stream) {
 //   128 tiles   M1024 N4096:  K512 17.7 / 18.0, K1536 20.8 / 20.6, K4096 28.5 / 26.6
 //   136 tiles   M2050 N2048:  K1536 19.4 / 19.7, K2048 21.0 / 21.1, K4096 26.6 / 25.8 (an odd row tile is half padding)
 //   128 tiles   M2048 N2048:  K512 17.6 / 17.3, K1024 19.1 / 18.5, K4096 28.3 / 25.7 (many row tiles share B)
-// so the k blocks that a pair walks, and those of the whole call, have to be enough.
-bool takes_pairs(int64_t M, int64_t N, int64_t k_blocks, int64_t sms) {
+// so the k blocks that a pair walks, and those of the whole call, have to be enough.  How many is enough depends on
+// the pitch of B's rows.  Boxes of 128 bytes on a pitch that is no multiple of 128 touch two lines of the L2 per row,
+// and the half of B that a pair does not fetch weighs twice:
+//   B [K,N]     M447 K4272 N1280 26.1 / 25.3, M319 K1728 N2816 19.6 / 20.6; M355 K4000 N2096 29.3 / 24.3
+//   B [N,K]     M768 N3616: K3584 22.9 / 23.6; M1008 N4064: K7104 33.5 / 33.0; M816 N1168: K6496 30.2 / 26.4
+// B [N,K] on lines of its own is fetched as one 256-row box by a lone CTA and gains nothing within one wave of pairs
+// (M1616 K3328 N2064 19.3 / 20.1, M496 K8064 N2144 30.8 / 31.5); with several waves it does for long walks (two waves:
+// M7104 K512 N624 15.4 / 15.8, M3248 K1280 N1392 19.9 / 19.3, M1776 K3840 N3040 35.2 / 32.2; more: M3568 K1536 N4784
+// 42.8 / 45.7, M2992 K1792 N3840 38.3 / 36.9).  Nor do few columns, unless there are many row tiles to stream, which
+// the deeper ring of a pair does better (N16: M4688 K5888 34.0 / 27.3, M7968 K5504 27.7 / 18.4, M2512 K6912 25.3 /
+// 26.0).  And where the last wave of lone tiles is all in a narrow last column while that of the pairs is not, a short
+// walk waits for the pairs' wide tiles (M1840 K1536 N7520 55.2 / 60.6, M825 K2080 N5472 29.8 / 35.6).
+bool takes_pairs(int64_t M, int64_t N, int64_t K, bool b_k_major, int64_t sms) {
   if (M <= BM) return false;
+  const int64_t k_blocks = (K + BK - 1) / BK;
   const int64_t row_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
   const int64_t tiles = row_tiles * n_tiles, pair_tiles = (row_tiles + 1) / 2 * n_tiles;
   const int64_t waves = (tiles + sms - 1) / sms, pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2);
   if (pair_waves * 9 > waves * 10) return false;
   const int64_t walk = pair_waves * k_blocks, all = tiles * k_blocks;
+  const int64_t tail = tiles - (waves - 1) * sms, pair_tail = pair_tiles - (pair_waves - 1) * (sms / 2);
+  const bool narrow_end = N % BN > 0 && N % BN <= BN / 2 && tail <= row_tiles && pair_tail > (row_tiles + 1) / 2;
+  if (pair_waves > 1 && narrow_end && k_blocks < 24) return false;
+  const bool whole_lines = (b_k_major ? K : N) % 128 == 0;
+  if (b_k_major) {
+    if (pair_waves > 2) return k_blocks >= (whole_lines ? 16 : 10);
+    if (N <= 32) return row_tiles >= 32;
+    if (whole_lines) return pair_waves == 2 && k_blocks >= 10;
+    if (N < 96 || (n_tiles == 1 && k_blocks < 32)) return false;   // little of B to share
+  } else {
+    if (pair_waves > 2 && k_blocks < 8) return false;
+    if (whole_lines && pair_waves == 1) {
+      if (n_tiles == 1) return false;
+      if (K % 128 != 0) return k_blocks >= 32 && all >= 672;      // (the lines of A count on both forms)
+      if (k_blocks >= 16)
+        return (all >= 672 && (row_tiles > 2 || k_blocks >= 32)) || (k_blocks >= 48 && all >= 480);
+    }
+  }
   if (walk >= 16) return all >= 256;
   if (row_tiles % 2 != 0) return false;
   return pair_waves == 1 ? (k_blocks >= 12 && all >= 768) || (row_tiles >= 16 && tiles >= 112)
@@ -371,7 +401,7 @@ int run(View2 a, View2 b, void* out, const int32_t* bias, const float* sa, const
   p.K = int(K);
   p.k_blocks = int((K + BK - 1) / BK);
   const I8Operands q{a, b, M, N, K};
-  if (sms >= 2 && takes_pairs(M, N, p.k_blocks, sms)) return launch<EPILOGUE, B_K_MAJOR, 2>(q, p, sms, stream);
+  if (sms >= 2 && takes_pairs(M, N, K, B_K_MAJOR, sms)) return launch<EPILOGUE, B_K_MAJOR, 2>(q, p, sms, stream);
   return launch<EPILOGUE, B_K_MAJOR, 1>(q, p, sms, stream);
 }
 

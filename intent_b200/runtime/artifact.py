@@ -56,9 +56,10 @@ class _LaunchFacts(ctypes.Structure):
 
 # entries made only of kernels that honour the dry-run observation
 _OBSERVABLE = ("intent_b200_weight_only_int4_matmul", "intent_b200_w4a16_gemv", "intent_b200_w4a16_gemm",
-               "intent_b200_gemm_i8", "intent_b200_w8a8_gemm", "intent_b200_ragged_grouped_gemm",
-               "intent_b200_routed_expert_projection", "intent_b200_moe_expert_ffn", "intent_b200_gemm_f16",
-               "intent_b200_bf16_gemm", "intent_b200_quantized_gemm", "intent_b200_moe_grouped_w4a16")
+               "intent_b200_gemm_i8", "intent_b200_w8a8_gemm", "intent_b200_w4a8_packed_matmul",
+               "intent_b200_ragged_grouped_gemm", "intent_b200_routed_expert_projection", "intent_b200_moe_expert_ffn",
+               "intent_b200_gemm_f16", "intent_b200_bf16_gemm", "intent_b200_quantized_gemm",
+               "intent_b200_moe_grouped_w4a16")
 
 
 class _Launched:

@@ -5,6 +5,7 @@ import torch
 
 import intent_b200 as ib
 import oracle
+from oracle.packed import unpack_w4a8
 
 pytestmark = pytest.mark.gpu
 
@@ -50,9 +51,16 @@ def test_pair_tiles_are_exact(cuda_device, M, K, N):
     assert torch.equal(out, oracle.gemm_i8_exact_f64(a, b, bias))
 
 
-def test_pair_tiles_with_the_second_operand_k_major(cuda_device):
-    """The packed programs hand their decoded weights over as [N, K]; both operands ragged, more tiles than pairs."""
-    M, K, N = 4112, 1056, 1400
+@pytest.mark.parametrize("M,K,N,kernel", [      # activation rows, k, weight rows (the rows of the product)
+    (4112, 1056, 1400, PAIRS),    # both operands ragged, more tiles than pairs
+    (1168, 6496, 816, PAIRS),     # one tile per pair; the rows of B share lines of the L2
+    (16, 2048, 4112, PAIRS),      # sixteen columns, many row tiles
+    (1168, 6528, 816, LONE),      # the rows of B on lines of their own
+    (272, 7168, 9400, LONE),      # 64 MB of A: three bands of the tile walk
+    (48, 2080, 816, LONE),        # little of B to share
+])
+def test_second_operand_k_major(cuda_device, M, K, N, kernel):
+    """The packed programs hand their decoded weights over as the first operand and the activations as B [N, K]."""
     g = torch.Generator().manual_seed(3)
     activation = torch.randint(-128, 128, (M, K), generator=g, dtype=torch.int8)
     packed = torch.randint(0, 256, (N, K // 2), generator=g, dtype=torch.uint8)
@@ -60,9 +68,8 @@ def test_pair_tiles_with_the_second_operand_k_major(cuda_device):
     out = artifact.run(activation.to(cuda_device), packed.to(cuda_device))        # [N, M]
     torch.cuda.synchronize()
     artifact.check()
-    assert torch.equal(out.cpu(), oracle.w4a8_packed_matmul(activation, packed))
-    # (this entry reports no facts; the rule reads the sizes of the product alone)
-    assert _run(cuda_device, *_operands(N, K, M))[1].startswith(PAIRS)
+    assert artifact.observation.kernel.startswith(kernel)
+    assert torch.equal(out.cpu(), oracle.gemm_i8_exact_f64(unpack_w4a8(packed), activation.T))
 
 
 @pytest.mark.parametrize("M,K,N,kernel", [
@@ -70,6 +77,8 @@ def test_pair_tiles_with_the_second_operand_k_major(cuda_device):
     (512, 1024, 2048, LONE), (512, 4096, 2048, PAIRS),       # too few k blocks to earn the pair launch back, and enough
     (129, 3072, 1024, LONE), (129, 8192, 1024, PAIRS),       # the same for eight tiles
     (2050, 1024, 2048, LONE), (2048, 1024, 2048, PAIRS),     # an odd row tile, many row tiles
+    (135, 2240, 4480, LONE), (135, 2240, 4496, PAIRS),       # rows of B on lines of their own, and sharing them
+    (3934, 576, 3664, LONE), (1840, 1536, 7520, LONE),       # several waves: few k blocks; a narrow last column
 ])
 def test_short_walks_run_on_lone_tiles(cuda_device, M, K, N, kernel):
     a, b, bias = (t.to(cuda_device) for t in _operands(M, K, N))
