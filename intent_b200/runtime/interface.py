@@ -19,7 +19,6 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 from enum import IntEnum
-from functools import cached_property
 
 from ..dtypes import DType, torch_dtype
 
@@ -124,28 +123,34 @@ class PublicInterface:
         # callables(dimensions: dict) -> None raising ValueError; derived relations such
         # as "packed rows * 8 == K" that tie symbolic dimensions together.
         self.dimension_rules = tuple(dimension_rules)
+        self._derived: tuple | None = None               # (views, inputs, outputs, pairs with a writable one)
+        self._allocation_errors: tuple | None = None
 
-    # -- views of the declaration: fixed by it, read on every call and put together by the first one ------------
-    @cached_property
+    # -- views of the declaration: fixed by it and put together by the first call ---------------------------------
+    def _derive(self) -> tuple:
+        views, inputs, outputs = [], [], []
+        for parameter in self.parameters:
+            if not isinstance(parameter, ViewParameter):
+                inputs.append(parameter)
+                continue
+            (outputs if parameter.access is ViewKind.OUT else inputs).append(parameter)
+            views.append(parameter)
+        pairs = [(left, right) for index, left in enumerate(views) for right in views[index + 1:]
+                 if left.access is not ViewKind.IN or right.access is not ViewKind.IN]
+        self._derived = (tuple(views), tuple(inputs), tuple(outputs), tuple(pairs))
+        return self._derived
+
+    @property
     def views(self) -> tuple:
-        return tuple(p for p in self.parameters if isinstance(p, ViewParameter))
+        return (self._derived or self._derive())[0]
 
-    @cached_property
+    @property
     def inputs(self) -> tuple:
-        return tuple(p for p in self.parameters if not isinstance(p, ViewParameter) or not p.output)
+        return (self._derived or self._derive())[1]
 
-    @cached_property
+    @property
     def outputs(self) -> tuple:
-        return tuple(p for p in self.views if p.output)
-
-    @cached_property
-    def _allocation_errors(self) -> tuple:
-        return self.output_allocation_errors()
-
-    @cached_property
-    def _writable_pairs(self) -> tuple:
-        return tuple((left, right) for index, left in enumerate(self.views)
-                     for right in self.views[index + 1:] if left.writable or right.writable)
+        return (self._derived or self._derive())[2]
 
     @property
     def mutable_inputs(self) -> tuple:
@@ -176,6 +181,8 @@ class PublicInterface:
 
     def require_output_allocation(self) -> None:
         errors = self._allocation_errors
+        if errors is None:
+            errors = self._allocation_errors = self.output_allocation_errors()
         if errors:
             raise NotImplementedError(
                 "Cannot allocate the declared outputs: " + "; ".join(errors) +
@@ -235,7 +242,8 @@ class PublicInterface:
         address facts, no entry-storage checks."""
         import torch
 
-        supplied = self.parameters if explicit_outputs else self.inputs
+        _, inputs, outputs, writable_pairs = self._derived or self._derive()
+        supplied = self.parameters if explicit_outputs else inputs
         if len(arguments) != len(supplied):
             raise TypeError(f"expected {len(supplied)} runtime arguments, got {len(arguments)}")
         if not explicit_outputs:
@@ -286,7 +294,7 @@ class PublicInterface:
             for rule in self.dimension_rules:
                 rule(dimensions)
         if not explicit_outputs:
-            for parameter in self.outputs:
+            for parameter in outputs:
                 shape = tuple(extent if isinstance(extent, int) else
                               (extent(dimensions) if isinstance(extent, Derived) else dimensions[extent])
                               for extent in parameter.shape)
@@ -296,10 +304,9 @@ class PublicInterface:
                 values[parameter.position] = value
                 facts[parameter.position] = observed
         if not abstract:
-            for left, right in self._writable_pairs:
+            for left, right in writable_pairs:
                 a, b = facts[left.position], facts[right.position]
                 if byte_spans_overlap((a.begin, a.end), (b.begin, b.end)):
                     raise NotImplementedError(
                         f"{left.name} and {right.name}: native entry requires nonoverlapping accessed byte spans")
-        outputs = tuple(values[p.position] for p in self.outputs)
-        return BoundArguments(tuple(values), outputs, tuple(facts), dimensions)
+        return BoundArguments(tuple(values), tuple(values[p.position] for p in outputs), tuple(facts), dimensions)

@@ -17,7 +17,7 @@ from ..errors import CompilationStageError
 _LOCK = Lock()
 _LIBRARY: ctypes.CDLL | None = None
 _ENTRIES: dict = {}
-_SELECTION: tuple | None = None        # address and bytes of the switches
+_SELECTION: ctypes.Array | None = None        # the switches, in the library's own memory
 
 _CARRIERS = {"ptr": ctypes.c_void_p, "bool": ctypes.c_bool, "i8": ctypes.c_int8, "i16": ctypes.c_int16,
              "i32": ctypes.c_int32, "i64": ctypes.c_int64, "f32": ctypes.c_float, "f64": ctypes.c_double}
@@ -79,8 +79,8 @@ def selection() -> bytes:
         where.restype, where.argtypes = ctypes.c_void_p, [ctypes.c_void_p]
         count = ctypes.c_int32()
         address = where(ctypes.byref(count))
-        _SELECTION = (address, 4 * count.value)
-    return ctypes.string_at(*_SELECTION)
+        _SELECTION = (ctypes.c_char * (4 * count.value)).from_address(address)
+    return _SELECTION.raw
 
 
 def status_string(status: int) -> str:
