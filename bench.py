@@ -56,7 +56,7 @@ FALLBACK_BF16_TFLOPS = 1590.0
 # captures summarised under profiles/, taken on ONE GPU with the full problem.  A rank of a sharded run
 # computes a different problem (a column shard against the whole of X), whose traffic was not captured and
 # does not scale with the shard: there the line reports null.
-NCU_TRAFFIC_BYTES_1GPU = {"decode": 30314496, "prefill": 529902848, "w8a8": 149691136, "grouped": 1231225192,
+NCU_TRAFFIC_BYTES_1GPU = {"decode": 30314496, "prefill": 521989632, "w8a8": 156809728, "grouped": 1231225192,
                           "moe": None}
 
 

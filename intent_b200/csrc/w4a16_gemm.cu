@@ -14,9 +14,9 @@
 //                 reads its packed words straight from global memory (a warp reads 128 contiguous
 //                 bytes per packed row; three blocks are kept in flight in registers), expands
 //                 them to values of T with the magic-number trick (prmt + lop3, exact subtract,
-//                 one rounding multiply by the scale) and writes them into the 128-byte row n of the K-major, 128B-swizzled B
-//                 operand tile.  Shared memory therefore carries each weight once (the operand
-//                 tile), not twice.
+//                 one rounding multiply by the scale) and writes them into the 128-byte row n of the
+//                 K-major, 128B-swizzled B operand tile.  Shared memory therefore carries each weight
+//                 once (the operand tile), not twice.
 //   warp 1        MMA issuer: one thread issues, per k block, four tcgen05.mma (M128 N=BN K16,
 //                 kind::f16, f32 accumulation in TMEM) for each of the MT row blocks - the row
 //                 blocks share the dequantised B tile - and commits to the mbarriers that free
@@ -98,7 +98,7 @@ struct GemmParams {
   int M, K;
   int WN;                    // columns of the weight matrix
   int k_blocks;              // ceil(K / 64)
-  int m_tiles, n_tiles;      // tiles of (MT*128) rows, tiles of 256 accumulator columns
+  int m_tiles, n_tiles;      // tiles of (MT*128) rows, tiles of BN accumulator columns
   int group_size;
   int twos_complement;
   int second_half_offset;    // weight-column distance of accumulator columns 128..255 (128, or I for up|gate)
@@ -591,10 +591,11 @@ int launch_gemm(const void* x, int64_t rows, int64_t K, const void* w, const voi
   p.route_weight = route_weight;
   p.routes = int(routes);
   p.top_k = top_k;
-  // Few rows per expert (at most 64 on average, `rows` counting 127 of padding for each): the weights come from HBM
-  // and three k blocks in flight do not cover its latency, so the L2 is asked eight blocks early.  64 tokens on 64
-  // experts of 4096 x 1408: 339 + 146 -> 307 + 135 us for the two contractions.  With many rows most of the weights
-  // are in the L2 already and the extra instructions cost 1 % (848 + 504 -> 858 + 508 us at 16384 tokens).
+  // Few rows per expert (at most 64 on average, `rows` counting 127 of padding for each, as blocks of 128 rows have
+  // it; blocks of 256 pad by more and never ask): the weights come from HBM and three k blocks in flight do not cover
+  // its latency, so the L2 is asked eight blocks early.  64 tokens on 64 experts of 4096 x 1408, the two contractions
+  // timed apart and in a row of their own: 339 + 146 -> 307 + 135 us.  With many rows most of the weights are in the
+  // L2 already and the extra instructions cost 1 % (848 + 504 -> 858 + 508 us at 16384 tokens).
   p.ahead = MODE != MODE_DENSE && !prelaid && rows <= experts * (64 + BM) ? 8 : 0;
 
   CUtensorMap map_x;
@@ -625,7 +626,7 @@ int launch_gemm(const void* x, int64_t rows, int64_t K, const void* w, const voi
 // weights are microseconds per k block measured on one tile per SM (bf16, group 128); the k blocks are the same
 // number for all forms.  A wide tile expands the most weights per microsecond, a narrow one spreads a small call over
 // the chip: M77 K14336 N4096 is 16 tiles of 256 columns (156 us), 32 of 128 (94), 64 of 64 (86) or 128 of 32 (81);
-// M512 K2048 N4096 8 pair tiles (33.6 us), 64 of 256 columns (25.6) or 128 of 128 (19.2); M1024 K4096 N4096 32 pair
+// M512 K2048 N4096 16 pair tiles (33.6 us), 64 of 256 columns (25.6) or 128 of 128 (19.2); M1024 K4096 N4096 32 pair
 // tiles (58.9 us) or 128 of 256 columns (50.3).  Large calls stay on the pairs (M2048 K4096 N4096 59.9 us against
 // 88.2).  All forms add the k blocks in the same order, so the bits of a row do not depend on the form.
 enum class Form { PAIR, TWO_BLOCKS, N256, N128, N64, N32 };

@@ -15,8 +15,9 @@
 // Roles per CTA (22 warps): warp 0 TMA producer (its own rows of X; the transaction bytes of
 // both CTAs complete on the leader's mbarrier), warps 6..21 dequantisers (four sets of four
 // warps, a thread per weight column, take turns at the k blocks; packed words straight from global
-// memory, two of a set's blocks ahead), warps 2..5 epilogue (own TMEM lanes).  Only the leader CTA (cluster rank 0) issues MMAs (one thread
-// of warp 1); its commits arrive on the stage barriers of both CTAs.
+// memory, two of a set's blocks ahead), warps 2..5 epilogue (own TMEM lanes).  Only the leader CTA
+// (cluster rank 0) issues MMAs (one thread of warp 1); its commits arrive on the stage barriers of
+// both CTAs.
 // In sets a dequantiser warp pays its hundred instructions of bookkeeping per k block on every
 // fourth block instead of on every one (it had two packed words a thread to show for it): 8192^3
 // 977 -> 927 us per call, M2048 K4096 N4096 67 -> 60 us.  Six operand stages, so that each set has
@@ -281,8 +282,9 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairPara
         static_assert(DQ_ROWS == 8, "the tiled layout is two halves of four words per column");
         const uint4 v = __ldg(reinterpret_cast<const uint4*>(f_w));
         const uint4 u = __ldg(reinterpret_cast<const uint4*>(f_w + (f_col_ok ? 128 * 4 : 0)));
-        b.w[0] = f_col_ok ? v.x : 0u; b.w[1] = f_col_ok ? v.y : 0u; b.w[2] = f_col_ok ? v.z : 0u; b.w[3] = f_col_ok ? v.w : 0u;
-        b.w[4] = f_col_ok ? u.x : 0u; b.w[5] = f_col_ok ? u.y : 0u; b.w[6] = f_col_ok ? u.z : 0u; b.w[7] = f_col_ok ? u.w : 0u;
+        const bool use = f_col_ok;
+        b.w[0] = use ? v.x : 0u; b.w[1] = use ? v.y : 0u; b.w[2] = use ? v.z : 0u; b.w[3] = use ? v.w : 0u;
+        b.w[4] = use ? u.x : 0u; b.w[5] = use ? u.y : 0u; b.w[6] = use ? u.z : 0u; b.w[7] = use ? u.w : 0u;
       } else if (f_col_ok && rows_left >= DQ_ROWS) {
         const uint32_t* q = f_w;
 #pragma unroll

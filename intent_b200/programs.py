@@ -314,8 +314,8 @@ def _lower_align(c, device):
         ViewParameter(2, "expert_blocks", dtypes.i32, (blocks,), OUT, alignment=4),
         ViewParameter(3, "total_padded", dtypes.i32, (1,), OUT, alignment=4),
     ), dimension_rules=(_rule(lambda d: d["T"] <= tokens, f"at most {tokens} tokens (TOKENS constexpr)"),))
-    return NativeProgram(interface=interface, entry_name="intent_b200_moe_align_routes", constants=(experts, block, routes),
-                         device=device)
+    return NativeProgram(interface=interface, entry_name="intent_b200_moe_align_routes",
+                         constants=(experts, block, routes), device=device)
 
 
 def _lower_positions(c, device):
@@ -494,8 +494,8 @@ moe_combine = KernelDefinition("moe_combine", {"ACCUMULATE": True}, _lower_combi
                                "examples/kernels/ragged/moe.py:48-53 (weighted scatter_reduce add)",
                                "y[t] += sum_c weight[t,c] * rows[position[t,c]] in choice order")
 
-ALL.update({d.name: d for d in (moe_align_routes, moe_count_routes, moe_prefix_routes, moe_scatter_routes, moe_mark_expert_blocks,
-                                moe_route_positions, moe_route_top2, moe_gather_rows, moe_grouped_upgate_silu,
+ALL.update({d.name: d for d in (moe_align_routes, moe_count_routes, moe_prefix_routes, moe_scatter_routes,
+                                moe_mark_expert_blocks, moe_route_positions, moe_route_top2, moe_gather_rows, moe_grouped_upgate_silu,
                                 moe_grouped_down, moe_grouped_down_scatter, moe_combine)})
 
 

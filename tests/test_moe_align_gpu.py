@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("tokens,given,experts,block", [(1, 1, 1, 128), (40, 33, 8, 128), (1000, 1000, 3, 16),
-                                                        (2049, 2049, 100, 256)])
+                                                        (2049, 2049, 100, 256), (300, 300, 8192, 128)])
 def test_one_launch_equals_the_stages(cuda_device, tokens, given, experts, block):
     g = torch.Generator().manual_seed(tokens + experts)
     ids = torch.randint(-1, experts + 1, (given, 2), generator=g, dtype=torch.int32)     # ids outside the table too

@@ -96,8 +96,9 @@ def test_gemm_full_size_prefill_rows(cuda_device):
 
 def test_reference_case_at_its_own_size(cuda_device):
     """The reference's own W4A16 case at its own size (M512 K2048 N4096, group 64, signed nibbles, f16;
-    experiments/cpu/providers/mojo/contraction.py:190-198), on tiles of 128 columns.  Checked against stored rows of the reference module's output at the reference's atol = 4e-2,
-    against the oracle on every row, and at the benchmark's 2e-2 * max|ref|."""
+    experiments/cpu/providers/mojo/contraction.py:190-198), on tiles of 128 columns.  Checked against stored rows of
+    the reference module's output at the reference's atol = 4e-2, against the oracle on every row, and at the
+    benchmark's 2e-2 * max|ref|."""
     import importlib.util
     from pathlib import Path
 

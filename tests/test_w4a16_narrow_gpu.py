@@ -20,7 +20,8 @@ pytestmark = pytest.mark.gpu
 ])
 def test_narrow_tiles_give_the_bits_of_the_wide_ones(cuda_device, dtype, M, K, N, group):
     """Every tile form adds the k blocks in the same order, so a row's bits do not depend on how many rows the call
-    has (4096 rows take a wider tile, or the same one where there are only 8 or 40 columns); the tolerances against the oracle are those of the wide tiles (test_w4a16_gemm_gpu.py)."""
+    has (4096 rows take a wider tile, or the same one where there are only 8 or 40 columns); the tolerances against
+    the oracle are those of the wide tiles (test_w4a16_gemm_gpu.py)."""
     x, p, s = ib.workloads.w4a16_inputs(4096, K, N, dtype=dtype, group_size=group, seed=M)
     artifact = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),
                           constexprs={"GROUP_SIZE": group, "ZERO_POINT": 8,
