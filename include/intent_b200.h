@@ -292,6 +292,10 @@ INTENT_B200_API int intent_b200_moe_route_positions(INTENT_B200_VIEW1(a0), INTEN
  * a0 x [T,H] 16-bit, a1 sorted_route_ids [P], a2 total_padded [1] -> a3 rows [P,H]; padding rows are zero. */
 INTENT_B200_API int intent_b200_moe_gather_rows(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2),
                                                 INTENT_B200_VIEW2(a3), int32_t top_k, void* stream);
+/* The same without the padding: rows of a3 that no route fills keep what they held. */
+INTENT_B200_API int intent_b200_moe_gather_routed_rows(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1),
+                                                       INTENT_B200_VIEW1(a2), INTENT_B200_VIEW2(a3), int32_t top_k,
+                                                       void* stream);
 /* Grouped int4 contractions over expert-sorted rows padded to block_rows (128 or 256, the alignment's
  * BLOCK_SIZE) per expert; a1 expert_blocks holds one expert id per block_rows rows (tcgen05 kernel of
  * weight_only_int4_matmul with a per-block expert; reference programs
@@ -309,6 +313,17 @@ INTENT_B200_API int intent_b200_moe_grouped_w4a16_upgate_silu_bf16(INTENT_B200_G
 INTENT_B200_API int intent_b200_moe_grouped_w4a16_upgate_silu_f16(INTENT_B200_GROUPED_SLOTS);
 INTENT_B200_API int intent_b200_moe_grouped_w4a16_down_f32_bf16(INTENT_B200_GROUPED_SLOTS);
 INTENT_B200_API int intent_b200_moe_grouped_w4a16_down_f32_f16(INTENT_B200_GROUPED_SLOTS);
+/* The up|gate projection of rows that the alignment's route list describes: a0 .. a4 as above, a5 sorted_route_ids
+ * [>= P] i32, a6 route_weights [T,K] f32 (only its extents are used: values of a5 outside [0, T*K) mark padding rows),
+ * a7 output [P,I] T.  Rows of padding may be left unwritten, and what they hold in a0 does not matter. */
+INTENT_B200_API int intent_b200_moe_grouped_w4a16_upgate_silu_routed_bf16(
+    INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2), INTENT_B200_VIEW3(a3), INTENT_B200_VIEW3(a4),
+    INTENT_B200_VIEW1(a5), INTENT_B200_VIEW2(a6), INTENT_B200_VIEW2(a7), int32_t group_size, int32_t zero_point,
+    int32_t block_rows, void* stream);
+INTENT_B200_API int intent_b200_moe_grouped_w4a16_upgate_silu_routed_f16(
+    INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2), INTENT_B200_VIEW3(a3), INTENT_B200_VIEW3(a4),
+    INTENT_B200_VIEW1(a5), INTENT_B200_VIEW2(a6), INTENT_B200_VIEW2(a7), int32_t group_size, int32_t zero_point,
+    int32_t block_rows, void* stream);
 /* Down projection with the weighted combine of examples/kernels/ragged/moe.py:43-53 in its epilogue:
  *   a0 hidden rows [P,K] T, a1 expert_blocks [B], a2 total_padded [1], a3 packed [E,K/8,WN], a4 scales [E,K/G,WN],
  *   a5 sorted_route_ids [>= P] i32 (route of every expert-sorted row; values outside [0, T*K) mark padding rows),

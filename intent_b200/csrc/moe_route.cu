@@ -228,7 +228,8 @@ __global__ void moe_positions_kernel(const int* __restrict__ sorted, const int* 
   }
 }
 
-// ---- gather: xs[p, :] = x[sorted[p] / top_k, :], zero rows for the padding ----
+// ---- gather: xs[p, :] = x[sorted[p] / top_k, :]; padding rows are zeros, or left alone without PADDING ----
+template <bool PADDING>
 __global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ sorted,
                                        const int* __restrict__ total, int capacity, int routes, int top_k,
                                        int row_vectors, uint4* __restrict__ out) {
@@ -236,6 +237,7 @@ __global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, const int* _
   for (int p = blockIdx.x; p < limit; p += gridDim.x) {
     const int r = sorted[p];
     const bool real = r >= 0 && r < routes;
+    if (!PADDING && !real) continue;
     const uint4* src = x + size_t(real ? r / top_k : 0) * row_vectors;
     uint4* dst = out + size_t(p) * row_vectors;
     for (int i = threadIdx.x; i < row_vectors; i += blockDim.x) dst[i] = real ? src[i] : make_uint4(0, 0, 0, 0);
@@ -368,20 +370,34 @@ extern "C" int intent_b200_moe_route_positions(INTENT_B200_VIEW1(a0), INTENT_B20
   return launch_status();
 }
 
+namespace ib200 {
+namespace {
+template <bool PADDING>
+int gather_rows(View2 x, View1 sorted, View1 total, View2 out, int top_k, cudaStream_t stream) {
+  if (out.d1 != x.d1 || out.d0 != sorted.d0 || total.d0 != 1 || top_k <= 0) return INTENT_B200_ERR_SHAPE;
+  if (sorted.d0 == 0 || x.d1 == 0) return INTENT_B200_OK;
+  if (!x.p || !sorted.p || !total.p || !out.p) return INTENT_B200_ERR_NULL;
+  if (!contiguous(x) || !contiguous(out) || !aligned16(x.p) || !aligned16(out.p)) return INTENT_B200_ERR_LAYOUT;
+  if (x.d1 % 8 != 0) return INTENT_B200_ERR_UNSUPPORTED;
+  moe_gather_rows_kernel<PADDING><<<grid_for(sorted.d0, 1, 148 * 16), 256, 0, stream>>>(
+      static_cast<const uint4*>(x.p), static_cast<const int*>(sorted.p), static_cast<const int*>(total.p),
+      int(sorted.d0), int(x.d0 * top_k), top_k, int(x.d1 / 8), static_cast<uint4*>(out.p));
+  note_launch();
+  return launch_status();
+}
+}  // namespace
+}  // namespace ib200
+
 // x [T,H] (16-bit), sorted_route_ids [capacity], total_padded [1] -> rows [capacity, H]; top_k scalar
 extern "C" int intent_b200_moe_gather_rows(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2),
                                            INTENT_B200_VIEW2(a3), int32_t top_k, void* stream) {
-  if (a3_d1 != a0_d1 || a3_d0 != a1_d0 || a2_d0 != 1 || top_k <= 0) return INTENT_B200_ERR_SHAPE;
-  if (a1_d0 == 0 || a0_d1 == 0) return INTENT_B200_OK;
-  if (!a0 || !a1 || !a2 || !a3) return INTENT_B200_ERR_NULL;
-  if (!contiguous(IB200_VIEW2_ARG(a0)) || !contiguous(IB200_VIEW2_ARG(a3)) || !aligned16(a0) || !aligned16(a3))
-    return INTENT_B200_ERR_LAYOUT;
-  if (a0_d1 % 8 != 0) return INTENT_B200_ERR_UNSUPPORTED;
-  moe_gather_rows_kernel<<<grid_for(a1_d0, 1, 148 * 16), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(a0), static_cast<const int*>(a1), static_cast<const int*>(a2), int(a1_d0),
-      int(a0_d0 * top_k), top_k, int(a0_d1 / 8), static_cast<uint4*>(a3));
-  note_launch();
-  return launch_status();
+  return gather_rows<true>(IB200_VIEW2_ARG(a0), IB200_VIEW1_ARG(a1), IB200_VIEW1_ARG(a2), IB200_VIEW2_ARG(a3), top_k,
+                           static_cast<cudaStream_t>(stream));
+}
+extern "C" int intent_b200_moe_gather_routed_rows(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2),
+                                                  INTENT_B200_VIEW2(a3), int32_t top_k, void* stream) {
+  return gather_rows<false>(IB200_VIEW2_ARG(a0), IB200_VIEW1_ARG(a1), IB200_VIEW1_ARG(a2), IB200_VIEW2_ARG(a3), top_k,
+                            static_cast<cudaStream_t>(stream));
 }
 
 // rows [P,H] f32, route_positions [T*K] i32, route_weights [T,K] f32, y [T,H] f32 (InOut; with

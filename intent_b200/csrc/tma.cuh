@@ -108,6 +108,38 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   return false;
 }
 
+// The same for a whole converged warp: the loop leaves by a vote, so the compiler knows the branch to be uniform and
+// keeps what depends on it in uniform registers, which the TMA and tensor-core instructions read.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint32_t limit = 1u << 16) {
+  for (uint32_t i = 0; i < limit; ++i)
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return false;
+}
+
+// Whether a phase has completed, without waiting: asked one step ahead, the answer is there when it is needed.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+// True in one lane of a converged warp, the same one each time.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t elected;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(elected)::"memory");
+  return elected != 0;
+}
+
 // 2-D tiled load, no multicast: coordinates are (c0 = innermost element index, c1 = row).
 // c0 * element size must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {

@@ -53,6 +53,7 @@
 #include "common.cuh"
 #include "tma.cuh"
 #include "umma.cuh"
+#include "w4a16_tmem.cuh"
 
 namespace ib200 {
 
@@ -691,12 +692,37 @@ int run(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, cuda
   }
 }
 
+// Whether a grouped call with the weights in tensor memory runs on CTA pairs: from 64 rows per expert on average on
+// (`rows` counts 127 of padding for each expert).
+bool grouped_pairs(int64_t rows, int64_t experts) { return rows > experts * (64 + BM); }
+
+// The kernel with the weights in tensor memory for a grouped call (sizes, layouts and alignments checked by the
+// caller); UNSUPPORTED when it does not take the call.
+template <typename T>
+int grouped_tmem(int mode, View2 x, View1 tile_expert, View1 total, View3 w, View3 s, void* out, int64_t out_cols,
+                 int group_size, int zero_point, int block_rows, const int* row_route, const float* route_weight,
+                 int64_t routes, int top_k, cudaStream_t stream) {
+  TmemCall q{};
+  q.x = x.p, q.rows = x.d0, q.K = x.d1;
+  q.w = w.p, q.s = s.p, q.experts = w.d0, q.WN = w.d2;
+  q.out = out, q.out_cols = out_cols;
+  q.group_size = group_size, q.zero_point = zero_point;
+  q.row_tile = 128, q.split = 1;
+  q.total_rows = static_cast<const int*>(total.p);
+  q.tile_expert = static_cast<const int*>(tile_expert.p);
+  q.block_rows = block_rows;
+  q.row_route = row_route, q.route_weight = route_weight, q.routes = routes, q.top_k = top_k;
+  return w4a16_tmem<T>(q, mode, grouped_pairs(x.d0, w.d0), stream);
+}
+
 // Grouped contractions over expert-sorted rows padded to `block_rows` (128 or 256) per expert; with 256
 // two row blocks share every dequantised weight tile.
-//   x [P, K]; tile_expert [>= P/block_rows]; total [1]; w [E, K/8, WN]; s [E, K/G, WN]; out [P, out_cols]
+//   x [P, K]; tile_expert [>= P/block_rows]; total [1]; w [E, K/8, WN]; s [E, K/G, WN]; out [P, out_cols];
+//   sorted_routes [>= P], or null: the route of every row; rows of no route in [0, routes) may be left out
 template <typename T, int MODE>
 int run_grouped(View2 x, View1 tile_expert, View1 total, View3 w, View3 s, View2 out, int group_size, int zero_point,
-                int block_rows, cudaStream_t stream, bool prelaid = false) {
+                int block_rows, cudaStream_t stream, bool prelaid = false, const int* sorted_routes = nullptr,
+                int64_t routes = 0) {
   const int64_t P = x.d0, K = x.d1, E = w.d0, WN = w.d2;
   const int64_t out_cols = MODE == MODE_UPGATE_SILU ? WN / 2 : WN;
   if (group_size != 32 && group_size != 64 && group_size != 128) return INTENT_B200_ERR_UNSUPPORTED;
@@ -713,6 +739,11 @@ int run_grouped(View2 x, View1 tile_expert, View1 total, View3 w, View3 s, View2
   if (K == 0 || WN % 8 != 0 || (MODE == MODE_UPGATE_SILU && (WN % 256 != 0)) ||
       P > (1 << 24) || K > (1 << 24) || WN > (1 << 24))
     return INTENT_B200_ERR_UNSUPPORTED;
+  if (!prelaid) {
+    const int status = grouped_tmem<T>(MODE, x, tile_expert, total, w, s, out.p, out_cols, group_size, zero_point,
+                                       block_rows, sorted_routes, nullptr, routes, 1, stream);
+    if (status != INTENT_B200_ERR_UNSUPPORTED) return status;
+  }
   if (block_rows == 2 * BM || (P + BM - 1) / BM <= PAIR_LIST_BLOCKS)   // 128-row blocks are paired by the kernel
     return launch_gemm<T, MODE, 2>(x.p, P, K, w.p, s.p, WN, out.p, out_cols, group_size, zero_point,
                                    static_cast<const int*>(total.p), static_cast<const int*>(tile_expert.p), stream,
@@ -746,6 +777,11 @@ int run_down_scatter(View2 x, View1 tile_expert, View1 total, View3 w, View3 s, 
     return INTENT_B200_ERR_UNSUPPORTED;
   const int* routes = static_cast<const int*>(sorted_routes.p);
   const float* route_weight = static_cast<const float*>(weights.p);
+  if (!prelaid) {
+    const int status = grouped_tmem<T>(MODE_DOWN_SCATTER, x, tile_expert, total, w, s, y.p, WN, group_size, zero_point,
+                                       block_rows, routes, route_weight, tokens * top_k, int(top_k), stream);
+    if (status != INTENT_B200_ERR_UNSUPPORTED) return status;
+  }
   if (block_rows == 2 * BM || (P + BM - 1) / BM <= PAIR_LIST_BLOCKS)
     return launch_gemm<T, MODE_DOWN_SCATTER, 2>(x.p, P, K, w.p, s.p, WN, y.p, WN, group_size, zero_point,
                                                 static_cast<const int*>(total.p),
@@ -782,17 +818,19 @@ int w4a16_gemm_bf16(View2 x, View2 w, View2 s, View2 y, int g, int zp, cudaStrea
 }  // namespace ib200
 
 // Reads (and clears) the status words of the tensor-core W4A16 kernels - the single-CTA kernel of this
-// file and the CTA-pair kernel, which keeps its own word - and synchronises the device.
+// file, the CTA-pair kernel and the kernel with the weights in tensor memory, which keep words of their own - and
+// synchronises the device.
 extern "C" int intent_b200_w4a16_gemm_device_status(void) {
-  int value = 0, pair_value = 0, zero = 0;
+  int value = 0, pair_value = 0, tmem_value = 0, zero = 0;
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return ib200::cuda_status(e);
   e = cudaMemcpyFromSymbol(&value, ib200::g_w4a16_gemm_status, sizeof(int));
   if (e != cudaSuccess) return ib200::cuda_status(e);
   if (value != 0) cudaMemcpyToSymbol(ib200::g_w4a16_gemm_status, &zero, sizeof(int));
-  const int status = ib200::w4a16_gemm_pair_take_status(&pair_value);
+  int status = ib200::w4a16_gemm_pair_take_status(&pair_value);
+  if (status == INTENT_B200_OK) status = ib200::w4a16_tmem_take_status(&tmem_value);
   if (status != INTENT_B200_OK) return status;
-  return value != 0 ? value : pair_value;
+  return value != 0 ? value : pair_value != 0 ? pair_value : tmem_value;
 }
 
 #define IB200_GROUPED_ENTRY(NAME, TYPE, MODE)                                                                   \
@@ -808,6 +846,23 @@ IB200_GROUPED_ENTRY(intent_b200_moe_grouped_w4a16_upgate_silu_bf16, __nv_bfloat1
 IB200_GROUPED_ENTRY(intent_b200_moe_grouped_w4a16_upgate_silu_f16, __half, MODE_UPGATE_SILU)
 IB200_GROUPED_ENTRY(intent_b200_moe_grouped_w4a16_down_f32_bf16, __nv_bfloat16, MODE_GROUPED_F32)
 IB200_GROUPED_ENTRY(intent_b200_moe_grouped_w4a16_down_f32_f16, __half, MODE_GROUPED_F32)
+
+// up|gate projection of routed rows: sorted routes and route weights as in the down projection (of the weights only the
+// extents are used: the number of routes)
+#define IB200_ROUTED_UPGATE_ENTRY(NAME, TYPE)                                                                       \
+  extern "C" int NAME(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2), INTENT_B200_VIEW3(a3),     \
+                      INTENT_B200_VIEW3(a4), INTENT_B200_VIEW1(a5), INTENT_B200_VIEW2(a6), INTENT_B200_VIEW2(a7),     \
+                      int32_t group_size, int32_t zero_point, int32_t block_rows, void* stream) {                    \
+    if (a5_d0 < a0_d0 || a6_d0 < 0 || a6_d1 < 0 || a6_d0 * a6_d1 > (1 << 30)) return INTENT_B200_ERR_SHAPE;            \
+    if (a0_d0 > 0 && !a5) return INTENT_B200_ERR_NULL;                                                               \
+    if (!ib200::contiguous(IB200_VIEW1_ARG(a5))) return INTENT_B200_ERR_LAYOUT;                                      \
+    return ib200::run_grouped<TYPE, ib200::MODE_UPGATE_SILU>(                                                        \
+        IB200_VIEW2_ARG(a0), IB200_VIEW1_ARG(a1), IB200_VIEW1_ARG(a2), IB200_VIEW3_ARG(a3), IB200_VIEW3_ARG(a4),     \
+        IB200_VIEW2_ARG(a7), group_size, zero_point, block_rows, static_cast<cudaStream_t>(stream), false,           \
+        static_cast<const int*>(a5), a6_d0 * a6_d1);                                                                 \
+  }
+IB200_ROUTED_UPGATE_ENTRY(intent_b200_moe_grouped_w4a16_upgate_silu_routed_bf16, __nv_bfloat16)
+IB200_ROUTED_UPGATE_ENTRY(intent_b200_moe_grouped_w4a16_upgate_silu_routed_f16, __half)
 
 #define IB200_DOWN_SCATTER_ENTRY(NAME, TYPE)                                                                        \
   extern "C" int NAME(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2), INTENT_B200_VIEW3(a3),     \

@@ -1,0 +1,705 @@
+// W4A16 contractions with the weights as the stationary operand in tensor memory (tcgen05, A from TMEM).
+//
+//   Y[m, n] = T( sum_k f32(X[m, k]) * f32( T( (q[k, n] - 8) * S[k / G, n] ) ) )
+//
+// Program: weight_only_int4_matmul (reference kernel body examples/kernels/contraction/weight_only_int4.py:18-51)
+// and the MoE grouped contractions (examples/kernels/ragged/grouped_gemm.py:11-70, ragged/moe.py:12-53 with int4
+// expert weights); the same arithmetic and the same order of the k blocks as w4a16_gemm.cu.
+//
+// Here the product is turned round: the M index of the MMA is the weight column, its N index the activation row.
+// A lane of tensor memory is one weight column, so the thread that expands a column's packed words stores them
+// straight into its own lane (tcgen05.st, 64 columns of 32 bits per 128 k) and the tensor core reads them from there.
+// The expanded weights never pass through shared memory, and a tile has as many rows as the call has, in steps of
+// 16, instead of 128.
+#include <type_traits>
+
+#include "cluster.cuh"
+#include "common.cuh"
+#include "tma.cuh"
+#include "umma.cuh"
+#include "w4a16_tmem.cuh"
+
+namespace ib200 {
+
+__device__ int g_w4a16_tmem_status = 0;
+
+namespace {
+
+constexpr int BK = 128;                    // k per stage
+constexpr int COLS = 128;                  // weight columns of a CTA's tile (lanes of tensor memory)
+constexpr int W_ROWS = BK / 8;             // packed rows of a stage
+constexpr int W_BYTES = W_ROWS * COLS * 4;
+constexpr int S_BYTES = 1024;              // room for the scales of a stage: up to four groups of 128 columns
+constexpr int W_STAGE = W_BYTES + S_BYTES;
+constexpr int SETS = 4;                    // sets of four dequantiser warps that take turns at the k blocks
+constexpr int A_STAGES = SETS;             // stages of expanded weights, 64 columns of tensor memory each
+constexpr int A_COLUMN = 256;              // first tensor-memory column of the expanded weights
+constexpr int ACC_COLUMNS = 256;           // tensor-memory columns of the accumulators (two sets up to 128 rows)
+constexpr int FIRST_EPILOGUE = 4, FIRST_DEQUANT = 8;   // multiples of four: warp % 4 is the TMEM quadrant
+constexpr int THREADS = (FIRST_DEQUANT + 4 * SETS) * 32;
+constexpr int LIST_BLOCKS = 1024;          // most 128-row blocks of a grouped call
+constexpr int SMEM_LIMIT = 227 * 1024;
+
+struct TmemParams {
+  void* y;
+  int M, K;                  // rows and width of the activations
+  int WN, out_cols;          // columns of the weight matrix and of the output
+  int k_blocks;              // ceil(K / 128)
+  int m_tiles, n_tiles;      // row tiles; column tiles of 128 * CG weight columns
+  int row_tile;              // most rows of a tile, a multiple of 16 * CG
+  int box_rows;              // rows of one activation box
+  int x_stages;              // stages of activations, A_STAGES .. 8
+  int w_stages;              // stages of packed words, SETS .. 16
+  int acc_sets;              // accumulator sets that alternate between tiles
+  int split;                 // CTAs of a cluster that share a tile's k blocks (1 = none)
+  int kb_each, kb_extra;     // k blocks of a CTA: the first kb_extra ranks of a cluster take one more
+  uint32_t tile_magic;       // ceil(2^32 / d), d the number of tiles that vary fastest (0 stands for d = 1)
+  int group_shift;           // log2 of the group size
+  int twos_complement;
+  // grouped modes
+  const int* total_rows;     // padded row count (device)
+  const int* tile_expert;    // expert of each block of `block_rows` rows
+  int block_rows;
+  int experts;
+  const int* row_route;      // route of every row; a row with no route in [0, routes) is padding; null: all rows count
+  const float* route_weight; // MODE_DOWN_SCATTER: [routes]
+  int routes, top_k;
+};
+
+constexpr int MODE_DENSE = 0, MODE_UPGATE_SILU = 1, MODE_GROUPED_F32 = 2, MODE_DOWN_SCATTER = 3;
+
+// D[tmem] (+)= A[tmem] * B[smem]
+template <int CG>
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                            bool accumulate) {
+  const uint32_t acc = accumulate ? 1u : 0u;
+  if (CG == 1)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+// 32 lanes x 32 consecutive 32-bit columns: thread i of the warp writes lane (base lane + i)
+__device__ __forceinline__ void tmem_store_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// 32 lanes x 16 columns
+__device__ __forceinline__ void tmem_load_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+  return v;
+}
+
+template <typename T, int MODE, int CG>
+__global__ void __launch_bounds__(THREADS, 1)
+w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                  const __grid_constant__ CUtensorMap map_s, const TmemParams p) {
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  const int x_rows = p.row_tile / CG;                  // activation rows this CTA stages
+  const uint32_t x_half = uint32_t(x_rows) * 128u;     // one box of 64 k
+  const uint32_t smem_x = base;
+  const uint32_t smem_w = smem_x + uint32_t(p.x_stages) * 2u * x_half;
+  const uint32_t bars = smem_w + uint32_t(p.w_stages) * W_STAGE;
+  const uint32_t full_w = bars;                        // [w_stages] packed words and scales landed
+  const uint32_t empty_w = full_w + 8 * p.w_stages;    // [w_stages] read by the dequantisers
+  // One pair of barriers per k block in flight (block i: number i % x_stages) covers both operands: its activations lie
+  // in stage i % x_stages of shared memory, its expanded weights in stage i % A_STAGES of tensor memory.
+  const uint32_t full = empty_w + 8 * p.w_stages;      // [x_stages] leader: activations landed, expanded weights stored
+  const uint32_t empty = full + 8 * p.x_stages;        // [x_stages] MMAs done with them
+  const uint32_t tmem_full = empty + 8 * p.x_stages;   // [2] accumulators complete
+  const uint32_t tmem_empty = tmem_full + 16;          // [2] leader: accumulators drained
+  const uint32_t tmem_slot = tmem_empty + 16;
+  volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
+  int2* list = reinterpret_cast<int2*>(base_ptr + (tmem_slot - base) + 16);   // grouped: {expert, rows} per block
+
+  const int tid = threadIdx.x;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // known to be uniform
+  const int lane = tid & 31;
+  const int rank = CG == 2 || p.split > 1 ? int(cluster_rank()) : 0;
+  const bool leader = CG == 1 || rank == 0;
+
+  if (warp == 0) {          // a lane per stage (at most 16 of a kind)
+    if (lane == 0) {
+      prefetch_tensormap(&map_w);
+      prefetch_tensormap(&map_s);
+      prefetch_tensormap(&map_x);
+    }
+    if (lane < p.w_stages) {
+      mbar_init(full_w + 8 * lane, 1);
+      mbar_init(empty_w + 8 * lane, 4);
+    }
+    if (lane < p.x_stages) {
+      mbar_init(full + 8 * lane, 4 * CG + 1);
+      mbar_init(empty + 8 * lane, 1);
+    }
+    if (lane < 2) {
+      mbar_init(tmem_full + 8 * lane, 1);
+      mbar_init(tmem_empty + 8 * lane, 4 * CG);
+    }
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    if (CG == 2) tmem_alloc_pair(tmem_slot, 512);
+    else tmem_alloc(tmem_slot, 512);
+  }
+  int m_tiles = p.m_tiles;
+  if (MODE != MODE_DENSE) {
+    // rows in use of every 128-row block: its routes come first, padding follows
+    m_tiles = min(m_tiles, (*p.total_rows + 127) / 128);
+    const int per_expert = p.block_rows / 128;
+    for (int b = warp; b < m_tiles; b += THREADS / 32) {
+      int rows = min(128, p.M - b * 128);
+      if (p.row_route != nullptr) {
+        int last = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = i * 32 + lane;
+          const int route = r < rows ? __ldg(p.row_route + b * 128 + r) : -1;
+          const unsigned used = __ballot_sync(0xffffffffu, route >= 0 && route < p.routes);
+          if (used) last = i * 32 + 32 - __clz(used);
+        }
+        rows = last;
+      }
+      if (lane == 0) {
+        int expert = p.tile_expert[b / per_expert];
+        if (unsigned(expert) >= unsigned(p.experts)) {
+          // an id that names no expert (a stale or sentinel table entry): never used as an index.  The plane past
+          // the last expert reads as zeros: zero scales, so zero weights
+          atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_INDEX);
+          expert = p.experts;
+        }
+        list[b] = make_int2(expert, rows);
+      }
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (CG == 2) cluster_sync();   // barriers are initialised before anything arrives remotely
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot_ptr;
+
+  const int items = m_tiles * p.n_tiles;
+  // split: the CTAs of a cluster (a row of the grid) work on one item, each on its own share of the k blocks
+  const int first_item = p.split > 1 ? int(blockIdx.y) : int(blockIdx.x) / CG;
+  const int item_step = p.split > 1 ? items : int(gridDim.x) / CG;
+  const int kb_first = p.split > 1 ? rank * p.kb_each + min(rank, p.kb_extra) : 0;
+  const int kb_count = p.kb_each + (p.split > 1 && rank < p.kb_extra ? 1 : 0);
+  // item / d without a division (items * d < 2^32)
+  auto tile_quotient = [&](int item) { return p.tile_magic ? int(__umulhi(uint32_t(item), p.tile_magic)) : item; };
+  struct Item {
+    int row0, n_tile, expert, rows, n;   // n: rows of the MMA, a multiple of 16 * CG
+  };
+  auto item_of = [&](int item) {
+    Item t;
+    if (MODE == MODE_DENSE) {
+      t.n_tile = tile_quotient(item);   // the row tile varies fastest
+      const int m_tile = item - t.n_tile * m_tiles;
+      t.row0 = m_tile * p.row_tile;
+      t.expert = 0;
+      t.rows = min(p.row_tile, p.M - t.row0);
+    } else {
+      const int block = tile_quotient(item);   // the column tile varies fastest
+      t.n_tile = item - block * p.n_tiles;
+      t.row0 = block * 128;
+      const int2 e = list[block];
+      t.expert = e.x;
+      t.rows = e.y;
+    }
+    t.n = max(16 * CG, (t.rows + 16 * CG - 1) / (16 * CG) * (16 * CG));
+    return t;
+  };
+
+  if (warp == 0) {
+    // ------------------------------ packed weights and scales ------------------
+    const int scale_rows = BK >> p.group_shift;
+    const uint32_t bytes = W_BYTES + uint32_t(scale_rows) * COLS * 2;
+    const int tile_columns = MODE == MODE_UPGATE_SILU ? 64 : COLS, tile_rank = CG == 2 ? rank : 0;
+    uint32_t s = 0, phase = 1;
+    bool ok = true, ready = true;   // ready: the stage was seen to be free
+    for (int item = first_item; item < items && ok; item += item_step) {
+      const Item t = item_of(item);
+      const int column = (t.n_tile * CG + tile_rank) * tile_columns;
+      int row = kb_first * W_ROWS, scale_row = kb_first * scale_rows;
+      for (int kb = 0; kb < kb_count; ++kb, row += W_ROWS, scale_row += scale_rows) {
+        const uint32_t bar = full_w + 8 * s, dst = smem_w + s * W_STAGE;
+        ok = __all_sync(0xffffffffu, ready) || mbar_wait_warp(empty_w + 8 * s, phase);
+        if (!ok) break;
+        if (++s == uint32_t(p.w_stages)) s = 0, phase ^= 1;
+        ready = mbar_test(empty_w + 8 * s, phase);
+        if (elect_one()) {
+          mbar_expect_tx(bar, bytes);
+          tma_load_3d(dst, &map_w, column, row, t.expert, bar);
+          tma_load_3d(dst + W_BYTES, &map_s, column, scale_row, t.expert, bar);
+          if (MODE == MODE_UPGATE_SILU) {   // 64 gate columns, then the 64 up columns that go with them
+            tma_load_3d(dst + W_BYTES / 2, &map_w, column + p.out_cols, row, t.expert, bar);
+            tma_load_3d(dst + W_BYTES + scale_rows * 128, &map_s, column + p.out_cols, scale_row, t.expert, bar);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (!ok && lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
+  } else if (warp == 2) {
+    // ------------------------------ activations --------------------------------
+    const uint32_t full_leader = CG == 2 ? map_to_rank(full, 0) : full;
+    uint32_t s = 0, phase = 1;
+    bool ok = true, ready = true;
+    for (int item = first_item; item < items && ok; item += item_step) {
+      const Item t = item_of(item);
+      const int rows = t.n / CG, row0 = t.row0 + (CG == 2 ? rank * rows : 0);
+      const int boxes = MODE == MODE_DENSE ? 1 : __shfl_sync(0xffffffffu, rows / 16, 0);
+      const uint32_t bytes = uint32_t(CG * boxes * p.box_rows) * 256u;
+      int k = kb_first * BK;
+      for (int kb = 0; kb < kb_count; ++kb, k += BK) {
+        const uint32_t own = full + 8 * s, bar = full_leader + 8 * s;
+        uint32_t dst = smem_x + s * 2u * x_half;
+        ok = __all_sync(0xffffffffu, ready) || mbar_wait_warp(empty + 8 * s, phase);
+        if (!ok) break;
+        if (++s == uint32_t(p.x_stages)) s = 0, phase ^= 1;
+        ready = mbar_test(empty + 8 * s, phase);
+        if (elect_one()) {
+          if (leader) mbar_expect_tx(own, bytes);
+          for (int box = 0, row = row0; box < boxes; ++box, row += 16, dst += 16 * 128) {
+            if (CG == 2) {
+              tma_load_2d_pair(dst, &map_x, k, row, bar);
+              tma_load_2d_pair(dst + x_half, &map_x, k + 64, row, bar);
+            } else {
+              tma_load_2d(dst, &map_x, k, row, bar);
+              tma_load_2d(dst + x_half, &map_x, k + 64, row, bar);
+            }
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (!ok && lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer ---------------------------------
+    // The whole warp walks the loop and one elected lane issues: with the loop inside `lane == 0` the descriptors live
+    // in per-thread registers and every MMA takes about 60 cycles to issue, whatever its size.
+    if (leader) {
+      constexpr uint32_t fmt = std::is_same<T, __half>::value ? 0u : 1u;
+      const bool issue = elect_one();
+      const uint64_t desc_x = umma_desc_k_major_sw128(smem_x);
+      const uint32_t desc_high = uint32_t(desc_x >> 32);
+      uint32_t s = 0, phase = 0, a = 0, local = 0;
+      bool ok = true, ready = false;   // ready: both operands of the k block were seen to be there
+      for (int item = first_item; item < items && ok; item += item_step, ++local) {
+        const Item t = item_of(item);
+        const uint32_t idesc = umma_idesc(1, fmt, fmt, 0, 0, CG * COLS, uint32_t(t.n));
+        const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = p.acc_sets == 2 ? local >> 1 : local;
+        ok = mbar_wait_warp(tmem_empty + 8 * acc, (use & 1) ^ 1);
+        if (!ok) break;
+        tcgen05_fence_after();
+        const uint32_t tmem_d = tmem_base + acc * (ACC_COLUMNS / 2);
+        for (int kb = 0; kb < kb_count; ++kb) {
+          const uint32_t tmem_a = tmem_base + A_COLUMN + a * 64, done = empty + 8 * s;
+          const uint32_t desc_low = uint32_t(desc_x) + s * (x_half >> 3);   // two halves of x_half / 16 units
+          ok = __all_sync(0xffffffffu, ready) || mbar_wait_warp(full + 8 * s, phase);
+          if (!ok) break;
+          if (++s == uint32_t(p.x_stages)) s = 0, phase ^= 1;
+          a = (a + 1) % A_STAGES;
+          ready = mbar_test(full + 8 * s, phase);   // of the next k block
+          tcgen05_fence_after();
+          if (issue) {
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk) {   // 16 k: 8 columns of A, 32 bytes of a row of B
+              const uint32_t low = desc_low + (kk >= 4 ? (x_half >> 4) : 0u) + 2 * (kk & 3);   // an address: no carry
+              umma_f16_ts<CG>(tmem_d, tmem_a + kk * 8, (uint64_t(desc_high) << 32) | low, idesc, (kb | kk) != 0);
+            }
+            if (CG == 2) umma_commit_pair(done);
+            else umma_commit(done);
+          }
+          __syncwarp();
+        }
+        if (ok && issue) {
+          if (CG == 2) umma_commit_pair(tmem_full + 8 * acc);
+          else umma_commit(tmem_full + 8 * acc);
+        }
+        __syncwarp();
+      }
+      if (!ok && lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
+    }
+  } else if (warp >= FIRST_DEQUANT) {
+    // ------------------------------ dequantisers --------------------------------
+    const int set = (warp - FIRST_DEQUANT) >> 2, quadrant = warp & 3;
+    const uint32_t magic = Elem<T>::kMagic2 ^ (p.twos_complement ? 0x00080008u : 0u);
+    // where this thread's column lies in a stage.  up|gate: a quadrant of lanes is 16 gate columns and the 16 up
+    // columns that go with them, so that the gate is applied inside a warp
+    uint32_t w_offset, w_pitch, s_offset, s_pitch;
+    const uint32_t scale_rows = uint32_t(BK) >> p.group_shift;
+    if (MODE == MODE_UPGATE_SILU) {
+      const uint32_t column = quadrant * 16 + (lane & 15), up = uint32_t(lane) >> 4;
+      w_pitch = 256, w_offset = up * (W_BYTES / 2) + column * 4;
+      s_pitch = 128, s_offset = W_BYTES + up * (scale_rows * 128) + column * 2;
+    } else {
+      const uint32_t column = quadrant * 32 + lane;
+      w_pitch = COLS * 4, w_offset = column * 4;
+      s_pitch = COLS * 2, s_offset = W_BYTES + column * 2;
+    }
+    uint32_t s_of[4];   // scale of k 32 g .. 32 g + 31
+#pragma unroll
+    for (int g = 0; g < 4; ++g) s_of[g] = s_offset + (uint32_t(g * 32) >> p.group_shift) * s_pitch;
+    const int my_items = items > first_item ? (items - first_item + item_step - 1) / item_step : 0;
+    const uint32_t total = uint32_t(my_items) * uint32_t(kb_count);
+    const uint32_t tmem_a = tmem_base + A_COLUMN + set * 64 + (uint32_t(quadrant * 32) << 16);
+    const uint32_t full_leader = CG == 2 ? map_to_rank(full, 0) : full;
+    // A set always writes the same stage of tensor memory: free when the block A_STAGES before has been multiplied.
+    // x is the barrier of the set's block, x_before that of its last one, A_STAGES before.
+    uint32_t s = set, phase = 0, x = set, phase_x = 0, x_before = 0, phase_before = 0;
+    bool ok = true;
+    for (uint32_t i = set; i < total; i += SETS) {
+      ok = mbar_wait_warp(full_w + 8 * s, phase);
+      if (!ok) break;
+      const uint32_t stage = smem_w + s * W_STAGE;
+      uint32_t words[W_ROWS], scale[4];
+#pragma unroll
+      for (int r = 0; r < W_ROWS; ++r) words[r] = lds32(stage + w_offset + r * w_pitch);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const uint32_t v = lds16(stage + s_of[g]);
+        scale[g] = v | (v << 16);
+      }
+      // the words are in registers before the stage is handed back: the arrival waits for the loads it depends on
+      asm volatile("" ::"r"(words[0]), "r"(words[W_ROWS - 1]), "r"(scale[3]) : "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty_w + 8 * s);
+      s += SETS;
+      if (s >= uint32_t(p.w_stages)) s -= p.w_stages, phase ^= 1;
+      if (i >= A_STAGES) {
+        ok = mbar_wait_warp(empty + 8 * x_before, phase_before);
+        if (!ok) break;
+      }
+      tcgen05_fence_after();
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t o[32];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t w = words[half * 8 + j], w4 = w >> 4, scale2 = scale[half * 2 + (j >> 2)];
+          o[4 * j + 0] = lop3_and_xor_u32(prmt(w, w4, 0x0400), 0x000F000Fu, magic);  // (k0, k1)
+          o[4 * j + 1] = lop3_and_xor_u32(prmt(w, w4, 0x0501), 0x000F000Fu, magic);  // (k2, k3)
+          o[4 * j + 2] = lop3_and_xor_u32(prmt(w, w4, 0x0602), 0x000F000Fu, magic);  // (k4, k5)
+          o[4 * j + 3] = lop3_and_xor_u32(prmt(w, w4, 0x0703), 0x000F000Fu, magic);  // (k6, k7)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            o[4 * j + c] = Elem<T>::mul2(Elem<T>::sub2(o[4 * j + c], Elem<T>::kBias2), scale2);
+        }
+        tmem_store_32x32(tmem_a + half * 32, o);
+      }
+      tmem_store_wait();
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_remote(full_leader + 8 * x);
+        else mbar_arrive(full_leader + 8 * x);
+      }
+      x_before = x, phase_before = phase_x;
+      x += SETS;
+      if (x >= uint32_t(p.x_stages)) x -= p.x_stages, phase_x ^= 1;
+    }
+    if (!ok && lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
+  } else if (warp >= FIRST_EPILOGUE) {
+    // ------------------------------ epilogue -----------------------------------
+    const int quadrant = warp & 3;
+    uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
+    float* yf = reinterpret_cast<float*>(p.y);
+    uint32_t local = 0;
+    for (int item = first_item; item < items; item += item_step, ++local) {
+      const Item t = item_of(item);
+      const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = p.acc_sets == 2 ? local >> 1 : local;
+      if (!mbar_wait_warp(tmem_full + 8 * acc, use & 1)) {
+        if (lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
+        break;
+      }
+      if (p.split > 1) break;   // the partial sums of the cluster are put together below
+      tcgen05_fence_after();
+      const uint32_t taddr = tmem_base + acc * (ACC_COLUMNS / 2) + (uint32_t(quadrant * 32) << 16);
+#pragma unroll 1
+      for (int c = 0; c < t.rows; c += 32) {
+        uint32_t v[32];
+        tmem_load_32x32(taddr + c, v);
+        if (MODE == MODE_UPGATE_SILU) {
+          tmem_load_wait();
+          // lanes 0..15 hold gate columns, lanes 16..31 the matching up columns: they swap half of the rows
+          const bool is_up = lane >= 16;
+          const int col = (t.n_tile * CG + (CG == 2 ? rank : 0)) * 64 + quadrant * 16 + (lane & 15);
+#pragma unroll 8
+          for (int i = 0; i < 16; ++i) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, is_up ? v[i] : v[16 + i], 16);
+            const float gv = __uint_as_float(is_up ? got : v[i]), uv = __uint_as_float(is_up ? v[16 + i] : got);
+            const int r = c + i + (is_up ? 16 : 0);
+            const float h = gv * (1.0f / (1.0f + __expf(-gv))) * uv;  // silu(gate) * up in f32, one rounding
+            if (r < t.rows) y[size_t(t.row0 + r) * p.out_cols + col] = Elem<T>::from_float(h);
+          }
+        } else {
+          const int col = (t.n_tile * CG + (CG == 2 ? rank : 0)) * COLS + quadrant * 32 + lane;
+          if (MODE == MODE_DOWN_SCATTER) {
+            // lane r of the chunk: where row r goes and with what weight
+            int token = -1;
+            float weight = 0.f;
+            if (c + lane < t.rows) {
+              const int route = __ldg(p.row_route + t.row0 + c + lane);
+              if (route >= 0 && route < p.routes) {
+                weight = __ldg(p.route_weight + route);
+                token = route / p.top_k;
+              }
+            }
+            tmem_load_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const int row_token = __shfl_sync(0xffffffffu, token, i);
+              const float w = __shfl_sync(0xffffffffu, weight, i);
+              if (row_token >= 0 && col < p.out_cols)
+                asm volatile("red.global.add.f32 [%0], %1;" ::"l"(yf + size_t(row_token) * p.out_cols + col),
+                             "f"(__fmul_rn(w, __uint_as_float(v[i])))
+                             : "memory");
+            }
+          } else {
+            tmem_load_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const int r = c + i;
+              if (r < t.rows && col < p.out_cols) {
+                if (MODE == MODE_GROUPED_F32) yf[size_t(t.row0 + r) * p.out_cols + col] = __uint_as_float(v[i]);
+                else y[size_t(t.row0 + r) * p.out_cols + col] = Elem<T>::from_float(__uint_as_float(v[i]));
+              }
+            }
+          }
+        }
+      }
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_remote(map_to_rank(tmem_empty + 8 * acc, 0));
+        else mbar_arrive(tmem_empty + 8 * acc);
+      }
+    }
+  }
+
+  __syncwarp();
+  tcgen05_fence_before();
+  __syncthreads();
+  if (MODE == MODE_DENSE && CG == 1 && p.split > 1 && first_item < items) {
+    // Every CTA of the cluster holds a partial sum of the whole tile.  The rows are dealt out in `split` slices: a
+    // CTA writes the others' slices into their shared memory (the operand stages are idle once all MMAs are done),
+    // then adds the partials of its own slice in rank order.
+    tcgen05_fence_after();
+    cluster_sync();
+    const Item t = item_of(first_item);
+    // slices of whole fours of rows; a column's rows lie together, four more than there are keep the lanes of a
+    // 16-byte access on different banks
+    const int slice = ((t.n + p.split - 1) / p.split + 3) & ~3, pitch = slice + 4;
+    const uint32_t taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
+    const uint32_t own_column = base + uint32_t((rank * COLS + (warp & 3) * 32 + lane) * pitch) * 4u;
+    for (int c = (warp >> 2) * 16; c < t.n; c += (THREADS / 128) * 16) {
+      uint32_t v[16];
+      tmem_load_32x16(taddr + c, v);
+      tmem_load_wait();
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        const int owner = (c + i) / slice, r = (c + i) - owner * slice;
+        asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(map_to_rank(own_column + r * 4, owner)),
+                     "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3])
+                     : "memory");
+      }
+    }
+    cluster_sync();
+    const float* parts = reinterpret_cast<const float*>(base_ptr);
+    uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
+    for (int i = tid; i < slice / 4 * COLS; i += THREADS) {
+      const int c = i % COLS, r = i / COLS * 4;
+      const int row = rank * slice + r, col = t.n_tile * COLS + c;
+      float4 sum = *reinterpret_cast<const float4*>(parts + size_t(c) * pitch + r);
+      for (int other = 1; other < p.split; ++other) {
+        const float4 v = *reinterpret_cast<const float4*>(parts + size_t(other * COLS + c) * pitch + r);
+        sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+      }
+      if (col >= p.out_cols) continue;
+      uint16_t* to = y + size_t(t.row0 + row) * p.out_cols + col;
+      if (row < t.rows) to[0] = Elem<T>::from_float(sum.x);
+      if (row + 1 < t.rows) to[p.out_cols] = Elem<T>::from_float(sum.y);
+      if (row + 2 < t.rows) to[2 * size_t(p.out_cols)] = Elem<T>::from_float(sum.z);
+      if (row + 3 < t.rows) to[3 * size_t(p.out_cols)] = Elem<T>::from_float(sum.w);
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+  }
+  if (CG == 2) cluster_sync();   // the peer's shared memory and TMEM stay alive until both CTAs are done
+  if (warp == 1) {
+    tcgen05_fence_after();
+    if (CG == 2) tmem_dealloc_pair(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
+  }
+}
+
+int device_sms() {
+  static int sms = [] {
+    int device = 0, value = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&value, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
+    return value;
+  }();
+  return sms;
+}
+
+template <typename T, int MODE, int CG>
+int launch(const TmemCall& q, cudaStream_t stream) {
+  const int sms = device_sms();
+  if (sms <= 0) return INTENT_B200_ERR_UNSUPPORTED;
+  TmemParams p{};
+  p.y = q.out;
+  p.M = int(q.rows);
+  p.K = int(q.K);
+  p.WN = int(q.WN);
+  p.out_cols = int(q.out_cols);
+  p.k_blocks = int((q.K + BK - 1) / BK);
+  p.row_tile = MODE == MODE_DENSE ? q.row_tile : 128;
+  p.m_tiles = int((q.rows + p.row_tile - 1) / p.row_tile);
+  p.n_tiles = MODE == MODE_UPGATE_SILU ? int(q.out_cols / (64 * CG)) : int((q.out_cols + COLS * CG - 1) / (COLS * CG));
+  p.box_rows = MODE == MODE_DENSE ? p.row_tile / CG : 16;
+  p.acc_sets = p.row_tile <= 128 ? 2 : 1;
+  p.split = q.split;
+  p.group_shift = q.group_size == 32 ? 5 : q.group_size == 64 ? 6 : 7;
+  p.twos_complement = q.zero_point == -1 ? 1 : 0;
+  p.total_rows = q.total_rows;
+  p.tile_expert = q.tile_expert;
+  p.block_rows = q.block_rows;
+  p.experts = int(q.experts);
+  p.row_route = q.row_route;
+  p.route_weight = q.route_weight;
+  p.routes = int(q.routes);
+  p.top_k = q.top_k;
+  if (p.row_tile % (16 * CG) != 0 || p.row_tile < 16 * CG || p.row_tile > 128 * CG) return INTENT_B200_ERR_UNSUPPORTED;
+  if (p.split < 1 || p.split > 8 || (p.split > 1 && (MODE != MODE_DENSE || CG != 1 || p.k_blocks < p.split)))
+    return INTENT_B200_ERR_UNSUPPORTED;
+  if (MODE != MODE_DENSE && (p.m_tiles > LIST_BLOCKS || q.block_rows % 128 != 0)) return INTENT_B200_ERR_UNSUPPORTED;
+
+  // Up to eight stages of activations: a stage comes back after its MMAs and a load from the L2, some 2000 cycles, of
+  // which four k blocks cover no more than that.  The rest is a ring for the packed words, which come from HBM.
+  const int list_bytes = MODE == MODE_DENSE ? 0 : p.m_tiles * 8;
+  const int fixed = 1024 + 512 + list_bytes, x_stage = p.row_tile / CG * 256;
+  p.x_stages = 8;
+  while (p.x_stages > A_STAGES && fixed + p.x_stages * x_stage + 9 * W_STAGE > SMEM_LIMIT) --p.x_stages;
+  p.w_stages = (SMEM_LIMIT - fixed - p.x_stages * x_stage) / W_STAGE;
+  if (p.w_stages > 16) p.w_stages = 16;
+  if (p.w_stages < SETS) return INTENT_B200_ERR_UNSUPPORTED;
+  const int smem = fixed + p.x_stages * x_stage + p.w_stages * W_STAGE;
+  if (p.split > 1) {   // the partial sums of a cluster meet where the operands were
+    const int slice = ((p.row_tile + p.split - 1) / p.split + 3) & ~3;
+    if (p.split * COLS * (slice + 4) * 4 > smem - 1536) return INTENT_B200_ERR_UNSUPPORTED;
+  }
+
+  const CUtensorMapDataType type =
+      std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const uint32_t box_cols = MODE == MODE_UPGATE_SILU ? 64 : COLS;
+  const uint64_t E = uint64_t(q.experts), K = uint64_t(q.K), WN = uint64_t(q.WN);
+  CUtensorMap map_x, map_w, map_s;
+  if (!make_tensor_map_2d(&map_x, type, q.x, uint64_t(q.rows), K, K * 2, uint32_t(p.box_rows), 64,
+                          CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !make_tensor_map_3d(&map_w, CU_TENSOR_MAP_DATA_TYPE_INT32, q.w, E, K / 8, WN, WN * 4, K / 8 * WN * 4, W_ROWS,
+                          box_cols, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+      !make_tensor_map_3d(&map_s, type, q.s, E, K / uint64_t(q.group_size), WN, WN * 2,
+                          K / uint64_t(q.group_size) * WN * 2, uint32_t(BK / q.group_size), box_cols,
+                          CU_TENSOR_MAP_SWIZZLE_NONE))
+    return INTENT_B200_ERR_UNSUPPORTED;
+
+  auto kernel = w4a16_tmem_kernel<T, MODE, CG>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return cuda_status(e);
+  const int64_t items = int64_t(p.m_tiles) * p.n_tiles;
+  const int64_t fastest = MODE == MODE_DENSE ? p.m_tiles : p.n_tiles;
+  if (items * fastest >= (int64_t(1) << 32) || (p.split > 1 && items > 65535)) return INTENT_B200_ERR_UNSUPPORTED;
+  p.tile_magic = fastest == 1 ? 0u : uint32_t(((uint64_t(1) << 32) + fastest - 1) / fastest);
+  p.kb_each = p.k_blocks / p.split;
+  p.kb_extra = p.k_blocks % p.split;
+  const int cluster = p.split > 1 ? p.split : CG;
+  const int grid = int(p.split > 1 ? items * p.split : CG * (items < sms / CG ? items : sms / CG));
+  if (LaunchFacts* sink = observe_sink())
+    return record_launch(sink, reinterpret_cast<const void*>(kernel),
+                         CG == 2       ? "w4a16_tmem_kernel CTA pairs, 256 columns"
+                         : p.split > 1 ? "w4a16_tmem_kernel k split over a cluster, 128 columns"
+                                       : "w4a16_tmem_kernel single CTA, 128 columns",
+                         grid, THREADS, smem, cluster);
+  cudaLaunchConfig_t config = {};
+  config.gridDim = p.split > 1 ? dim3(unsigned(p.split), unsigned(items), 1) : dim3(unsigned(grid), 1, 1);
+  config.blockDim = dim3(THREADS, 1, 1);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = unsigned(cluster);
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = cluster > 1 ? 1 : 0;
+  e = cudaLaunchKernelEx(&config, kernel, map_x, map_w, map_s, p);
+  if (e != cudaSuccess) return cuda_status(e);
+  note_launch();
+  return launch_status();
+}
+
+}  // namespace
+
+template <typename T>
+int w4a16_tmem(const TmemCall& q, int mode, bool pairs, cudaStream_t stream) {
+  switch (mode) {
+    case MODE_DENSE: return pairs ? launch<T, MODE_DENSE, 2>(q, stream) : launch<T, MODE_DENSE, 1>(q, stream);
+    case MODE_UPGATE_SILU:
+      return pairs ? launch<T, MODE_UPGATE_SILU, 2>(q, stream) : launch<T, MODE_UPGATE_SILU, 1>(q, stream);
+    case MODE_GROUPED_F32:
+      return pairs ? launch<T, MODE_GROUPED_F32, 2>(q, stream) : launch<T, MODE_GROUPED_F32, 1>(q, stream);
+    case MODE_DOWN_SCATTER:
+      return pairs ? launch<T, MODE_DOWN_SCATTER, 2>(q, stream) : launch<T, MODE_DOWN_SCATTER, 1>(q, stream);
+  }
+  return INTENT_B200_ERR_UNSUPPORTED;
+}
+template int w4a16_tmem<__half>(const TmemCall&, int, bool, cudaStream_t);
+template int w4a16_tmem<__nv_bfloat16>(const TmemCall&, int, bool, cudaStream_t);
+
+// Reads and clears this file's status word (the device is idle when it is called).
+int w4a16_tmem_take_status(int* value) {
+  int zero = 0;
+  cudaError_t e = cudaMemcpyFromSymbol(value, g_w4a16_tmem_status, sizeof(int));
+  if (e != cudaSuccess) return cuda_status(e);
+  if (*value != 0) cudaMemcpyToSymbol(g_w4a16_tmem_status, &zero, sizeof(int));
+  return INTENT_B200_OK;
+}
+
+}  // namespace ib200

@@ -172,6 +172,17 @@ class MoEW4A16FFN:
         # bits as the ordered combine.  More choices keep the ordered combine kernel.
         self.fused_combine = top_k <= 2
         self.down_scatter = _compile(programs.moe_grouped_down_scatter, target=target, constexprs=grouped)
+        # The fused chain reads no padding row, so on the reference layout it neither writes nor multiplies them.
+        self._chain = (self.gather, self.up_gate)
+        if self.fused_combine and not prelayout:
+            self._chain = (_compile(programs.moe_gather_rows, target=target,
+                                    constexprs={"ACT_DTYPE": act_dtype, "TOP_K": top_k, "PADDING": False}),
+                           _compile(programs.moe_grouped_upgate_silu, target=target,
+                                    constexprs=dict(grouped, ROUTED=True)))
+
+    def _up_gate_inputs(self, rows, blocks, total, packed, scales, sorted_routes, topk_weights):
+        inputs = (rows, blocks, total, packed, scales)
+        return inputs if self._chain[1] is self.up_gate else inputs + (sorted_routes, topk_weights)
 
     def route(self, logits):
         """logits [T, E_total] f32 -> (ids [T,2] i32, weights [T,2] f32)."""
@@ -211,8 +222,10 @@ class MoEW4A16FFN:
         if self.fused_combine:
             up_gate_packed, down_packed = self._weights(up_gate_packed, down_packed)
             sorted_routes, expert_blocks, total = self.alignment.run(topk_ids)
-            rows = self.gather.run(x, sorted_routes, total)
-            hidden = self.up_gate.run(rows, expert_blocks, total, up_gate_packed, up_gate_scales)
+            gather, up_gate = self._chain
+            rows = gather.run(x, sorted_routes, total)
+            hidden = up_gate.run(*self._up_gate_inputs(rows, expert_blocks, total, up_gate_packed, up_gate_scales,
+                                                       sorted_routes, topk_weights))
             self.down_scatter(hidden, expert_blocks, total, down_packed, down_scales, sorted_routes, topk_weights, y)
             return y
         rows, positions = self.experts_forward(x, topk_ids, up_gate_packed, up_gate_scales, down_packed,
@@ -233,8 +246,10 @@ class MoEW4A16FFN:
         align = self.alignment.prepare(topk_ids)
         sorted_routes, expert_blocks, total = align.result()
         if self.fused_combine and not clear_positions:
-            gather_call = self.gather.prepare(x, sorted_routes, total)
-            up_call = self.up_gate.prepare(gather_call.result(), expert_blocks, total, up_gate_packed, up_gate_scales)
+            gather, up_gate = self._chain
+            gather_call = gather.prepare(x, sorted_routes, total)
+            up_call = up_gate.prepare(*self._up_gate_inputs(gather_call.result(), expert_blocks, total, up_gate_packed,
+                                                            up_gate_scales, sorted_routes, topk_weights))
             scatter_call = self.down_scatter.prepare(up_call.result(), expert_blocks, total, down_packed, down_scales,
                                                      sorted_routes, topk_weights, y)
             return PreparedFusedFFN(align, gather_call, up_call, scatter_call, y)

@@ -372,13 +372,14 @@ def _lower_gather(c, device):
         ViewParameter(2, "total_padded", dtypes.i32, (1,), IN, alignment=4),
         ViewParameter(3, "rows", act, ("P", "H"), OUT),
     ))
-    return NativeProgram(interface=interface, entry_name="intent_b200_moe_gather_rows",
-                         constants=(int(c["TOP_K"]),), device=device)
+    entry = "intent_b200_moe_gather_rows" if c["PADDING"] else "intent_b200_moe_gather_routed_rows"
+    return NativeProgram(interface=interface, entry_name=entry, constants=(int(c["TOP_K"]),), device=device)
 
 
-moe_gather_rows = KernelDefinition("moe_gather_rows", {"ACT_DTYPE": "bf16", "TOP_K": 2}, _lower_gather,
+moe_gather_rows = KernelDefinition("moe_gather_rows", {"ACT_DTYPE": "bf16", "TOP_K": 2, "PADDING": True}, _lower_gather,
                                    "examples/kernels/ragged/moe.py:34-36 (I.gather of token rows)",
-                                   "rows[p] = x[sorted[p] // TOP_K], zero rows for padding")
+                                   "rows[p] = x[sorted[p] // TOP_K], zero rows for padding (PADDING=False: those are "
+                                   "left alone)")
 
 
 def _grouped_constants(c):
@@ -400,19 +401,24 @@ def _lower_grouped(c, device, *, gated):
         raise CompilationStageError("provider_native_compilation", "BLOCK_ROWS must be 128 or 256")
     out_cols = Derived("I", lambda d: d["WN"] // 2) if gated else "WN"
     weight, weight_rule, suffix = _grouped_weight(c, group)
-    interface = PublicInterface((
-        ViewParameter(0, "rows", act, ("P", "K"), IN),
-        ViewParameter(1, "expert_blocks", dtypes.i32, ("B",), IN, alignment=4),
-        ViewParameter(2, "total_padded", dtypes.i32, (1,), IN, alignment=4),
-        weight,
-        ViewParameter(4, "scales", act, ("E", "KG", "WN"), IN),
-        ViewParameter(5, "output", act if gated else dtypes.f32, ("P", out_cols), OUT),
-    ), dimension_rules=(
-        weight_rule,
-        _rule(lambda d: d["B"] * block >= d["P"], f"expert_blocks must cover every {block}-row block of rows"),
-    ))
+    views = [ViewParameter(0, "rows", act, ("P", "K"), IN),
+             ViewParameter(1, "expert_blocks", dtypes.i32, ("B",), IN, alignment=4),
+             ViewParameter(2, "total_padded", dtypes.i32, (1,), IN, alignment=4),
+             weight,
+             ViewParameter(4, "scales", act, ("E", "KG", "WN"), IN)]
+    rules = [weight_rule,
+             _rule(lambda d: d["B"] * block >= d["P"], f"expert_blocks must cover every {block}-row block of rows")]
     stem = "upgate_silu" if gated else "down_f32"
-    return NativeProgram(interface=interface, entry_name=f"intent_b200_moe_grouped_w4a16_{stem}{suffix}_{act.name}",
+    if gated and c["ROUTED"]:
+        if suffix:
+            raise CompilationStageError("provider_native_compilation", "ROUTED needs WEIGHT_LAYOUT 'reference'")
+        stem += "_routed"
+        views += [ViewParameter(5, "sorted_route_ids", dtypes.i32, ("S",), IN, alignment=4),
+                  ViewParameter(6, "route_weights", dtypes.f32, ("T", "TOP_K"), IN, alignment=4)]
+        rules.append(_rule(lambda d: d["S"] >= d["P"], "sorted_route_ids must cover every row"))
+    views.append(ViewParameter(len(views), "output", act if gated else dtypes.f32, ("P", out_cols), OUT))
+    return NativeProgram(interface=PublicInterface(tuple(views), dimension_rules=tuple(rules)),
+                         entry_name=f"intent_b200_moe_grouped_w4a16_{stem}{suffix}_{act.name}",
                          constants=(group, zp, block), device=device)
 
 
@@ -437,10 +443,11 @@ def _grouped_weight(c, group):
 _GROUPED_CONSTEXPRS = {"GROUP_SIZE": 128, "ZERO_POINT": 8, "ACT_DTYPE": "bf16", "BLOCK_ROWS": 128,
                        "WEIGHT_LAYOUT": "reference"}
 moe_grouped_upgate_silu = KernelDefinition(
-    "moe_grouped_upgate_silu", dict(_GROUPED_CONSTEXPRS), lambda c, d: _lower_grouped(c, d, gated=True),
+    "moe_grouped_upgate_silu", dict(_GROUPED_CONSTEXPRS, ROUTED=False), lambda c, d: _lower_grouped(c, d, gated=True),
     "examples/kernels/ragged/grouped_gemm.py:42-70, examples/kernels/ragged/moe.py:37-42, "
     "examples/kernels/activation/swiglu.py:27-46",
-    "hidden = silu(rows @ Wgate[e]) * (rows @ Wup[e]) per expert block, int4 weights")
+    "hidden = silu(rows @ Wgate[e]) * (rows @ Wup[e]) per expert block, int4 weights (ROUTED: rows that no route fills "
+    "are left out)")
 moe_grouped_down = KernelDefinition(
     "moe_grouped_down", dict(_GROUPED_CONSTEXPRS), lambda c, d: _lower_grouped(c, d, gated=False),
     "examples/kernels/ragged/grouped_gemm.py:42-70, examples/kernels/ragged/moe.py:43-47",
