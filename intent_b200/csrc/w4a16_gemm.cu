@@ -74,6 +74,7 @@ constexpr int DQ_ROWS = BK / 8;       // packed words per thread and k block
 constexpr int THREADS = (6 + DEQUANT_WARPS) * 32;
 constexpr int BAND_TILES = 8;         // row tiles per band of the tile walk
 
+constexpr int TMEM_MAX_ROWS = 2048;   // dense calls of fewer rows may run with the weights in tensor memory
 constexpr int PAIR_LIST_BLOCKS = 8192;  // most 128-row blocks the in-kernel block pairing handles
 
 template <int MT, int BN>
@@ -632,7 +633,7 @@ int launch_gemm(const void* x, int64_t rows, int64_t K, const void* w, const voi
 // 88.2).  All forms add the k blocks in the same order, so the bits of a row do not depend on the form.
 enum class Form { PAIR, TWO_BLOCKS, N256, N128, N64, N32 };
 
-Form choose_form(int64_t M, int64_t N, bool pairs) {
+Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
   const int64_t sms = device_sms() > 0 ? device_sms() : 1;
   struct Candidate {
     Form form;
@@ -654,7 +655,64 @@ Form choose_form(int64_t M, int64_t N, bool pairs) {
       least = cost;
     }
   }
+  // the whole call: what it takes besides its k blocks is 4 us, with pairs 9 (epilogues of 512 rows)
+  *time = (best == Form::PAIR ? 9.0 : 4.0) + least * double((K + BK - 1) / BK);
   return best;
+}
+
+// Whether a dense call runs with the weights in tensor memory (w4a16_tmem.cu), and on which tile: the least of the
+// times below, if that is less than what the forms above take.  Microseconds, bf16, group 128, replayed as a graph over
+// weights that do not stay in the L2; `blocks` are k blocks of 128 per CTA:
+//   lone CTA of r <= 128 rows x 128 columns   4.2 + 0.014 r + waves * blocks * (0.24 + 0.0014 r)
+//   the k blocks over a cluster of 2 or 4     + 2.0 or 2.5, one wave
+//   CTA pair of r rows x 256 columns          5 + 0.012 r + waves * blocks * (0.405 at 128 rows, 0.52 at 192, 0.735 at 256)
+// Measured against the forms above: M17 K4096 N4096 27.2 -> 9.2 us, M77 K14336 N4096 81.1 -> 18.0, M256 K8192 N1024
+// 48.8 -> 13.1, M256 K4096 N14336 52.9 -> 30.4, M512 K2048 N4096 19.8 -> 13.5, M1024 K4096 N4096 50.9 -> 30.3.
+// Calls of K < 2048 stay above: they take 8 to 16 us either way, most of it not in the k blocks.  So do unsplit calls
+// with less than a tile for every second SM.  A split changes the order of a row's sum, so that its bits depend on the
+// number of rows of the call; it is taken from K > 2048 on, where it gives a third or more.
+bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, double other, TmemCall* call, bool* pairs) {
+  const int64_t sms = device_sms(), blocks = (K + 127) / 128;
+  if (sms <= 0 || K < 2048 || M >= TMEM_MAX_ROWS) return false;
+  double best = other;
+  const auto consider = [&](bool pair, int64_t row_tiles, int split) {
+    const int64_t unit = pair ? 32 : 16, most = pair ? 256 : 128;
+    const int64_t rows = ((M + row_tiles - 1) / row_tiles + unit - 1) / unit * unit;
+    if (rows > most) return;
+    const int64_t tiles = (M + rows - 1) / rows * ((N + (pair ? 255 : 127)) / (pair ? 256 : 128));
+    const int64_t ctas = tiles * (pair ? 2 : split);
+    double cost;
+    if (split > 1) {
+      // clusters of four do not fill every part of the chip: 33 of them were seen side by side
+      if (K <= 2048 || blocks < 4 * split || ctas > (split == 2 ? sms : sms * 9 / 10)) return;
+      cost = (split == 2 ? 6.2 : 6.7) + 0.014 * double(rows) +
+             double((blocks + split - 1) / split) * (0.24 + 0.0014 * double(rows));
+    } else {
+      if (2 * ctas < sms) return;
+      const int64_t at_once = pair ? sms / 2 : sms, waves = (tiles + at_once - 1) / at_once;
+      const double r = double(rows);
+      const double block = !pair       ? 0.24 + 0.0014 * r
+                           : r <= 128  ? 0.285 + 0.00094 * r
+                           : r <= 192  ? 0.405 + 0.0018 * (r - 128)
+                                       : 0.52 + 0.00336 * (r - 192);
+      cost = (pair ? 5.0 + 0.012 * r : 4.2 + 0.014 * r) + double(waves * blocks) * block;
+    }
+    if (cost < best) {
+      best = cost;
+      call->row_tile = int(rows);
+      call->split = split;
+      *pairs = pair;
+    }
+  };
+  const int64_t most_tiles = (M + 31) / 32;
+  for (int64_t t = (M + 255) / 256; t <= (M + 63) / 64 && t <= most_tiles; ++t) {
+    if (pairs_allowed) consider(true, t, 1);
+    for (const int split : {1, 2, 4}) consider(false, t, split);
+  }
+  if (M < 64) {
+    for (const int split : {1, 2, 4}) consider(false, 1, split);
+  }
+  return best < other;
 }
 
 template <typename T>
@@ -670,7 +728,21 @@ int run(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, cuda
   if (!contiguous(x) || !contiguous(w) || !contiguous(s) || !contiguous(y)) return INTENT_B200_ERR_LAYOUT;
   if (!aligned16(x.p) || !aligned16(w.p) || !aligned16(s.p) || !aligned16(y.p)) return INTENT_B200_ERR_LAYOUT;
   if (K == 0 || N % 8 != 0 || M > (1 << 24) || K > (1 << 24) || N > (1 << 24)) return INTENT_B200_ERR_UNSUPPORTED;
-  const Form form = choose_form(M, N, selection().gemm_pairs != 0);
+  double time = 0.0;
+  const Form form = choose_form(M, K, N, selection().gemm_pairs != 0, &time);
+  if (!prelaid) {
+    TmemCall q{};
+    bool pairs = false;
+    if (choose_tmem(M, K, N, selection().gemm_pairs != 0, time, &q, &pairs)) {
+      q.x = x.p, q.rows = M, q.K = K;
+      q.w = w.p, q.s = s.p, q.experts = 1, q.WN = N;
+      q.out = y.p, q.out_cols = N;
+      q.group_size = group_size, q.zero_point = zero_point;
+      q.block_rows = BM, q.top_k = 1;
+      const int status = w4a16_tmem<T>(q, MODE_DENSE, pairs, stream);
+      if (status != INTENT_B200_ERR_UNSUPPORTED) return status;
+    }
+  }
   if (form == Form::PAIR) {  // CTA pairs, each CTA dequantises half of every weight tile
     const int status = w4a16_gemm_pair<T>(x.p, M, K, w.p, s.p, N, y.p, group_size, zero_point, stream, prelaid);
     if (status != INTENT_B200_ERR_UNSUPPORTED) return status;

@@ -1,0 +1,74 @@
+"""The W4A16 kernel with the weights in tensor memory: edges of its tiles in rows, columns and k.  Tiled weight copies
+run on the other kernels, which add the k blocks in the same order, so unsplit calls must agree with them bit for bit;
+the tolerances against the oracle are those of test_w4a16_gemm_gpu.py."""
+import pytest
+import torch
+
+import intent_b200 as ib
+import oracle
+from intent_b200 import prelayout
+from intent_b200.moe import MoEW4A16FFN
+from conftest import max_abs_rel
+
+pytestmark = pytest.mark.gpu
+
+LONE, PAIRS, SPLIT = ("w4a16_tmem_kernel " + s for s in ("single CTA", "CTA pairs", "k split over a cluster"))
+
+
+@pytest.mark.parametrize("dtype,zero_point,group,M,K,N,kernel", [
+    (torch.float16, 8, 128, 17, 4096, 4096, SPLIT),                    # one tile of 32 rows, four CTAs a tile
+    (torch.bfloat16, "twos_complement", 32, 77, 4128, 2056, SPLIT),    # a quarter of a k block at the end, 33 blocks
+    (torch.bfloat16, 8, 64, 130, 2112, 9224, LONE),                    # half a k block, a ragged second row tile
+    (torch.float16, "twos_complement", 64, 512, 2048, 4096, LONE),
+    (torch.bfloat16, 8, 128, 511, 8192, 8200, PAIRS),                  # 256-row tiles, one accumulator
+    (torch.float16, 8, 128, 1030, 4096, 4104, PAIRS),                  # 128-row tiles, eight columns in the last tile
+])
+def test_dense_tiles(cuda_device, dtype, zero_point, group, M, K, N, kernel):
+    x, p, s = ib.workloads.w4a16_inputs(M, K, N, dtype=dtype, group_size=group, seed=M)
+    constants = {"GROUP_SIZE": group, "ZERO_POINT": zero_point, "ACT_DTYPE": "f16" if dtype == torch.float16 else "bf16"}
+    artifact = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0), constexprs=constants)
+    tiled = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),
+                       constexprs=dict(constants, WEIGHT_LAYOUT="tiled", KERNEL="gemm"))
+    xd, pd, sd = x.to(cuda_device), p.to(cuda_device), s.to(cuda_device)
+    out = artifact.run(xd, pd, sd)
+    assert artifact.observation.kernel.startswith(kernel), artifact.observation.kernel
+    assert torch.equal(artifact.run(xd, pd, sd), out)
+    other = tiled.run(xd, prelayout.tile(pd).tensor, sd)
+    torch.cuda.synchronize()
+    artifact.check()
+    if kernel is not SPLIT:
+        assert torch.equal(out, other)
+    rows = torch.randperm(M, generator=torch.Generator().manual_seed(1))[:128].sort().values
+    rows = torch.cat([torch.tensor([0]), rows, torch.tensor([M - 1])])
+    rounded = oracle.weight_only_int4_matmul_rounded(x[rows], p, s, group_size=group,
+                                                     zero_point=8 if zero_point == 8 else None)
+    assert max_abs_rel(out[rows.to(cuda_device)].cpu(), rounded) <= (2e-3 if dtype == torch.float16 else 1.6e-2)
+
+
+@pytest.mark.parametrize("rows_of_expert,hidden,intermediate,block", [
+    ((1, 16, 17, 0, 32, 33, 15, 2), 512, 128, 128),            # few rows: lone CTAs
+    ((127, 128, 129, 0, 256, 1, 300, 31), 1024, 384, 128),     # blocks full and nearly empty: CTA pairs
+    ((127, 128, 129, 0, 256, 1, 300, 31), 256, 128, 256),      # blocks of 256 rows, the second half empty
+])
+def test_routed_rows(cuda_device, rows_of_expert, hidden, intermediate, block):
+    experts = len(rows_of_expert)
+    flat = torch.repeat_interleave(torch.arange(experts), torch.tensor(rows_of_expert))
+    flat = flat[torch.randperm(flat.numel(), generator=torch.Generator().manual_seed(2))]
+    ids = flat[: flat.numel() // 2 * 2].reshape(-1, 2).to(torch.int32)
+    tokens = ids.shape[0]
+    data = ib.workloads.moe_inputs(tokens, hidden, experts, intermediate, dtype=torch.bfloat16, seed=3)
+    dev = {k: v.to(cuda_device) for k, v in data.items()}
+    weights = torch.rand((tokens, 2), generator=torch.Generator().manual_seed(4))
+    sizes = dict(tokens=tokens, hidden=hidden, intermediate=intermediate, experts=experts, block_size=block,
+                 target=ib.B200Target(0))
+    args = (dev["x"], ids.to(cuda_device), weights.to(cuda_device), dev["up_gate_packed"], dev["up_gate_scales"],
+            dev["down_packed"], dev["down_scales"])
+    plain, tiled = MoEW4A16FFN(**sizes), MoEW4A16FFN(prelayout=True, **sizes)
+    y = plain(*args)
+    assert plain._chain[1].observation.kernel.startswith("w4a16_tmem_kernel")
+    torch.cuda.synchronize()
+    plain.down_scatter.check()
+    assert torch.equal(y, tiled(*args))
+    ref = oracle.moe_w4a16_swiglu_ffn(data["x"], ids, weights, data["up_gate_packed"], data["up_gate_scales"],
+                                      data["down_packed"], data["down_scales"])
+    assert max_abs_rel(y.cpu(), ref) <= 2e-2
