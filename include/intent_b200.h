@@ -52,6 +52,10 @@ enum intent_b200_status {
 
 /* Library identity: returns a static string "intent_b200 <version> sm_100a". */
 INTENT_B200_API const char* intent_b200_version(void);
+/* A program entry as a function of an array of 64-bit slots, in the order of the entry's own parameters (stream last);
+ * null when `name` is no program entry.  `slots` receives their number. */
+typedef int (*intent_b200_packed_fn)(const int64_t* slots);
+INTENT_B200_API intent_b200_packed_fn intent_b200_packed_call(const char* name, int32_t* slots);
 /* Human-readable name of a status code (static string). */
 INTENT_B200_API const char* intent_b200_status_string(int status);
 /* Number of kernels this library has launched in the calling process (all

@@ -1,7 +1,7 @@
-"""In-tree build of ``libintent_b200.so`` (sm_100a only).
+"""In-tree build of ``libintent_b200.so`` (sm_100a only) and of the host extension ``intent_b200_binder.so``.
 
 ``python -m intent_b200.build`` compiles every ``csrc/*.cu`` with nvcc and links
-one shared library under ``intent_b200/lib/``.  Nothing is JIT-compiled at run
+one shared library under ``intent_b200/lib/``, and ``csrc/host/binder.cpp`` against torch.  Nothing is JIT-compiled at run
 time: the runtime loads this prebuilt library and fails loudly if it is absent.
 """
 from __future__ import annotations
@@ -17,6 +17,8 @@ ROOT = Path(__file__).resolve().parent
 CSRC = ROOT / "csrc"
 OBJ = CSRC / "build"
 LIB = ROOT / "lib" / "libintent_b200.so"
+BINDER_SOURCE = CSRC / "host" / "binder.cpp"
+BINDER = ROOT / "lib" / "intent_b200_binder.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -83,7 +85,30 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         done = subprocess.run(command, capture_output=True, text=True)
         if done.returncode != 0:
             raise RuntimeError(f"link failed:\n{done.stdout}\n{done.stderr}")
+    build_binder(force)
     return LIB
+
+
+def build_binder(force: bool = False) -> Path:
+    """The native call path (runtime/native.py: ``binder``), a CPython extension linked against torch."""
+    import sysconfig
+
+    import torch
+
+    if not force and not _stale(BINDER, [BINDER_SOURCE]):
+        return BINDER
+    root = Path(torch.__file__).resolve().parent
+    include = root / "include"
+    command = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               f"-I{include}", f"-I{include / 'torch' / 'csrc' / 'api' / 'include'}",
+               f"-I{sysconfig.get_paths()['include']}", f"-I{Path(_nvcc()).resolve().parent.parent / 'include'}",
+               str(BINDER_SOURCE), "-o", str(BINDER), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
+               "-lc10", "-lc10_cuda"]
+    done = subprocess.run(command, capture_output=True, text=True)
+    if done.returncode != 0:
+        raise RuntimeError(f"the host extension does not build:\n{done.stdout}\n{done.stderr}")
+    return BINDER
 
 
 if __name__ == "__main__":

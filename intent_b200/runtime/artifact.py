@@ -21,7 +21,8 @@ from typing import Any
 
 from ..errors import CompilationStageError
 from . import native
-from .interface import BoundArguments, PublicInterface, ScalarParameter, ViewParameter
+from ..dtypes import torch_dtype
+from .interface import BoundArguments, PublicInterface, ScalarParameter, ViewFacts, ViewParameter
 
 
 @dataclass(frozen=True, slots=True)
@@ -151,7 +152,7 @@ class PreparedCall:
             launched = self._launched = _Launched(
                 self._slots, self.invocation.views,
                 sum(w.numel() * w.element_size() for w in self._workspace), int(status), selection)
-        program._launched = launched
+        program.record(launched)
         if status:
             native.check(status, program.entry_name, launched.observation(program))
 
@@ -208,6 +209,8 @@ class NativeProgram:
         self._carriers_head = tuple(carriers)
         self._function = None
         self._workspace_count = None
+        self.binder = None                   # native caller, from the first accepted call on (native.binder)
+        self._binder_asked = False
 
     # ---- C entry -----------------------------------------------------------------
     def function(self, workspace_count: int | None = None):
@@ -221,7 +224,47 @@ class NativeProgram:
 
     @property
     def observation(self):
-        return None if self._launched is None else self._launched.observation(self)
+        launched = self.latest()
+        return None if launched is None else launched.observation(self)
+
+    # ---- native call path ----------------------------------------------------------
+    def record(self, launched: _Launched) -> None:
+        """``launched`` is the latest call."""
+        self._launched = launched
+        if self.binder is not None:
+            self.binder.forget()
+
+    def latest(self) -> _Launched | None:
+        """The record of the latest call; a native one is put together when it is asked for."""
+        seen = None if self.binder is None else self.binder.last()
+        if seen is not None:
+            slots, workspace_bytes, status, selection = seen
+            views, at = [], 0
+            for parameter in self.interface.parameters:
+                rank = len(parameter.shape)
+                views.append(ViewFacts(slots[at + 1:at + 1 + rank], slots[at + 1 + rank:at + 1 + 2 * rank],
+                                       None, None, None, None))
+                at += 1 + 2 * rank
+            self.record(_Launched(slots, tuple(views), workspace_bytes, status, selection))
+        return self._launched
+
+    def native_failure(self, status: int) -> None:
+        native.check(status, self.entry_name, self.latest().observation(self))
+
+    def _teach(self, bound: BoundArguments, selection: bytes):
+        """The native caller (or None), told that these shapes are accepted.  Everything it learns follows from the
+        shapes and the selection switches alone."""
+        if not self._binder_asked:
+            self._binder_asked = True
+            parameters = self.interface.parameters
+            if all(isinstance(p, ViewParameter) and p.layout == "contiguous" for p in parameters):
+                views = tuple((int(p.access), torch_dtype(p.dtype), len(p.shape), p.alignment) for p in parameters)
+                self.binder = native.binder(self.entry_name, self.device, views, self.constants,
+                                            None if self._workspace_spec is None else self._stream_workspaces)
+        if self.binder is not None:
+            size = -1 if self._workspace_spec is None else int(self._workspace_spec(bound.dimensions))
+            self.binder.learn(tuple(e for f in bound.views for e in f.shape), size, self.is_empty(bound), selection)
+        return self.binder
 
     @cached_property
     def _torch_device(self):
@@ -244,8 +287,9 @@ class NativeProgram:
         facts = _LaunchFacts()
         if library.intent_b200_observe_begin_selected(ctypes.byref(facts), selection, len(selection) // 4) != 0:
             return {}
+        workspaces = (len(slots) - len(self._carriers_head)) // 2      # a pointer and a size each
         try:
-            status = self.function()(*slots, self.current_stream())
+            status = self.function(workspaces)(*slots, self.current_stream())
         finally:
             library.intent_b200_observe_end()
         if status != 0 or not facts.valid:
@@ -335,13 +379,31 @@ class NativeProgram:
         return self.prepare(*arguments, outputs=outputs)
 
     def run(self, *arguments):
+        selection = native.selection()
         bound = self.interface.bind(tuple(arguments), device=self._torch_device)
-        call = PreparedCall(self, bound, self.allocate_workspace(bound, per_stream=True))
+        workspace = self.allocate_workspace(bound, per_stream=True)
+        binder = self._teach(bound, selection)
+        if binder is not None:
+            status = binder.start(bound.arguments)
+            if status is None:
+                return bound.result()
+            if status is not NotImplemented:
+                self.native_failure(status)
+        call = PreparedCall(self, bound, workspace)
         call.launch()
         return call.result()
 
     def launch(self, *arguments) -> None:
-        self.prepare(*arguments, explicit_outputs=True).launch()
+        selection = native.selection()
+        bound = self.interface.bind(tuple(arguments), device=self._torch_device, explicit_outputs=True)
+        binder = self._teach(bound, selection)
+        if binder is not None:
+            status = binder.launch(bound.arguments)
+            if status is None:
+                return
+            if status is not NotImplemented:
+                self.native_failure(status)
+        PreparedCall(self, bound).launch()
 
     def infer_outputs(self, arguments: tuple):
         """Shape inference for fake tensors: no pointers, no launch."""
@@ -418,6 +480,13 @@ class CompiledArtifact:
 
     def run(self, *arguments: Any):
         """Allocate declared Out buffers and execute with inputs in declaration order."""
+        binder = getattr(self.runtime, "binder", None)
+        if binder is not None:
+            result = binder.run(arguments)
+            if result is not NotImplemented:
+                if type(result) is int:
+                    self.runtime.native_failure(result)
+                return result
         return self._invoke(self.runtime.run, arguments)
 
     def prepare(self, *arguments: Any, outputs: tuple | None = None) -> PreparedCall:
@@ -426,6 +495,13 @@ class CompiledArtifact:
 
     def launch(self, *arguments: Any) -> None:
         """Execute with every runtime argument, including explicit Out buffers."""
+        binder = getattr(self.runtime, "binder", None)
+        if binder is not None:
+            result = binder.launch(arguments)
+            if result is not NotImplemented:
+                if result is not None:
+                    self.runtime.native_failure(result)
+                return
         self._invoke(self.runtime.launch, arguments)
 
     __call__ = launch

@@ -18,6 +18,8 @@ _LOCK = Lock()
 _LIBRARY: ctypes.CDLL | None = None
 _ENTRIES: dict = {}
 _SELECTION: ctypes.Array | None = None        # the switches, in the library's own memory
+_BINDER = None                                # the Binder type of the host extension; False: not built
+_PACKED: dict = {}                            # entry name -> (address, slots) of its packed form; None: it has none
 
 _CARRIERS = {"ptr": ctypes.c_void_p, "bool": ctypes.c_bool, "i8": ctypes.c_int8, "i16": ctypes.c_int16,
              "i32": ctypes.c_int32, "i64": ctypes.c_int64, "f32": ctypes.c_float, "f64": ctypes.c_double}
@@ -81,6 +83,47 @@ def selection() -> bytes:
         address = where(ctypes.byref(count))
         _SELECTION = (ctypes.c_char * (4 * count.value)).from_address(address)
     return _SELECTION.raw
+
+
+def _binder_type():
+    """The native call path (csrc/host/binder.cpp), or False where it is not built: every call then takes the Python
+    path, which does the same."""
+    global _BINDER
+    if _BINDER is None:
+        from importlib.util import module_from_spec, spec_from_file_location
+
+        import torch  # noqa: F401  (the extension links against its libraries)
+
+        path = Path(__file__).resolve().parent.parent / "lib" / "intent_b200_binder.so"
+        _BINDER = False
+        if path.exists():
+            spec = spec_from_file_location("intent_b200_binder", path)
+            try:
+                module = module_from_spec(spec)
+                spec.loader.exec_module(module)
+            except ImportError as error:
+                raise CompilationStageError("native_loading", f"cannot load {path}: {error}") from error
+            _BINDER = module.Binder
+    return _BINDER
+
+
+def binder(entry_name: str, device: int, views: tuple, constants: tuple, workspaces: dict | None):
+    """A native caller of one entry: ``views`` are (access, torch dtype, rank, alignment) in declaration order.
+    None where the entry has no packed form."""
+    kind = _binder_type()
+    if not kind:
+        return None
+    packed = _PACKED.get(entry_name, False)
+    if packed is False:
+        find = library()["intent_b200_packed_call"]
+        find.restype, find.argtypes = ctypes.c_void_p, [ctypes.c_char_p, ctypes.c_void_p]
+        slots = ctypes.c_int32()
+        address = find(entry_name.encode(), ctypes.byref(slots))
+        packed = _PACKED[entry_name] = (address, slots.value) if address and slots.value <= 63 else None
+    if packed is None or len(views) > 16 or any(not 1 <= v[2] <= 3 for v in views):
+        return None
+    size = len(selection())
+    return kind(*packed, device, ctypes.addressof(_SELECTION), size, workspaces, views, constants)
 
 
 def status_string(status: int) -> str:
