@@ -452,24 +452,28 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + acc * (ACC_COLUMNS / 2) + (uint32_t(quadrant * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < t.rows; c += 32) {
-        uint32_t v[32];
-        tmem_load_32x32(taddr + c, v);
+      for (int c = 0; c < t.rows; c += MODE == MODE_UPGATE_SILU ? 16 : 32) {
+        // Predicated, not branched: a branch a row keeps the work of different rows apart, and the epilogue of a tile with
+        // few k blocks then takes longer than its MMAs (16384 tokens on 64 experts of 4096 x 1408: up|gate 807 -> 640 us).
         if (MODE == MODE_UPGATE_SILU) {
-          tmem_load_wait();
-          // lanes 0..15 hold gate columns, lanes 16..31 the matching up columns: they swap half of the rows
+          // lanes 0..15 hold gate columns, lanes 16..31 the matching up columns: of 16 rows each takes eight
           const bool is_up = lane >= 16;
           const int col = (t.n_tile * CG + (CG == 2 ? rank : 0)) * 64 + quadrant * 16 + (lane & 15);
-#pragma unroll 8
-          for (int i = 0; i < 16; ++i) {
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, is_up ? v[i] : v[16 + i], 16);
-            const float gv = __uint_as_float(is_up ? got : v[i]), uv = __uint_as_float(is_up ? v[16 + i] : got);
-            const int r = c + i + (is_up ? 16 : 0);
-            const float h = gv * (1.0f / (1.0f + __expf(-gv))) * uv;  // silu(gate) * up in f32, one rounding
+          uint32_t v[16];
+          tmem_load_32x16(taddr + c, v);
+          tmem_load_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, is_up ? v[i] : v[8 + i], 16);
+            const float gv = __uint_as_float(is_up ? got : v[i]), uv = __uint_as_float(is_up ? v[8 + i] : got);
+            const int r = c + i + (is_up ? 8 : 0);
+            const float h = gv * __frcp_rn(1.0f + __expf(-gv)) * uv;  // silu(gate) * up in f32, one rounding
             if (r < t.rows) y[size_t(t.row0 + r) * p.out_cols + col] = Elem<T>::from_float(h);
           }
         } else {
           const int col = (t.n_tile * CG + (CG == 2 ? rank : 0)) * COLS + quadrant * 32 + lane;
+          uint32_t v[32];
+          tmem_load_32x32(taddr + c, v);
           if (MODE == MODE_DOWN_SCATTER) {
             // lane r of the chunk: where row r goes and with what weight
             int token = -1;
@@ -482,23 +486,42 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
               }
             }
             tmem_load_wait();
+            // Four lanes swap four rows of their four columns, so that each adds 16 bytes of one row: adds of four bytes a
+            // lane stop at 1 TB/s (16384 tokens on 64 experts, whole layer: 1493 us with them, 1400 so).
+            const bool odd = lane & 1, upper = lane & 2;
+            const int first_col = col & ~3, off = first_col < p.out_cols ? 0 : int(0x80000000);
+            float* to = yf + first_col;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int row_token = __shfl_sync(0xffffffffu, token, i);
-              const float w = __shfl_sync(0xffffffffu, weight, i);
-              if (row_token >= 0 && col < p.out_cols)
-                asm volatile("red.global.add.f32 [%0], %1;" ::"l"(yf + size_t(row_token) * p.out_cols + col),
-                             "f"(__fmul_rn(w, __uint_as_float(v[i])))
-                             : "memory");
+            for (int i = 0; i < 32; i += 4) {
+              const uint32_t got0 = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
+              const uint32_t got1 = __shfl_xor_sync(0xffffffffu, odd ? v[i + 2] : v[i + 3], 1);
+              const uint32_t a0 = odd ? got0 : v[i], a1 = odd ? v[i + 1] : got0;          // row 0 or 1
+              const uint32_t b0 = odd ? got1 : v[i + 2], b1 = odd ? v[i + 3] : got1;      // row 2 or 3
+              const uint32_t got2 = __shfl_xor_sync(0xffffffffu, upper ? a0 : b0, 2);
+              const uint32_t got3 = __shfl_xor_sync(0xffffffffu, upper ? a1 : b1, 2);
+              const int row_token = __shfl_sync(0xffffffffu, token, i + (lane & 3)) | off;
+              const float w = __shfl_sync(0xffffffffu, weight, i + (lane & 3));
+              const float c0 = __fmul_rn(w, __uint_as_float(upper ? got2 : a0));
+              const float c1 = __fmul_rn(w, __uint_as_float(upper ? got3 : a1));
+              const float c2 = __fmul_rn(w, __uint_as_float(upper ? b0 : got2));
+              const float c3 = __fmul_rn(w, __uint_as_float(upper ? b1 : got3));
+              asm volatile(
+                  "{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %5, 0;\n\t"
+                  "@p red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n\t}"
+                  ::"l"(to + int64_t(row_token) * p.out_cols), "f"(c0), "f"(c1), "f"(c2), "f"(c3), "r"(row_token)
+                  : "memory");
             }
           } else {
             tmem_load_wait();
+            const int left = col < p.out_cols ? t.rows - c : 0;
+            size_t at = size_t(t.row0 + c) * p.out_cols + col;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int r = c + i;
-              if (r < t.rows && col < p.out_cols) {
-                if (MODE == MODE_GROUPED_F32) yf[size_t(t.row0 + r) * p.out_cols + col] = __uint_as_float(v[i]);
-                else y[size_t(t.row0 + r) * p.out_cols + col] = Elem<T>::from_float(__uint_as_float(v[i]));
+            for (int i = 0; i < 32; ++i, at += p.out_cols) {
+              if (MODE == MODE_GROUPED_F32) {
+                if (i < left) yf[at] = __uint_as_float(v[i]);
+              } else {
+                const uint16_t value = Elem<T>::from_float(__uint_as_float(v[i]));
+                if (i < left) y[at] = value;
               }
             }
           }
