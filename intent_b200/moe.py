@@ -14,6 +14,7 @@ no step reads a device value back to the host.
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import cached_property
 
 from . import programs
 from .compiler import compile as _compile
@@ -153,36 +154,57 @@ class MoEW4A16FFN:
         if block_size not in (128, 256):
             raise ValueError("block_size must be 128 or 256 (rows of one tile of the grouped contraction)")
         quant = {"GROUP_SIZE": group_size, "ZERO_POINT": zero_point, "ACT_DTYPE": act_dtype}
-        self.router = _compile(programs.moe_route_top2, target=target)
-        self.positions = _compile(programs.moe_route_positions, target=target, constexprs=align)
-        self.gather = _compile(programs.moe_gather_rows, target=target,
-                               constexprs={"ACT_DTYPE": act_dtype, "TOP_K": top_k})
+        gathered = {"ACT_DTYPE": act_dtype, "TOP_K": top_k}
         grouped = dict(quant, BLOCK_ROWS=block_size, WEIGHT_LAYOUT="tiled" if prelayout else "reference")
+        self._bind = lambda definition, constexprs=None: _compile(definition, target=target, constexprs=constexprs)
+        self._align, self._gathered, self._grouped = align, gathered, grouped
+        self.router = self._bind(programs.moe_route_top2)
         self.prelayout = None
         if prelayout:
             from .prelayout import PrelayoutCache
 
             self.prelayout = PrelayoutCache()
-        self.up_gate = _compile(programs.moe_grouped_upgate_silu, target=target, constexprs=grouped)
-        self.down = _compile(programs.moe_grouped_down, target=target, constexprs=grouped)
-        self.combine = _compile(programs.moe_combine, target=target)
-        self.combine_overwrite = _compile(programs.moe_combine, target=target, constexprs={"ACCUMULATE": False})
         # With at most two choices per token the weighted combine runs in the down projection's epilogue
         # (relaxed vector atomics on y): on a zeroed y two additions commute exactly, so the result has the same
         # bits as the ordered combine.  More choices keep the ordered combine kernel.
         self.fused_combine = top_k <= 2
-        self.down_scatter = _compile(programs.moe_grouped_down_scatter, target=target, constexprs=grouped)
+        self.down_scatter = self._bind(programs.moe_grouped_down_scatter, grouped)
         # The fused chain reads no padding row, so on the reference layout it neither writes nor multiplies them.
-        self._chain = (self.gather, self.up_gate)
-        if self.fused_combine and not prelayout:
-            self._chain = (_compile(programs.moe_gather_rows, target=target,
-                                    constexprs={"ACT_DTYPE": act_dtype, "TOP_K": top_k, "PADDING": False}),
-                           _compile(programs.moe_grouped_upgate_silu, target=target,
-                                    constexprs=dict(grouped, ROUTED=True)))
+        self._routed = self.fused_combine and not prelayout
+        if self._routed:
+            self._chain = (self._bind(programs.moe_gather_rows, dict(gathered, PADDING=False)),
+                           self._bind(programs.moe_grouped_upgate_silu, dict(grouped, ROUTED=True)))
+        else:
+            self._chain = (self.gather, self.up_gate)
+
+    # What only the other chains use is bound at its first use.
+    @cached_property
+    def positions(self):
+        return self._bind(programs.moe_route_positions, self._align)
+
+    @cached_property
+    def gather(self):
+        return self._bind(programs.moe_gather_rows, self._gathered)
+
+    @cached_property
+    def up_gate(self):
+        return self._bind(programs.moe_grouped_upgate_silu, self._grouped)
+
+    @cached_property
+    def down(self):
+        return self._bind(programs.moe_grouped_down, self._grouped)
+
+    @cached_property
+    def combine(self):
+        return self._bind(programs.moe_combine)
+
+    @cached_property
+    def combine_overwrite(self):
+        return self._bind(programs.moe_combine, {"ACCUMULATE": False})
 
     def _up_gate_inputs(self, rows, blocks, total, packed, scales, sorted_routes, topk_weights):
         inputs = (rows, blocks, total, packed, scales)
-        return inputs if self._chain[1] is self.up_gate else inputs + (sorted_routes, topk_weights)
+        return inputs + (sorted_routes, topk_weights) if self._routed else inputs
 
     def route(self, logits):
         """logits [T, E_total] f32 -> (ids [T,2] i32, weights [T,2] f32)."""
