@@ -122,6 +122,8 @@ def binder(entry_name: str, device: int, views: tuple, constants: tuple, workspa
         packed = _PACKED[entry_name] = (address, slots.value) if address and slots.value <= 63 else None
     if packed is None or len(views) > 16 or any(not 1 <= v[2] <= 3 for v in views):
         return None
+    if sum(1 + 2 * v[2] for v in views) + len(constants) + (0 if workspaces is None else 2) + 1 != packed[1]:
+        return None          # not this entry's parameters
     size = len(selection())
     return kind(*packed, device, ctypes.addressof(_SELECTION), size, workspaces, views, constants)
 
