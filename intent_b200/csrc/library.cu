@@ -13,6 +13,8 @@ void note_launch(int count) { g_launches.fetch_add(count, std::memory_order_rela
 int w4a16_stream_f16(View2, View2, View2, View2, int, int, void*, int64_t, cudaStream_t);
 int w4a16_stream_bf16(View2, View2, View2, View2, int, int, void*, int64_t, cudaStream_t);
 int64_t w4a16_stream_workspace_bytes(int64_t M, int64_t K, int64_t N);
+int w4a16_skinny_f16(View2, View2, View2, View2, int, int, void*, int64_t, cudaStream_t);
+int w4a16_skinny_bf16(View2, View2, View2, View2, int, int, void*, int64_t, cudaStream_t);
 int w4a16_gemm_f16(View2, View2, View2, View2, int, int, cudaStream_t);
 int w4a16_gemm_bf16(View2, View2, View2, View2, int, int, cudaStream_t);
 
@@ -110,6 +112,11 @@ extern "C" int64_t intent_b200_launch_count(void) { return ib200::g_launches.loa
                       int64_t workspace_bytes, void* stream) {                                            \
     const bool skinny = SELECT;                                                                           \
     if (skinny && (TABLE)) {                                                                              \
+      const int wide = ib200::w4a16_skinny_##TYPE(IB200_VIEW2_ARG(a0), IB200_VIEW2_ARG(a1),               \
+                                                  IB200_VIEW2_ARG(a2), IB200_VIEW2_ARG(a3), group_size,   \
+                                                  zero_point, workspace, workspace_bytes,                 \
+                                                  static_cast<cudaStream_t>(stream));                     \
+      if (wide != ib200::kTableDeclined) return wide;                                                     \
       const int status = ib200::w4a16_table_single_##TYPE(                                                \
           IB200_VIEW2_ARG(a0), IB200_VIEW2_ARG(a1), IB200_VIEW2_ARG(a2), IB200_VIEW2_ARG(a3), group_size, \
           zero_point, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));                     \

@@ -66,7 +66,12 @@ struct TmemParams {
   int routes, top_k;
 };
 
-constexpr int MODE_DENSE = 0, MODE_UPGATE_SILU = 1, MODE_GROUPED_F32 = 2, MODE_DOWN_SCATTER = 3;
+// MODE_SKINNY: dense calls of at most SKINNY_ROWS rows, as precise as the bandwidth kernels that serve the others: the
+// weights go to the tensor core as the integers q - 8, exactly; every quantisation group has an accumulator of its own,
+// which the epilogue warps scale and add up in f32 while the next k blocks are multiplied.
+constexpr int MODE_DENSE = 0, MODE_UPGATE_SILU = 1, MODE_GROUPED_F32 = 2, MODE_DOWN_SCATTER = 3, MODE_SKINNY = 4;
+constexpr int SKINNY_ROWS = 16, RING = 4;    // accumulators of RING k blocks in flight, up to four groups each
+__host__ __device__ constexpr bool dense_mode(int mode) { return mode == MODE_DENSE || mode == MODE_SKINNY; }
 
 // D[tmem] (+)= A[tmem] * B[smem]
 template <int CG>
@@ -99,6 +104,14 @@ __device__ __forceinline__ void tmem_store_32x32(uint32_t taddr, const uint32_t 
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
         "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
         "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+// 32 lanes x 16 columns
+__device__ __forceinline__ void tmem_store_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -142,9 +155,9 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   // in stage i % x_stages of shared memory, its expanded weights in stage i % A_STAGES of tensor memory.
   const uint32_t full = empty_w + 8 * p.w_stages;      // [x_stages] leader: activations landed, expanded weights stored
   const uint32_t empty = full + 8 * p.x_stages;        // [x_stages] MMAs done with them
-  const uint32_t tmem_full = empty + 8 * p.x_stages;   // [2] accumulators complete
-  const uint32_t tmem_empty = tmem_full + 16;          // [2] leader: accumulators drained
-  const uint32_t tmem_slot = tmem_empty + 16;
+  const uint32_t tmem_full = empty + 8 * p.x_stages;   // [2; RING] accumulators complete
+  const uint32_t tmem_empty = tmem_full + 8 * RING;    // [2; RING] leader: accumulators drained
+  const uint32_t tmem_slot = tmem_empty + 8 * RING;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
   int2* list = reinterpret_cast<int2*>(base_ptr + (tmem_slot - base) + 16);   // grouped: {expert, rows} per block
 
@@ -162,13 +175,13 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
     if (lane < p.w_stages) {
       mbar_init(full_w + 8 * lane, 1);
-      mbar_init(empty_w + 8 * lane, 4);
+      mbar_init(empty_w + 8 * lane, MODE == MODE_SKINNY ? 8 : 4);   // (the epilogue reads the scales of a stage)
     }
     if (lane < p.x_stages) {
       mbar_init(full + 8 * lane, 4 * CG + 1);
       mbar_init(empty + 8 * lane, 1);
     }
-    if (lane < 2) {
+    if (lane < RING) {
       mbar_init(tmem_full + 8 * lane, 1);
       mbar_init(tmem_empty + 8 * lane, 4 * CG);
     }
@@ -179,7 +192,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     else tmem_alloc(tmem_slot, 512);
   }
   int m_tiles = p.m_tiles;
-  if (MODE != MODE_DENSE) {
+  if (!dense_mode(MODE)) {
     // rows in use of every 128-row block: its routes come first, padding follows
     m_tiles = min(m_tiles, (*p.total_rows + 127) / 128);
     const int per_expert = p.block_rows / 128;
@@ -227,7 +240,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   };
   auto item_of = [&](int item) {
     Item t;
-    if (MODE == MODE_DENSE) {
+    if (dense_mode(MODE)) {
       t.n_tile = tile_quotient(item);   // the row tile varies fastest
       const int m_tile = item - t.n_tile * m_tiles;
       t.row0 = m_tile * p.row_tile;
@@ -283,7 +296,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     for (int item = first_item; item < items && ok; item += item_step) {
       const Item t = item_of(item);
       const int rows = t.n / CG, row0 = t.row0 + (CG == 2 ? rank * rows : 0);
-      const int boxes = MODE == MODE_DENSE ? 1 : __shfl_sync(0xffffffffu, rows / 16, 0);
+      const int boxes = dense_mode(MODE) ? 1 : __shfl_sync(0xffffffffu, rows / 16, 0);
       const uint32_t bytes = uint32_t(CG * boxes * p.box_rows) * 256u;
       int k = kb_first * BK;
       for (int kb = 0; kb < kb_count; ++kb, k += BK) {
@@ -318,26 +331,45 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       const bool issue = elect_one();
       const uint64_t desc_x = umma_desc_k_major_sw128(smem_x);
       const uint32_t desc_high = uint32_t(desc_x >> 32);
-      uint32_t s = 0, phase = 0, a = 0, local = 0;
+      uint32_t s = 0, phase = 0, a = 0, local = 0, ring = 0, ring_phase = 0;
       bool ok = true, ready = false;   // ready: both operands of the k block were seen to be there
       for (int item = first_item; item < items && ok; item += item_step, ++local) {
         const Item t = item_of(item);
         const uint32_t idesc = umma_idesc(1, fmt, fmt, 0, 0, CG * COLS, uint32_t(t.n));
         const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = p.acc_sets == 2 ? local >> 1 : local;
-        ok = mbar_wait_warp(tmem_empty + 8 * acc, (use & 1) ^ 1);
-        if (!ok) break;
-        tcgen05_fence_after();
+        if (MODE != MODE_SKINNY) {
+          ok = mbar_wait_warp(tmem_empty + 8 * acc, (use & 1) ^ 1);
+          if (!ok) break;
+          tcgen05_fence_after();
+        }
         const uint32_t tmem_d = tmem_base + acc * (ACC_COLUMNS / 2);
         for (int kb = 0; kb < kb_count; ++kb) {
           const uint32_t tmem_a = tmem_base + A_COLUMN + a * 64, done = empty + 8 * s;
           const uint32_t desc_low = uint32_t(desc_x) + s * (x_half >> 3);   // two halves of x_half / 16 units
           ok = __all_sync(0xffffffffu, ready) || mbar_wait_warp(full + 8 * s, phase);
           if (!ok) break;
+          if (MODE == MODE_SKINNY) {
+            ok = mbar_wait_warp(tmem_empty + 8 * ring, ring_phase ^ 1);
+            if (!ok) break;
+          }
           if (++s == uint32_t(p.x_stages)) s = 0, phase ^= 1;
           a = (a + 1) % A_STAGES;
           ready = mbar_test(full + 8 * s, phase);   // of the next k block
           tcgen05_fence_after();
-          if (issue) {
+          if (MODE == MODE_SKINNY) {
+            if (issue) {
+              const int steps = 1 << (p.group_shift - 4);   // MMAs of 16 k in a group
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk) {
+                const uint32_t low = desc_low + (kk >= 4 ? (x_half >> 4) : 0u) + 2 * (kk & 3);
+                umma_f16_ts<CG>(tmem_base + ring * 64 + (kk >> (p.group_shift - 4)) * SKINNY_ROWS, tmem_a + kk * 8,
+                                (uint64_t(desc_high) << 32) | low, idesc, (kk & (steps - 1)) != 0);
+              }
+              umma_commit(done);
+              umma_commit(tmem_full + 8 * ring);
+            }
+            if (++ring == RING) ring = 0, ring_phase ^= 1;
+          } else if (issue) {
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {   // 16 k: 8 columns of A, 32 bytes of a row of B
               const uint32_t low = desc_low + (kk >= 4 ? (x_half >> 4) : 0u) + 2 * (kk & 3);   // an address: no carry
@@ -348,7 +380,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           }
           __syncwarp();
         }
-        if (ok && issue) {
+        if (MODE != MODE_SKINNY && ok && issue) {
           if (CG == 2) umma_commit_pair(tmem_full + 8 * acc);
           else umma_commit(tmem_full + 8 * acc);
         }
@@ -393,7 +425,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       for (int r = 0; r < W_ROWS; ++r) words[r] = lds32(stage + w_offset + r * w_pitch);
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        const uint32_t v = lds16(stage + s_of[g]);
+        const uint32_t v = MODE == MODE_SKINNY ? 0u : lds16(stage + s_of[g]);
         scale[g] = v | (v << 16);
       }
       // the words are in registers before the stage is handed back: the arrival waits for the loads it depends on
@@ -418,8 +450,10 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           o[4 * j + 2] = lop3_and_xor_u32(prmt(w, w4, 0x0602), 0x000F000Fu, magic);  // (k4, k5)
           o[4 * j + 3] = lop3_and_xor_u32(prmt(w, w4, 0x0703), 0x000F000Fu, magic);  // (k6, k7)
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            o[4 * j + c] = Elem<T>::mul2(Elem<T>::sub2(o[4 * j + c], Elem<T>::kBias2), scale2);
+          for (int c = 0; c < 4; ++c) {
+            o[4 * j + c] = Elem<T>::sub2(o[4 * j + c], Elem<T>::kBias2);
+            if (MODE != MODE_SKINNY) o[4 * j + c] = Elem<T>::mul2(o[4 * j + c], scale2);
+          }
         }
         tmem_store_32x32(tmem_a + half * 32, o);
       }
@@ -433,6 +467,56 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       x_before = x, phase_before = phase_x;
       x += SETS;
       if (x >= uint32_t(p.x_stages)) x -= p.x_stages, phase_x ^= 1;
+    }
+    if (!ok && lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
+  } else if (MODE == MODE_SKINNY && warp >= FIRST_EPILOGUE) {
+    // ------------------------------ scaling and sum over the groups ------------
+    const int quadrant = warp & 3, column = quadrant * 32 + lane, groups = BK >> p.group_shift;
+    const uint32_t s_offset = W_BYTES + uint32_t(column) * 2;
+    uint32_t s = 0, phase = 0, ring = 0, ring_phase = 0;
+    bool ok = true;
+    for (int item = first_item; item < items && ok; item += item_step) {
+      const Item t = item_of(item);
+      float sum[SKINNY_ROWS];
+#pragma unroll
+      for (int r = 0; r < SKINNY_ROWS; ++r) sum[r] = 0.f;
+      for (int kb = 0; kb < kb_count; ++kb) {
+        ok = mbar_wait_warp(tmem_full + 8 * ring, ring_phase) && mbar_wait_warp(full_w + 8 * s, phase);
+        if (!ok) break;
+        tcgen05_fence_after();
+        const uint32_t stage = smem_w + s * W_STAGE + s_offset;
+        const uint32_t taddr = tmem_base + ring * 64 + (uint32_t(quadrant * 32) << 16);
+        for (int g = 0; g < groups; ++g) {
+          uint32_t v[SKINNY_ROWS];
+          tmem_load_32x16(taddr + g * SKINNY_ROWS, v);
+          const float scale = Elem<T>::to_float(uint16_t(lds16(stage + g * (COLS * 2))));
+          tmem_load_wait();
+#pragma unroll
+          for (int r = 0; r < SKINNY_ROWS; ++r) sum[r] = fmaf(__uint_as_float(v[r]), scale, sum[r]);
+        }
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(tmem_empty + 8 * ring);
+          mbar_arrive(empty_w + 8 * s);
+        }
+        if (++ring == RING) ring = 0, ring_phase ^= 1;
+        if (++s == uint32_t(p.w_stages)) s = 0, phase ^= 1;
+      }
+      const int col = t.n_tile * COLS + column;
+      if (p.split > 1) {   // back to tensor memory (all MMAs are done), from where the cluster's partial sums are put together
+        uint32_t v[SKINNY_ROWS];
+#pragma unroll
+        for (int r = 0; r < SKINNY_ROWS; ++r) v[r] = __float_as_uint(sum[r]);
+        tmem_store_32x16(tmem_base + (uint32_t(quadrant * 32) << 16), v);
+        tmem_store_wait();
+        tcgen05_fence_before();
+      } else if (ok && col < p.out_cols) {
+        uint16_t* y = reinterpret_cast<uint16_t*>(p.y) + col;
+#pragma unroll
+        for (int r = 0; r < SKINNY_ROWS; ++r)
+          if (r < t.rows) y[size_t(r) * p.out_cols] = Elem<T>::from_float(sum[r]);
+      }
     }
     if (!ok && lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
   } else if (warp >= FIRST_EPILOGUE) {
@@ -539,7 +623,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
-  if (MODE == MODE_DENSE && CG == 1 && p.split > 1 && first_item < items) {
+  if (dense_mode(MODE) && CG == 1 && p.split > 1 && first_item < items) {
     // Every CTA of the cluster holds a partial sum of the whole tile.  The rows are dealt out in `split` slices: a
     // CTA writes the others' slices into their shared memory (the operand stages are idle once all MMAs are done),
     // then adds the partials of its own slice in rank order.
@@ -613,10 +697,10 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   p.WN = int(q.WN);
   p.out_cols = int(q.out_cols);
   p.k_blocks = int((q.K + BK - 1) / BK);
-  p.row_tile = MODE == MODE_DENSE ? q.row_tile : 128;
+  p.row_tile = dense_mode(MODE) ? q.row_tile : 128;
   p.m_tiles = int((q.rows + p.row_tile - 1) / p.row_tile);
   p.n_tiles = MODE == MODE_UPGATE_SILU ? int(q.out_cols / (64 * CG)) : int((q.out_cols + COLS * CG - 1) / (COLS * CG));
-  p.box_rows = MODE == MODE_DENSE ? p.row_tile / CG : 16;
+  p.box_rows = dense_mode(MODE) ? p.row_tile / CG : 16;
   p.acc_sets = p.row_tile <= 128 ? 2 : 1;
   p.split = q.split;
   p.group_shift = q.group_size == 32 ? 5 : q.group_size == 64 ? 6 : 7;
@@ -630,13 +714,14 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   p.routes = int(q.routes);
   p.top_k = q.top_k;
   if (p.row_tile % (16 * CG) != 0 || p.row_tile < 16 * CG || p.row_tile > 128 * CG) return INTENT_B200_ERR_UNSUPPORTED;
-  if (p.split < 1 || p.split > 8 || (p.split > 1 && (MODE != MODE_DENSE || CG != 1 || p.k_blocks < p.split)))
+  if (p.split < 1 || p.split > 8 || (p.split > 1 && (!dense_mode(MODE) || CG != 1 || p.k_blocks < p.split)))
     return INTENT_B200_ERR_UNSUPPORTED;
-  if (MODE != MODE_DENSE && (p.m_tiles > LIST_BLOCKS || q.block_rows % 128 != 0)) return INTENT_B200_ERR_UNSUPPORTED;
+  if (MODE == MODE_SKINNY && (p.row_tile != SKINNY_ROWS || p.M > SKINNY_ROWS)) return INTENT_B200_ERR_UNSUPPORTED;
+  if (!dense_mode(MODE) && (p.m_tiles > LIST_BLOCKS || q.block_rows % 128 != 0)) return INTENT_B200_ERR_UNSUPPORTED;
 
   // Up to eight stages of activations: a stage comes back after its MMAs and a load from the L2, some 2000 cycles, of
   // which four k blocks cover no more than that.  The rest is a ring for the packed words, which come from HBM.
-  const int list_bytes = MODE == MODE_DENSE ? 0 : p.m_tiles * 8;
+  const int list_bytes = dense_mode(MODE) ? 0 : p.m_tiles * 8;
   const int fixed = 1024 + 512 + list_bytes, x_stage = p.row_tile / CG * 256;
   p.x_stages = 8;
   while (p.x_stages > A_STAGES && fixed + p.x_stages * x_stage + 9 * W_STAGE > SMEM_LIMIT) --p.x_stages;
@@ -667,7 +752,7 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_status(e);
   const int64_t items = int64_t(p.m_tiles) * p.n_tiles;
-  const int64_t fastest = MODE == MODE_DENSE ? p.m_tiles : p.n_tiles;
+  const int64_t fastest = dense_mode(MODE) ? p.m_tiles : p.n_tiles;
   if (items * fastest >= (int64_t(1) << 32) || (p.split > 1 && items > 65535)) return INTENT_B200_ERR_UNSUPPORTED;
   p.tile_magic = fastest == 1 ? 0u : uint32_t(((uint64_t(1) << 32) + fastest - 1) / fastest);
   p.kb_each = p.k_blocks / p.split;
@@ -676,7 +761,9 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   const int grid = int(p.split > 1 ? items * p.split : CG * (items < sms / CG ? items : sms / CG));
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel),
-                         CG == 2       ? "w4a16_tmem_kernel CTA pairs, 256 columns"
+                         MODE == MODE_SKINNY ? (p.split > 1 ? "w4a16_tmem_kernel 16 rows, scaled in f32, k split over a cluster"
+                                                            : "w4a16_tmem_kernel 16 rows, scaled in f32")
+                         : CG == 2       ? "w4a16_tmem_kernel CTA pairs, 256 columns"
                          : p.split > 1 ? "w4a16_tmem_kernel k split over a cluster, 128 columns"
                                        : "w4a16_tmem_kernel single CTA, 128 columns",
                          grid, THREADS, smem, cluster);
@@ -704,6 +791,7 @@ template <typename T>
 int w4a16_tmem(const TmemCall& q, int mode, bool pairs, cudaStream_t stream) {
   switch (mode) {
     case MODE_DENSE: return pairs ? launch<T, MODE_DENSE, 2>(q, stream) : launch<T, MODE_DENSE, 1>(q, stream);
+    case MODE_SKINNY: return launch<T, MODE_SKINNY, 1>(q, stream);
     case MODE_UPGATE_SILU:
       return pairs ? launch<T, MODE_UPGATE_SILU, 2>(q, stream) : launch<T, MODE_UPGATE_SILU, 1>(q, stream);
     case MODE_GROUPED_F32:

@@ -45,6 +45,31 @@ def test_dense_tiles(cuda_device, dtype, zero_point, group, M, K, N, kernel):
     assert max_abs_rel(out[rows.to(cuda_device)].cpu(), rounded) <= (2e-3 if dtype == torch.float16 else 1.6e-2)
 
 
+@pytest.mark.parametrize("dtype,zero_point,group,M,K,N", [
+    (torch.float16, 8, 128, 16, 4096, 4096),                     # four CTAs a tile
+    (torch.bfloat16, "twos_complement", 32, 9, 1056, 136),       # four groups a k block, a quarter block at the end
+    (torch.float16, "twos_complement", 64, 13, 2112, 1000),
+    (torch.bfloat16, 8, 128, 12, 2048, 19208),                   # more tiles than SMs
+])
+def test_nine_to_sixteen_rows(cuda_device, dtype, zero_point, group, M, K, N):
+    """Scales in f32, as in the bandwidth kernels: no further from the result in 64 bits than they are."""
+    x, p, s = ib.workloads.w4a16_inputs(M, K, N, dtype=dtype, group_size=group, seed=M)
+    constants = {"GROUP_SIZE": group, "ZERO_POINT": zero_point, "ACT_DTYPE": "f16" if dtype == torch.float16 else "bf16"}
+    artifact, other = (ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),
+                                  constexprs=dict(constants, KERNEL=kernel)) for kernel in ("auto", "gemv"))
+    xd, pd, sd = x.to(cuda_device), p.to(cuda_device), s.to(cuda_device)
+    out, stream = artifact.run(xd, pd, sd), other.run(xd, pd, sd)
+    assert artifact.observation.kernel.startswith("w4a16_tmem_kernel 16 rows"), artifact.observation.kernel
+    assert torch.equal(artifact.run(xd, pd, sd), out)
+    torch.cuda.synchronize()
+    artifact.check()
+    q = oracle.unpack_int4(p).double()
+    q = q - 8 if zero_point == 8 else torch.where(q > 7, q - 16, q)
+    exact = x.double() @ (q * s.double().repeat_interleave(group, dim=0))
+    error, before = ((o.cpu().double() - exact).norm() / exact.norm() for o in (out, stream))
+    assert error <= before * 1.02       # both are the rounding of the result; 2 % for sums in another order
+
+
 @pytest.mark.parametrize("rows_of_expert,hidden,intermediate,block", [
     ((1, 16, 17, 0, 32, 33, 15, 2), 512, 128, 128),            # few rows: lone CTAs
     ((127, 128, 129, 0, 256, 1, 300, 31), 1024, 384, 128),     # blocks full and nearly empty: CTA pairs
