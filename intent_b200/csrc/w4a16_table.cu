@@ -210,7 +210,7 @@ w4a16_table_kernel(const __grid_constant__ TableMaps maps, const __grid_constant
   __shared__ int total_units;
   __shared__ int abort_flag;
 
-  if (p.overlap) asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.launch_dependents;");   // as in w4a16_stream.cu
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int cta = int(blockIdx.x);
@@ -288,9 +288,10 @@ w4a16_table_kernel(const __grid_constant__ TableMaps maps, const __grid_constant
   };
   // First wave: slot s is owned by warp s % WARPS.  With launch overlap the packed weights (static) are requested
   // before the wait for the kernel ahead of this one; activations, which that kernel may have produced, after it.
+  if (!p.overlap) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (lane == 0)
     for (int seq = warp; seq < min(total, S); seq += WARPS) issue(seq, 0);
-  if (p.overlap) asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   uint32_t magic_a, magic_b;
   Expand<T>::magic(p.twos_complement != 0, magic_a, magic_b);
@@ -627,7 +628,7 @@ w4a16_ride_kernel(const __grid_constant__ TableMaps maps, const __grid_constant_
   __shared__ int next_unit;                    // the next unit of the CTA's sequence nobody has taken yet
 
   if (p.probe == 7) return;   // measurement: what the bare launch of this kernel costs
-  if (p.overlap) asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.launch_dependents;");   // as in w4a16_stream.cu
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int cta = int(blockIdx.x);
@@ -715,6 +716,7 @@ w4a16_ride_kernel(const __grid_constant__ TableMaps maps, const __grid_constant_
       }
       first += n;
     }
+    if (!p.overlap) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (early_unit) issue(early_ent, uint32_t(lane), 1);
   }
   if (warp == 0) {
@@ -776,8 +778,9 @@ w4a16_ride_kernel(const __grid_constant__ TableMaps maps, const __grid_constant_
     sched[e] = ent;
     if (e == tid) mine_ent = ent;
   }
+  if (!p.overlap) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (tid >= early && tid < min(total, S)) issue(mine_ent, uint32_t(tid), 1);
-  if (p.overlap) asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (early_unit) issue(early_ent, uint32_t(lane), 2);
   if (tid >= early && tid < min(total, S)) issue(mine_ent, uint32_t(tid), 2);
   __syncthreads();   // the schedule is complete
@@ -1293,7 +1296,7 @@ int launch_table(const TableMaps& maps, const TableParams& p, int grid, size_t s
   attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
-  config.numAttrs = p.overlap ? 1 : 0;
+  config.numAttrs = 1;
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel), "w4a16_table_kernel staged activations", grid,
                          WARPS * 32, int(smem), 1);
@@ -1317,7 +1320,7 @@ int launch_ride(const TableMaps& maps, const TableParams& p, int grid, size_t sm
   attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
-  config.numAttrs = p.overlap ? 1 : 0;
+  config.numAttrs = 1;
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel), "w4a16_ride_kernel activations ride with the units",
                          grid, 1024, int(smem), 1);
