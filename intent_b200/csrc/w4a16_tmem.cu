@@ -14,8 +14,8 @@
 //
 // What bounds it: per 128 k 530 to 565 cycles for a lone tile or a pair of up to 128 rows - the issue loop, beside 330 issue
 // slots of every scheduler for the dequantisers and, at 128 rows of a pair, 512 cycles of MMAs; 1058 at 256 rows of a pair
-// (MMAs 1024).  With all SMs at work the operands come from the L2 at 8 TB/s: 0.40 us per 128 k.  Against the forms with the
-// weights in shared memory: M77 K14336 N4096 81.1 -> 18.0 us, M1024 K4096 N4096 50.9 -> 30.3, 64 tokens on 64 experts of
+// (MMAs 1024).  With all SMs at work a pair takes 0.40 us per 128 k, with the tensor pipe 44 % and the L2 16 % busy (M1024
+// K4096 N4096): the hand-overs between the roles, not a throughput.  Against the forms with the weights in shared memory: M77 K14336 N4096 81.1 -> 18.0 us, M1024 K4096 N4096 50.9 -> 30.3, 64 tokens on 64 experts of
 // 4096 x 1408 277 + 120 -> 103 + 56.
 #include <type_traits>
 
