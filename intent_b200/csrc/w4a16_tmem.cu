@@ -759,8 +759,10 @@ int launch(const TmemCall& q, cudaStream_t stream) {
                           CU_TENSOR_MAP_SWIZZLE_NONE))
     return INTENT_B200_ERR_UNSUPPORTED;
 
+  // The limit belongs to the kernel, not to the launch: the same value from every call, so that no thread lowers it
+  // between another one's request and its launch.
   auto kernel = w4a16_tmem_kernel<T, MODE, CG>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
   if (e != cudaSuccess) return cuda_status(e);
   const int64_t items = int64_t(p.m_tiles) * p.n_tiles;
   const int64_t fastest = dense_mode(MODE) ? p.m_tiles : p.n_tiles;

@@ -1,6 +1,8 @@
 """The W4A16 kernel with the weights in tensor memory: edges of its tiles in rows, columns and k.  Tiled weight copies
 run on the other kernels, which add the k blocks in the same order, so unsplit calls must agree with them bit for bit;
 the tolerances against the oracle are those of test_w4a16_gemm_gpu.py."""
+import threading
+
 import pytest
 import torch
 
@@ -97,3 +99,39 @@ def test_routed_rows(cuda_device, rows_of_expert, hidden, intermediate, block):
     ref = oracle.moe_w4a16_swiglu_ffn(data["x"], ids, weights, data["up_gate_packed"], data["up_gate_scales"],
                                       data["down_packed"], data["down_scales"])
     assert max_abs_rel(y.cpu(), ref) <= 2e-2
+
+
+@pytest.mark.parametrize("sizes", [
+    ((32, 2176, 512), (128, 2176, 512)),     # one instance of this kernel, 214528 and 224768 bytes of shared memory
+])
+def test_threads_launch_one_instance(cuda_device, sizes):
+    """Calls of one kernel instance with different shared memory do not get in each other's way: a launch must not fail
+    because another thread has asked for less in between."""
+    failures, threads = [], []
+
+    def work(M, K, N):
+        x, p, s = (t.to(cuda_device) for t in ib.workloads.w4a16_inputs(M, K, N, dtype=torch.bfloat16, seed=M))
+        artifact = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),
+                              constexprs={"GROUP_SIZE": 128, "ZERO_POINT": 8, "ACT_DTYPE": "bf16"})
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                expected = artifact.run(x, p, s)
+                ready.wait(60)
+                for _ in range(40):
+                    for _ in range(100):
+                        out = artifact.run(x, p, s)
+                    torch.cuda.current_stream().synchronize()      # (a full queue would keep the threads apart)
+            if not torch.equal(out, expected):
+                failures.append((M, "other bits"))
+        except Exception as error:
+            failures.append((M, str(error)))
+            ready.abort()
+
+    ready = threading.Barrier(4 * len(sizes))
+    torch.cuda.synchronize()
+    for size in 4 * sizes:
+        threads.append(threading.Thread(target=work, args=size))
+        threads[-1].start()
+    for t in threads:
+        t.join()
+    assert not failures, failures[:1]
