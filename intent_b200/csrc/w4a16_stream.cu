@@ -582,7 +582,8 @@ template <typename T, int MB, int STEPS, int WARPS, bool XSTAGED, int RING>
 int launch_kernel(const CUtensorMap& map_w, const CUtensorMap& map_s, const CUtensorMap& map_x, const StreamParams& p, const Plan& plan,
                   cudaStream_t stream) {
   auto kernel = w4a16_stream_kernel<T, MB, STEPS, WARPS, XSTAGED, RING>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(plan.smem_bytes));
+  // (the limit belongs to the kernel: the same value from every thread, not each plan's own)
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   if (e != cudaSuccess) return cuda_status(e);
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(plan.grid, 1, 1);

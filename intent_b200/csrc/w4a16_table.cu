@@ -1285,7 +1285,7 @@ template <typename T, int MB, int STEPS>
 int launch_table(const TableMaps& maps, const TableParams& p, int grid, size_t smem, cudaStream_t stream) {
   constexpr int WARPS = MB == 1 ? 32 : 16;
   auto kernel = w4a16_table_kernel<T, MB, STEPS, WARPS>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);   // as in w4a16_stream.cu
   if (e != cudaSuccess) return cuda_status(e);
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(grid, 1, 1);
@@ -1309,7 +1309,7 @@ int launch_table(const TableMaps& maps, const TableParams& p, int grid, size_t s
 template <typename T, int STEPS, int UR, bool CORR_MMA>
 int launch_ride(const TableMaps& maps, const TableParams& p, int grid, size_t smem, cudaStream_t stream) {
   auto kernel = w4a16_ride_kernel<T, STEPS, UR, CORR_MMA>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);   // as in w4a16_stream.cu
   if (e != cudaSuccess) return cuda_status(e);
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(grid, 1, 1);

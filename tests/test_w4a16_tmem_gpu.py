@@ -103,6 +103,8 @@ def test_routed_rows(cuda_device, rows_of_expert, hidden, intermediate, block):
 
 @pytest.mark.parametrize("sizes", [
     ((32, 2176, 512), (128, 2176, 512)),     # one instance of this kernel, 214528 and 224768 bytes of shared memory
+    ((1, 1024, 512), (1, 4096, 4096)),       # the bandwidth kernel: rings of a few slots and of many
+    ((4, 1024, 512), (4, 4096, 4096)),       # a table of one problem
 ])
 def test_threads_launch_one_instance(cuda_device, sizes):
     """Calls of one kernel instance with different shared memory do not get in each other's way: a launch must not fail
