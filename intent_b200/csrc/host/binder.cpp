@@ -152,6 +152,7 @@ PyObject* invoke(Binder* self, PyObject* arguments, bool explicit_outputs, bool 
         return not_plain();
 
   if (!plan->empty) {
+    at::Tensor workspace;   // kept over the call: another thread may replace the stream's buffer meanwhile
     for (int64_t c : *self->constants) slots[at_slot++] = c;
     int64_t workspace_bytes = 0;
     if (self->has_workspace) {
@@ -166,10 +167,10 @@ PyObject* invoke(Binder* self, PyObject* arguments, bool explicit_outputs, bool 
           return not_plain();
         }
         if (!THPVariable_CheckExact(held)) return not_plain();
-        const at::Tensor& buffer = THPVariable_Unpack(held);
-        if (buffer.numel() < plan->workspace) return not_plain();
-        pointer = reinterpret_cast<int64_t>(buffer.data_ptr());
-        workspace_bytes = buffer.numel();
+        workspace = THPVariable_Unpack(held);
+        if (workspace.numel() < plan->workspace) return not_plain();
+        pointer = reinterpret_cast<int64_t>(workspace.data_ptr());
+        workspace_bytes = workspace.numel();
       }
       slots[at_slot++] = pointer;
       slots[at_slot++] = workspace_bytes;

@@ -127,3 +127,41 @@ def test_several_threads(cuda_device):
     for t in threads:
         t.join()
     assert not failures
+
+
+def _binder_of(entry, workspaces):
+    """A native caller of ``entry`` (a Python function of the slots) with one f32 input and one f32 output of one axis each.
+    Nothing is launched: the entry stands where the library's would."""
+    import ctypes
+
+    function = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.POINTER(ctypes.c_int64))(entry)
+    switches = ctypes.create_string_buffer(4)
+    views = ((0, torch.float32, 1, 4), (1, torch.float32, 1, 4))
+    slots = 3 * len(views) + (0 if workspaces is None else 2) + 1
+    binder = native._binder_type()(ctypes.cast(function, ctypes.c_void_p).value, slots, 0, ctypes.addressof(switches), 4,
+                                   workspaces, views, ())
+    return binder, (function, switches)
+
+
+def test_a_workspace_outlives_the_call_that_uses_it(cuda_device):
+    """Another thread may replace the stream's workspace while a call is under way without the interpreter lock; the
+    call's buffer must not go back to the allocator before it has been launched on."""
+    size = 4 << 20
+    stream = torch.cuda.current_stream().cuda_stream
+    workspaces = {stream: torch.zeros(size, dtype=torch.uint8, device=cuda_device)}
+    given_back = []
+
+    def entry(slots):
+        before = torch.cuda.memory_allocated()
+        workspaces[stream] = None                # as a call that needs a larger one does
+        given_back.append(before - torch.cuda.memory_allocated())
+        return 0
+
+    binder, keep = _binder_of(entry, workspaces)
+    binder.learn((8, 8), size, False, bytes(4))
+    x = torch.zeros(8, device=cuda_device)
+    before = torch.cuda.memory_allocated()
+    out = binder.run((x,))
+    assert out.shape == (8,) and given_back == [0]
+    del out
+    assert torch.cuda.memory_allocated() == before - size      # and it does go back afterwards
