@@ -19,6 +19,7 @@
 #include <Python.h>
 
 #include <cstring>
+#include <memory>
 #include <new>
 #include <vector>
 
@@ -61,9 +62,15 @@ struct Binder {
   bool has_workspace;
   std::vector<View>* views;
   std::vector<int64_t>* constants;
-  std::vector<Plan>* plans;
+  std::vector<std::shared_ptr<const Plan>>* plans;
   std::size_t next;                  // plan to replace when there are kMaxPlans
   Record* last;
+};
+
+// Gives the interpreter lock up for its lifetime, also where an exception ends it.
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
 };
 
 PyObject* not_plain() { Py_RETURN_NOTIMPLEMENTED; }
@@ -112,14 +119,14 @@ PyObject* invoke(Binder* self, PyObject* arguments, bool explicit_outputs, bool 
   if (next != count) return not_plain();
 
   // the plan of these shapes, found under the switches as they are
-  const Plan* plan = nullptr;
-  for (const Plan& p : *self->plans) {
-    const int64_t* extent = p.shapes.data();
+  std::shared_ptr<const Plan> plan;   // (learn() of another thread may drop it from the list)
+  for (const auto& p : *self->plans) {
+    const int64_t* extent = p->shapes.data();
     bool same = true;
     for (std::size_t i = 0; i < n && same; extent += views[i].rank, ++i)
       if (supplied[i]) same = std::memcmp(extent, supplied[i]->sizes().data(), views[i].rank * sizeof(int64_t)) == 0;
     if (same) {
-      plan = &p;
+      plan = p;
       break;
     }
   }
@@ -130,13 +137,16 @@ PyObject* invoke(Binder* self, PyObject* arguments, bool explicit_outputs, bool 
   int at_slot = 0;
   at::Tensor made[16];
   int64_t begin[16], end[16];
-  const int64_t* extent = plan->shapes.data();
-  for (std::size_t i = 0; i < n; extent += views[i].rank, ++i) {
+  if (!explicit_outputs) {
+    Unlocked unlocked;   // an allocation may reach the driver and take milliseconds
+    const int64_t* extent = plan->shapes.data();
+    for (std::size_t i = 0; i < n; extent += views[i].rank, ++i)
+      if (!supplied[i])
+        made[i] = at::empty(at::IntArrayRef(extent, views[i].rank),
+                            at::TensorOptions().dtype(views[i].type).device(at::kCUDA, self->device));
+  }
+  for (std::size_t i = 0; i < n; ++i) {
     const int rank = views[i].rank;
-    if (!supplied[i]) {
-      const at::IntArrayRef shape(extent, rank);
-      made[i] = at::empty(shape, at::TensorOptions().dtype(views[i].type).device(at::kCUDA, self->device));
-    }
     const at::Tensor& t = supplied[i] ? *supplied[i] : made[i];
     const int64_t pointer = reinterpret_cast<int64_t>(t.data_ptr());
     if (pointer % views[i].alignment != 0 || !t.is_contiguous()) return not_plain();
@@ -246,18 +256,18 @@ PyObject* binder_learn(PyObject* object, PyObject* arguments) {
     return nullptr;
   }
   try {
-    Plan plan;
+    auto plan = std::make_shared<Plan>();
     for (std::size_t i = 0; i < extents; ++i) {
       const long long extent = PyLong_AsLongLong(PyTuple_GET_ITEM(shapes, Py_ssize_t(i)));
       if (extent == -1 && PyErr_Occurred()) return nullptr;
-      plan.shapes.push_back(extent);
+      plan->shapes.push_back(extent);
     }
-    plan.selection.assign(selection, selection + selection_bytes);
-    plan.workspace = workspace;
-    plan.empty = empty != 0;
+    plan->selection.assign(selection, selection + selection_bytes);
+    plan->workspace = workspace;
+    plan->empty = empty != 0;
     auto& plans = *self->plans;
-    for (Plan& p : plans)
-      if (p.shapes == plan.shapes) {   // found again under other switches
+    for (auto& p : plans)
+      if (p->shapes == plan->shapes) {   // found again under other switches
         p = std::move(plan);
         Py_RETURN_NONE;
       }
@@ -323,7 +333,7 @@ PyObject* binder_new(PyTypeObject* type, PyObject* arguments, PyObject*) {
   try {
     self->views = new std::vector<View>();
     self->constants = new std::vector<int64_t>();
-    self->plans = new std::vector<Plan>();
+    self->plans = new std::vector<std::shared_ptr<const Plan>>();
     self->last = new Record();
     for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(views); ++i) {
       View v;

@@ -165,3 +165,44 @@ def test_a_workspace_outlives_the_call_that_uses_it(cuda_device):
     assert out.shape == (8,) and given_back == [0]
     del out
     assert torch.cuda.memory_allocated() == before - size      # and it does go back afterwards
+
+
+def test_other_threads_run_while_an_output_is_allocated(cuda_device):
+    """An allocation that reaches the driver takes milliseconds: the interpreter lock is released for it, as torch.empty
+    does."""
+    import sys
+    import time
+
+    counter, at_entry, stop = [0], [], threading.Event()
+
+    def entry(slots):
+        at_entry.append(counter[0])
+        return 0
+
+    binder, keep = _binder_of(entry, None)
+    binder.learn((8, 1 << 31), -1, False, bytes(4))
+
+    def count():
+        while not stop.is_set():
+            counter[0] += 1
+            time.sleep(0)
+
+    x = torch.zeros(8, device=cuda_device)
+    interval = sys.getswitchinterval()
+    thread = threading.Thread(target=count)
+    progress = []
+    try:
+        sys.setswitchinterval(30.0)             # the other thread only gets what is given up
+        thread.start()
+        for _ in range(5):
+            torch.cuda.empty_cache()
+            before = counter[0]
+            out = binder.run((x,))              # 8 GiB that no cached block serves
+            progress.append(at_entry[-1] - before)
+            del out
+    finally:
+        stop.set()
+        sys.setswitchinterval(interval)
+        thread.join()
+        torch.cuda.empty_cache()
+    assert max(progress) > 5, progress          # (the call of the entry itself gives the lock up once)
