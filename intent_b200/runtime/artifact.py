@@ -228,6 +228,11 @@ class NativeProgram:
         return None if launched is None else launched.observation(self)
 
     # ---- native call path ----------------------------------------------------------
+    @property
+    def launcher(self):
+        """The native caller of ``launch``: a launch owns its workspace, so a program that needs one has none."""
+        return self.binder if self._workspace_spec is None else None
+
     def record(self, launched: _Launched) -> None:
         """``launched`` is the latest call."""
         self._launched = launched
@@ -261,9 +266,10 @@ class NativeProgram:
                 views = tuple((int(p.access), torch_dtype(p.dtype), len(p.shape), p.alignment) for p in parameters)
                 self.binder = native.binder(self.entry_name, self.device, views, self.constants,
                                             None if self._workspace_spec is None else self._stream_workspaces)
-        if self.binder is not None:
-            size = -1 if self._workspace_spec is None else int(self._workspace_spec(bound.dimensions))
-            self.binder.learn(tuple(e for f in bound.views for e in f.shape), size, self.is_empty(bound), selection)
+        if self.binder is None or not native.PLAIN.issuperset(map(type, bound.arguments)):
+            return None                      # (it does not take subclasses)
+        size = -1 if self._workspace_spec is None else int(self._workspace_spec(bound.dimensions))
+        self.binder.learn(tuple(e for f in bound.views for e in f.shape), size, self.is_empty(bound), selection)
         return self.binder
 
     @cached_property
@@ -396,7 +402,7 @@ class NativeProgram:
     def launch(self, *arguments) -> None:
         selection = native.selection()
         bound = self.interface.bind(tuple(arguments), device=self._torch_device, explicit_outputs=True)
-        binder = self._teach(bound, selection)
+        binder = self._teach(bound, selection) if self._workspace_spec is None else None
         if binder is not None:
             status = binder.launch(bound.arguments)
             if status is None:
@@ -495,7 +501,7 @@ class CompiledArtifact:
 
     def launch(self, *arguments: Any) -> None:
         """Execute with every runtime argument, including explicit Out buffers."""
-        binder = getattr(self.runtime, "binder", None)
+        binder = getattr(self.runtime, "launcher", None)
         if binder is not None:
             result = binder.launch(arguments)
             if result is not NotImplemented:

@@ -19,6 +19,7 @@ _LIBRARY: ctypes.CDLL | None = None
 _ENTRIES: dict = {}
 _SELECTION: ctypes.Array | None = None        # the switches, in the library's own memory
 _BINDER = None                                # the Binder type of the host extension; False: not built
+PLAIN: frozenset = frozenset()                # the tensor types that a native caller takes
 _PACKED: dict = {}                            # entry name -> (address, slots) of its packed form; None: it has none
 
 _CARRIERS = {"ptr": ctypes.c_void_p, "bool": ctypes.c_bool, "i8": ctypes.c_int8, "i16": ctypes.c_int16,
@@ -88,11 +89,13 @@ def selection() -> bytes:
 def _binder_type():
     """The native call path (csrc/host/binder.cpp), or False where it is not built: every call then takes the Python
     path, which does the same."""
-    global _BINDER
+    global _BINDER, PLAIN
     if _BINDER is None:
         from importlib.util import module_from_spec, spec_from_file_location
 
-        import torch  # noqa: F401  (the extension links against its libraries)
+        import torch         # (the extension links against its libraries)
+
+        PLAIN = frozenset((torch.Tensor, torch.nn.Parameter))
 
         path = Path(__file__).resolve().parent.parent / "lib" / "intent_b200_binder.so"
         _BINDER = False

@@ -206,3 +206,33 @@ def test_other_threads_run_while_an_output_is_allocated(cuda_device):
         thread.join()
         torch.cuda.empty_cache()
     assert max(progress) > 5, progress          # (the call of the entry itself gives the lock up once)
+
+
+def test_launch_with_a_workspace_does_not_ask_the_native_path(cuda_device):
+    """Such a call owns its workspace, which the native path does not make."""
+    artifact = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),
+                          constexprs={"GROUP_SIZE": 128, "ZERO_POINT": 8})
+    x, p, s = (t.to(cuda_device) for t in ib.workloads.w4a16_inputs(1, 1024, 512, dtype=torch.float16, seed=1))
+    expected = artifact.run(x, p, s)
+    assert torch.equal(artifact.run(x, p, s), expected)
+    asked = []
+
+    class Watched:
+        def __init__(self, binder):
+            self.binder = binder
+
+        def __getattr__(self, name):
+            asked.append(name)
+            return getattr(self.binder, name)
+
+    artifact.runtime.binder = Watched(artifact.runtime.binder)
+    out = torch.empty_like(expected)
+    artifact.launch(x, p, s, out)
+    assert torch.equal(out, expected) and not {"launch", "start", "learn"} & set(asked), asked
+    # nor does a call of tensors that the native path never takes teach it anything
+    class Subclass(torch.Tensor):
+        pass
+
+    asked.clear()
+    assert torch.equal(artifact.run(x.as_subclass(Subclass), p, s), expected)
+    assert not {"start", "learn"} & set(asked), asked
