@@ -256,8 +256,8 @@ class NativeProgram:
     def native_failure(self, status: int) -> None:
         native.check(status, self.entry_name, self.latest().observation(self))
 
-    def _teach(self, bound: BoundArguments, selection: bytes):
-        """The native caller (or None), told that these shapes are accepted.  Everything it learns follows from the
+    def _teach(self, bound: BoundArguments, selection: bytes, size: int):
+        """The native caller (or None), told that these shapes are accepted, with a workspace of ``size`` bytes.  Everything it learns follows from the
         shapes and the selection switches alone."""
         if not self._binder_asked:
             self._binder_asked = True
@@ -268,7 +268,6 @@ class NativeProgram:
                                             None if self._workspace_spec is None else self._stream_workspaces)
         if self.binder is None or not native.PLAIN.issuperset(map(type, bound.arguments)):
             return None                      # (it does not take subclasses)
-        size = -1 if self._workspace_spec is None else int(self._workspace_spec(bound.dimensions))
         self.binder.learn(tuple(e for f in bound.views for e in f.shape), size, self.is_empty(bound), selection)
         return self.binder
 
@@ -334,7 +333,11 @@ class NativeProgram:
     def is_empty(self, bound: BoundArguments) -> bool:
         return bool(self._empty(bound.dimensions)) if self._empty is not None else False
 
-    def allocate_workspace(self, bound: BoundArguments, *, per_stream: bool = False) -> tuple:
+    def workspace_size(self, bound: BoundArguments) -> int:
+        """Bytes of scratch of one call; -1 where the entry takes none."""
+        return -1 if self._workspace_spec is None else int(self._workspace_spec(bound.dimensions))
+
+    def allocate_workspace(self, bound: BoundArguments, *, per_stream: bool = False, size: int | None = None) -> tuple:
         """Scratch for one binding.  Entries keep their scratch zero-filled across
         launches, so it is zeroed once here.  ``per_stream`` reuses one buffer for
         successive calls on the current stream (what ``run`` does); a prepared
@@ -343,7 +346,8 @@ class NativeProgram:
 
         if self._workspace_spec is None:
             return ()
-        size = int(self._workspace_spec(bound.dimensions))
+        if size is None:
+            size = self.workspace_size(bound)
         if size <= 0:
             return (torch.empty((0,), dtype=torch.uint8, device=self._torch_device),)
         if not per_stream:
@@ -387,8 +391,9 @@ class NativeProgram:
     def run(self, *arguments):
         selection = native.selection()
         bound = self.interface.bind(tuple(arguments), device=self._torch_device)
-        workspace = self.allocate_workspace(bound, per_stream=True)
-        binder = self._teach(bound, selection)
+        size = self.workspace_size(bound)
+        workspace = self.allocate_workspace(bound, per_stream=True, size=size)
+        binder = self._teach(bound, selection, size)
         if binder is not None:
             status = binder.start(bound.arguments)
             if status is None:
@@ -402,7 +407,7 @@ class NativeProgram:
     def launch(self, *arguments) -> None:
         selection = native.selection()
         bound = self.interface.bind(tuple(arguments), device=self._torch_device, explicit_outputs=True)
-        binder = self._teach(bound, selection) if self._workspace_spec is None else None
+        binder = self._teach(bound, selection, -1) if self._workspace_spec is None else None
         if binder is not None:
             status = binder.launch(bound.arguments)
             if status is None:
