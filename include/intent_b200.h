@@ -94,8 +94,19 @@ INTENT_B200_API int intent_b200_observe_begin_selected(void* facts, const int32_
  * M == 0 or N == 0 succeed without a launch).
  * The plain entries pick the kernel from M (M = 1: the single-problem bandwidth
  * kernel; M = 2 .. 8: the ride-along kernel of the table entries below, as a table
- * of one problem; M = 9 .. 16: the bandwidth kernel; above: the tcgen05 tensor-core
- * kernel); the _gemv / _gemm entries force the bandwidth / tensor-core kernel.
+ * of one problem; M = 9 .. 16: a tcgen05 kernel that scales in f32, or the bandwidth
+ * kernel for K < 1024 or N < 128; above: the tcgen05 tensor-core kernels); the
+ * _gemv / _gemm entries force the bandwidth / tensor-core kernels.  Calls of 9 to 16
+ * rows that the bandwidth kernel has no plan for (the workspace query returns 0: M = 9
+ * with K = 14336 and N = 4096, for one) are refused, whichever kernel would run.
+ *
+ * Bits.  Every entry gives the same bits for the same call.  In the _gemm entries
+ * (and the tiled ones below) the bits of a row do not depend on what else the call
+ * holds: not on the number of rows, not on the columns beside it (a column shard has
+ * the bits of the whole), not on the layout of the weights.  The plain entries cut K
+ * into two or four parts where whole tiles would leave most of the chip idle (K > 2048
+ * and fewer than 2048 rows; which calls follows from M, N, K and the GPU), so that there
+ * the same row agrees between calls of other sizes to the rounding of f32 sums.
  *
  * workspace: device scratch of at least ..._workspace_bytes(M, K, N) bytes,
  * 16-byte aligned (NULL / 0 when that query returns 0).  It must be zero-filled

@@ -15,8 +15,8 @@ int w4a16_stream_bf16(View2, View2, View2, View2, int, int, void*, int64_t, cuda
 int64_t w4a16_stream_workspace_bytes(int64_t M, int64_t K, int64_t N);
 int w4a16_skinny_f16(View2, View2, View2, View2, int, int, void*, int64_t, cudaStream_t);
 int w4a16_skinny_bf16(View2, View2, View2, View2, int, int, void*, int64_t, cudaStream_t);
-int w4a16_gemm_f16(View2, View2, View2, View2, int, int, cudaStream_t);
-int w4a16_gemm_bf16(View2, View2, View2, View2, int, int, cudaStream_t);
+int w4a16_gemm_f16(View2, View2, View2, View2, int, int, bool, cudaStream_t);
+int w4a16_gemm_bf16(View2, View2, View2, View2, int, int, bool, cudaStream_t);
 
 // Rows of activation up to which the bandwidth kernel is used.
 constexpr int64_t kSkinnyMaxM = 16;
@@ -106,7 +106,8 @@ extern "C" const char* intent_b200_status_string(int status) {
 
 extern "C" int64_t intent_b200_launch_count(void) { return ib200::g_launches.load(std::memory_order_relaxed); }
 
-#define IB200_W4A16_ENTRY(NAME, TYPE, SELECT, TABLE)                                                              \
+// SPLIT: the tensor-core kernel may cut K into parts (a row's bits then depend on the call around it)
+#define IB200_W4A16_ENTRY(NAME, TYPE, SELECT, TABLE, SPLIT)                                               \
   extern "C" int NAME(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW2(a1), INTENT_B200_VIEW2(a2),                \
                       INTENT_B200_VIEW2(a3), int32_t group_size, int32_t zero_point, void* workspace,     \
                       int64_t workspace_bytes, void* stream) {                                            \
@@ -127,16 +128,16 @@ extern "C" int64_t intent_b200_launch_count(void) { return ib200::g_launches.loa
                                         IB200_VIEW2_ARG(a3), group_size, zero_point, workspace,           \
                                         workspace_bytes, static_cast<cudaStream_t>(stream));              \
     return ib200::w4a16_gemm_##TYPE(IB200_VIEW2_ARG(a0), IB200_VIEW2_ARG(a1), IB200_VIEW2_ARG(a2),        \
-                                    IB200_VIEW2_ARG(a3), group_size, zero_point,                          \
+                                    IB200_VIEW2_ARG(a3), group_size, zero_point, SPLIT,                   \
                                     static_cast<cudaStream_t>(stream));                                   \
   }
 
-IB200_W4A16_ENTRY(intent_b200_weight_only_int4_matmul_f16, f16, a0_d0 <= ib200::kSkinnyMaxM, a0_d0 >= 2)
-IB200_W4A16_ENTRY(intent_b200_weight_only_int4_matmul_bf16, bf16, a0_d0 <= ib200::kSkinnyMaxM, a0_d0 >= 2)
-IB200_W4A16_ENTRY(intent_b200_w4a16_gemv_f16, f16, true, false)
-IB200_W4A16_ENTRY(intent_b200_w4a16_gemv_bf16, bf16, true, false)
-IB200_W4A16_ENTRY(intent_b200_w4a16_gemm_f16, f16, false, false)
-IB200_W4A16_ENTRY(intent_b200_w4a16_gemm_bf16, bf16, false, false)
+IB200_W4A16_ENTRY(intent_b200_weight_only_int4_matmul_f16, f16, a0_d0 <= ib200::kSkinnyMaxM, a0_d0 >= 2, true)
+IB200_W4A16_ENTRY(intent_b200_weight_only_int4_matmul_bf16, bf16, a0_d0 <= ib200::kSkinnyMaxM, a0_d0 >= 2, true)
+IB200_W4A16_ENTRY(intent_b200_w4a16_gemv_f16, f16, true, false, false)
+IB200_W4A16_ENTRY(intent_b200_w4a16_gemv_bf16, bf16, true, false, false)
+IB200_W4A16_ENTRY(intent_b200_w4a16_gemm_f16, f16, false, false, false)
+IB200_W4A16_ENTRY(intent_b200_w4a16_gemm_bf16, bf16, false, false, false)
 
 extern "C" int64_t intent_b200_weight_only_int4_matmul_workspace_bytes(int64_t M, int64_t K, int64_t N) {
   if (M > ib200::kSkinnyMaxM) return 0;

@@ -633,7 +633,7 @@ int launch_gemm(const void* x, int64_t rows, int64_t K, const void* w, const voi
 // the chip: M77 K14336 N4096 is 16 tiles of 256 columns (156 us), 32 of 128 (94), 64 of 64 (86) or 128 of 32 (81);
 // M512 K2048 N4096 16 pair tiles (33.6 us), 64 of 256 columns (25.6) or 128 of 128 (19.2); M1024 K4096 N4096 32 pair
 // tiles (58.9 us) or 128 of 256 columns (50.3).  Large calls stay on the pairs (M2048 K4096 N4096 59.9 us against
-// 88.2).  All forms add the k blocks in the same order, so the bits of a row do not depend on the form.
+// 88.2).  All these forms add the k blocks in the same order, so the bits of a row do not depend on the form.
 enum class Form { PAIR, TWO_BLOCKS, N256, N128, N64, N32 };
 
 Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
@@ -672,9 +672,14 @@ Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
 // Measured against the forms above: M17 K4096 N4096 27.2 -> 9.2 us, M77 K14336 N4096 81.1 -> 18.0, M256 K8192 N1024
 // 48.8 -> 13.1, M256 K4096 N14336 52.9 -> 30.4, M512 K2048 N4096 19.8 -> 13.5, M1024 K4096 N4096 50.9 -> 30.3.
 // Calls of K < 2048 stay above: they take 8 to 16 us either way, most of it not in the k blocks.  So do unsplit calls
-// with less than a tile for every second SM.  A split changes the order of a row's sum, so that its bits depend on the
-// number of rows of the call; it is taken from K > 2048 on, where it gives a third or more.
-bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, double other, TmemCall* call, bool* pairs) {
+// with less than a tile for every second SM.  A split changes the order of a row's sum: which split a call takes follows
+// from its rows, its columns, the number of SMs and the pairs switch, so where one is allowed (the entry that chooses
+// among all kernels) a row agrees with the same row of another call, and a column shard with the whole, to rounding only.
+// Up to K = 2048 nothing is split and the bits are the same.  The entry of the tensor-core kernels and the tiled layout
+// never split and take whole tiles however few there are: M77 K4096 N4096 14.2 us against 10.8 with a split, M77 K14336
+// N4096 37.1 against 17.0, M511 K8192 N1024 23.8 against 16.4 (27.1, 81.0 and 48.7 with the weights in shared memory).
+bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split_allowed, double other, TmemCall* call,
+                 bool* pairs) {
   const int64_t sms = device_sms(), blocks = (K + 127) / 128;
   if (sms <= 0 || K < 2048 || M >= TMEM_MAX_ROWS) return false;
   double best = other;
@@ -686,12 +691,13 @@ bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, double oth
     const int64_t ctas = tiles * (pair ? 2 : split);
     double cost;
     if (split > 1) {
+      if (!split_allowed) return;
       // clusters of four do not fill every part of the chip: 33 of them were seen side by side
       if (K <= 2048 || blocks < 4 * split || ctas > (split == 2 ? sms : sms * 9 / 10)) return;
       cost = (split == 2 ? 6.2 : 6.7) + 0.014 * double(rows) +
              double((blocks + split - 1) / split) * (0.24 + 0.0014 * double(rows));
     } else {
-      if (2 * ctas < sms) return;
+      if (split_allowed && 2 * ctas < sms) return;
       const int64_t at_once = pair ? sms / 2 : sms, waves = (tiles + at_once - 1) / at_once;
       const double r = double(rows);
       const double block = !pair       ? 0.24 + 0.0014 * r
@@ -719,7 +725,7 @@ bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, double oth
 }
 
 template <typename T>
-int run(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, cudaStream_t stream,
+int run(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, bool split, cudaStream_t stream,
         bool prelaid = false) {
   const int64_t M = x.d0, K = x.d1, N = w.d1;
   if (group_size != 32 && group_size != 64 && group_size != 128) return INTENT_B200_ERR_UNSUPPORTED;
@@ -736,7 +742,7 @@ int run(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, cuda
   if (!prelaid) {
     TmemCall q{};
     bool pairs = false;
-    if (choose_tmem(M, K, N, selection().gemm_pairs != 0, time, &q, &pairs)) {
+    if (choose_tmem(M, K, N, selection().gemm_pairs != 0, split, time, &q, &pairs)) {
       q.x = x.p, q.rows = M, q.K = K;
       q.w = w.p, q.s = s.p, q.experts = 1, q.WN = N;
       q.out = y.p, q.out_cols = N;
@@ -918,11 +924,11 @@ inline bool tiled_as_experts(View2 tiled, int64_t K, int64_t WN, View3* w) {
 }  // namespace ib200
 
 namespace ib200 {
-int w4a16_gemm_f16(View2 x, View2 w, View2 s, View2 y, int g, int zp, cudaStream_t stream) {
-  return run<__half>(x, w, s, y, g, zp, stream);
+int w4a16_gemm_f16(View2 x, View2 w, View2 s, View2 y, int g, int zp, bool split, cudaStream_t stream) {
+  return run<__half>(x, w, s, y, g, zp, split, stream);
 }
-int w4a16_gemm_bf16(View2 x, View2 w, View2 s, View2 y, int g, int zp, cudaStream_t stream) {
-  return run<__nv_bfloat16>(x, w, s, y, g, zp, stream);
+int w4a16_gemm_bf16(View2 x, View2 w, View2 s, View2 y, int g, int zp, bool split, cudaStream_t stream) {
+  return run<__nv_bfloat16>(x, w, s, y, g, zp, split, stream);
 }
 int w4a16_skinny_f16(View2 x, View2 w, View2 s, View2 y, int g, int zp, void* ws, int64_t ws_bytes, cudaStream_t stream) {
   return skinny<__half>(x, w, s, y, g, zp, ws, ws_bytes, stream);
@@ -998,7 +1004,7 @@ IB200_DOWN_SCATTER_ENTRY(intent_b200_moe_grouped_w4a16_down_scatter_f16, __half)
     ib200::View2 w;                                                                                                \
     if (!ib200::tiled_as_matrix(IB200_VIEW1_ARG(a1), a0_d1, a2_d1, &w)) return INTENT_B200_ERR_SHAPE;              \
     return ib200::run<TYPE>(IB200_VIEW2_ARG(a0), w, IB200_VIEW2_ARG(a2), IB200_VIEW2_ARG(a3), group_size,          \
-                            zero_point, static_cast<cudaStream_t>(stream), true);                                  \
+                            zero_point, false, static_cast<cudaStream_t>(stream), true);                           \
   }
 IB200_TILED_GEMM_ENTRY(intent_b200_w4a16_gemm_tiled_f16, __half)
 IB200_TILED_GEMM_ENTRY(intent_b200_w4a16_gemm_tiled_bf16, __nv_bfloat16)

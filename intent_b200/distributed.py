@@ -7,6 +7,9 @@ benchmark configurations ask for.
   * Dense W4A16 prefill and W8A8 shard over output columns: rank r owns a
     contiguous block of columns of the weight (and of its scales), activations are
     replicated, every rank writes its own block of Y.  No collective on the path.
+    A shard has the bits of the whole product, except that the default W4A16 program
+    may cut K > 2048 into parts for calls of fewer than 2048 rows, by their size: there
+    they agree to rounding, and ``KERNEL='gemm'`` keeps the bits.
   * MoE is expert-parallel: rank r owns experts [r*E/g, (r+1)*E/g).  Tokens are
     routed where they live, token rows travel to the owners of their experts with
     one all-to-all, the expert FFN runs on the received rows, the f32 result rows

@@ -190,7 +190,8 @@ weight_only_int4_matmul = KernelDefinition(
                 "WEIGHT_LAYOUT": "reference", "PRELAYOUT": False},
     lower=_lower_w4a16,
     reference="examples/kernels/contraction/weight_only_int4.py:18-51",
-    summary="Y = X @ dequant(int4 packed along K, per-group scales); f32 accumulation",
+    summary="Y = X @ dequant(int4 packed along K, per-group scales); f32 accumulation (KERNEL 'gemm': the bits of a "
+            "row are those of any other call with that row; 'auto' may cut K into parts, which agree to rounding)",
 )
 
 

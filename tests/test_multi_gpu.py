@@ -1,6 +1,7 @@
 """Two-rank GPU checks (skipped on a single GPU): the expert-parallel MoE must reproduce the
 single-GPU result bit for bit (f32 rows travel, the combine order is fixed), and a column shard of
-the dense prefill must equal the same columns of the unsharded product."""
+the dense prefill must equal the same columns of the unsharded product (K = 1024 here; from K > 2048 on the default
+may cut K into parts by the shard's size, and KERNEL='gemm' keeps the bits)."""
 import os
 import socket
 

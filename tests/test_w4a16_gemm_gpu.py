@@ -148,7 +148,8 @@ def test_cta_pair_kernel_equals_single_cta_kernel(cuda_device, M, K, N):
 
 def test_host_pipeline_of_row_pieces_gives_the_whole_product(cuda_device):
     """ColumnShardedRows on one GPU: rows uploaded, multiplied and downloaded in (tapered) pieces give the bits
-    of one launch over all rows (a row's sums do not depend on which rows share its tile)."""
+    of one launch over all rows (up to K = 2048, and with KERNEL='gemm' for any K, a row's sums do not depend on which
+    rows share its call)."""
     from intent_b200.distributed import ColumnShardedRows
     M, K, N = 2048, 1024, 512
     x, p, s = ib.workloads.w4a16_inputs(M, K, N, dtype=torch.bfloat16, group_size=128, seed=4)

@@ -19,8 +19,8 @@ pytestmark = pytest.mark.gpu
     (torch.float16, 511, 1152, 2048, 128),
 ])
 def test_narrow_tiles_give_the_bits_of_the_wide_ones(cuda_device, dtype, M, K, N, group):
-    """Every tile form adds the k blocks in the same order, so a row's bits do not depend on how many rows the call
-    has (4096 rows take a wider tile, or the same one where there are only 8 or 40 columns); the tolerances against
+    """Up to K = 2048 every tile form adds the k blocks in the same order, so a row's bits do not depend on how many rows
+    the call has (longer K: test_w4a16_tmem_gpu.py; 4096 rows take a wider tile, or the same one where there are only 8 or 40 columns); the tolerances against
     the oracle are those of the wide tiles (test_w4a16_gemm_gpu.py)."""
     x, p, s = ib.workloads.w4a16_inputs(4096, K, N, dtype=dtype, group_size=group, seed=M)
     artifact = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),

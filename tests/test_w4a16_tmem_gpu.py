@@ -137,3 +137,41 @@ def test_threads_launch_one_instance(cuda_device, sizes):
     for t in threads:
         t.join()
     assert not failures, failures[:1]
+
+
+@pytest.mark.parametrize("dtype,group,K,N", [
+    (torch.bfloat16, 128, 4096, 4096),
+    (torch.float16, 64, 2112, 2056),         # half a k block at the end, eight columns in the last tile
+])
+def test_rows_of_one_kernel_keep_their_bits(cuda_device, dtype, group, K, N):
+    """KERNEL='gemm' adds the k blocks in one order whatever else a call holds: the bits of a row depend neither on the
+    number of rows, nor on the columns beside it, nor on the layout of the weights.  The default may cut K into two or four
+    parts for few rows; the same products are then added in f32 in another order, so that results agree to the rounding
+    of the output type (half a unit in the last place each: 2^-8 of the value in bf16, 2^-11 in f16; cancellation leaves
+    sums that are small against their terms, hence the root mean square beside the value)."""
+    M = 2100                                 # runs on another kernel
+    x, p, s = ib.workloads.w4a16_inputs(M, K, N, dtype=dtype, group_size=group, seed=K)
+    constants = {"GROUP_SIZE": group, "ZERO_POINT": 8, "ACT_DTYPE": "f16" if dtype == torch.float16 else "bf16"}
+    compiled = lambda **more: ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),
+                                         constexprs=dict(constants, **more))
+    auto, gemm, tiled = compiled(), compiled(KERNEL="gemm"), compiled(KERNEL="gemm", WEIGHT_LAYOUT="tiled")
+    xd, pd, sd = x.to(cuda_device), p.to(cuda_device), s.to(cuda_device)
+    whole = gemm.run(xd, pd, sd)
+    assert not gemm.observation.kernel.startswith("w4a16_tmem_kernel")
+    assert torch.equal(tiled.run(xd, prelayout.tile(pd).tensor, sd), whole)
+    half = slice(0, N // 16 * 8)
+    shard = pd[:, half].contiguous(), sd[:, half].contiguous()
+    split = 0
+    for rows in (1, 17, 32, 77, 128, 200, 511, 1300):
+        part = xd[:rows].contiguous()
+        assert torch.equal(gemm.run(part, pd, sd), whole[:rows]), rows
+        assert "split" not in gemm.observation.kernel
+        assert torch.equal(gemm.run(part, *shard), whole[:rows, half]), rows
+        if rows > 16:
+            out = auto.run(part, pd, sd).double()
+            split += "split" in auto.observation.kernel
+            scale = whole[:rows].double().abs().clamp(min=whole.double().pow(2).mean().sqrt().item())
+            assert ((out - whole[:rows].double()).abs() / scale).max() <= (2 ** -10 if dtype == torch.float16 else 2 ** -7)
+    assert split
+    torch.cuda.synchronize()
+    gemm.check()
