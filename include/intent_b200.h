@@ -138,7 +138,8 @@ INTENT_B200_API int intent_b200_w4a16_gemv_workspace_status(void* workspace, int
  * bounded device-side wait expired in an earlier launch, or INTENT_B200_ERR_INDEX if a grouped entry met an
  * expert id outside [0, E).  Synchronises the device and clears the word. */
 INTENT_B200_API int intent_b200_w4a16_gemm_device_status(void);
-/* Large dense W4A16 calls run on CTA pairs (tcgen05 cta_group::2); 0 forces the single-CTA kernel.
+/* Large dense W4A16 calls and grouped calls with many rows per expert run on CTA pairs (tcgen05 cta_group::2); 0 forces
+ * the kernels without them.
  * For measurement and tests; process-global. */
 INTENT_B200_API int intent_b200_w4a16_gemm_pairs(int32_t enable);
 /* Launch-latency overlap of the bandwidth kernel (programmatic dependent

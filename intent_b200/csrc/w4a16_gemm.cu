@@ -774,8 +774,10 @@ int run(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, bool
 }
 
 // Whether a grouped call with the weights in tensor memory runs on CTA pairs: from 64 rows per expert on average on
-// (`rows` counts 127 of padding for each expert).
-bool grouped_pairs(int64_t rows, int64_t experts) { return rows > experts * (64 + BM); }
+// (`rows` counts 127 of padding for each expert) and where pairs are allowed.
+bool grouped_pairs(int64_t rows, int64_t experts) {
+  return selection().gemm_pairs != 0 && rows > experts * (64 + BM);
+}
 
 // The kernel with the weights in tensor memory for a grouped call (sizes, layouts and alignments checked by the
 // caller); UNSUPPORTED when it does not take the call.

@@ -10,6 +10,7 @@ import intent_b200 as ib
 import oracle
 from intent_b200 import prelayout
 from intent_b200.moe import MoEW4A16FFN
+from intent_b200.runtime import native
 from conftest import max_abs_rel
 
 pytestmark = pytest.mark.gpu
@@ -175,3 +176,23 @@ def test_rows_of_one_kernel_keep_their_bits(cuda_device, dtype, group, K, N):
     assert split
     torch.cuda.synchronize()
     gemm.check()
+
+
+def test_the_pairs_switch_holds_for_grouped_calls(cuda_device):
+    """With pairs switched off the grouped contractions run on lone CTAs, with the same bits."""
+    library = native.library()
+    tokens, hidden, intermediate, experts = 1024, 512, 256, 4
+    data = ib.workloads.moe_inputs(tokens, hidden, experts, intermediate, dtype=torch.bfloat16, seed=5)
+    dev = {k: v.to(cuda_device) for k, v in data.items()}
+    layer = MoEW4A16FFN(tokens=tokens, hidden=hidden, intermediate=intermediate, experts=experts, target=ib.B200Target(0))
+    ids, weights = layer.route(dev["logits"])
+    args = (dev["x"], ids, weights, dev["up_gate_packed"], dev["up_gate_scales"], dev["down_packed"], dev["down_scales"])
+    paired = layer(*args)
+    assert layer.down_scatter.observation.kernel.startswith(PAIRS)
+    try:
+        assert library.intent_b200_w4a16_gemm_pairs(0) == 0
+        single = layer(*args)
+        assert layer.down_scatter.observation.kernel.startswith(LONE)
+    finally:
+        library.intent_b200_w4a16_gemm_pairs(1)
+    assert torch.equal(single, paired)
