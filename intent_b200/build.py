@@ -1,4 +1,4 @@
-"""In-tree build of ``libintent_b200.so`` (sm_100a only) and of the host extension ``intent_b200_binder.so``.
+"""In-tree build of ``libintent_b200.so`` (sm_100a only) and of the host extension ``intent_b200_binder-*.so``.
 
 ``python -m intent_b200.build`` compiles every ``csrc/*.cu`` with nvcc and links
 one shared library under ``intent_b200/lib/``, and ``csrc/host/binder.cpp`` against torch.  Nothing is JIT-compiled at run
@@ -18,7 +18,6 @@ CSRC = ROOT / "csrc"
 OBJ = CSRC / "build"
 LIB = ROOT / "lib" / "libintent_b200.so"
 BINDER_SOURCE = CSRC / "host" / "binder.cpp"
-BINDER = ROOT / "lib" / "intent_b200_binder.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -95,20 +94,23 @@ def build_binder(force: bool = False) -> Path:
 
     import torch
 
-    if not force and not _stale(BINDER, [BINDER_SOURCE]):
-        return BINDER
+    from .runtime.native import binder_path
+
+    target = binder_path()
+    if not force and not _stale(target, [BINDER_SOURCE]):
+        return target
     root = Path(torch.__file__).resolve().parent
     include = root / "include"
     command = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
                f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
                f"-I{include}", f"-I{include / 'torch' / 'csrc' / 'api' / 'include'}",
                f"-I{sysconfig.get_paths()['include']}", f"-I{Path(_nvcc()).resolve().parent.parent / 'include'}",
-               str(BINDER_SOURCE), "-o", str(BINDER), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
+               str(BINDER_SOURCE), "-o", str(target), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
                "-lc10", "-lc10_cuda"]
     done = subprocess.run(command, capture_output=True, text=True)
     if done.returncode != 0:
         raise RuntimeError(f"the host extension does not build:\n{done.stdout}\n{done.stderr}")
-    return BINDER
+    return target
 
 
 if __name__ == "__main__":

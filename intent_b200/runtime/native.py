@@ -18,6 +18,7 @@ _LOCK = Lock()
 _LIBRARY: ctypes.CDLL | None = None
 _ENTRIES: dict = {}
 _SELECTION: ctypes.Array | None = None        # the switches, in the library's own memory
+_LIB = Path(__file__).resolve().parent.parent / "lib"
 _BINDER = None                                # the Binder type of the host extension; False: not built
 PLAIN: frozenset = frozenset()                # the tensor types that a native caller takes
 _PACKED: dict = {}                            # entry name -> (address, slots) of its packed form; None: it has none
@@ -86,9 +87,21 @@ def selection() -> bytes:
     return _SELECTION.raw
 
 
+def binder_path() -> Path:
+    """Where the host extension for this interpreter and this torch lies: it is compiled against internals of both
+    (dispatch keys, the layout of tensor objects), so one that was built for others must not be loaded."""
+    import sysconfig
+
+    import torch
+
+    key = (torch.__version__, str(torch.version.git_version)[:8], f"abi{int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           sysconfig.get_config_var("SOABI"))
+    return _LIB / ("intent_b200_binder-" + "-".join(key) + ".so")
+
+
 def _binder_type():
-    """The native call path (csrc/host/binder.cpp), or False where it is not built: every call then takes the Python
-    path, which does the same."""
+    """The native call path (csrc/host/binder.cpp), or False where it is not built for this interpreter and this torch:
+    every call then takes the Python path, which does the same."""
     global _BINDER, PLAIN
     if _BINDER is None:
         from importlib.util import module_from_spec, spec_from_file_location
@@ -97,7 +110,7 @@ def _binder_type():
 
         PLAIN = frozenset((torch.Tensor, torch.nn.Parameter))
 
-        path = Path(__file__).resolve().parent.parent / "lib" / "intent_b200_binder.so"
+        path = binder_path()
         _BINDER = False
         if path.exists():
             spec = spec_from_file_location("intent_b200_binder", path)
@@ -107,6 +120,11 @@ def _binder_type():
             except ImportError as error:
                 raise CompilationStageError("native_loading", f"cannot load {path}: {error}") from error
             _BINDER = module.Binder
+        elif any(_LIB.glob("intent_b200_binder*.so")):
+            import warnings
+
+            warnings.warn(f"the native call path was built for another torch or Python ({path.name} is not there): calls "
+                          "take the Python path; `python -m intent_b200.build` builds it", RuntimeWarning, stacklevel=2)
     return _BINDER
 
 

@@ -213,3 +213,23 @@ def test_torch_operator_schema_and_fake_inference_without_a_device():
     for bad in ("no_namespace", "a::b::c", "9a::b", "a::"):
         with pytest.raises(ValueError):
             artifact.as_torch_op(bad)
+
+
+def test_the_host_extension_is_of_this_torch(monkeypatch, tmp_path):
+    """It is compiled against internals of torch and Python: after a change of either the old file is neither loaded nor
+    taken for up to date, and calls go on through Python."""
+    from intent_b200 import build
+    from intent_b200.runtime import native
+
+    monkeypatch.setattr(native, "_LIB", tmp_path)
+    monkeypatch.setattr(native, "_BINDER", None)
+    built = native.binder_path()
+    built.write_bytes(b"not a library")
+    assert not build._stale(built, [])
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    assert native.binder_path() != built and build._stale(native.binder_path(), [])
+    with pytest.warns(RuntimeWarning, match="another torch"):
+        assert native._binder_type() is False
+    built.unlink()
+    monkeypatch.setattr(native, "_BINDER", None)
+    assert native._binder_type() is False            # not built at all: nothing to say
