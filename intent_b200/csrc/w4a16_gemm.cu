@@ -598,9 +598,10 @@ int launch_gemm(const void* x, int64_t rows, int64_t K, const void* w, const voi
   p.top_k = top_k;
   // Few rows per expert (at most 64 on average, `rows` counting 127 of padding for each, as blocks of 128 rows have
   // it; blocks of 256 pad by more and never ask): the weights come from HBM and three k blocks in flight do not cover
-  // its latency, so the L2 is asked eight blocks early.  64 tokens on 64 experts of 4096 x 1408, the two contractions
-  // timed apart and in a row of their own: 339 + 146 -> 307 + 135 us.  With many rows most of the weights are in the
-  // L2 already and the extra instructions cost 1 % (848 + 504 -> 858 + 508 us at 16384 tokens).
+  // its latency, so the L2 is asked eight blocks early.  Such calls come here with more than 1024 row blocks only (the
+  // kernel with the weights in tensor memory takes the others), which means 683 experts or more: 512, 4096 and 16384
+  // tokens on 1040 experts of 1024 x 512, up|gate 567 -> 558, 943 -> 925 and 946 -> 932 us, down and 64 tokens the same.
+  // With many rows most of the weights are in the L2 already and the extra instructions cost 1 %.
   p.ahead = MODE != MODE_DENSE && !prelaid && rows <= experts * (64 + BM) ? 8 : 0;
 
   CUtensorMap map_x;
@@ -780,7 +781,8 @@ bool grouped_pairs(int64_t rows, int64_t experts) {
 }
 
 // The kernel with the weights in tensor memory for a grouped call (sizes, layouts and alignments checked by the
-// caller); UNSUPPORTED when it does not take the call.
+// caller); UNSUPPORTED when it does not take the call: more than 1024 blocks of 128 rows, for which its list of blocks
+// has no room.
 template <typename T>
 int grouped_tmem(int mode, View2 x, View1 tile_expert, View1 total, View3 w, View3 s, void* out, int64_t out_cols,
                  int group_size, int zero_point, int block_rows, const int* row_route, const float* route_weight,

@@ -196,3 +196,25 @@ def test_the_pairs_switch_holds_for_grouped_calls(cuda_device):
     finally:
         library.intent_b200_w4a16_gemm_pairs(1)
     assert torch.equal(single, paired)
+
+
+def test_more_row_blocks_than_the_kernel_lists(cuda_device):
+    """Above 1024 blocks of 128 rows a grouped call runs on the kernel with the weights in shared memory, here with a row
+    or none for each of many experts; the rows of padding hold whatever was there before."""
+    tokens, hidden, intermediate, experts = 96, 384, 128, 1040
+    data = ib.workloads.moe_inputs(tokens, hidden, experts, intermediate, dtype=torch.bfloat16, seed=7)
+    dev = {k: v.to(cuda_device) for k, v in data.items()}
+    sizes = dict(tokens=tokens, hidden=hidden, intermediate=intermediate, experts=experts, target=ib.B200Target(0))
+    plain, tiled = MoEW4A16FFN(**sizes), MoEW4A16FFN(prelayout=True, **sizes)
+    ids, weights = plain.route(dev["logits"])
+    args = (dev["x"], ids, weights, dev["up_gate_packed"], dev["up_gate_scales"], dev["down_packed"], dev["down_scales"])
+    stale = torch.full((1 << 26,), float("nan"), dtype=torch.bfloat16, device=cuda_device)
+    del stale                                    # the rows and the hidden rows of the call come from this block
+    y = plain(*args)
+    assert plain.down_scatter.observation.kernel.startswith("w4a16_gemm_kernel")
+    assert torch.equal(y, tiled(*args))
+    torch.cuda.synchronize()
+    plain.down_scatter.check()
+    ref = oracle.moe_w4a16_swiglu_ffn(data["x"], ids.cpu(), weights.cpu(), data["up_gate_packed"], data["up_gate_scales"],
+                                      data["down_packed"], data["down_scales"])
+    assert max_abs_rel(y.cpu(), ref) <= 2e-2
