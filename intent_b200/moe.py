@@ -177,6 +177,11 @@ class MoEW4A16FFN:
         else:
             self._chain = (self.gather, self.up_gate)
 
+    @property
+    def chain(self):
+        """The programs that a call runs after the alignment, in order."""
+        return (*self._chain, self.down_scatter) if self.fused_combine else (self.gather, self.up_gate, self.down, self.combine)
+
     # What only the other chains use is bound at its first use.
     @cached_property
     def positions(self):
@@ -184,11 +189,19 @@ class MoEW4A16FFN:
 
     @cached_property
     def gather(self):
-        return self._bind(programs.moe_gather_rows, self._gathered)
+        """All rows with zeros for the padding.  A call may run another program in its place (``chain``), which its
+        observation then describes until it is called itself."""
+        return self._in_place_of(0, self._bind(programs.moe_gather_rows, self._gathered))
 
     @cached_property
     def up_gate(self):
-        return self._bind(programs.moe_grouped_upgate_silu, self._grouped)
+        """All rows, those of the padding among them; beside ``chain`` as :attr:`gather`."""
+        return self._in_place_of(1, self._bind(programs.moe_grouped_upgate_silu, self._grouped))
+
+    def _in_place_of(self, step, artifact):
+        if self._routed:
+            artifact.runtime.stand_in = self._chain[step].runtime
+        return artifact
 
     @cached_property
     def down(self):

@@ -211,6 +211,7 @@ class NativeProgram:
         self._workspace_count = None
         self.binder = None                   # native caller, from the first accepted call on (native.binder)
         self._binder_asked = False
+        self.stand_in: NativeProgram | None = None   # runs in this program's place; observed until this one runs itself
 
     # ---- C entry -----------------------------------------------------------------
     def function(self, workspace_count: int | None = None):
@@ -225,7 +226,9 @@ class NativeProgram:
     @property
     def observation(self):
         launched = self.latest()
-        return None if launched is None else launched.observation(self)
+        if launched is None:
+            return None if self.stand_in is None else self.stand_in.observation
+        return launched.observation(self)
 
     # ---- native call path ----------------------------------------------------------
     @property

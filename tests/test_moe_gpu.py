@@ -234,3 +234,24 @@ def test_host_pipelined_ffn_gives_the_whole_batch_bits(cuda_device):
         piped.run(logits[:100], x[:100], out[:100])
     with pytest.raises(ValueError):
         HostPipelinedFFN(tokens=510, hidden=hidden, intermediate=intermediate, experts=experts, chunks=4)
+
+
+@pytest.mark.parametrize("prelayout", [False, True])
+def test_a_layer_says_what_a_call_ran(cuda_device, prelayout):
+    """``chain`` holds the programs of a call; ``gather`` and ``up_gate``, which take all rows, describe the call of the
+    program that ran in their place until they are called themselves."""
+    tokens, hidden, intermediate, experts = 64, 256, 128, 4
+    data = ib.workloads.moe_inputs(tokens, hidden, experts, intermediate, dtype=torch.bfloat16, seed=6)
+    dev = {k: v.to(cuda_device) for k, v in data.items()}
+    layer = MoEW4A16FFN(tokens=tokens, hidden=hidden, intermediate=intermediate, experts=experts, target=ib.B200Target(0),
+                        prelayout=prelayout)
+    ids, weights = layer.route(dev["logits"])
+    layer(dev["x"], ids, weights, dev["up_gate_packed"], dev["up_gate_scales"], dev["down_packed"], dev["down_scales"])
+    assert [p.observation.status for p in layer.chain] == [0, 0, 0]
+    assert layer.chain[2] is layer.down_scatter
+    for step, program in zip(layer.chain, (layer.gather, layer.up_gate)):
+        seen, ran = program.observation, step.observation
+        assert seen.status == 0 and (seen.entry, seen.arguments) == (ran.entry, ran.arguments)
+    sorted_routes, _, total = layer.alignment.run(ids)
+    layer.gather.run(dev["x"], sorted_routes, total)
+    assert layer.gather.observation.entry == "intent_b200_moe_gather_rows"

@@ -93,7 +93,7 @@ def test_routed_rows(cuda_device, rows_of_expert, hidden, intermediate, block):
             dev["down_packed"], dev["down_scales"])
     plain, tiled = MoEW4A16FFN(**sizes), MoEW4A16FFN(prelayout=True, **sizes)
     y = plain(*args)
-    assert plain._chain[1].observation.kernel.startswith("w4a16_tmem_kernel")
+    assert plain.chain[1].observation.kernel.startswith("w4a16_tmem_kernel")
     torch.cuda.synchronize()
     plain.down_scatter.check()
     assert torch.equal(y, tiled(*args))
