@@ -21,7 +21,16 @@ def test_router_top2_bit_exact(cuda_device):
     ref_ids, ref_weights = oracle.moe_route_top2(logits)
     assert ids.dtype == torch.int32 and torch.equal(ids.cpu(), ref_ids)
     assert ids[5].tolist() == [7, 40] and ids[9].tolist() == [0, 1]
-    assert torch.allclose(weights.cpu(), ref_weights, rtol=2e-6, atol=0)
+    weights = weights.cpu()
+    if not torch.allclose(weights, ref_weights, rtol=2e-6, atol=0):
+        # which rows, and which side is off: both lie within 3e-7 of 64 bits where they are sound
+        exact = torch.softmax(logits.double(), dim=1).gather(1, ref_ids.long())
+        away = ((weights - ref_weights).abs() / ref_weights).amax(dim=1)
+        rows = away.argsort(descending=True)[:4].tolist()
+        again = router.run(logits.to(cuda_device))[1].cpu()
+        pytest.fail(f"{int((away > 2e-6).sum())} rows differ; the worst (row, kernel, oracle, 64 bits, kernel once more): " +
+                    "; ".join(f"{r} {weights[r].tolist()} {ref_weights[r].tolist()} {exact[r].tolist()} {again[r].tolist()}"
+                              for r in rows))
     g = load_golden("insertion_top_k")                                           # reference golden, k = 8 -> first two
     ids, _ = router.run(g["logits"].to(cuda_device))
     assert torch.equal(ids.cpu(), g["indices"][:, :2])
