@@ -213,3 +213,22 @@ def test_errors_and_edges_on_device(cuda_device):
     with pytest.raises(ib.CompilationStageError) as info:
         artifact.run(x2.to(cuda_device), p2.to(cuda_device), s2.to(cuda_device))
     assert info.value.stage == "provider_invocation" and info.value.status == 3
+
+
+@pytest.mark.parametrize("kernel,rows", [("auto", (1, 4, 1, 12, 8, 2)), ("gemv", (1, 16, 5, 1, 9))])
+def test_one_workspace_serves_every_shape(cuda_device, kernel, rows):
+    """A launch leaves its scratch zero-filled, so that the next one on it may have another shape or run on another kernel:
+    a program's calls on one stream share one buffer.  The results are those of programs of their own."""
+    constants = {"GROUP_SIZE": 128, "ZERO_POINT": 8, "KERNEL": kernel}
+    compiled = lambda: ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0), constexprs=constants)
+    shared = compiled()
+    for K, N in ((4096, 1024), (2176, 2176), (1024, 4096), (4096, 4104)):
+        for M in rows:
+            x, p, s = (t.to(cuda_device) for t in ib.workloads.w4a16_inputs(M, K, N, dtype=torch.float16, seed=M + K))
+            expected = compiled().run(x, p, s)
+            out = shared.run(x, p, s)
+            torch.cuda.synchronize()
+            (buffer,) = shared.runtime._stream_workspaces.values()
+            assert not buffer.any(), (M, K, N, shared.observation.kernel)
+            assert torch.equal(out, expected), (M, K, N)
+    shared.check()
