@@ -218,3 +218,36 @@ def test_more_row_blocks_than_the_kernel_lists(cuda_device):
     ref = oracle.moe_w4a16_swiglu_ffn(data["x"], ids.cpu(), weights.cpu(), data["up_gate_packed"], data["up_gate_scales"],
                                       data["down_packed"], data["down_scales"])
     assert max_abs_rel(y.cpu(), ref) <= 2e-2
+
+
+def test_dependent_calls_without_synchronisation(cuda_device):
+    """Programmatic launches: a call starts while the one before it is still running, and must see what that one wrote -
+    activations from another kernel of this library, and weights that were copied just before.  Twelve rows, four, one and
+    77 by turns; the same chain with a synchronisation after every step gives the expected bits."""
+    width, steps = 2176, 48
+    artifact = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),
+                          constexprs={"GROUP_SIZE": 128, "ZERO_POINT": 8, "ACT_DTYPE": "bf16"})
+    x, p, s = ib.workloads.w4a16_inputs(77, width, width, dtype=torch.bfloat16, seed=8)
+    others = [ib.workloads.w4a16_inputs(1, width, width, dtype=torch.bfloat16, seed=9 + i)[1].to(cuda_device) for i in (0, 1)]
+    xd, sd = x.to(cuda_device), s.to(cuda_device)
+    kernels = set()
+
+    def chain(synchronise):
+        weight, state = others[0].clone(), xd.clone()
+        for step in range(steps):
+            rows = (12, 4, 1, 77)[step % 4]
+            weight.copy_(others[step % 2])
+            out = artifact.run(state[:rows], weight, sd)
+            if synchronise:
+                torch.cuda.synchronize()
+                kernels.add(artifact.observation.kernel.split(",")[0])
+            state = torch.cat((out, state[rows:]))
+            if rows == 77:       # and one call straight after another
+                state = artifact.run(artifact.run(state[:16], weight, sd), weight, sd).repeat(5, 1)[:77]
+            state = state / state.abs().amax(dim=1, keepdim=True)
+        return state
+
+    expected = chain(True)
+    assert torch.isfinite(expected).all() and len(kernels) == 4, kernels
+    for _ in range(10):
+        assert torch.equal(chain(False), expected)
