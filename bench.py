@@ -1007,7 +1007,7 @@ def run_moe(args, rank: int, world: int, device):
                                      "profiles/moe_step_launch_list.md, not one figure",
                      "peak_source": peaks["source"] + " (burst cuBLAS bf16); whole step, not one kernel",
                      "frac_of_sustained": round(achieved / peaks["bf16_tflops_sustained"], 4),
-                     "kernel": "w4a16_gemm_kernel (grouped modes)"},
+                     "kernel": ("w4a16_gemm_kernel" if args.prelayout else "w4a16_tmem_kernel") + " (grouped modes)"},
         "kernels": split,
         "e2e": {"value": round(flops / (e2e_s / e2e_steps) / 1e12, 2), "unit": "TFLOP/s",
                 "h2d_bytes_per_step": t_local * (64 * 4 + hidden * 2), "d2h_bytes_per_step": t_local * hidden * 4,

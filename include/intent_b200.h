@@ -134,7 +134,7 @@ INTENT_B200_API int64_t intent_b200_w4a16_gemv_workspace_bytes(int64_t M, int64_
  * INTENT_B200_ERR_TIMEOUT) and, when it is set, zero-fills the workspace again so that it can be reused.
  * Call it wherever the host synchronises anyway (end of a decode step, before results are consumed). */
 INTENT_B200_API int intent_b200_w4a16_gemv_workspace_status(void* workspace, int64_t workspace_bytes, void* stream);
-/* Status word of the tensor-core W4A16 kernels (single-CTA and CTA-pair): 0, INTENT_B200_ERR_TIMEOUT if a
+/* Status word of the tensor-core W4A16 kernels (single-CTA, CTA-pair, weights in tensor memory): 0, INTENT_B200_ERR_TIMEOUT if a
  * bounded device-side wait expired in an earlier launch, or INTENT_B200_ERR_INDEX if a grouped entry met an
  * expert id outside [0, E).  Synchronises the device and clears the word. */
 INTENT_B200_API int intent_b200_w4a16_gemm_device_status(void);
@@ -146,7 +146,8 @@ INTENT_B200_API int intent_b200_w4a16_gemm_pairs(int32_t enable);
  * launch).  When enabled, a launch may start and request its packed weights
  * while the kernel before it on the stream is still running; it waits for that
  * kernel before it reads the activations or writes the output.  Only enable it when the packed weights are not written by the kernel
- * launched immediately before (they are static model state in a decode loop).
+ * launched immediately before, nor by one ahead of a row of W4A16 launches of this library that come before: those may
+ * still be under way themselves (the weights are static model state in a decode loop).
  * Process-global; off by default. */
 INTENT_B200_API int intent_b200_w4a16_gemv_overlap(int32_t enable);
 /* Number of CTAs of the bandwidth kernel (0 = one per SM).  For measurement

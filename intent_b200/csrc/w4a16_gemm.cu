@@ -35,7 +35,8 @@
 // Every wait is bounded; a wait that gives up records INTENT_B200_ERR_TIMEOUT and the CTA drains
 // and frees its TMEM.
 //
-// The same kernel serves the MoE grouped contractions (reference programs
+// The same kernel serves the MoE grouped contractions on tiled weights and above 1024 row blocks (the others run on
+// w4a16_tmem.cu; reference programs
 // examples/kernels/ragged/grouped_gemm.py:11-70 and examples/kernels/ragged/moe.py:12-53 with
 // int4 expert weights): rows are sorted by expert and padded to 128 per expert, so a 128-row
 // block belongs to one expert, read from the block -> expert table of the route alignment; the
@@ -672,8 +673,14 @@ Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
 //   CTA pair of r rows x 256 columns          5 + 0.012 r + waves * blocks * (0.405 at 128 rows, 0.52 at 192, 0.735 at 256)
 // Measured against the forms above: M17 K4096 N4096 27.2 -> 9.2 us, M77 K14336 N4096 81.1 -> 18.0, M256 K8192 N1024
 // 48.8 -> 13.1, M256 K4096 N14336 52.9 -> 30.4, M512 K2048 N4096 19.8 -> 13.5, M1024 K4096 N4096 50.9 -> 30.3.
-// Calls of K < 2048 stay above: they take 8 to 16 us either way, most of it not in the k blocks.  So do unsplit calls
-// with less than a tile for every second SM.  A split changes the order of a row's sum: which split a call takes follows
+// Four lines stand outside the estimate.  The fit covers K >= 2048 and fewer than 2048 rows, and tests of the forms above
+// ask for them by sizes beyond that.  With the lines taken out, graph replay, this kernel against the form that runs:
+//   K < 2048    M17 K1024 N1024 6.7 of 9.6 us, M300 K1536 N2048 8.5 of 13.9, M512 K1920 N4096 15.1 of 24.1; but M1024 K1024
+//               N8192 26.2 of 23.0, M1900 K1024 N4096 26.4 of 22.9
+//   M >= 2048   M2500 K8192 N1024 33.2 of 85.7, M4096 K4096 N1024 31.2 of 47.1, M2500 K4096 N8192 130.9 of 159; but M2048
+//               K4096 N4096 60.8 of 53.7, M4096 K4096 N4096 120.8 of 117.7, 8192 cubed 917 of 921
+//   no split up to K = 2048 (there a row keeps its bits, see below)   M32 K2048 N2048 9.7 of 20.3, M77 K2048 N4104 14.2 of 20.8
+// and, where a split is allowed, unsplit calls with less than a tile for every second SM.  A split changes the order of a row's sum: which split a call takes follows
 // from its rows, its columns, the number of SMs and the pairs switch, so where one is allowed (the entry that chooses
 // among all kernels) a row agrees with the same row of another call, and a column shard with the whole, to rounding only.
 // Up to K = 2048 nothing is split and the bits are the same.  The entry of the tensor-core kernels and the tiled layout
@@ -775,6 +782,9 @@ int run(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, bool
 }
 
 // Whether a grouped call with the weights in tensor memory runs on CTA pairs: from 64 rows per expert on average on
+// (4096 x 1408, up|gate + down: 64 experts 146 + 78 us on lone CTAs, 133 + 76 on pairs, 8 experts 47 + 22 and 47 + 24; at
+// 256 rows 363 + 225 and 348 + 217.  Below the line pairs are ahead too where there are many experts, 125 + 66 and 118 + 64
+// at 16 rows, but not with few, 43 + 20 and 43 + 21 at 32.)
 // (`rows` counts 127 of padding for each expert) and where pairs are allowed.
 bool grouped_pairs(int64_t rows, int64_t experts) {
   return selection().gemm_pairs != 0 && rows > experts * (64 + BM);

@@ -127,7 +127,10 @@ class PrelayoutProgram:
     reference's, but the weights are taken to be static model state.  Calls with more than 16 activation rows
     run on a tiled copy of the weight that is made the first time a weight tensor is seen and kept in a
     :class:`intent_b200.prelayout.PrelayoutCache`; calls with at most 16 rows go to the bandwidth kernel, which
-    reads the reference layout directly."""
+    reads the reference layout directly.
+
+    Measured, it does not pay: the tiled copy keeps a call off the kernel with the weights in tensor memory (bf16, group
+    128: M77 K14336 N4096 80 us against 17, M1024 K4096 N4096 50 against 31, 8192 cubed 893 against 883)."""
 
     SKINNY_ROWS = 16
 
