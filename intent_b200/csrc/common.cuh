@@ -142,6 +142,11 @@ struct Elem<__half> {
   __device__ static __forceinline__ uint16_t from_float(float v) {
     return __half_as_ushort(__float2half_rn(v));
   }
+  __device__ static __forceinline__ uint32_t pack2(float low, float high) {
+    uint32_t d;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(high), "f"(low));
+    return d;
+  }
   __device__ static __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                                   uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -172,6 +177,11 @@ struct Elem<__nv_bfloat16> {
   }
   __device__ static __forceinline__ uint16_t from_float(float v) {
     return __bfloat16_as_ushort(__float2bfloat16_rn(v));
+  }
+  __device__ static __forceinline__ uint32_t pack2(float low, float high) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(high), "f"(low));
+    return d;
   }
   __device__ static __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                                   uint32_t a3, uint32_t b0, uint32_t b1) {

@@ -143,6 +143,16 @@ __device__ __forceinline__ uint32_t lds16(uint32_t addr) {
   return v;
 }
 
+// Four neighbouring lanes hold a column each, with rows 0 and 1 in `low` and rows 2 and 3 in `high`: each gets row
+// `lane & 3` of the four columns.
+__device__ __forceinline__ uint2 swap_rows(uint32_t low, uint32_t high, int lane) {
+  const bool odd = lane & 1, upper = lane & 2;
+  const uint32_t got = __shfl_xor_sync(0xffffffffu, prmt(low, high, odd ? 0x5410 : 0x7632), 1);
+  const uint32_t a = prmt(low, got, odd ? 0x3254 : 0x5410), b = prmt(high, got, odd ? 0x3276 : 0x7610);
+  const uint32_t other = __shfl_xor_sync(0xffffffffu, upper ? a : b, 2);
+  return upper ? make_uint2(other, b) : make_uint2(a, other);
+}
+
 template <typename T, int MODE, int CG>
 __global__ void __launch_bounds__(THREADS, 1)
 w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
@@ -150,7 +160,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   extern __shared__ unsigned char smem_raw[];
   // Programmatic launch: a CTA of the next such launch may set itself up on an SM that this one has left, and this launch
   // touches no global memory before everything ahead of it in the stream has completed.  One call after another:
-  // M16 K4096 N4096 10.3 -> 8.4 us, M77 K14336 N4096 19.1 -> 17.4, M512 K2048 N4096 14.4 -> 13.0.
+  // M16 K4096 N4096 10.3 -> 8.4 us, M77 K14336 N4096 19.1 -> 17.4, M512 K2048 N4096 14.4 -> 13.0 (each as it was then).
   asm volatile("griddepcontrol.launch_dependents;");
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -530,15 +540,21 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       }
     }
     if (!ok && lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
-  } else if (warp >= FIRST_EPILOGUE) {
+  }
+  if (MODE != MODE_SKINNY && warp >= FIRST_EPILOGUE && (p.split == 1 || warp < FIRST_DEQUANT) && items > first_item) {
     // ------------------------------ epilogue -----------------------------------
-    const int quadrant = warp & 3;
+    // The dequantisers, whose work is done by then, take four fifths of the last tile: nothing is left to overlap it with.
+    // Bound by the stores: two bytes a lane and four warps took 4 of the 13 us of a call of M512 K2048 N4096 (a tile a
+    // CTA); eight bytes a lane and twenty warps, 13.06 -> 10.77 us.
+    const int quadrant = warp & 3, last = (items - 1 - first_item) / item_step;
+    const int share = warp >= FIRST_DEQUANT ? 1 + ((warp - FIRST_DEQUANT) >> 2) : 0;
     uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
     float* yf = reinterpret_cast<float*>(p.y);
-    uint32_t local = 0;
-    for (int item = first_item; item < items; item += item_step, ++local) {
+    constexpr int CHUNK = MODE == MODE_UPGATE_SILU ? 16 : 32;   // rows at a time
+    for (int local = share ? last : 0; local <= last; ++local) {
+      const int item = first_item + local * item_step;
       const Item t = item_of(item);
-      const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = p.acc_sets == 2 ? local >> 1 : local;
+      const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = uint32_t(p.acc_sets == 2 ? local >> 1 : local);
       if (!mbar_wait_warp(tmem_full + 8 * acc, use & 1)) {
         if (lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
         break;
@@ -547,7 +563,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + acc * (ACC_COLUMNS / 2) + (uint32_t(quadrant * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < t.rows; c += MODE == MODE_UPGATE_SILU ? 16 : 32) {
+      for (int c = share * CHUNK; c < t.rows; c += local == last ? (1 + SETS) * CHUNK : CHUNK) {
         // Predicated, not branched: a branch a row keeps the work of different rows apart, and the epilogue of a tile with
         // few k blocks then takes longer than its MMAs (16384 tokens on 64 experts of 4096 x 1408: up|gate 807 -> 640 us).
         if (MODE == MODE_UPGATE_SILU) {
@@ -557,13 +573,18 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           uint32_t v[16];
           tmem_load_32x16(taddr + c, v);
           tmem_load_wait();
+          float h[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const uint32_t got = __shfl_xor_sync(0xffffffffu, is_up ? v[i] : v[8 + i], 16);
             const float gv = __uint_as_float(is_up ? got : v[i]), uv = __uint_as_float(is_up ? v[8 + i] : got);
-            const int r = c + i + (is_up ? 8 : 0);
-            const float h = gv * __frcp_rn(1.0f + __expf(-gv)) * uv;  // silu(gate) * up in f32, one rounding
-            if (r < t.rows) y[size_t(t.row0 + r) * p.out_cols + col] = Elem<T>::from_float(h);
+            h[i] = gv * __frcp_rn(1.0f + __expf(-gv)) * uv;  // silu(gate) * up in f32, one rounding
+          }
+#pragma unroll
+          for (int i = 0; i < 8; i += 4) {
+            const uint2 four = swap_rows(Elem<T>::pack2(h[i], h[i + 1]), Elem<T>::pack2(h[i + 2], h[i + 3]), lane);
+            const int r = c + i + (lane & 3) + (is_up ? 8 : 0);
+            if (r < t.rows) *reinterpret_cast<uint2*>(y + size_t(t.row0 + r) * p.out_cols + (col & ~3)) = four;
           }
         } else {
           const int col = (t.n_tile * CG + (CG == 2 ? rank : 0)) * COLS + quadrant * 32 + lane;
@@ -609,14 +630,18 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           } else {
             tmem_load_wait();
             const int left = col < p.out_cols ? t.rows - c : 0;
-            size_t at = size_t(t.row0 + c) * p.out_cols + col;
+            if (MODE == MODE_GROUPED_F32) {
+              size_t at = size_t(t.row0 + c) * p.out_cols + col;
 #pragma unroll
-            for (int i = 0; i < 32; ++i, at += p.out_cols) {
-              if (MODE == MODE_GROUPED_F32) {
+              for (int i = 0; i < 32; ++i, at += p.out_cols)
                 if (i < left) yf[at] = __uint_as_float(v[i]);
-              } else {
-                const uint16_t value = Elem<T>::from_float(__uint_as_float(v[i]));
-                if (i < left) y[at] = value;
+            } else {
+              uint16_t* to = y + size_t(t.row0 + c + (lane & 3)) * p.out_cols + (col & ~3);
+#pragma unroll
+              for (int i = 0; i < 32; i += 4, to += 4 * size_t(p.out_cols)) {
+                const uint2 four = swap_rows(Elem<T>::pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
+                                             Elem<T>::pack2(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), lane);
+                if (i + (lane & 3) < left) *reinterpret_cast<uint2*>(to) = four;
               }
             }
           }
@@ -624,7 +649,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       }
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) {
+      if (lane == 0 && local < last) {
         if (CG == 2) mbar_arrive_remote(map_to_rank(tmem_empty + 8 * acc, 0));
         else mbar_arrive(tmem_empty + 8 * acc);
       }

@@ -25,6 +25,7 @@ LONE, PAIRS, SPLIT = ("w4a16_tmem_kernel " + s for s in ("single CTA", "CTA pair
     (torch.float16, "twos_complement", 64, 512, 2048, 4096, LONE),
     (torch.bfloat16, 8, 128, 511, 8192, 8200, PAIRS),                  # 256-row tiles, one accumulator
     (torch.float16, 8, 128, 1030, 4096, 4104, PAIRS),                  # 128-row tiles, eight columns in the last tile
+    (torch.bfloat16, 8, 128, 35, 2048, 19208, LONE),                   # more tiles than SMs, three rows past a chunk of 32
 ])
 def test_dense_tiles(cuda_device, dtype, zero_point, group, M, K, N, kernel):
     x, p, s = ib.workloads.w4a16_inputs(M, K, N, dtype=dtype, group_size=group, seed=M)
