@@ -17,6 +17,9 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// its two halves: everything before the first in all threads of the cluster comes before what follows the second
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // shared::cluster address of the same shared-memory offset in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
   uint32_t remote;
@@ -31,6 +34,21 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 // release above makes the thread wait about a microsecond for its earlier accesses.)
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// mbar_wait_warp (tma.cuh) for a barrier whose phase completes by what other CTAs of the cluster wrote
+__device__ __forceinline__ bool mbar_wait_warp_cluster(uint32_t bar, uint32_t parity, uint32_t limit = 1u << 16) {
+  for (uint32_t i = 0; i < limit; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity), "r"(20000u)
+        : "memory");
+    if (__all_sync(0xffffffffu, done != 0)) return true;
+  }
+  return false;
 }
 // plain (non-multicast) 2-D tiled load of a CTA pair: data to this CTA, bytes complete on `cluster_bar`
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1,

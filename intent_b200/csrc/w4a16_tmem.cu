@@ -59,6 +59,7 @@ struct TmemParams {
   int acc_sets;              // accumulator sets that alternate between tiles
   int split;                 // CTAs of a cluster that share a tile's k blocks (1 = none)
   int kb_each, kb_extra;     // k blocks of a CTA: the first kb_extra ranks of a cluster take one more
+  uint32_t exchange;         // split: offset of the room for the cluster's partial sums, 0 = where the operands were
   uint32_t tile_magic;       // ceil(2^32 / d), d the number of tiles that vary fastest (0 stands for d = 1)
   int group_shift;           // log2 of the group size
   int twos_complement;
@@ -112,14 +113,6 @@ __device__ __forceinline__ void tmem_store_32x32(uint32_t taddr, const uint32_t 
         "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
-// 32 lanes x 16 columns
-__device__ __forceinline__ void tmem_store_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // 32 lanes x 16 columns
@@ -153,6 +146,15 @@ __device__ __forceinline__ uint2 swap_rows(uint32_t low, uint32_t high, int lane
   return upper ? make_uint2(other, b) : make_uint2(a, other);
 }
 
+// 16 bytes to another CTA of the cluster, counted on a barrier beside them
+__device__ __forceinline__ void store_async_v4(uint32_t cluster_addr, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3,
+                                               uint32_t cluster_bar) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+      ::"r"(cluster_addr), "r"(v0), "r"(v1), "r"(v2), "r"(v3), "r"(cluster_bar)
+      : "memory");
+}
+
 template <typename T, int MODE, int CG>
 __global__ void __launch_bounds__(THREADS, 1)
 w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
@@ -179,6 +181,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   const uint32_t tmem_empty = tmem_full + 8 * RING;    // [2; RING] leader: accumulators drained
   const uint32_t tmem_slot = tmem_empty + 8 * RING;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
+  const uint32_t parts_full = tmem_slot + 8;           // split: the partial sums of this CTA's rows have arrived
   int2* list = reinterpret_cast<int2*>(base_ptr + (tmem_slot - base) + 16);   // grouped: {expert, rows} per block
 
   const int tid = threadIdx.x;
@@ -192,6 +195,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       prefetch_tensormap(&map_w);
       prefetch_tensormap(&map_s);
       prefetch_tensormap(&map_x);
+      mbar_init(parts_full, 1);
     }
     if (lane < p.w_stages) {
       mbar_init(full_w + 8 * lane, 1);
@@ -245,6 +249,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   tcgen05_fence_before();
   __syncthreads();
   if (CG == 2) cluster_sync();   // barriers are initialised before anything arrives remotely
+  else if (p.split > 1) cluster_arrive();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 
@@ -277,6 +282,21 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
     t.n = max(16 * CG, (t.rows + 16 * CG - 1) / (16 * CG) * (16 * CG));
     return t;
+  };
+
+  // split: the rows of a tile are dealt out in slices of whole fours, one for each CTA of the cluster; a CTA sends its sums of
+  // every slice to the CTA that owns it.  Its room there: [rank][four of rows][column], 16 bytes each, so that the lanes of
+  // a warp write and read 512 bytes in a row.
+  const uint32_t parts = base + p.exchange;
+  bool waited = false;    // for the other CTAs of the cluster to be there
+  auto slice_fours = [&](int fours) { return (fours + p.split - 1) / p.split; };
+  auto send_part = [&](int four, int column, int fours, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
+    const int slice = slice_fours(fours), owner = four / slice;
+    const uint32_t to = parts + uint32_t((rank * slice + four - owner * slice) * COLS + column) * 16u;
+    if (owner == rank)
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(to), "r"(v0), "r"(v1), "r"(v2), "r"(v3) : "memory");
+    else
+      store_async_v4(map_to_rank(to, owner), v0, v1, v2, v3, map_to_rank(parts_full, owner));
   };
 
   if (warp == 0) {
@@ -525,13 +545,14 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         if (++s == uint32_t(p.w_stages)) s = 0, phase ^= 1;
       }
       const int col = t.n_tile * COLS + column;
-      if (p.split > 1) {   // back to tensor memory (all MMAs are done), from where the cluster's partial sums are put together
-        uint32_t v[SKINNY_ROWS];
+      if (p.split > 1) {
+        cluster_wait();
+        waited = true;
+        if (ok)
 #pragma unroll
-        for (int r = 0; r < SKINNY_ROWS; ++r) v[r] = __float_as_uint(sum[r]);
-        tmem_store_32x16(tmem_base + (uint32_t(quadrant * 32) << 16), v);
-        tmem_store_wait();
-        tcgen05_fence_before();
+          for (int g = 0; g < SKINNY_ROWS / 4; ++g)
+            send_part(g, column, t.n / 4, __float_as_uint(sum[4 * g]), __float_as_uint(sum[4 * g + 1]),
+                      __float_as_uint(sum[4 * g + 2]), __float_as_uint(sum[4 * g + 3]));
       } else if (ok && col < p.out_cols) {
         uint16_t* y = reinterpret_cast<uint16_t*>(p.y) + col;
 #pragma unroll
@@ -659,47 +680,47 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
-  if (dense_mode(MODE) && CG == 1 && p.split > 1 && first_item < items) {
-    // Every CTA of the cluster holds a partial sum of the whole tile.  The rows are dealt out in `split` slices: a
-    // CTA writes the others' slices into their shared memory (the operand stages are idle once all MMAs are done),
-    // then adds the partials of its own slice in rank order.
+  if (dense_mode(MODE) && CG == 1 && p.split > 1) {
+    // Every CTA of the cluster holds a partial sum of the whole tile; its owner adds up a slice in rank order.  Bound by the
+    // round trips between the SMs: plain remote stores, 96 bytes from lane to lane, between two cluster barriers took 5 of
+    // the 17.3 us of a call of M77 K14336 N4096, 15.1 with these (M16 K4096 N4096 8.4 -> 7.8, M128 13.7 -> 11.1; the own slice
+    // through the same asynchronous stores: 15.5, 7.7, 11.9, and M256 K8192 N4096 20.3 instead of 18.8).
     tcgen05_fence_after();
-    cluster_sync();
+    if (!waited) cluster_wait();
+    if (MODE != MODE_SKINNY && p.exchange == 0) cluster_sync();   // the MMAs of all CTAs are done with the operand stages
     const Item t = item_of(first_item);
-    // slices of whole fours of rows; a column's rows lie together, four more than there are keep the lanes of a
-    // 16-byte access on different banks
-    const int slice = ((t.n + p.split - 1) / p.split + 3) & ~3, pitch = slice + 4;
-    const uint32_t taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
-    const uint32_t own_column = base + uint32_t((rank * COLS + (warp & 3) * 32 + lane) * pitch) * 4u;
-    for (int c = (warp >> 2) * 16; c < t.n; c += (THREADS / 128) * 16) {
-      uint32_t v[16];
-      tmem_load_32x16(taddr + c, v);
-      tmem_load_wait();
+    const int fours = t.n / 4, slice = slice_fours(fours), mine = max(0, min(slice, fours - rank * slice));
+    if (tid == 0) mbar_expect_tx(parts_full, uint32_t((p.split - 1) * mine * COLS) * 16u);
+    if (MODE != MODE_SKINNY) {
+      const uint32_t taddr = tmem_base + (uint32_t((warp & 3) * 32) << 16);
+      for (int c = (warp >> 2) * 16; c < t.n; c += (THREADS / 128) * 16) {
+        uint32_t v[16];
+        tmem_load_32x16(taddr + c, v);
+        tmem_load_wait();
 #pragma unroll
-      for (int i = 0; i < 16; i += 4) {
-        const int owner = (c + i) / slice, r = (c + i) - owner * slice;
-        asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(map_to_rank(own_column + r * 4, owner)),
-                     "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3])
-                     : "memory");
+        for (int i = 0; i < 16; i += 4)
+          send_part((c + i) / 4, (warp & 3) * 32 + lane, fours, v[i], v[i + 1], v[i + 2], v[i + 3]);
       }
     }
-    cluster_sync();
-    const float* parts = reinterpret_cast<const float*>(base_ptr);
-    uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
-    for (int i = tid; i < slice / 4 * COLS; i += THREADS) {
-      const int c = i % COLS, r = i / COLS * 4;
-      const int row = rank * slice + r, col = t.n_tile * COLS + c;
-      float4 sum = *reinterpret_cast<const float4*>(parts + size_t(c) * pitch + r);
-      for (int other = 1; other < p.split; ++other) {
-        const float4 v = *reinterpret_cast<const float4*>(parts + size_t(other * COLS + c) * pitch + r);
-        sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    cluster_arrive();
+    if (MODE != MODE_SKINNY) __syncthreads();
+    if (mbar_wait_warp_cluster(parts_full, 0)) {
+      const float4* from = reinterpret_cast<const float4*>(base_ptr + p.exchange);
+      uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
+      for (int i = tid; i < mine * COLS; i += THREADS) {   // a four of rows has four warps
+        const int c = i % COLS, first = (rank * slice + i / COLS) * 4, row = first + (lane & 3);
+        const int col = t.n_tile * COLS + (c & ~3);
+        float4 sum = from[i];
+        for (int other = 1; other < p.split; ++other) {
+          const float4 v = from[other * slice * COLS + i];
+          sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+        }
+        const uint2 four = swap_rows(Elem<T>::pack2(sum.x, sum.y), Elem<T>::pack2(sum.z, sum.w), lane);
+        if (row < t.rows && col < p.out_cols)
+          *reinterpret_cast<uint2*>(y + size_t(t.row0 + row) * p.out_cols + col) = four;
       }
-      if (col >= p.out_cols) continue;
-      uint16_t* to = y + size_t(t.row0 + row) * p.out_cols + col;
-      if (row < t.rows) to[0] = Elem<T>::from_float(sum.x);
-      if (row + 1 < t.rows) to[p.out_cols] = Elem<T>::from_float(sum.y);
-      if (row + 2 < t.rows) to[2 * size_t(p.out_cols)] = Elem<T>::from_float(sum.z);
-      if (row + 3 < t.rows) to[3 * size_t(p.out_cols)] = Elem<T>::from_float(sum.w);
+    } else if (lane == 0) {
+      atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
     }
     tcgen05_fence_before();
     __syncthreads();
@@ -710,6 +731,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     if (CG == 2) tmem_dealloc_pair(tmem_base, 512);
     else tmem_dealloc(tmem_base, 512);
   }
+  if (CG == 1 && p.split > 1) cluster_wait();   // nothing of the other CTAs is on its way to this one's shared memory
 }
 
 int device_sms() {
@@ -758,17 +780,20 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   // Up to eight stages of activations: a stage comes back after its MMAs and a load from the L2, some 2000 cycles, of
   // which four k blocks cover no more than that.  The rest is a ring for the packed words, which come from HBM.
   const int list_bytes = dense_mode(MODE) ? 0 : p.m_tiles * 8;
-  const int fixed = 1024 + 512 + list_bytes, x_stage = p.row_tile / CG * 256;
+  const int x_stage = p.row_tile / CG * 256;
+  // split: the partial sums of a cluster have room of their own where that leaves five stages of activations, and lie where
+  // the operands were otherwise
+  const int sums = p.split > 1 ? p.split * ((p.row_tile / 4 + p.split - 1) / p.split) * COLS * 16 : 0;
+  int fixed = 1024 + 512 + list_bytes + sums;
+  if (sums > 0 && fixed + 5 * x_stage + 9 * W_STAGE > SMEM_LIMIT) fixed -= sums;
   p.x_stages = 8;
   while (p.x_stages > A_STAGES && fixed + p.x_stages * x_stage + 9 * W_STAGE > SMEM_LIMIT) --p.x_stages;
   p.w_stages = (SMEM_LIMIT - fixed - p.x_stages * x_stage) / W_STAGE;
   if (p.w_stages > 16) p.w_stages = 16;
   if (p.w_stages < SETS) return INTENT_B200_ERR_UNSUPPORTED;
-  const int smem = fixed + p.x_stages * x_stage + p.w_stages * W_STAGE;
-  if (p.split > 1) {   // the partial sums of a cluster meet where the operands were
-    const int slice = ((p.row_tile + p.split - 1) / p.split + 3) & ~3;
-    if (p.split * COLS * (slice + 4) * 4 > smem - 1536) return INTENT_B200_ERR_UNSUPPORTED;
-  }
+  const int smem = fixed + p.x_stages * x_stage + p.w_stages * W_STAGE, operands = p.x_stages * x_stage + p.w_stages * W_STAGE;
+  if (sums > operands) return INTENT_B200_ERR_UNSUPPORTED;
+  if (sums > 0 && fixed >= 1024 + 512 + sums) p.exchange = uint32_t(operands + 512);
 
   const CUtensorMapDataType type =
       std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
