@@ -215,6 +215,13 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     if (CG == 2) tmem_alloc_pair(tmem_slot, 512);
     else tmem_alloc(tmem_slot, 512);
   }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (CG == 2) cluster_sync();   // barriers are initialised before anything arrives remotely
+  else if (p.split > 1) cluster_arrive();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot_ptr;
+  // everything above is done while the kernel before is still at work, everything below may read what that one wrote
   asm volatile("griddepcontrol.wait;" ::: "memory");
   int m_tiles = p.m_tiles;
   if (!dense_mode(MODE)) {
@@ -245,13 +252,8 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         list[b] = make_int2(expert, rows);
       }
     }
+    __syncthreads();
   }
-  tcgen05_fence_before();
-  __syncthreads();
-  if (CG == 2) cluster_sync();   // barriers are initialised before anything arrives remotely
-  else if (p.split > 1) cluster_arrive();
-  tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot_ptr;
 
   const int items = m_tiles * p.n_tiles;
   // split: the CTAs of a cluster (a row of the grid) work on one item, each on its own share of the k blocks
