@@ -477,11 +477,6 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       if (lane == 0) mbar_arrive(empty_w + 8 * s);
       s += SETS;
       if (s >= uint32_t(p.w_stages)) s -= p.w_stages, phase ^= 1;
-      if (i >= A_STAGES) {
-        ok = mbar_wait_warp(empty + 8 * x_before, phase_before);
-        if (!ok) break;
-      }
-      tcgen05_fence_after();
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         uint32_t o[32];
@@ -498,8 +493,17 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             if (MODE != MODE_SKINNY) o[4 * j + c] = Elem<T>::mul2(o[4 * j + c], scale2);
           }
         }
+        if (half == 0) {
+          // The first half is expanded while the block that still lies in this stage is being multiplied.
+#pragma unroll
+          for (int j = 0; j < 32; ++j) asm volatile("" : "+r"(o[j]));
+          if (i >= A_STAGES) ok = mbar_wait_warp(empty + 8 * x_before, phase_before);
+          if (!ok) break;
+          tcgen05_fence_after();
+        }
         tmem_store_32x32(tmem_a + half * 32, o);
       }
+      if (!ok) break;
       tmem_store_wait();
       tcgen05_fence_before();
       __syncwarp();
