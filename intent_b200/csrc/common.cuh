@@ -117,6 +117,14 @@ __device__ __forceinline__ uint2 ldg_stream_v2(const void* p) {
   return v;
 }
 
+// silu(gate) * up in f32.  The reciprocal is the hardware's (one unit in the last place, infinity gives zero), the exponential's
+// error is larger: the correctly rounded one is a branch per value, which kept the values of a thread from overlapping.
+__device__ __forceinline__ float silu_times(float gate, float up) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.0f + __expf(-gate)));
+  return gate * r * up;
+}
+
 // Element-type traits for the 16-bit activation types.
 template <typename T>
 struct Elem;

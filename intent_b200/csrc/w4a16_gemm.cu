@@ -340,7 +340,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
                   for (int e = 0; e < 2; ++e) {
                     const float gv = __uint_as_float(gate[8 * q + 2 * j + e]);
                     const float uv = __uint_as_float(up[8 * q + 2 * j + e]);
-                    h[e] = gv * (1.0f / (1.0f + __expf(-gv))) * uv;  // silu(gate) * up in f32, one rounding
+                    h[e] = silu_times(gv, uv);  // one rounding
                   }
                   o[j] = uint32_t(Elem<T>::from_float(h[0])) | (uint32_t(Elem<T>::from_float(h[1])) << 16);
                 }

@@ -578,10 +578,27 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
     float* yf = reinterpret_cast<float*>(p.y);
     constexpr int CHUNK = MODE == MODE_UPGATE_SILU ? 16 : 32;   // rows at a time
+    // Lane r of a chunk: where row r goes and with what weight, asked for a chunk ahead (two dependent loads took most of
+    // the epilogue's time).
+    int next_token = -1;
+    float next_weight = 0.f;
+    auto next_route = [&](const Item& t, int c) {
+      next_token = -1;
+      next_weight = 0.f;
+      if (c + lane < t.rows) {
+        const int route = __ldg(p.row_route + t.row0 + c + lane);
+        if (route >= 0 && route < p.routes) {
+          next_weight = __ldg(p.route_weight + route);
+          next_token = route / p.top_k;
+        }
+      }
+    };
     for (int local = share ? last : 0; local <= last; ++local) {
       const int item = first_item + local * item_step;
       const Item t = item_of(item);
       const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = uint32_t(p.acc_sets == 2 ? local >> 1 : local);
+      const int step = local == last ? (1 + SETS) * CHUNK : CHUNK;
+      if (MODE == MODE_DOWN_SCATTER) next_route(t, share * CHUNK);
       if (!mbar_wait_warp(tmem_full + 8 * acc, use & 1)) {
         if (lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
         break;
@@ -590,7 +607,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + acc * (ACC_COLUMNS / 2) + (uint32_t(quadrant * 32) << 16);
 #pragma unroll 1
-      for (int c = share * CHUNK; c < t.rows; c += local == last ? (1 + SETS) * CHUNK : CHUNK) {
+      for (int c = share * CHUNK; c < t.rows; c += step) {
         // Predicated, not branched: a branch a row keeps the work of different rows apart, and the epilogue of a tile with
         // few k blocks then takes longer than its MMAs (16384 tokens on 64 experts of 4096 x 1408: up|gate 807 -> 640 us).
         if (MODE == MODE_UPGATE_SILU) {
@@ -605,7 +622,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           for (int i = 0; i < 8; ++i) {
             const uint32_t got = __shfl_xor_sync(0xffffffffu, is_up ? v[i] : v[8 + i], 16);
             const float gv = __uint_as_float(is_up ? got : v[i]), uv = __uint_as_float(is_up ? v[8 + i] : got);
-            h[i] = gv * __frcp_rn(1.0f + __expf(-gv)) * uv;  // silu(gate) * up in f32, one rounding
+            h[i] = silu_times(gv, uv);  // one rounding
           }
 #pragma unroll
           for (int i = 0; i < 8; i += 4) {
@@ -618,16 +635,9 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           uint32_t v[32];
           tmem_load_32x32(taddr + c, v);
           if (MODE == MODE_DOWN_SCATTER) {
-            // lane r of the chunk: where row r goes and with what weight
-            int token = -1;
-            float weight = 0.f;
-            if (c + lane < t.rows) {
-              const int route = __ldg(p.row_route + t.row0 + c + lane);
-              if (route >= 0 && route < p.routes) {
-                weight = __ldg(p.route_weight + route);
-                token = route / p.top_k;
-              }
-            }
+            const int token = next_token;
+            const float weight = next_weight;
+            next_route(t, c + step);
             tmem_load_wait();
             // Four lanes swap four rows of their four columns, so that each adds 16 bytes of one row: adds of four bytes a
             // lane stop at 1 TB/s (16384 tokens on 64 experts, whole layer: 1493 us with them, 1400 so).
