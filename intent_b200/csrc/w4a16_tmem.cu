@@ -67,6 +67,8 @@ struct TmemParams {
   const int* total_rows;     // padded row count (device)
   const int* tile_expert;    // expert of each block of `block_rows` rows
   int block_rows;
+  int list_items;            // entries of the list of tiles: most items of a CTA (list_by_item), or all tiles
+  int list_by_item;
   int experts;
   const int* row_route;      // route of every row; a row with no route in [0, routes) is padding; null: all rows count
   const float* route_weight; // MODE_DOWN_SCATTER: [routes]
@@ -182,7 +184,8 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   const uint32_t tmem_slot = tmem_empty + 8 * RING;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
   const uint32_t parts_full = tmem_slot + 8;           // split: the partial sums of this CTA's rows have arrived
-  int2* list = reinterpret_cast<int2*>(base_ptr + (tmem_slot - base) + 16);   // grouped: {expert, rows} per block
+  // grouped: {expert, rows in use} of this CTA's items, or of every tile where those are fewer
+  int2* list = reinterpret_cast<int2*>(base_ptr + (tmem_slot - base) + 16);
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // known to be uniform
@@ -224,37 +227,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   // everything above is done while the kernel before is still at work, everything below may read what that one wrote
   asm volatile("griddepcontrol.wait;" ::: "memory");
   int m_tiles = p.m_tiles;
-  if (!dense_mode(MODE)) {
-    // rows in use of every 128-row block: its routes come first, padding follows
-    m_tiles = min(m_tiles, (*p.total_rows + 127) / 128);
-    const int per_expert = p.block_rows / 128;
-    for (int b = warp; b < m_tiles; b += THREADS / 32) {
-      int rows = min(128, p.M - b * 128);
-      if (p.row_route != nullptr) {
-        int last = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = i * 32 + lane;
-          const int route = r < rows ? __ldg(p.row_route + b * 128 + r) : -1;
-          const unsigned used = __ballot_sync(0xffffffffu, route >= 0 && route < p.routes);
-          if (used) last = i * 32 + 32 - __clz(used);
-        }
-        rows = last;
-      }
-      if (lane == 0) {
-        int expert = p.tile_expert[b / per_expert];
-        if (unsigned(expert) >= unsigned(p.experts)) {
-          // an id that names no expert (a stale or sentinel table entry): never used as an index.  The plane past
-          // the last expert reads as zeros: zero scales, so zero weights
-          atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_INDEX);
-          expert = p.experts;
-        }
-        list[b] = make_int2(expert, rows);
-      }
-    }
-    __syncthreads();
-  }
-
+  if (!dense_mode(MODE)) m_tiles = min(m_tiles, (*p.total_rows + 127) / 128);
   const int items = m_tiles * p.n_tiles;
   // split: the CTAs of a cluster (a row of the grid) work on one item, each on its own share of the k blocks
   const int first_item = p.split > 1 ? int(blockIdx.y) : int(blockIdx.x) / CG;
@@ -266,7 +239,8 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   struct Item {
     int row0, n_tile, expert, rows, n;   // n: rows of the MMA, a multiple of 16 * CG
   };
-  auto item_of = [&](int item) {
+  const int my_items = items > first_item ? (items - 1 - first_item) / item_step + 1 : 0;
+  auto item_of = [&](int item, int local) {   // the local-th one of this CTA
     Item t;
     if (dense_mode(MODE)) {
       t.n_tile = tile_quotient(item);   // the row tile varies fastest
@@ -275,16 +249,49 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       t.expert = 0;
       t.rows = min(p.row_tile, p.M - t.row0);
     } else {
-      const int block = tile_quotient(item);   // the column tile varies fastest
-      t.n_tile = item - block * p.n_tiles;
-      t.row0 = block * 128;
-      const int2 e = list[block];
+      const int tile = tile_quotient(item);   // the column tile varies fastest
+      t.n_tile = item - tile * p.n_tiles;
+      t.row0 = tile * 128;
+      const int2 e = list[p.list_by_item ? local : tile];
       t.expert = e.x;
       t.rows = e.y;
     }
     t.n = max(16 * CG, (t.rows + 16 * CG - 1) / (16 * CG) * (16 * CG));
     return t;
   };
+
+  if (!dense_mode(MODE)) {
+    // Rows in use of a 128-row block: its routes come first, padding follows.  Bound by the latency of the loads, hence one
+    // round of them, which does not wait for the number of rows: as a loop over all blocks, a warp and block at a time, this
+    // took 17 of the 650 us of the up|gate contraction of 16384 tokens on 64 experts and 2 to 4 us at 64 tokens.
+    const int per_expert = p.block_rows / 128;
+    for (int e = warp; e < p.list_items; e += THREADS / 32) {
+      const int tile = p.list_by_item ? tile_quotient(first_item + e * item_step) : e;
+      if (tile >= p.m_tiles) break;
+      int rows = min(128, p.M - tile * 128), expert = __ldg(p.tile_expert + tile / per_expert);
+      if (p.row_route != nullptr) {
+        int last = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = i * 32 + lane;
+          const int route = r < rows ? __ldg(p.row_route + tile * 128 + r) : -1;
+          const unsigned used = __ballot_sync(0xffffffffu, route >= 0 && route < p.routes);
+          if (used) last = i * 32 + 32 - __clz(used);
+        }
+        rows = last;
+      }
+      if (lane == 0) {
+        if (unsigned(expert) >= unsigned(p.experts)) {
+          // an id that names no expert (a stale or sentinel table entry): never used as an index.  The plane past
+          // the last expert reads as zeros: zero scales, so zero weights
+          if (tile < m_tiles) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_INDEX);
+          expert = p.experts;
+        }
+        list[e] = make_int2(expert, rows);
+      }
+    }
+    __syncthreads();
+  }
 
   // split: the rows of a tile are dealt out in slices of whole fours, one for each CTA of the cluster; a CTA sends its sums of
   // every slice to the CTA that owns it.  Its room there: [rank][four of rows][column], 16 bytes each, so that the lanes of
@@ -308,8 +315,8 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const int tile_columns = MODE == MODE_UPGATE_SILU ? 64 : COLS, tile_rank = CG == 2 ? rank : 0;
     uint32_t s = 0, phase = 1;
     bool ok = true, ready = true;   // ready: the stage was seen to be free
-    for (int item = first_item; item < items && ok; item += item_step) {
-      const Item t = item_of(item);
+    for (int item = first_item, local = 0; item < items && ok; item += item_step, ++local) {
+      const Item t = item_of(item, local);
       const int column = (t.n_tile * CG + tile_rank) * tile_columns;
       int row = kb_first * W_ROWS, scale_row = kb_first * scale_rows;
       for (int kb = 0; kb < kb_count; ++kb, row += W_ROWS, scale_row += scale_rows) {
@@ -336,8 +343,8 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const uint32_t full_leader = CG == 2 ? map_to_rank(full, 0) : full;
     uint32_t s = 0, phase = 1;
     bool ok = true, ready = true;
-    for (int item = first_item; item < items && ok; item += item_step) {
-      const Item t = item_of(item);
+    for (int item = first_item, local = 0; item < items && ok; item += item_step, ++local) {
+      const Item t = item_of(item, local);
       const int rows = t.n / CG, row0 = t.row0 + (CG == 2 ? rank * rows : 0);
       const int boxes = dense_mode(MODE) ? 1 : __shfl_sync(0xffffffffu, rows / 16, 0);
       const uint32_t bytes = uint32_t(CG * boxes * p.box_rows) * 256u;
@@ -377,7 +384,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       uint32_t s = 0, phase = 0, a = 0, local = 0, ring = 0, ring_phase = 0;
       bool ok = true, ready = false;   // ready: both operands of the k block were seen to be there
       for (int item = first_item; item < items && ok; item += item_step, ++local) {
-        const Item t = item_of(item);
+        const Item t = item_of(item, int(local));
         const uint32_t idesc = umma_idesc(1, fmt, fmt, 0, 0, CG * COLS, uint32_t(t.n));
         const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = p.acc_sets == 2 ? local >> 1 : local;
         if (MODE != MODE_SKINNY) {
@@ -451,7 +458,6 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     uint32_t s_of[4];   // scale of k 32 g .. 32 g + 31
 #pragma unroll
     for (int g = 0; g < 4; ++g) s_of[g] = s_offset + (uint32_t(g * 32) >> p.group_shift) * s_pitch;
-    const int my_items = items > first_item ? (items - first_item + item_step - 1) / item_step : 0;
     const uint32_t total = uint32_t(my_items) * uint32_t(kb_count);
     const uint32_t tmem_a = tmem_base + A_COLUMN + set * 64 + (uint32_t(quadrant * 32) << 16);
     const uint32_t full_leader = CG == 2 ? map_to_rank(full, 0) : full;
@@ -523,7 +529,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     uint32_t s = 0, phase = 0, ring = 0, ring_phase = 0;
     bool ok = true;
     for (int item = first_item; item < items && ok; item += item_step) {
-      const Item t = item_of(item);
+      const Item t = item_of(item, 0);
       float sum[SKINNY_ROWS];
 #pragma unroll
       for (int r = 0; r < SKINNY_ROWS; ++r) sum[r] = 0.f;
@@ -568,12 +574,12 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
     if (!ok && lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
   }
-  if (MODE != MODE_SKINNY && warp >= FIRST_EPILOGUE && (p.split == 1 || warp < FIRST_DEQUANT) && items > first_item) {
+  if (MODE != MODE_SKINNY && warp >= FIRST_EPILOGUE && (p.split == 1 || warp < FIRST_DEQUANT) && my_items > 0) {
     // ------------------------------ epilogue -----------------------------------
     // The dequantisers, whose work is done by then, take four fifths of the last tile: nothing is left to overlap it with.
     // Bound by the stores: two bytes a lane and four warps took 4 of the 13 us of a call of M512 K2048 N4096 (a tile a
     // CTA); eight bytes a lane and twenty warps, 13.06 -> 10.77 us.
-    const int quadrant = warp & 3, last = (items - 1 - first_item) / item_step;
+    const int quadrant = warp & 3, last = my_items - 1;
     const int share = warp >= FIRST_DEQUANT ? 1 + ((warp - FIRST_DEQUANT) >> 2) : 0;
     uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
     float* yf = reinterpret_cast<float*>(p.y);
@@ -595,7 +601,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     };
     for (int local = share ? last : 0; local <= last; ++local) {
       const int item = first_item + local * item_step;
-      const Item t = item_of(item);
+      const Item t = item_of(item, local);
       const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = uint32_t(p.acc_sets == 2 ? local >> 1 : local);
       const int step = local == last ? (1 + SETS) * CHUNK : CHUNK;
       if (MODE == MODE_DOWN_SCATTER) next_route(t, share * CHUNK);
@@ -704,7 +710,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     tcgen05_fence_after();
     if (!waited) cluster_wait();
     if (MODE != MODE_SKINNY && p.exchange == 0) cluster_sync();   // the MMAs of all CTAs are done with the operand stages
-    const Item t = item_of(first_item);
+    const Item t = item_of(first_item, 0);
     const int fours = t.n / 4, slice = slice_fours(fours), mine = max(0, min(slice, fours - rank * slice));
     if (tid == 0) mbar_expect_tx(parts_full, uint32_t((p.split - 1) * mine * COLS) * 16u);
     if (MODE != MODE_SKINNY) {
@@ -771,7 +777,7 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   p.WN = int(q.WN);
   p.out_cols = int(q.out_cols);
   p.k_blocks = int((q.K + BK - 1) / BK);
-  p.row_tile = dense_mode(MODE) ? q.row_tile : 128;
+  p.row_tile = q.row_tile;
   p.m_tiles = int((q.rows + p.row_tile - 1) / p.row_tile);
   p.n_tiles = MODE == MODE_UPGATE_SILU ? int(q.out_cols / (64 * CG)) : int((q.out_cols + COLS * CG - 1) / (COLS * CG));
   p.box_rows = dense_mode(MODE) ? p.row_tile / CG : 16;
@@ -791,11 +797,16 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   if (p.split < 1 || p.split > 8 || (p.split > 1 && (!dense_mode(MODE) || CG != 1 || p.k_blocks < p.split)))
     return INTENT_B200_ERR_UNSUPPORTED;
   if (MODE == MODE_SKINNY && (p.row_tile != SKINNY_ROWS || p.M > SKINNY_ROWS)) return INTENT_B200_ERR_UNSUPPORTED;
-  if (!dense_mode(MODE) && (p.m_tiles > LIST_BLOCKS || q.block_rows % 128 != 0)) return INTENT_B200_ERR_UNSUPPORTED;
+  if (!dense_mode(MODE) && (p.m_tiles > LIST_BLOCKS || q.block_rows % 128 != 0 || p.row_tile != 128))
+    return INTENT_B200_ERR_UNSUPPORTED;
 
   // Up to eight stages of activations: a stage comes back after its MMAs and a load from the L2, some 2000 cycles, of
   // which four k blocks cover no more than that.  The rest is a ring for the packed words, which come from HBM.
-  const int list_bytes = dense_mode(MODE) ? 0 : p.m_tiles * 8;
+  const int64_t items = int64_t(p.m_tiles) * p.n_tiles, at_once = sms / CG;
+  const int64_t most_items = (items + at_once - 1) / at_once;   // of a CTA or a pair
+  p.list_by_item = most_items < p.m_tiles;
+  p.list_items = dense_mode(MODE) ? 0 : int(p.list_by_item ? most_items : p.m_tiles);
+  const int list_bytes = p.list_items * 8;
   const int x_stage = p.row_tile / CG * 256;
   // split: the partial sums of a cluster have room of their own where that leaves five stages of activations, and lie where
   // the operands were otherwise
@@ -830,14 +841,13 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   auto kernel = w4a16_tmem_kernel<T, MODE, CG>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
   if (e != cudaSuccess) return cuda_status(e);
-  const int64_t items = int64_t(p.m_tiles) * p.n_tiles;
   const int64_t fastest = dense_mode(MODE) ? p.m_tiles : p.n_tiles;
   if (items * fastest >= (int64_t(1) << 32) || (p.split > 1 && items > 65535)) return INTENT_B200_ERR_UNSUPPORTED;
   p.tile_magic = fastest == 1 ? 0u : uint32_t(((uint64_t(1) << 32) + fastest - 1) / fastest);
   p.kb_each = p.k_blocks / p.split;
   p.kb_extra = p.k_blocks % p.split;
   const int cluster = p.split > 1 ? p.split : CG;
-  const int grid = int(p.split > 1 ? items * p.split : CG * (items < sms / CG ? items : sms / CG));
+  const int grid = int(p.split > 1 ? items * p.split : CG * (items < at_once ? items : at_once));
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel),
                          MODE == MODE_SKINNY ? (p.split > 1 ? "w4a16_tmem_kernel 16 rows, scaled in f32, k split over a cluster"

@@ -15,7 +15,7 @@ struct TmemCall {
   void* out;
   int64_t out_cols;
   int group_size, zero_point;
-  int row_tile;                // dense: rows of a tile, a multiple of 16 up to 128 (with pairs of 32 up to 256)
+  int row_tile;                // rows of a tile, a multiple of 16 up to 128 (with pairs of 32 up to 256; grouped: 128)
   int split;                   // dense: CTAs of a cluster that share the k blocks of a tile
   const int* total_rows;       // grouped modes, as in w4a16_gemm.cu
   const int* tile_expert;
