@@ -78,12 +78,40 @@ inline bool contiguous(const View3& v) {
 }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// A programmatic launch: the kernel may start on SMs that the kernel ahead of it has left, and waits inside
+// (programmatic_wait) for everything ahead of it in the stream before it touches global memory.  What it does before that -
+// barriers, tensor memory, indexes - and the launch itself then cost nothing beside the kernel ahead.
+template <typename... P, typename... A>
+cudaError_t launch_programmatic(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
+                                const A&... arguments) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[2];
+  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  attribute[1].id = cudaLaunchAttributeClusterDimension;
+  attribute[1].val.clusterDim.x = unsigned(cluster);
+  attribute[1].val.clusterDim.y = 1;
+  attribute[1].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<P>(arguments)...);
+}
+
 #define IB200_VIEW1_ARG(p) ib200::View1{p, p##_d0, p##_s0}
 #define IB200_VIEW2_ARG(p) ib200::View2{p, p##_d0, p##_d1, p##_s0, p##_s1}
 #define IB200_VIEW3_ARG(p) ib200::View3{p, p##_d0, p##_d1, p##_d2, p##_s0, p##_s1, p##_s2}
 
 // ---- device side ---------------------------------------------------------
 #ifdef __CUDACC__
+
+// lets the next programmatic launch start as soon as every CTA of this one has
+__device__ __forceinline__ void programmatic_begin() { asm volatile("griddepcontrol.launch_dependents;"); }
+// everything ahead in the stream has completed and its writes are visible
+__device__ __forceinline__ void programmatic_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;

@@ -35,6 +35,8 @@ __device__ __forceinline__ void top2_insert(Top2& t, float v, int i) {
 
 __global__ void moe_route_top2_kernel(const float* __restrict__ logits, int tokens, int experts,
                                       int* __restrict__ ids, float* __restrict__ weights) {
+  programmatic_begin();
+  programmatic_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= tokens) return;
@@ -160,6 +162,8 @@ __global__ void __launch_bounds__(1024)
 moe_align_kernel(const int* __restrict__ ids, int routes, int experts, int block, int* __restrict__ sorted,
                  int sorted_capacity, int fill, int* __restrict__ blocks, int blocks_capacity,
                  int* __restrict__ total_padded) {
+  programmatic_begin();
+  programmatic_wait();
   extern __shared__ int counts[];      // [experts]
   __shared__ int warp_count[32];
   __shared__ int bounds[2];            // padded start of this CTA's span, padded total
@@ -233,6 +237,8 @@ template <bool PADDING>
 __global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ sorted,
                                        const int* __restrict__ total, int capacity, int routes, int top_k,
                                        int row_vectors, uint4* __restrict__ out) {
+  programmatic_begin();
+  programmatic_wait();
   const int limit = min(capacity, *total);
   for (int p = blockIdx.x; p < limit; p += gridDim.x) {
     const int r = sorted[p];
@@ -285,10 +291,11 @@ extern "C" int intent_b200_moe_route_top2(INTENT_B200_VIEW2(a0), INTENT_B200_VIE
   if (!contiguous(IB200_VIEW2_ARG(a0)) || !contiguous(IB200_VIEW2_ARG(a1)) || !contiguous(IB200_VIEW2_ARG(a2)))
     return INTENT_B200_ERR_LAYOUT;
   const int tokens = int(a0_d0);
-  moe_route_top2_kernel<<<(tokens + 7) / 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const float*>(a0), tokens, int(a0_d1), static_cast<int*>(a1), static_cast<float*>(a2));
+  const int status = cuda_status(launch_programmatic(
+      moe_route_top2_kernel, (tokens + 7) / 8, 256, 0, static_cast<cudaStream_t>(stream), 1, static_cast<const float*>(a0),
+      tokens, int(a0_d1), static_cast<int*>(a1), static_cast<float*>(a2)));
   note_launch();
-  return launch_status();
+  return status;
 }
 
 // topk_ids [T,K] i32, expert_counts [E] i32 (InOut, accumulated)
@@ -351,11 +358,12 @@ extern "C" int intent_b200_moe_align_routes(INTENT_B200_VIEW2(a0), INTENT_B200_V
   if (!contiguous(IB200_VIEW2_ARG(a0)) || !contiguous(IB200_VIEW1_ARG(a1)) || !contiguous(IB200_VIEW1_ARG(a2)))
     return INTENT_B200_ERR_LAYOUT;
   if (experts > 8192) return INTENT_B200_ERR_UNSUPPORTED;
-  moe_align_kernel<<<experts, 1024, size_t(experts) * 4, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const int*>(a0), int(a0_d0 * a0_d1), experts, block_size, static_cast<int*>(a1), int(a1_d0),
-      fill, static_cast<int*>(a2), int(a2_d0), static_cast<int*>(a3));
+  const int status = cuda_status(launch_programmatic(
+      moe_align_kernel, experts, 1024, size_t(experts) * 4, static_cast<cudaStream_t>(stream), 1,
+      static_cast<const int*>(a0), int(a0_d0 * a0_d1), experts, block_size, static_cast<int*>(a1), int(a1_d0), fill,
+      static_cast<int*>(a2), int(a2_d0), static_cast<int*>(a3)));
   note_launch();
-  return launch_status();
+  return status;
 }
 
 // sorted_route_ids [capacity], total_padded [1] -> route_positions [R]
@@ -379,11 +387,12 @@ int gather_rows(View2 x, View1 sorted, View1 total, View2 out, int top_k, cudaSt
   if (!x.p || !sorted.p || !total.p || !out.p) return INTENT_B200_ERR_NULL;
   if (!contiguous(x) || !contiguous(out) || !aligned16(x.p) || !aligned16(out.p)) return INTENT_B200_ERR_LAYOUT;
   if (x.d1 % 8 != 0) return INTENT_B200_ERR_UNSUPPORTED;
-  moe_gather_rows_kernel<PADDING><<<grid_for(sorted.d0, 1, 148 * 16), 256, 0, stream>>>(
-      static_cast<const uint4*>(x.p), static_cast<const int*>(sorted.p), static_cast<const int*>(total.p),
-      int(sorted.d0), int(x.d0 * top_k), top_k, int(x.d1 / 8), static_cast<uint4*>(out.p));
+  const int status = cuda_status(launch_programmatic(
+      moe_gather_rows_kernel<PADDING>, grid_for(sorted.d0, 1, 148 * 16), 256, 0, stream, 1, static_cast<const uint4*>(x.p),
+      static_cast<const int*>(sorted.p), static_cast<const int*>(total.p), int(sorted.d0), int(x.d0 * top_k), top_k,
+      int(x.d1 / 8), static_cast<uint4*>(out.p)));
   note_launch();
-  return launch_status();
+  return status;
 }
 }  // namespace
 }  // namespace ib200

@@ -23,6 +23,8 @@ __device__ __forceinline__ uint32_t sign_extend_nibbles(uint32_t nibbles) {
 
 // 16 packed bytes (32 nibbles) -> 32 int8, k order: byte b holds k = 2b (low) and 2b + 1 (high)
 __global__ void expand_w4_kernel(const uint4* __restrict__ packed, uint4* __restrict__ out, int64_t vectors) {
+  programmatic_begin();
+  programmatic_wait();
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < vectors; i += int64_t(gridDim.x) * blockDim.x) {
     const uint4 v = ldg_stream_v4(packed + i);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -42,6 +44,8 @@ __global__ void expand_w4_kernel(const uint4* __restrict__ packed, uint4* __rest
 // One 4-byte word holds 16 two-bit values: value k sits in byte k % 4 at bit 2 * (k / 4), so
 // (word >> 2L) & 0x03030303 is the four values 4L .. 4L+3 in output byte order.
 __global__ void expand_int2_kernel(const uint32_t* __restrict__ packed, uint4* __restrict__ out, int64_t words) {
+  programmatic_begin();
+  programmatic_wait();
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < words; i += int64_t(gridDim.x) * blockDim.x) {
     const uint32_t w = __ldg(packed + i);
     out[i] = make_uint4(w & 0x03030303u, (w >> 2) & 0x03030303u, (w >> 4) & 0x03030303u, (w >> 6) & 0x03030303u);
@@ -58,6 +62,8 @@ __device__ __forceinline__ uint32_t fp4_bits_to_bf16(uint32_t bits) {
 // 4 packed bytes = two big-endian 16-bit words = 8 codes -> 8 bf16 (16 bytes)
 __global__ void expand_fp4_kernel(const uint32_t* __restrict__ packed, uint4* __restrict__ out, int64_t words,
                                   int32_t* row_span, int32_t rows) {
+  programmatic_begin();
+  programmatic_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     row_span[0] = 0;
     row_span[1] = rows;
@@ -86,6 +92,8 @@ __global__ void expand_fp4_kernel(const uint32_t* __restrict__ packed, uint4* __
 template <int ROWS>
 __global__ void int2_gemv_kernel(const int8_t* __restrict__ activation, const uint32_t* __restrict__ packed,
                                  int32_t* __restrict__ out, int M, int N, int K) {
+  programmatic_begin();
+  programmatic_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -153,10 +161,9 @@ extern "C" int intent_b200_w4a8_packed_matmul(INTENT_B200_VIEW2(a0), INTENT_B200
   if (!workspace || !aligned16(workspace) || workspace_bytes < align256(N * K)) return INTENT_B200_ERR_WORKSPACE;
   if (!observe_sink()) {      // (the contraction behind the expansion is what gets observed)
     const int64_t vectors = N * P / 16;
-    expand_w4_kernel<<<grid_for(vectors, 256), 256, 0, stream>>>(static_cast<const uint4*>(a1),
-                                                                static_cast<uint4*>(workspace), vectors);
+    status = cuda_status(launch_programmatic(expand_w4_kernel, grid_for(vectors, 256), 256, 0, stream, 1,
+                                             static_cast<const uint4*>(a1), static_cast<uint4*>(workspace), vectors));
     note_launch();
-    status = launch_status();
     if (status != INTENT_B200_OK) return status;
   }
   // rows of the product are the weight rows: out[N,M] = W8[N,K] . A[M,K]^T
@@ -177,21 +184,17 @@ extern "C" int intent_b200_bitnet_int2_matmul(INTENT_B200_VIEW2(a0), INTENT_B200
   if (M <= 16) {  // decode: one pass over the packed weights
     const int64_t warps_needed = N;
     const int blocks = int(warps_needed / 8 < 148 * 8 ? (warps_needed + 7) / 8 : 148 * 8);
-    if (M <= 4)
-      int2_gemv_kernel<4><<<blocks, 256, 0, stream>>>(static_cast<const int8_t*>(a0), static_cast<const uint32_t*>(a1),
-                                                     static_cast<int32_t*>(a2), int(M), int(N), int(K));
-    else
-      int2_gemv_kernel<8><<<blocks, 256, 0, stream>>>(static_cast<const int8_t*>(a0), static_cast<const uint32_t*>(a1),
-                                                     static_cast<int32_t*>(a2), int(M), int(N), int(K));
+    status = cuda_status(launch_programmatic(M <= 4 ? int2_gemv_kernel<4> : int2_gemv_kernel<8>, blocks, 256, 0, stream, 1,
+                                             static_cast<const int8_t*>(a0), static_cast<const uint32_t*>(a1),
+                                             static_cast<int32_t*>(a2), int(M), int(N), int(K)));
     note_launch();
-    return launch_status();
+    return status;
   }
   if (!workspace || !aligned16(workspace) || workspace_bytes < align256(N * K)) return INTENT_B200_ERR_WORKSPACE;
   const int64_t words = N * P / 4;
-  expand_int2_kernel<<<grid_for(words, 256), 256, 0, stream>>>(static_cast<const uint32_t*>(a1),
-                                                              static_cast<uint4*>(workspace), words);
+  status = cuda_status(launch_programmatic(expand_int2_kernel, grid_for(words, 256), 256, 0, stream, 1,
+                                           static_cast<const uint32_t*>(a1), static_cast<uint4*>(workspace), words));
   note_launch();
-  status = launch_status();
   if (status != INTENT_B200_OK) return status;
   return i8_gemm_nt(a0, M, K, workspace, N, static_cast<int32_t*>(a2), stream);
 }
@@ -212,11 +215,10 @@ extern "C" int intent_b200_dequant_bf16_fp4_matmul(INTENT_B200_VIEW2(a0), INTENT
   if (!workspace || !aligned16(workspace) || workspace_bytes < decoded_bytes + 256) return INTENT_B200_ERR_WORKSPACE;
   int32_t* row_span = reinterpret_cast<int32_t*>(static_cast<unsigned char*>(workspace) + decoded_bytes);
   const int64_t words = N * P / 4;
-  expand_fp4_kernel<<<grid_for(words, 256), 256, 0, stream>>>(static_cast<const uint32_t*>(a1),
-                                                             static_cast<uint4*>(workspace), words, row_span,
-                                                             int32_t(M));
+  status = cuda_status(launch_programmatic(expand_fp4_kernel, grid_for(words, 256), 256, 0, stream, 1,
+                                           static_cast<const uint32_t*>(a1), static_cast<uint4*>(workspace), words, row_span,
+                                           int32_t(M)));
   note_launch();
-  status = launch_status();
   if (status != INTENT_B200_OK) return status;
   return bf16_gemm_nt(a0, M, K, workspace, N, a2, row_span, stream);
 }

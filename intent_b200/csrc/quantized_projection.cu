@@ -21,6 +21,8 @@ constexpr int kQ4Bytes = 144, kQ8Bytes = 292, kRecordValues = 256;
 // one warp per record; lane l holds values 8l .. 8l+7
 __global__ void q8_k_quantize_kernel(const float* __restrict__ activation, int records,
                                      unsigned char* __restrict__ out) {
+  programmatic_begin();
+  programmatic_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= records) return;
@@ -71,6 +73,8 @@ __global__ void q8_k_quantize_kernel(const float* __restrict__ activation, int r
 // one warp per output row
 __global__ void q4_k_projection_kernel(const unsigned char* __restrict__ weights, const unsigned char* __restrict__ xq,
                                        int rows, int records, float* __restrict__ out) {
+  programmatic_begin();
+  programmatic_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -141,16 +145,17 @@ extern "C" int intent_b200_quantized_projection(INTENT_B200_VIEW3(a0), INTENT_B2
   if (G > 0 && (!workspace || !aligned16(workspace) || workspace_bytes < align256(G * kQ8Bytes)))
     return INTENT_B200_ERR_WORKSPACE;
   if (G > 0) {
-    q8_k_quantize_kernel<<<int((G + 7) / 8), 256, 0, stream>>>(static_cast<const float*>(a1), int(G),
-                                                               static_cast<unsigned char*>(workspace));
+    const int status = cuda_status(launch_programmatic(q8_k_quantize_kernel, int((G + 7) / 8), 256, 0, stream, 1,
+                                                       static_cast<const float*>(a1), int(G),
+                                                       static_cast<unsigned char*>(workspace)));
     note_launch();
-    const int status = launch_status();
     if (status != INTENT_B200_OK) return status;
   }
   const int64_t blocks = (N + 7) / 8;
-  q4_k_projection_kernel<<<int(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream>>>(
+  const int status = cuda_status(launch_programmatic(
+      q4_k_projection_kernel, int(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream, 1,
       static_cast<const unsigned char*>(a0), static_cast<const unsigned char*>(workspace), int(N), int(G),
-      static_cast<float*>(a2));
+      static_cast<float*>(a2)));
   note_launch();
-  return launch_status();
+  return status;
 }

@@ -146,6 +146,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
   constexpr int A_STAGES = Plan::A, B_STAGES = Plan::B, B_BYTES = Plan::B_BYTES, DQ_SETS = Plan::SETS;
   constexpr int ACC_BUFFERS = 2 / MT;       // accumulator sets that alternate between tiles
   extern __shared__ unsigned char smem_raw[];
+  programmatic_begin();
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t smem_a = base;
@@ -185,6 +186,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const GemmParams p)
     fence_mbar_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
+  programmatic_wait();
   if (CAN_PAIR && paired && warp == 0) {
     // Pair neighbouring 128-row blocks of one expert: a block whose position inside its expert's run
     // is even starts a tile; the tile has a second half when the next block has the same expert.
@@ -624,9 +626,9 @@ int launch_gemm(const void* x, int64_t rows, int64_t K, const void* w, const voi
                          : BN == 64  ? "w4a16_gemm_kernel single CTA, 128x64 tiles"
                                      : "w4a16_gemm_kernel single CTA, 128x32 tiles",
                          grid, THREADS, smem, 1);
-  kernel<<<grid, THREADS, smem, stream>>>(map_x, p);
+  e = launch_programmatic(kernel, grid, THREADS, smem, stream, 1, map_x, p);
   note_launch();
-  return launch_status();
+  return cuda_status(e);
 }
 
 // Which tile a dense call runs on: the fewest waves of tiles, weighted by what a k block costs on each form.  The

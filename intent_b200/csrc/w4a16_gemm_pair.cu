@@ -76,6 +76,7 @@ template <typename T>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairParams p) {
   extern __shared__ unsigned char smem_raw[];
+  programmatic_begin();
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t smem_a = base;
@@ -117,6 +118,7 @@ w4a16_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const PairPara
   cluster_sync();   // barriers of both CTAs are initialised before anything arrives remotely
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  programmatic_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
@@ -392,9 +394,9 @@ int w4a16_gemm_pair(const void* x, int64_t M, int64_t K, const void* w, const vo
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel), "w4a16_gemm_pair_kernel CTA pairs, 512x256 tiles",
                          2 * pairs, THREADS, SMEM_BYTES, 2);
-  kernel<<<2 * pairs, THREADS, SMEM_BYTES, stream>>>(map_x, p);
+  e = launch_programmatic(kernel, 2 * pairs, THREADS, SMEM_BYTES, stream, 1, map_x, p);   // (clusters of two: __cluster_dims__)
   note_launch();
-  return launch_status();
+  return cuda_status(e);
 }
 
 // Reads the pair kernel's status word into *value and clears it when it was set (the caller has

@@ -82,6 +82,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                const I8Params p) {
   constexpr int STAGES = Ring<CG>::STAGES, B_BYTES = Ring<CG>::B_BYTES;
   extern __shared__ unsigned char smem_raw[];
+  programmatic_begin();
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t smem_a = base;
@@ -121,6 +122,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (CG == 2) cluster_sync();   // barriers of both CTAs are initialised before anything arrives remotely
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  programmatic_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -307,19 +309,7 @@ int launch(const I8Operands& q, I8Params& p, int sms, cudaStream_t stream) {
     return record_launch(sink, reinterpret_cast<const void*>(kernel),
                          CG == 2 ? "i8_gemm_kernel CTA pairs, 256x256 tiles" : "i8_gemm_kernel 128x256 tiles, two accumulators",
                          grid, THREADS, smem, CG);
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(unsigned(grid), 1, 1);
-  config.blockDim = dim3(THREADS, 1, 1);
-  config.dynamicSmemBytes = smem;
-  config.stream = stream;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeClusterDimension;
-  attribute[0].val.clusterDim.x = CG;
-  attribute[0].val.clusterDim.y = 1;
-  attribute[0].val.clusterDim.z = 1;
-  config.attrs = attribute;
-  config.numAttrs = CG > 1 ? 1 : 0;
-  e = cudaLaunchKernelEx(&config, kernel, map_a, map_b, p);
+  e = launch_programmatic(kernel, grid, THREADS, smem, stream, CG, map_a, map_b, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();
