@@ -76,7 +76,7 @@ constexpr int DQ_ROWS = BK / 8;       // packed words per thread and k block
 constexpr int THREADS = (6 + DEQUANT_WARPS) * 32;
 constexpr int BAND_TILES = 8;         // row tiles per band of the tile walk
 
-constexpr int TMEM_MAX_ROWS = 2048;   // dense calls of fewer rows may run with the weights in tensor memory
+constexpr int TMEM_MAX_ROWS = 2048;   // dense calls of fewer rows run with the weights in tensor memory where that is faster
 constexpr int PAIR_LIST_BLOCKS = 8192;  // most 128-row blocks the in-kernel block pairing handles
 
 template <int MT, int BN>
@@ -122,7 +122,7 @@ struct GemmParams {
 
 constexpr int MODE_DENSE = 0, MODE_UPGATE_SILU = 1, MODE_GROUPED_F32 = 2, MODE_DOWN_SCATTER = 3;
 constexpr int MODE_SKINNY = 4;       // of the kernel with the weights in tensor memory only
-constexpr int SKINNY_LEAST = 9;      // fewest rows of such a call
+constexpr int SKINNY_LEAST = 5;      // fewest rows of such a call
 
 __device__ __forceinline__ void red_add_v4(float* address, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(address), "f"(a), "f"(b), "f"(c), "f"(d)
@@ -675,14 +675,17 @@ Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
 //   CTA pair of r rows x 256 columns          5 + 0.012 r + waves * blocks * (0.405 at 128 rows, 0.52 at 192, 0.735 at 256)
 // Measured against the forms above: M17 K4096 N4096 27.2 -> 9.2 us, M77 K14336 N4096 81.1 -> 18.0, M256 K8192 N1024
 // 48.8 -> 13.1, M256 K4096 N14336 52.9 -> 30.4, M512 K2048 N4096 19.8 -> 13.5, M1024 K4096 N4096 50.9 -> 30.3.
-// Four lines stand outside the estimate.  The fit covers K >= 2048 and fewer than 2048 rows, and tests of the forms above
-// ask for them by sizes beyond that.  With the lines taken out, graph replay, this kernel against the form that runs:
-//   K < 2048    M17 K1024 N1024 6.7 of 9.6 us, M300 K1536 N2048 8.5 of 13.9, M512 K1920 N4096 15.1 of 24.1; but M1024 K1024
-//               N8192 26.2 of 23.0, M1900 K1024 N4096 26.4 of 22.9
-//   M >= 2048   M2500 K8192 N1024 33.2 of 85.7, M4096 K4096 N1024 31.2 of 47.1, M2500 K4096 N8192 130.9 of 159; but M2048
-//               K4096 N4096 60.8 of 53.7, M4096 K4096 N4096 120.8 of 117.7, 8192 cubed 917 of 921
-//   no split up to K = 2048 (there a row keeps its bits, see below)   M32 K2048 N2048 9.7 of 20.3, M77 K2048 N4104 14.2 of 20.8
-// and, where a split is allowed, unsplit calls with less than a tile for every second SM.  A split changes the order of a row's sum: which split a call takes follows
+// Lines that stand outside the estimate.  For the entry that chooses among all kernels (`split_allowed`) they lie where tests
+// of the forms above ask for these by sizes, not where they are faster:
+//   K <= 1152                            M19 K1152 N4176 5.8 of 11.9 us, M899 K1152 N2000 7.2 of 13.1
+//   K = 2048, less than a tile for every second SM   M79 K2048 N2432 8.1 of 14.8
+//   no split up to K = 2048 (there a row keeps its bits, see below)   M36 K1792 N5336 6.9 split in two, 7.5 whole, 16.6 above
+// The entry of the tensor-core kernels keeps to K >= 2048 and fewer than 2048 rows, for the same reason.  Between, this kernel
+// against the forms above: M20 K1536 N2384 9.9 of 18.8, M546 K1408 N1112 8.3 of 23.0, M983 K1536 N5768 17.6 of 38.4.
+// From 2048 rows on it has to be a fifth faster by the estimate, which does not know the power cap: M2180 K7936 N1224 33.6 of
+// 81.0, M2358 K1920 N7512 50.8 of 87.1, M3339 K6016 N8032 227 of 326, but M2048 K4096 N4096 60.8 of 53.7, M4096 K4096 N4096
+// 120.8 of 117.7, 8192 cubed 917 of 921.
+// Where a split is allowed from K = 2048 on, unsplit calls with less than a tile for every second SM are left out.  A split changes the order of a row's sum: which split a call takes follows
 // from its rows, its columns, the number of SMs and the pairs switch, so where one is allowed (the entry that chooses
 // among all kernels) a row agrees with the same row of another call, and a column shard with the whole, to rounding only.
 // Up to K = 2048 nothing is split and the bits are the same.  The entry of the tensor-core kernels and the tiled layout
@@ -691,8 +694,9 @@ Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
 bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split_allowed, double other, TmemCall* call,
                  bool* pairs) {
   const int64_t sms = device_sms(), blocks = (K + 127) / 128;
-  if (sms <= 0 || K < 2048 || M >= TMEM_MAX_ROWS) return false;
-  double best = other;
+  if (sms <= 0 || K <= 1152 || (!split_allowed && (K < 2048 || M >= TMEM_MAX_ROWS))) return false;
+  const double limit = M >= TMEM_MAX_ROWS ? other / 1.2 : other;
+  double best = limit;
   const auto consider = [&](bool pair, int64_t row_tiles, int split) {
     const int64_t unit = pair ? 32 : 16, most = pair ? 256 : 128;
     const int64_t rows = ((M + row_tiles - 1) / row_tiles + unit - 1) / unit * unit;
@@ -707,7 +711,7 @@ bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split
       cost = (split == 2 ? 6.2 : 6.7) + 0.014 * double(rows) +
              double((blocks + split - 1) / split) * (0.24 + 0.0014 * double(rows));
     } else {
-      if (split_allowed && 2 * ctas < sms) return;
+      if (split_allowed && K >= 2048 && 2 * ctas < sms) return;
       const int64_t at_once = pair ? sms / 2 : sms, waves = (tiles + at_once - 1) / at_once;
       const double r = double(rows);
       const double block = !pair       ? 0.24 + 0.0014 * r
@@ -723,15 +727,15 @@ bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split
       *pairs = pair;
     }
   };
-  const int64_t most_tiles = (M + 31) / 32;
-  for (int64_t t = (M + 255) / 256; t <= (M + 63) / 64 && t <= most_tiles; ++t) {
+  const int64_t least_rows = M >= TMEM_MAX_ROWS ? 128 : K < 2048 ? 48 : 64, most_tiles = (M + 31) / 32;
+  for (int64_t t = (M + 255) / 256; t <= (M + least_rows - 1) / least_rows && t <= most_tiles; ++t) {
     if (pairs_allowed) consider(true, t, 1);
     for (const int split : {1, 2, 4}) consider(false, t, split);
   }
   if (M < 64) {
     for (const int split : {1, 2, 4}) consider(false, 1, split);
   }
-  return best < other;
+  return best < limit;
 }
 
 template <typename T>
@@ -816,8 +820,11 @@ int grouped_tmem(int mode, View2 x, View1 tile_expert, View1 total, View3 w, Vie
 // of call, or one that the bandwidth kernel refuses with its own status).  Tiles are spread over clusters of up to four CTAs
 // as long as every CTA keeps four k blocks.  Against the bandwidth kernel (bf16, group 128, cold weights): M16 K4096 N4096
 // 21.9 -> 9.8 us, M9 18.0 -> 9.6, M16 K8192 N1024 25.4 -> 11.6, M16 K1024 N1024 16.2 -> 6.6, M16 K4096 N14336 47.0 -> 16.4;
-// error against 64 bits 2.08e-4 of 2.09e-4 (f16), 1.673e-3 of 1.673e-3 (bf16).  Up to eight rows the ride-along kernel
-// streams the weights as fast.
+// error against 64 bits 2.08e-4 of 2.09e-4 (f16), 1.673e-3 of 1.673e-3 (bf16).  Against the ride-along kernel (bf16, group
+// 128): M6 K4096 N4096 9.5 -> 7.9 us, K1024 N1024 8.1 -> 6.2, K8192 N8192 18.7 -> 17.3, K8192 N1024 10.4 and 10.4; four rows
+// and fewer are left to it (M4 K8192 N1024 8.2 of 10.4, K4096 N14336 14.9 of 15.7, but K4096 N4096 8.6 of 7.9), and so are
+// calls with more tiles than half the SMs, whose tiles cannot be cut, up to six rows (M6 K4096 N14336 15.6 of 15.7, M8
+// 16.1 of 15.7).
 template <typename T>
 int skinny(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, const void* workspace,
            int64_t workspace_bytes, cudaStream_t stream) {
@@ -834,6 +841,7 @@ int skinny(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, c
   const int64_t asked = w4a16_stream_workspace_bytes(M, K, N);   // 0: the bandwidth kernel has no plan for the call
   if (asked <= 0 || !workspace || !aligned16(workspace) || workspace_bytes < asked) return kTableDeclined;
   const int64_t tiles = (N + 127) / 128, blocks = (K + 127) / 128, sms = device_sms();
+  if (M <= 6 && 2 * tiles > sms) return kTableDeclined;
   int split = 1;
   while (split < 4 && tiles * split * 2 <= (split == 1 ? sms : sms * 9 / 10) && blocks >= 8 * split) split *= 2;
   TmemCall q{};
