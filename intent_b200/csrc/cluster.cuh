@@ -50,6 +50,20 @@ __device__ __forceinline__ bool mbar_wait_warp_cluster(uint32_t bar, uint32_t pa
   }
   return false;
 }
+// 16 bytes to another CTA of the cluster, counted on a barrier beside them
+__device__ __forceinline__ void store_async_v4(uint32_t cluster_addr, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3,
+                                               uint32_t cluster_bar) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+      ::"r"(cluster_addr), "r"(v0), "r"(v1), "r"(v2), "r"(v3), "r"(cluster_bar)
+      : "memory");
+}
+// shared memory of this CTA to another one of the cluster, counted on a barrier there; 16-byte addresses and size
+__device__ __forceinline__ void copy_to_cluster(uint32_t cluster_addr, uint32_t from, uint32_t bytes, uint32_t cluster_bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(cluster_addr), "r"(from), "r"(bytes), "r"(cluster_bar)
+               : "memory");
+}
 // plain (non-multicast) 2-D tiled load of a CTA pair: data to this CTA, bytes complete on `cluster_bar`
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1,
                                                  uint32_t cluster_bar) {

@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "dense.cuh"
+#include "split_k.cuh"
 #include "tma.cuh"
 #include "umma.cuh"
 
@@ -50,6 +51,7 @@ struct Params {
   const int32_t* offsets;      // [groups + 1]; null = one group covering every row
   int groups, rows, N, K;
   int k_blocks, n_tiles;
+  int split;                   // CTAs of a cluster that share the k blocks of a tile (1 = none)
   void* out;
   int64_t out_rows;
   const int32_t* row_map;      // output row (or route) of member row r; null = r itself
@@ -99,6 +101,7 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const uint32_t tmem_full = empty + 8 * STAGES;
   const uint32_t tmem_empty = tmem_full + 16;
   const uint32_t tmem_slot = tmem_empty + 16;
+  const uint32_t parts_full = tmem_slot + 8;   // split: the other CTAs' sums of this one's chunks have arrived
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
   int* s_begin = reinterpret_cast<int*>(base_ptr + (bars - base) + 256);
   int* s_count = s_begin + MAX_GROUPS + 1;
@@ -117,6 +120,7 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       mbar_init(tmem_full + 8 * s, 1);
       mbar_init(tmem_empty + 8 * s, 4);
     }
+    mbar_init(parts_full, 1);
     fence_mbar_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
@@ -149,17 +153,24 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
   const int tiles = s_prefix[p.groups];
+  // split: a row of the grid is a cluster, and has one tile or none.  (Offsets that do not rise can ask for more tiles than
+  // there are clusters: every CTA then walks whole tiles.)
+  const bool split = p.split > 1 && tiles <= int(gridDim.y);
+  const SplitShare share{split ? int(cluster_rank()) : 0, p.split};
+  const int first_tile = split ? int(blockIdx.y) : int(blockIdx.x + gridDim.x * blockIdx.y);
+  const int tile_step = split ? max(tiles, 1) : int(gridDim.x * gridDim.y);
+  const int kb_first = split ? share.first(p.k_blocks) : 0, kb_count = split ? share.count(p.k_blocks) : p.k_blocks;
 
   if (warp == 0) {
     if (lane == 0) {
       TileWalk walk(s_begin, s_count, s_prefix, p.groups);
       uint32_t it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
         int g, m_block, n_tile;
         walk.locate(tile, g, m_block, n_tile);
         const int row0 = s_begin[g] + m_block * BM;
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        for (int kb = kb_first; kb < kb_first + kb_count; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           if (!mbar_wait(empty + 8 * s, ((it / STAGES) & 1) ^ 1)) { ok = false; break; }
           const uint32_t bar = full + 8 * s;
@@ -182,12 +193,12 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       constexpr uint32_t idesc = umma_idesc(1, format, format, 0, B_K_MAJOR ? 0 : 1, BM, BN);
       uint32_t it = 0, local = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++local) {
+      for (int tile = first_tile; tile < tiles && ok; tile += tile_step, ++local) {
         const uint32_t acc = local & 1;
         if (!mbar_wait(tmem_empty + 8 * acc, ((local >> 1) & 1) ^ 1)) { ok = false; break; }
         tcgen05_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        for (int kb = 0; kb < kb_count; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           if (!mbar_wait(full + 8 * s, (it / STAGES) & 1)) { ok = false; break; }
           tcgen05_fence_after();
@@ -206,11 +217,87 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       }
       if (!ok) atomicExch(&g_grouped16_status, INTENT_B200_ERR_TIMEOUT);
     }
-  } else {
+  }
+  // Where this lane's row of a tile goes, and with what weight.
+  struct Place {
+    int64_t out_row;
+    float weight;
+    bool valid;
+  };
+  auto place_of = [&](int g, int m_block, int in_tile) {
+    const int in_group = m_block * BM + in_tile;
+    const int member = s_begin[g] + in_group;
+    Place at{member, 1.f, in_group < s_count[g]};
+    if (at.valid && p.row_map) at.out_row = p.row_map[member];
+    if (EPILOGUE == kWeightedAdd) {
+      at.valid = at.valid && at.out_row >= 0 && at.out_row < p.routes;
+      if (at.valid) {
+        at.weight = p.route_weights[at.out_row];
+        at.out_row = p.route_token[at.out_row];
+      }
+    }
+    at.valid = at.valid && at.out_row >= 0 && at.out_row < p.out_rows;
+    return at;
+  };
+  // One chunk of 32 columns of a row
+  auto finish = [&](const uint32_t (&v)[32], const Place& at, int col) {
+    if (!at.valid) return;
+    const int64_t out_row = at.out_row;
+    const float weight = at.weight;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int n0 = col + q * 8;
+      if (n0 < p.N) {  // N is a multiple of 8
+        if (EPILOGUE == kQuantize) {
+          // i8(trunc(clamp((relu(acc + bias) + residual) / scale, -128, 127))), all in f32
+          const float4 b0 = __ldg(reinterpret_cast<const float4*>(p.bias + n0));
+          const float4 b1 = __ldg(reinterpret_cast<const float4*>(p.bias + n0 + 4));
+          const float4 s0 = __ldg(reinterpret_cast<const float4*>(p.out_scale + n0));
+          const float4 s1 = __ldg(reinterpret_cast<const float4*>(p.out_scale + n0 + 4));
+          const uint4 r = __ldg(reinterpret_cast<const uint4*>(
+              reinterpret_cast<const uint16_t*>(p.residual) + size_t(out_row) * p.N + n0));
+          const float bias[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+          const float scale[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+          const uint32_t res[4] = {r.x, r.y, r.z, r.w};
+          uint32_t packed[2] = {0u, 0u};
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float residual = Elem<T>::to_float(uint16_t(res[j >> 1] >> (16 * (j & 1))));
+            float value = fmaxf(__uint_as_float(v[8 * q + j]) + bias[j], 0.f) + residual;
+            value = __fdiv_rn(value, scale[j]);
+            value = fminf(fmaxf(value, -128.f), 127.f);
+            packed[j >> 2] |= (uint32_t(__float2int_rz(value)) & 0xFFu) << (8 * (j & 3));
+          }
+          *reinterpret_cast<uint2*>(reinterpret_cast<int8_t*>(p.out) + size_t(out_row) * p.N + n0) =
+              make_uint2(packed[0], packed[1]);
+        } else if (EPILOGUE == kWeightedAdd) {
+          float* dst = reinterpret_cast<float*>(p.out) + size_t(out_row) * p.N + n0;
+          red_add_v4(dst, weight * __uint_as_float(v[8 * q + 0]), weight * __uint_as_float(v[8 * q + 1]),
+                     weight * __uint_as_float(v[8 * q + 2]), weight * __uint_as_float(v[8 * q + 3]));
+          red_add_v4(dst + 4, weight * __uint_as_float(v[8 * q + 4]), weight * __uint_as_float(v[8 * q + 5]),
+                     weight * __uint_as_float(v[8 * q + 6]), weight * __uint_as_float(v[8 * q + 7]));
+        } else {
+          uint32_t o[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float lo = __uint_as_float(v[8 * q + 2 * j]), hi = __uint_as_float(v[8 * q + 2 * j + 1]);
+            if (EPILOGUE == kReluCast) {
+              lo = fmaxf(lo, 0.f);
+              hi = fmaxf(hi, 0.f);
+            }
+            o[j] = uint32_t(Elem<T>::from_float(lo)) | (uint32_t(Elem<T>::from_float(hi)) << 16);
+          }
+          *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + size_t(out_row) * p.N + n0) =
+              make_uint4(o[0], o[1], o[2], o[3]);
+        }
+      }
+    }
+  };
+  if (warp >= 2) {
     const int quadrant = warp & 3;
     TileWalk walk(s_begin, s_count, s_prefix, p.groups);
     uint32_t local = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
+    for (int tile = first_tile; tile < tiles; tile += tile_step, ++local) {
       int g, m_block, n_tile;
       walk.locate(tile, g, m_block, n_tile);
       const uint32_t acc = local & 1;
@@ -218,78 +305,16 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         if (lane == 0) atomicExch(&g_grouped16_status, INTENT_B200_ERR_TIMEOUT);
         break;
       }
+      if (split) break;   // the partial sums of the cluster are put together below
       tcgen05_fence_after();
-      const int in_group = m_block * BM + quadrant * 32 + lane;
-      const int member = s_begin[g] + in_group;
-      bool valid = in_group < s_count[g];
-      int64_t out_row = member;
-      float weight = 1.f;
-      if (valid && p.row_map) out_row = p.row_map[member];
-      if (EPILOGUE == kWeightedAdd) {
-        valid = valid && out_row >= 0 && out_row < p.routes;
-        if (valid) {
-          weight = p.route_weights[out_row];
-          out_row = p.route_token[out_row];
-        }
-      }
-      valid = valid && out_row >= 0 && out_row < p.out_rows;
+      const Place at = place_of(g, m_block, quadrant * 32 + lane);
       const uint32_t taddr = tmem_base + acc * BN + (uint32_t(quadrant * 32) << 16);
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
         uint32_t v[32];
         tmem_load_32x32(taddr + c * 32, v);
         tmem_load_wait();
-        const int col = n_tile * BN + c * 32;
-        if (valid) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int n0 = col + q * 8;
-            if (n0 < p.N) {  // N is a multiple of 8
-              if (EPILOGUE == kQuantize) {
-                // i8(trunc(clamp((relu(acc + bias) + residual) / scale, -128, 127))), all in f32
-                const float4 b0 = __ldg(reinterpret_cast<const float4*>(p.bias + n0));
-                const float4 b1 = __ldg(reinterpret_cast<const float4*>(p.bias + n0 + 4));
-                const float4 s0 = __ldg(reinterpret_cast<const float4*>(p.out_scale + n0));
-                const float4 s1 = __ldg(reinterpret_cast<const float4*>(p.out_scale + n0 + 4));
-                const uint4 r = __ldg(reinterpret_cast<const uint4*>(
-                    reinterpret_cast<const uint16_t*>(p.residual) + size_t(out_row) * p.N + n0));
-                const float bias[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-                const float scale[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-                const uint32_t res[4] = {r.x, r.y, r.z, r.w};
-                uint32_t packed[2] = {0u, 0u};
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  const float residual = Elem<T>::to_float(uint16_t(res[j >> 1] >> (16 * (j & 1))));
-                  float value = fmaxf(__uint_as_float(v[8 * q + j]) + bias[j], 0.f) + residual;
-                  value = __fdiv_rn(value, scale[j]);
-                  value = fminf(fmaxf(value, -128.f), 127.f);
-                  packed[j >> 2] |= (uint32_t(__float2int_rz(value)) & 0xFFu) << (8 * (j & 3));
-                }
-                *reinterpret_cast<uint2*>(reinterpret_cast<int8_t*>(p.out) + size_t(out_row) * p.N + n0) =
-                    make_uint2(packed[0], packed[1]);
-              } else if (EPILOGUE == kWeightedAdd) {
-                float* dst = reinterpret_cast<float*>(p.out) + size_t(out_row) * p.N + n0;
-                red_add_v4(dst, weight * __uint_as_float(v[8 * q + 0]), weight * __uint_as_float(v[8 * q + 1]),
-                           weight * __uint_as_float(v[8 * q + 2]), weight * __uint_as_float(v[8 * q + 3]));
-                red_add_v4(dst + 4, weight * __uint_as_float(v[8 * q + 4]), weight * __uint_as_float(v[8 * q + 5]),
-                           weight * __uint_as_float(v[8 * q + 6]), weight * __uint_as_float(v[8 * q + 7]));
-              } else {
-                uint32_t o[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  float lo = __uint_as_float(v[8 * q + 2 * j]), hi = __uint_as_float(v[8 * q + 2 * j + 1]);
-                  if (EPILOGUE == kReluCast) {
-                    lo = fmaxf(lo, 0.f);
-                    hi = fmaxf(hi, 0.f);
-                  }
-                  o[j] = uint32_t(Elem<T>::from_float(lo)) | (uint32_t(Elem<T>::from_float(hi)) << 16);
-                }
-                *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + size_t(out_row) * p.N + n0) =
-                    make_uint4(o[0], o[1], o[2], o[3]);
-              }
-            }
-          }
-        }
+        finish(v, at, n_tile * BN + c * 32);
       }
       tcgen05_fence_before();
       __syncwarp();
@@ -297,8 +322,41 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
   }
 
+  __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
+  if (split) {
+    tcgen05_fence_after();
+    cluster_sync();   // the MMAs of all CTAs are done with the operand stages, where the sums go
+    if (first_tile < tiles && warp >= 2) {
+      int g, m_block, n_tile;
+      TileWalk walk(s_begin, s_count, s_prefix, p.groups);
+      walk.locate(first_tile, g, m_block, n_tile);
+      const int quadrant = warp & 3, in_tile = quadrant * 32 + lane;
+      const int chunks = min(kPartChunks, (p.N - n_tile * BN + 31) / 32);
+      const int warps = min(4, (s_count[g] - m_block * BM + 31) / 32);
+      const uint32_t taddr = tmem_base + (uint32_t(quadrant * 32) << 16);
+      const PartRoom room{smem_a, warps};
+      if (warp == 2 && lane == 0) mbar_expect_tx(parts_full, expected_parts(share, chunks, warps));
+      if (quadrant < warps) {
+        send_parts(share, room, parts_full, taddr, chunks, quadrant, lane);
+        if (mbar_wait_warp_cluster(parts_full, 0)) {
+          const Place at = place_of(g, m_block, in_tile);
+          for (int c = share.rank; c < chunks; c += share.split) {
+            uint32_t v[32];
+            add_parts(share, room, taddr, c, quadrant, lane,
+                      [](uint32_t x, uint32_t y) { return __float_as_uint(__uint_as_float(x) + __uint_as_float(y)); }, v);
+            finish(v, at, n_tile * BN + c * 32);
+          }
+        } else if (lane == 0) {
+          atomicExch(&g_grouped16_status, INTENT_B200_ERR_TIMEOUT);
+        }
+      }
+    }
+    __syncwarp();
+    tcgen05_fence_before();
+    cluster_sync();   // nothing is on its way to a CTA that is gone
+  }
   if (warp == 1) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, 512);
@@ -403,15 +461,18 @@ int launch(const Problem& q, cudaStream_t stream) {
   auto kernel = grouped_gemm16_kernel<T, B_K_MAJOR, EPILOGUE>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_status(e);
-  const int grid = int(tile_bound < sms ? (tile_bound > 0 ? tile_bound : 1) : sms);
+  p.split = tile_bound > 0 ? split_of(tile_bound, p.k_blocks / 2, q.rows, 0.45, sms) : 1;   // (blocks of 64 k)
+  const int grid = int(p.split > 1 ? tile_bound * p.split : tile_bound < sms ? (tile_bound > 0 ? tile_bound : 1) : sms);
   if (LaunchFacts* sink = observe_sink())
-    return record_launch(sink, reinterpret_cast<const void*>(kernel), "grouped_gemm16_kernel 128x256 tiles", grid,
-                         THREADS, SMEM_BYTES, 1);
+    return record_launch(sink, reinterpret_cast<const void*>(kernel), p.split > 1 ? "grouped_gemm16_kernel 128x256 tiles, k split over a cluster"
+                                     : "grouped_gemm16_kernel 128x256 tiles",
+                         grid, THREADS, SMEM_BYTES, p.split);
   // Up to a wave of tiles a programmatic launch saves a good microsecond (rows 111 26 347 22 22 of 1368 x 1280 15.4 -> 13.4
   // us).  Above, it costs: the CTAs take the SMs in the order in which these come free, and neighbouring tiles, which
   // share an operand, then run far apart (expert FFN of 688 rows 197 -> 210 us, of 4096 rows 1777 -> 1841).
   if (tile_bound <= sms) {
-    e = launch_programmatic(kernel, grid, THREADS, SMEM_BYTES, stream, 1, map_a, map_b, p);
+    const dim3 ctas = p.split > 1 ? dim3(unsigned(p.split), unsigned(tile_bound), 1) : dim3(unsigned(grid), 1, 1);
+    e = launch_programmatic(kernel, ctas, THREADS, SMEM_BYTES, stream, p.split, map_a, map_b, p);
   } else {
     kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(map_a, map_b, p);
     e = cudaGetLastError();

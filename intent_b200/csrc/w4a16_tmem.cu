@@ -148,15 +148,6 @@ __device__ __forceinline__ uint2 swap_rows(uint32_t low, uint32_t high, int lane
   return upper ? make_uint2(other, b) : make_uint2(a, other);
 }
 
-// 16 bytes to another CTA of the cluster, counted on a barrier beside them
-__device__ __forceinline__ void store_async_v4(uint32_t cluster_addr, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3,
-                                               uint32_t cluster_bar) {
-  asm volatile(
-      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-      ::"r"(cluster_addr), "r"(v0), "r"(v1), "r"(v2), "r"(v3), "r"(cluster_bar)
-      : "memory");
-}
-
 template <typename T, int MODE, int CG>
 __global__ void __launch_bounds__(THREADS, 1)
 w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,

@@ -23,6 +23,7 @@
 #include "cluster.cuh"
 #include "common.cuh"
 #include "dense.cuh"
+#include "split_k.cuh"
 #include "tma.cuh"
 #include "umma.cuh"
 
@@ -56,6 +57,7 @@ struct I8Params {
   int M, N, K;
   int k_blocks, m_tiles, n_tiles;
   int band;                 // row tiles of a band of the tile walk
+  int split;                // CTAs of a cluster that share the k blocks of a tile (1 = none; lone tiles only)
 };
 
 // Tile walk: the row tile varies fastest, so that the columns of B in flight are few.  Where A is too large to stay in
@@ -93,14 +95,19 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const uint32_t tmem_full = empty + 8 * STAGES;
   const uint32_t tmem_empty = tmem_full + 16;
   const uint32_t tmem_slot = tmem_empty + 16;
+  const uint32_t parts_full = tmem_slot + 8;   // split: the other CTAs' sums of this one's chunks have arrived
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const int tiles = p.m_tiles * p.n_tiles;
+  const bool split = CG == 1 && p.split > 1;
   const int rank = CG == 2 ? int(cluster_rank()) : 0;
-  const int first_tile = int(blockIdx.x) / CG, tile_step = int(gridDim.x) / CG;
+  const SplitShare share{split ? int(cluster_rank()) : 0, p.split};
+  // split: a row of the grid is a cluster, and has one tile
+  const int first_tile = split ? int(blockIdx.y) : int(blockIdx.x) / CG, tile_step = split ? tiles : int(gridDim.x) / CG;
+  const int kb_first = split ? share.first(p.k_blocks) : 0, kb_count = split ? share.count(p.k_blocks) : p.k_blocks;
 
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -111,6 +118,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_init(tmem_full + 8 * s, 1);
       mbar_init(tmem_empty + 8 * s, 4 * CG);
     }
+    mbar_init(parts_full, 1);
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -131,7 +139,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       for (int tile = first_tile; tile < tiles && ok; tile += tile_step) {
         int m_tile, n_tile;
         tile_coords(tile, p, m_tile, n_tile);
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        for (int kb = kb_first; kb < kb_first + kb_count; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           if (!mbar_wait(empty + 8 * s, ((it / STAGES) & 1) ^ 1)) { ok = false; break; }
           const int row0 = (m_tile * CG + rank) * BM, col0 = n_tile * BN + rank * (BN / CG);
@@ -167,7 +175,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (!mbar_wait(tmem_empty + 8 * acc, ((local >> 1) & 1) ^ 1)) { ok = false; break; }
         tcgen05_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        for (int kb = 0; kb < kb_count; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           if (!mbar_wait(full + 8 * s, (it / STAGES) & 1)) { ok = false; break; }
           tcgen05_fence_after();
@@ -192,7 +200,47 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
       if (!ok) atomicExch(&g_w8a8_gemm_status, INTENT_B200_ERR_TIMEOUT);
     }
-  } else {
+  }
+  // One chunk of 32 columns of a row
+  auto finish = [&](const uint32_t (&v)[32], int row, float row_scale, int col) {
+    if (row >= p.M) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int n0 = col + q * 8;
+      if (n0 < p.N) {  // N is a multiple of 16
+        if (EPILOGUE == 0) {
+          const float4 s0 = __ldg(reinterpret_cast<const float4*>(p.b_scales + n0));
+          const float4 s1 = __ldg(reinterpret_cast<const float4*>(p.b_scales + n0 + 4));
+          const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+          uint32_t o[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float lo = (float(int32_t(v[8 * q + 2 * j])) * row_scale) * sc[2 * j];
+            const float hi = (float(int32_t(v[8 * q + 2 * j + 1])) * row_scale) * sc[2 * j + 1];
+            o[j] = uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(lo))) |
+                   (uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(hi))) << 16);
+          }
+          *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + size_t(row) * p.N + n0) =
+              make_uint4(o[0], o[1], o[2], o[3]);
+        } else {
+          int32_t* dst = reinterpret_cast<int32_t*>(p.out) + size_t(row) * p.N + n0;
+          int4 b0 = make_int4(0, 0, 0, 0), b1 = make_int4(0, 0, 0, 0);
+          if (p.bias) {
+            b0 = __ldg(reinterpret_cast<const int4*>(p.bias + n0));
+            b1 = __ldg(reinterpret_cast<const int4*>(p.bias + n0 + 4));
+          }
+          // integer addition wraps (two's complement), as the reference's numerics require
+          *reinterpret_cast<uint4*>(dst) =
+              make_uint4(v[8 * q + 0] + uint32_t(b0.x), v[8 * q + 1] + uint32_t(b0.y),
+                         v[8 * q + 2] + uint32_t(b0.z), v[8 * q + 3] + uint32_t(b0.w));
+          *reinterpret_cast<uint4*>(dst + 4) =
+              make_uint4(v[8 * q + 4] + uint32_t(b1.x), v[8 * q + 5] + uint32_t(b1.y),
+                         v[8 * q + 6] + uint32_t(b1.z), v[8 * q + 7] + uint32_t(b1.w));
+        }
+      }
+    }
+  };
+  if (warp >= 2) {
     const int quadrant = warp & 3;
     uint32_t local = 0;
     for (int tile = first_tile; tile < tiles; tile += tile_step, ++local) {
@@ -203,6 +251,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (lane == 0) atomicExch(&g_w8a8_gemm_status, INTENT_B200_ERR_TIMEOUT);
         break;
       }
+      if (split) break;   // the partial sums of the cluster are put together below
       tcgen05_fence_after();
       const int row = (m_tile * CG + rank) * BM + quadrant * 32 + lane;
       const uint32_t taddr = tmem_base + acc * BN + (uint32_t(quadrant * 32) << 16);
@@ -213,44 +262,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         uint32_t v[32];
         tmem_load_32x32(taddr + c * 32, v);
         tmem_load_wait();
-        const int col = n_tile * BN + c * 32;
-        if (row < p.M) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int n0 = col + q * 8;
-            if (n0 < p.N) {  // N is a multiple of 16
-              if (EPILOGUE == 0) {
-                const float4 s0 = __ldg(reinterpret_cast<const float4*>(p.b_scales + n0));
-                const float4 s1 = __ldg(reinterpret_cast<const float4*>(p.b_scales + n0 + 4));
-                const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-                uint32_t o[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float lo = (float(int32_t(v[8 * q + 2 * j])) * row_scale) * sc[2 * j];
-                  const float hi = (float(int32_t(v[8 * q + 2 * j + 1])) * row_scale) * sc[2 * j + 1];
-                  o[j] = uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(lo))) |
-                         (uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(hi))) << 16);
-                }
-                *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + size_t(row) * p.N + n0) =
-                    make_uint4(o[0], o[1], o[2], o[3]);
-              } else {
-                int32_t* dst = reinterpret_cast<int32_t*>(p.out) + size_t(row) * p.N + n0;
-                int4 b0 = make_int4(0, 0, 0, 0), b1 = make_int4(0, 0, 0, 0);
-                if (p.bias) {
-                  b0 = __ldg(reinterpret_cast<const int4*>(p.bias + n0));
-                  b1 = __ldg(reinterpret_cast<const int4*>(p.bias + n0 + 4));
-                }
-                // integer addition wraps (two's complement), as the reference's numerics require
-                *reinterpret_cast<uint4*>(dst) =
-                    make_uint4(v[8 * q + 0] + uint32_t(b0.x), v[8 * q + 1] + uint32_t(b0.y),
-                               v[8 * q + 2] + uint32_t(b0.z), v[8 * q + 3] + uint32_t(b0.w));
-                *reinterpret_cast<uint4*>(dst + 4) =
-                    make_uint4(v[8 * q + 4] + uint32_t(b1.x), v[8 * q + 5] + uint32_t(b1.y),
-                               v[8 * q + 6] + uint32_t(b1.z), v[8 * q + 7] + uint32_t(b1.w));
-              }
-            }
-          }
-        }
+        finish(v, row, row_scale, n_tile * BN + c * 32);
       }
       tcgen05_fence_before();
       __syncwarp();
@@ -261,8 +273,39 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   }
 
+  __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
+  if (split) {
+    tcgen05_fence_after();
+    cluster_sync();   // the MMAs of all CTAs are done with the operand stages, where the sums go
+    if (first_tile < tiles && warp >= 2) {
+      int m_tile, n_tile;
+      tile_coords(first_tile, p, m_tile, n_tile);
+      const int quadrant = warp & 3, in_tile = quadrant * 32 + lane, row = m_tile * BM + in_tile;
+      const int chunks = min(kPartChunks, (p.N - n_tile * BN + 31) / 32), warps = min(4, (p.M - m_tile * BM + 31) / 32);
+      const uint32_t taddr = tmem_base + (uint32_t(quadrant * 32) << 16);
+      const PartRoom room{smem_a, warps};
+      if (warp == 2 && lane == 0) mbar_expect_tx(parts_full, expected_parts(share, chunks, warps));
+      if (quadrant < warps) {
+        send_parts(share, room, parts_full, taddr, chunks, quadrant, lane);
+        if (mbar_wait_warp_cluster(parts_full, 0)) {
+          float row_scale = 0.f;
+          if (EPILOGUE == 0 && row < p.M) row_scale = p.a_scales[row];
+          for (int c = share.rank; c < chunks; c += share.split) {
+            uint32_t v[32];
+            add_parts(share, room, taddr, c, quadrant, lane, [](uint32_t x, uint32_t y) { return x + y; }, v);
+            finish(v, row, row_scale, n_tile * BN + c * 32);
+          }
+        } else if (lane == 0) {
+          atomicExch(&g_w8a8_gemm_status, INTENT_B200_ERR_TIMEOUT);
+        }
+      }
+    }
+    __syncwarp();
+    tcgen05_fence_before();
+    cluster_sync();   // nothing is on its way to a CTA that is gone
+  }
   if (CG == 2) cluster_sync();   // the peer's shared memory and TMEM stay alive until both CTAs are done
   if (warp == 1) {
     tcgen05_fence_after();
@@ -304,12 +347,16 @@ int launch(const I8Operands& q, I8Params& p, int sms, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_status(e);
   const int tiles = p.m_tiles * p.n_tiles;
-  const int grid = CG * std::min(tiles, sms / CG);
+  p.split = CG == 1 && tiles <= 65535 ? split_of(tiles, p.k_blocks, q.M, B_K_MAJOR ? 0.25 : 0.45, sms) : 1;
+  const int grid = p.split > 1 ? tiles * p.split : CG * std::min(tiles, sms / CG);
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel),
-                         CG == 2 ? "i8_gemm_kernel CTA pairs, 256x256 tiles" : "i8_gemm_kernel 128x256 tiles, two accumulators",
-                         grid, THREADS, smem, CG);
-  e = launch_programmatic(kernel, grid, THREADS, smem, stream, CG, map_a, map_b, p);
+                         CG == 2       ? "i8_gemm_kernel CTA pairs, 256x256 tiles"
+                         : p.split > 1 ? "i8_gemm_kernel 128x256 tiles, k split over a cluster"
+                                       : "i8_gemm_kernel 128x256 tiles, two accumulators",
+                         grid, THREADS, smem, p.split > 1 ? p.split : CG);
+  const dim3 ctas = p.split > 1 ? dim3(unsigned(p.split), unsigned(tiles), 1) : dim3(unsigned(grid), 1, 1);
+  e = launch_programmatic(kernel, ctas, THREADS, smem, stream, p.split > 1 ? p.split : CG, map_a, map_b, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();
