@@ -341,6 +341,16 @@ INTENT_B200_API int intent_b200_moe_grouped_w4a16_upgate_silu_routed_f16(
     INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2), INTENT_B200_VIEW3(a3), INTENT_B200_VIEW3(a4),
     INTENT_B200_VIEW1(a5), INTENT_B200_VIEW2(a6), INTENT_B200_VIEW2(a7), int32_t group_size, int32_t zero_point,
     int32_t block_rows, void* stream);
+/* The same with a8 y [T,K] f32, which is zero afterwards: the buffer that the down projection below adds to, filled beside
+ * the contraction. */
+INTENT_B200_API int intent_b200_moe_grouped_w4a16_upgate_silu_clear_bf16(
+    INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2), INTENT_B200_VIEW3(a3), INTENT_B200_VIEW3(a4),
+    INTENT_B200_VIEW1(a5), INTENT_B200_VIEW2(a6), INTENT_B200_VIEW2(a7), INTENT_B200_VIEW2(a8), int32_t group_size,
+    int32_t zero_point, int32_t block_rows, void* stream);
+INTENT_B200_API int intent_b200_moe_grouped_w4a16_upgate_silu_clear_f16(
+    INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2), INTENT_B200_VIEW3(a3), INTENT_B200_VIEW3(a4),
+    INTENT_B200_VIEW1(a5), INTENT_B200_VIEW2(a6), INTENT_B200_VIEW2(a7), INTENT_B200_VIEW2(a8), int32_t group_size,
+    int32_t zero_point, int32_t block_rows, void* stream);
 /* Down projection with the weighted combine of examples/kernels/ragged/moe.py:43-53 in its epilogue:
  *   a0 hidden rows [P,K] T, a1 expert_blocks [B], a2 total_padded [1], a3 packed [E,K/8,WN], a4 scales [E,K/G,WN],
  *   a5 sorted_route_ids [>= P] i32 (route of every expert-sorted row; values outside [0, T*K) mark padding rows),

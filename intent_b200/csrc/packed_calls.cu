@@ -54,6 +54,8 @@ const Row kRows[] = {
     IB200_PACKED(intent_b200_moe_grouped_w4a16_down_scatter_tiled_bf16),
     IB200_PACKED(intent_b200_moe_grouped_w4a16_down_scatter_tiled_f16),
     IB200_PACKED(intent_b200_moe_grouped_w4a16_upgate_silu_bf16),
+    IB200_PACKED(intent_b200_moe_grouped_w4a16_upgate_silu_clear_bf16),
+    IB200_PACKED(intent_b200_moe_grouped_w4a16_upgate_silu_clear_f16),
     IB200_PACKED(intent_b200_moe_grouped_w4a16_upgate_silu_f16),
     IB200_PACKED(intent_b200_moe_grouped_w4a16_upgate_silu_routed_bf16),
     IB200_PACKED(intent_b200_moe_grouped_w4a16_upgate_silu_routed_f16),

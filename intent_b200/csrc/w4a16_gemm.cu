@@ -802,8 +802,9 @@ bool grouped_pairs(int64_t rows, int64_t experts) {
 template <typename T>
 int grouped_tmem(int mode, View2 x, View1 tile_expert, View1 total, View3 w, View3 s, void* out, int64_t out_cols,
                  int group_size, int zero_point, int block_rows, const int* row_route, const float* route_weight,
-                 int64_t routes, int top_k, cudaStream_t stream) {
+                 int64_t routes, int top_k, cudaStream_t stream, View2 clear = {}) {
   TmemCall q{};
+  q.clear = static_cast<float*>(clear.p), q.clear_vectors = clear.d0 * clear.d1 / 4;
   q.x = x.p, q.rows = x.d0, q.K = x.d1;
   q.w = w.p, q.s = s.p, q.experts = w.d0, q.WN = w.d2;
   q.out = out, q.out_cols = out_cols;
@@ -861,7 +862,7 @@ int skinny(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, c
 template <typename T, int MODE>
 int run_grouped(View2 x, View1 tile_expert, View1 total, View3 w, View3 s, View2 out, int group_size, int zero_point,
                 int block_rows, cudaStream_t stream, bool prelaid = false, const int* sorted_routes = nullptr,
-                int64_t routes = 0) {
+                int64_t routes = 0, View2 clear = {}) {
   const int64_t P = x.d0, K = x.d1, E = w.d0, WN = w.d2;
   const int64_t out_cols = MODE == MODE_UPGATE_SILU ? WN / 2 : WN;
   if (group_size != 32 && group_size != 64 && group_size != 128) return INTENT_B200_ERR_UNSUPPORTED;
@@ -870,7 +871,12 @@ int run_grouped(View2 x, View1 tile_expert, View1 total, View3 w, View3 s, View2
       out.d1 != out_cols || total.d0 < 1 || (block_rows != BM && block_rows != 2 * BM) ||
       tile_expert.d0 * block_rows < P)
     return INTENT_B200_ERR_SHAPE;
-  if (P == 0 || WN == 0 || E == 0) return INTENT_B200_OK;
+  // what no kernel below fills beside its work
+  const auto clear_alone = [&]() -> int {
+    if (clear.p == nullptr || observe_sink()) return INTENT_B200_OK;
+    return cuda_status(cudaMemsetAsync(clear.p, 0, size_t(clear.d0) * size_t(clear.d1) * sizeof(float), stream));
+  };
+  if (P == 0 || WN == 0 || E == 0) return clear_alone();
   if (!x.p || !w.p || !s.p || !out.p || !tile_expert.p || !total.p) return INTENT_B200_ERR_NULL;
   if (!contiguous(x) || !contiguous(w) || !contiguous(s) || !contiguous(out) || !contiguous(tile_expert))
     return INTENT_B200_ERR_LAYOUT;
@@ -880,9 +886,11 @@ int run_grouped(View2 x, View1 tile_expert, View1 total, View3 w, View3 s, View2
     return INTENT_B200_ERR_UNSUPPORTED;
   if (!prelaid) {
     const int status = grouped_tmem<T>(MODE, x, tile_expert, total, w, s, out.p, out_cols, group_size, zero_point,
-                                       block_rows, sorted_routes, nullptr, routes, 1, stream);
+                                       block_rows, sorted_routes, nullptr, routes, 1, stream, clear);
     if (status != INTENT_B200_ERR_UNSUPPORTED) return status;
   }
+  const int cleared = clear_alone();
+  if (cleared != INTENT_B200_OK) return cleared;
   if (block_rows == 2 * BM || (P + BM - 1) / BM <= PAIR_LIST_BLOCKS)   // 128-row blocks are paired by the kernel
     return launch_gemm<T, MODE, 2>(x.p, P, K, w.p, s.p, WN, out.p, out_cols, group_size, zero_point,
                                    static_cast<const int*>(total.p), static_cast<const int*>(tile_expert.p), stream,
@@ -1008,6 +1016,26 @@ IB200_GROUPED_ENTRY(intent_b200_moe_grouped_w4a16_down_f32_f16, __half, MODE_GRO
   }
 IB200_ROUTED_UPGATE_ENTRY(intent_b200_moe_grouped_w4a16_upgate_silu_routed_bf16, __nv_bfloat16)
 IB200_ROUTED_UPGATE_ENTRY(intent_b200_moe_grouped_w4a16_upgate_silu_routed_f16, __half)
+
+// the same with a buffer y [T, K] f32 that is zero afterwards
+#define IB200_CLEARING_UPGATE_ENTRY(NAME, TYPE)                                                                     \
+  extern "C" int NAME(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2), INTENT_B200_VIEW3(a3),     \
+                      INTENT_B200_VIEW3(a4), INTENT_B200_VIEW1(a5), INTENT_B200_VIEW2(a6), INTENT_B200_VIEW2(a7),     \
+                      INTENT_B200_VIEW2(a8), int32_t group_size, int32_t zero_point, int32_t block_rows,             \
+                      void* stream) {                                                                                \
+    if (a5_d0 < a0_d0 || a6_d0 < 0 || a6_d1 < 0 || a6_d0 * a6_d1 > (1 << 30)) return INTENT_B200_ERR_SHAPE;            \
+    if (a8_d0 != a6_d0 || a8_d1 != a0_d1) return INTENT_B200_ERR_SHAPE;                                              \
+    if ((a0_d0 > 0 && !a5) || (a8_d0 * a8_d1 > 0 && !a8)) return INTENT_B200_ERR_NULL;                               \
+    if (!ib200::contiguous(IB200_VIEW1_ARG(a5)) || !ib200::contiguous(IB200_VIEW2_ARG(a8)) || !ib200::aligned16(a8)) \
+      return INTENT_B200_ERR_LAYOUT;                                                                                 \
+    if (a8_d1 % 4 != 0) return INTENT_B200_ERR_UNSUPPORTED;                                                          \
+    return ib200::run_grouped<TYPE, ib200::MODE_UPGATE_SILU>(                                                        \
+        IB200_VIEW2_ARG(a0), IB200_VIEW1_ARG(a1), IB200_VIEW1_ARG(a2), IB200_VIEW3_ARG(a3), IB200_VIEW3_ARG(a4),     \
+        IB200_VIEW2_ARG(a7), group_size, zero_point, block_rows, static_cast<cudaStream_t>(stream), false,           \
+        static_cast<const int*>(a5), a6_d0 * a6_d1, IB200_VIEW2_ARG(a8));                                            \
+  }
+IB200_CLEARING_UPGATE_ENTRY(intent_b200_moe_grouped_w4a16_upgate_silu_clear_bf16, __nv_bfloat16)
+IB200_CLEARING_UPGATE_ENTRY(intent_b200_moe_grouped_w4a16_upgate_silu_clear_f16, __half)
 
 #define IB200_DOWN_SCATTER_ENTRY(NAME, TYPE)                                                                        \
   extern "C" int NAME(INTENT_B200_VIEW2(a0), INTENT_B200_VIEW1(a1), INTENT_B200_VIEW1(a2), INTENT_B200_VIEW3(a3),     \

@@ -73,6 +73,8 @@ struct TmemParams {
   const int* row_route;      // route of every row; a row with no route in [0, routes) is padding; null: all rows count
   const float* route_weight; // MODE_DOWN_SCATTER: [routes]
   int routes, top_k;
+  float4* clear;             // MODE_UPGATE_SILU: filled with zeros by a warp that has nothing else to do; may be null
+  int64_t clear_vectors;
 };
 
 // MODE_SKINNY: dense calls of at most SKINNY_ROWS rows, as precise as the bandwidth kernels that serve the others: the
@@ -429,6 +431,17 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       }
       if (!ok && lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
     }
+  } else if (MODE == MODE_UPGATE_SILU && warp == 3) {
+    // ------------------------------ zeros for the kernel that adds to this buffer ----
+    // In pieces of 2 KiB with a pause between them, about 1 TB/s over all SMs: far from the operands' loads in the way, and
+    // done before them (16384 tokens of 4096: 268 MB beside 600 us of contraction; a fill of its own took 38).
+    const int64_t step = int64_t(gridDim.x) * 128;
+    for (int64_t at = int64_t(blockIdx.x) * 128; at < p.clear_vectors; at += step) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (at + i * 32 + lane < p.clear_vectors) p.clear[at + i * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+      __nanosleep(200);
+    }
   } else if (warp >= FIRST_DEQUANT) {
     // ------------------------------ dequantisers --------------------------------
     const int set = (warp - FIRST_DEQUANT) >> 2, quadrant = warp & 3;
@@ -784,6 +797,8 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   p.route_weight = q.route_weight;
   p.routes = int(q.routes);
   p.top_k = q.top_k;
+  p.clear = reinterpret_cast<float4*>(q.clear);
+  p.clear_vectors = q.clear ? q.clear_vectors : 0;
   if (p.row_tile % (16 * CG) != 0 || p.row_tile < 16 * CG || p.row_tile > 128 * CG) return INTENT_B200_ERR_UNSUPPORTED;
   if (p.split < 1 || p.split > 8 || (p.split > 1 && (!dense_mode(MODE) || CG != 1 || p.k_blocks < p.split)))
     return INTENT_B200_ERR_UNSUPPORTED;

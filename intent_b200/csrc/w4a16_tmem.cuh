@@ -24,6 +24,8 @@ struct TmemCall {
   const float* route_weight;
   int64_t routes;
   int top_k;
+  float* clear;                // up|gate: a buffer that the call fills with zeros beside its work, or null
+  int64_t clear_vectors;       // its size in 16 bytes
 };
 
 // mode: the MODE_* numbers of w4a16_gemm.cu

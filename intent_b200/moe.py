@@ -174,8 +174,9 @@ class MoEW4A16FFN:
         # The fused chain reads no padding row, so on the reference layout it neither writes nor multiplies them.
         self._routed = self.fused_combine and not prelayout
         if self._routed:
+            # (the up|gate contraction clears the result that the down projection adds to)
             self._chain = (self._bind(programs.moe_gather_rows, dict(gathered, PADDING=False)),
-                           self._bind(programs.moe_grouped_upgate_silu, dict(grouped, ROUTED=True)))
+                           self._bind(programs.moe_grouped_upgate_silu, dict(grouped, ROUTED=True, CLEAR=True)))
         else:
             self._chain = (self.gather, self.up_gate)
 
@@ -199,6 +200,11 @@ class MoEW4A16FFN:
     def up_gate(self):
         """All rows, those of the padding among them; beside ``chain`` as :attr:`gather`."""
         return self._in_place_of(1, self._bind(programs.moe_grouped_upgate_silu, self._grouped))
+
+    @cached_property
+    def _routed_up_gate(self):
+        """The up|gate contraction of the routed rows for a ``y`` that is there already."""
+        return self._bind(programs.moe_grouped_upgate_silu, dict(self._grouped, ROUTED=True))
 
     def _in_place_of(self, step, artifact):
         if self._routed:
@@ -254,15 +260,20 @@ class MoEW4A16FFN:
         """y[t] (+)= sum_c topk_weights[t, c] * FFN_{topk_ids[t, c]}(x[t]); y f32 [T, H]."""
         import torch
 
-        if y is None:
+        clears = y is None and self._routed and tuple(x.shape) == (topk_weights.shape[0], self.hidden)
+        if y is None and not clears:
             y = torch.zeros((x.shape[0], self.hidden), dtype=torch.float32, device=x.device)
         if self.fused_combine:
             up_gate_packed, down_packed = self._weights(up_gate_packed, down_packed)
             sorted_routes, expert_blocks, total = self.alignment.run(topk_ids)
             gather, up_gate = self._chain
             rows = gather.run(x, sorted_routes, total)
-            hidden = up_gate.run(*self._up_gate_inputs(rows, expert_blocks, total, up_gate_packed, up_gate_scales,
-                                                       sorted_routes, topk_weights))
+            inputs = self._up_gate_inputs(rows, expert_blocks, total, up_gate_packed, up_gate_scales, sorted_routes,
+                                          topk_weights)
+            if clears:
+                hidden, y = up_gate.run(*inputs)
+            else:
+                hidden = (self._routed_up_gate if self._routed else up_gate).run(*inputs)
             self.down_scatter(hidden, expert_blocks, total, down_packed, down_scales, sorted_routes, topk_weights, y)
             return y
         rows, positions = self.experts_forward(x, topk_ids, up_gate_packed, up_gate_scales, down_packed,
@@ -284,6 +295,8 @@ class MoEW4A16FFN:
         sorted_routes, expert_blocks, total = align.result()
         if self.fused_combine and not clear_positions:
             gather, up_gate = self._chain
+            if self._routed:
+                up_gate = self._routed_up_gate
             gather_call = gather.prepare(x, sorted_routes, total)
             up_call = up_gate.prepare(*self._up_gate_inputs(gather_call.result(), expert_blocks, total, up_gate_packed,
                                                             up_gate_scales, sorted_routes, topk_weights))

@@ -416,11 +416,15 @@ def _lower_grouped(c, device, *, gated):
     if gated and c["ROUTED"]:
         if suffix:
             raise CompilationStageError("provider_native_compilation", "ROUTED needs WEIGHT_LAYOUT 'reference'")
-        stem += "_routed"
+        stem += "_clear" if c["CLEAR"] else "_routed"
         views += [ViewParameter(5, "sorted_route_ids", dtypes.i32, ("S",), IN, alignment=4),
                   ViewParameter(6, "route_weights", dtypes.f32, ("T", "TOP_K"), IN, alignment=4)]
         rules.append(_rule(lambda d: d["S"] >= d["P"], "sorted_route_ids must cover every row"))
     views.append(ViewParameter(len(views), "output", act if gated else dtypes.f32, ("P", out_cols), OUT))
+    if gated and c["CLEAR"]:
+        if not c["ROUTED"]:
+            raise CompilationStageError("provider_native_compilation", "CLEAR needs ROUTED")
+        views.append(ViewParameter(len(views), "y", dtypes.f32, ("T", "K"), OUT))
     return NativeProgram(interface=PublicInterface(tuple(views), dimension_rules=tuple(rules)),
                          entry_name=f"intent_b200_moe_grouped_w4a16_{stem}{suffix}_{act.name}",
                          constants=(group, zp, block), device=device)
@@ -447,11 +451,11 @@ def _grouped_weight(c, group):
 _GROUPED_CONSTEXPRS = {"GROUP_SIZE": 128, "ZERO_POINT": 8, "ACT_DTYPE": "bf16", "BLOCK_ROWS": 128,
                        "WEIGHT_LAYOUT": "reference"}
 moe_grouped_upgate_silu = KernelDefinition(
-    "moe_grouped_upgate_silu", dict(_GROUPED_CONSTEXPRS, ROUTED=False), lambda c, d: _lower_grouped(c, d, gated=True),
+    "moe_grouped_upgate_silu", dict(_GROUPED_CONSTEXPRS, ROUTED=False, CLEAR=False), lambda c, d: _lower_grouped(c, d, gated=True),
     "examples/kernels/ragged/grouped_gemm.py:42-70, examples/kernels/ragged/moe.py:37-42, "
     "examples/kernels/activation/swiglu.py:27-46",
     "hidden = silu(rows @ Wgate[e]) * (rows @ Wup[e]) per expert block, int4 weights (ROUTED: rows that no route fills "
-    "are left out)")
+    "are left out; CLEAR, with it: a second result y [T, K] of zeros, for the down projection to add to)")
 moe_grouped_down = KernelDefinition(
     "moe_grouped_down", dict(_GROUPED_CONSTEXPRS), lambda c, d: _lower_grouped(c, d, gated=False),
     "examples/kernels/ragged/grouped_gemm.py:42-70, examples/kernels/ragged/moe.py:43-47",

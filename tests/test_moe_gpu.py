@@ -264,3 +264,26 @@ def test_a_layer_says_what_a_call_ran(cuda_device, prelayout):
     sorted_routes, _, total = layer.alignment.run(ids)
     layer.gather.run(dev["x"], sorted_routes, total)
     assert layer.gather.observation.entry == "intent_b200_moe_gather_rows"
+
+
+@pytest.mark.parametrize("tokens,hidden", [(1, 128), (33, 1152), (300, 256)])
+def test_a_call_clears_its_result(cuda_device, tokens, hidden):
+    """The up|gate contraction zero-fills the result: whatever its memory held before, a call gives what adding to a zeroed
+    ``y`` gives, bit for bit, and an unrouted token's row is zero."""
+    intermediate, experts = 128, 4
+    data, _, _ = _ffn_case(tokens, hidden, intermediate, experts, torch.bfloat16, seed=8)
+    dev = {k: v.to(cuda_device) for k, v in data.items()}
+    layer = MoEW4A16FFN(tokens=tokens, hidden=hidden, intermediate=intermediate, experts=experts, target=ib.B200Target(0))
+    ids, weights = layer.route(dev["logits"])
+    ids[-1] = -1                                                   # the last token goes nowhere
+    args = (dev["x"], ids, weights, dev["up_gate_packed"], dev["up_gate_scales"], dev["down_packed"], dev["down_scales"])
+    expected = layer(*args, y=torch.zeros((tokens, hidden), dtype=torch.float32, device=cuda_device))
+    for _ in range(4):
+        stale = torch.full((tokens, hidden), float("nan"), dtype=torch.float32, device=cuda_device)
+        del stale                                                  # (the result comes from this block)
+        assert torch.equal(layer(*args), expected)
+    assert not expected[-1].any()
+    onto = torch.ones((tokens, hidden), dtype=torch.float32, device=cuda_device)
+    assert layer(*args, y=onto) is onto and torch.equal(onto[-1], torch.ones_like(onto[-1]))
+    with pytest.raises((TypeError, ValueError, RuntimeError)):     # one token more than there are weights
+        layer(torch.cat((dev["x"], dev["x"][:1])), *args[1:])
