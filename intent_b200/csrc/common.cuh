@@ -162,6 +162,15 @@ struct Elem<__half> {
   // 0x6400 | q is the half 1024 + q (ulp is 1 at 2^10); subtracting 1032 gives q - 8 exactly.
   static constexpr uint32_t kMagic2 = 0x64006400u;
   static constexpr uint32_t kBias2 = 0x64086408u;  // half2(1032, 1032)
+  // The bits q alone are the half q * 2^-24: times 2^15, less 2^-6, they give (q - 8) * 2^-9 exactly.
+  __device__ static __forceinline__ uint32_t tiny2(uint32_t q) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(q), "r"(0x78007800u), "r"(0xA400A400u));
+    return d;
+  }
+  static constexpr float kTinyScale = 512.f;
+  static constexpr uint32_t kTinyScale2 = 0x60006000u;
+  static constexpr bool kWideScale = false;        // a scale times that may leave the type's range
   __device__ static __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -198,6 +207,15 @@ struct Elem<__nv_bfloat16> {
   // 0x4300 | q is the bfloat16 128 + q (ulp is 1 at 2^7); subtracting 136 gives q - 8 exactly.
   static constexpr uint32_t kMagic2 = 0x43004300u;
   static constexpr uint32_t kBias2 = 0x43084308u;  // bf16x2(136, 136)
+  // The bits q alone are the bfloat16 q * 2^-133: times 2^127, less 2^-3, they give (q - 8) * 2^-6 exactly.
+  __device__ static __forceinline__ uint32_t tiny2(uint32_t q) {
+    uint32_t d;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(q), "r"(0x7F007F00u), "r"(0xBE00BE00u));
+    return d;
+  }
+  static constexpr float kTinyScale = 64.f;
+  static constexpr uint32_t kTinyScale2 = 0x42804280u;
+  static constexpr bool kWideScale = true;         // a scale times that stays in the type's range (up to 2^121)
   __device__ static __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
