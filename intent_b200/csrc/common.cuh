@@ -98,7 +98,9 @@ cudaError_t launch_programmatic(void (*kernel)(P...), dim3 grid, dim3 block, siz
   attribute[1].val.clusterDim.z = 1;
   config.attrs = attribute;
   config.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&config, kernel, static_cast<P>(arguments)...);
+  const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<P>(arguments)...);
+  if (e != cudaSuccess) cudaGetLastError();   // (returned here, and not left for the next one who asks)
+  return e;
 }
 
 #define IB200_VIEW1_ARG(p) ib200::View1{p, p##_d0, p##_s0}

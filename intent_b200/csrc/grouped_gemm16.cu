@@ -20,6 +20,7 @@
 // its group loads rows of the next group (or zeros past the last row); the epilogue writes
 // only rows of its own group.  Programs whose rows are selected through an index list gather
 // them once into a workspace in member order; the epilogue scatters through the same list.
+// Calls with few tiles share a tile's k blocks among the CTAs of a cluster (split_k.cuh).
 // Every wait is bounded; a wait that gives up records a timeout status and the kernel drains.
 #include <type_traits>
 
@@ -44,6 +45,7 @@ constexpr int THREADS = 6 * 32;
 constexpr int MAX_GROUPS = 1024;
 constexpr int TABLE_BYTES = 3 * (MAX_GROUPS + 1) * 4;
 constexpr int SMEM_BYTES = 1024 + STAGES * (A_BYTES + B_BYTES) + 256 + TABLE_BYTES;
+static_assert(STAGES * (A_BYTES + B_BYTES) >= kPartRoom, "the sums of a cluster lie where the operands were");
 
 enum Epilogue { kCast = 0, kReluCast = 1, kWeightedAdd = 2, kQuantize = 3 };
 

@@ -705,7 +705,7 @@ bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split
     const int64_t ctas = tiles * (pair ? 2 : split);
     double cost;
     if (split > 1) {
-      if (!split_allowed) return;
+      if (!split_allowed || M >= TMEM_MAX_ROWS) return;
       // clusters of four do not fill every part of the chip: 33 of them were seen side by side
       if (K <= 2048 || blocks < 4 * split || ctas > (split == 2 ? sms : sms * 9 / 10)) return;
       cost = (split == 2 ? 6.2 : 6.7) + 0.014 * double(rows) +
@@ -843,6 +843,7 @@ int skinny(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, c
   if (asked <= 0 || !workspace || !aligned16(workspace) || workspace_bytes < asked) return kTableDeclined;
   const int64_t tiles = (N + 127) / 128, blocks = (K + 127) / 128, sms = device_sms();
   if (M <= 6 && 2 * tiles > sms) return kTableDeclined;
+  if (M <= 8 && (!selection().table_single || !selection().table_ride)) return kTableDeclined;   // (asked not to take them)
   int split = 1;
   while (split < 4 && tiles * split * 2 <= (split == 1 ? sms : sms * 9 / 10) && blocks >= 8 * split) split *= 2;
   TmemCall q{};

@@ -12,11 +12,12 @@
 // The expanded weights never pass through shared memory, and a tile has as many rows as the call has, in steps of
 // 16, instead of 128.
 //
-// What bounds it: per 128 k 530 to 565 cycles for a lone tile or a pair of up to 128 rows - the issue loop, beside 330 issue
-// slots of every scheduler for the dequantisers and, at 128 rows of a pair, 512 cycles of MMAs; 1058 at 256 rows of a pair
-// (MMAs 1024).  With all SMs at work a pair takes 0.40 us per 128 k, with the tensor pipe 44 % and the L2 16 % busy (M1024
-// K4096 N4096): the hand-overs between the roles, not a throughput.  Against the forms with the weights in shared memory: M77 K14336 N4096 81.1 -> 18.0 us, M1024 K4096 N4096 50.9 -> 30.3, 64 tokens on 64 experts of
-// 4096 x 1408 277 + 120 -> 103 + 56.
+// What bounds it: per 128 k 600 cycles for a lone tile or a pair of up to 128 rows with all SMs at work - the issue loop (450 of
+// them) and the dequantisers, 290 issue slots of every scheduler (f16 320), hand their blocks to each other; with neither
+// conversion nor more than one MMA a block it is 560.  At 256 rows of a pair the MMAs' 1024 cycles count.  A small call is start-up (the
+// wait for the kernel ahead ends 1.3 us after that kernel, first words 1 us later), its k blocks and the exchange between
+// the CTAs of a cluster (2 us).  Against the forms with the weights in shared memory: M77 K14336 N4096 81.1 -> 14.5 us,
+// M1024 K4096 N4096 50.9 -> 28, 64 tokens on 64 experts of 4096 x 1408 414 -> 155 (the whole layer).
 #include <type_traits>
 
 #include "cluster.cuh"

@@ -15,6 +15,7 @@
 // K32 MMAs per stage, warps 2..5 drain the two TMEM accumulators.  What bounds it is the rate at
 // which operands get into and out of shared memory; the pair reads two thirds of the bytes per
 // operation.  4096 x 8192 x 8192 scaled, calls back to back: 214.7 -> 200.5 us (2.56 -> 2.74 POP/s).
+// Calls with few tiles share a tile's k blocks among the CTAs of a cluster (split_k.cuh).
 // With B_K_MAJOR the second operand is given as [N,K] (K contiguous, e.g. decoded packed weights)
 // and is loaded as one 256-row K-major box.
 // Every wait is bounded (see tma.cuh); a wait that gives up records a timeout status.
@@ -46,6 +47,8 @@ struct Ring {
   static constexpr int B_BYTES = 2 * B_BOX_BYTES / CG;
   static constexpr int SMEM_BYTES = 1024 + STAGES * (A_BYTES + B_BYTES) + 256;
 };
+
+static_assert(Ring<1>::STAGES * (A_BYTES + Ring<1>::B_BYTES) >= kPartRoom, "the sums of a cluster lie where the operands were");
 
 constexpr int64_t BAND_BYTES = int64_t(64) << 20;   // of A, from which on rows are walked in bands
 
