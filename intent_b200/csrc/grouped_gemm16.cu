@@ -87,7 +87,8 @@ struct TileWalk {
   }
 };
 
-template <typename T, bool B_K_MAJOR, int EPILOGUE>
+// SPLIT: an instance of its own (in one with both ways whole tiles took a hundredth longer)
+template <typename T, bool B_K_MAJOR, int EPILOGUE, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
 grouped_gemm16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const Params p) {
@@ -157,10 +158,10 @@ grouped_gemm16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const int tiles = s_prefix[p.groups];
   // split: a row of the grid is a cluster, and has one tile or none.  (Offsets that do not rise can ask for more tiles than
   // there are clusters: every CTA then walks whole tiles.)
-  const bool split = p.split > 1 && tiles <= int(gridDim.y);
+  const bool split = SPLIT && tiles <= int(gridDim.y);
   const SplitShare share{split ? int(cluster_rank()) : 0, p.split};
-  const int first_tile = split ? int(blockIdx.y) : int(blockIdx.x + gridDim.x * blockIdx.y);
-  const int tile_step = split ? max(tiles, 1) : int(gridDim.x * gridDim.y);
+  const int first_tile = split ? int(blockIdx.y) : int(SPLIT ? blockIdx.x + gridDim.x * blockIdx.y : blockIdx.x);
+  const int tile_step = split ? max(tiles, 1) : int(SPLIT ? gridDim.x * gridDim.y : gridDim.x);
   const int kb_first = split ? share.first(p.k_blocks) : 0, kb_count = split ? share.count(p.k_blocks) : p.k_blocks;
 
   if (warp == 0) {
@@ -460,10 +461,10 @@ int launch(const Problem& q, cudaStream_t stream) {
                                   uint64_t(q.N), uint64_t(q.N) * 2, uint64_t(q.K) * uint64_t(q.N) * 2, BK, 64,
                                   CU_TENSOR_MAP_SWIZZLE_128B);
   if (!ok) return INTENT_B200_ERR_UNSUPPORTED;
-  auto kernel = grouped_gemm16_kernel<T, B_K_MAJOR, EPILOGUE>;
+  p.split = tile_bound > 0 ? split_of(tile_bound, p.k_blocks / 2, q.rows, 0.45, sms) : 1;   // (blocks of 64 k)
+  auto kernel = p.split > 1 ? grouped_gemm16_kernel<T, B_K_MAJOR, EPILOGUE, true> : grouped_gemm16_kernel<T, B_K_MAJOR, EPILOGUE, false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return cuda_status(e);
-  p.split = tile_bound > 0 ? split_of(tile_bound, p.k_blocks / 2, q.rows, 0.45, sms) : 1;   // (blocks of 64 k)
   const int grid = int(p.split > 1 ? tile_bound * p.split : tile_bound < sms ? (tile_bound > 0 ? tile_bound : 1) : sms);
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel), p.split > 1 ? "grouped_gemm16_kernel 128x256 tiles, k split over a cluster"

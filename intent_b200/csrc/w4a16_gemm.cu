@@ -682,9 +682,9 @@ Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
 //   no split up to K = 2048 (there a row keeps its bits, see below)   M36 K1792 N5336 6.9 split in two, 7.5 whole, 16.6 above
 // The entry of the tensor-core kernels keeps to K >= 2048 and fewer than 2048 rows, for the same reason.  Between, this kernel
 // against the forms above: M20 K1536 N2384 9.9 of 18.8, M546 K1408 N1112 8.3 of 23.0, M983 K1536 N5768 17.6 of 38.4.
-// From 2048 rows on it has to be a fifth faster by the estimate, which does not know the power cap: M2180 K7936 N1224 33.6 of
-// 81.0, M2358 K1920 N7512 50.8 of 87.1, M3339 K6016 N8032 227 of 326, but M2048 K4096 N4096 60.8 of 53.7, M4096 K4096 N4096
-// 120.8 of 117.7, 8192 cubed 917 of 921.
+// From 2048 rows on it has to be faster by the estimate, which does not know the power cap, by a fifth, or by a third where
+// the other form takes 100 us: M2180 K7936 N1224 33.6 of 81.0, M2358 K1920 N7512 50.8 of 87.1, M3339 K6016 N8032 227 of 326,
+// but M2048 K4096 N4096 60.8 of 53.7, M4096 K4096 N4096 120.8 of 117.7, 8192 cubed 939 of 916 (a fifth by the estimate).
 // Where a split is allowed from K = 2048 on, unsplit calls with less than a tile for every second SM are left out.  A split changes the order of a row's sum: which split a call takes follows
 // from its rows, its columns, the number of SMs and the pairs switch, so where one is allowed (the entry that chooses
 // among all kernels) a row agrees with the same row of another call, and a column shard with the whole, to rounding only.
@@ -695,7 +695,7 @@ bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split
                  bool* pairs) {
   const int64_t sms = device_sms(), blocks = (K + 127) / 128;
   if (sms <= 0 || K <= 1152 || (!split_allowed && (K < 2048 || M >= TMEM_MAX_ROWS))) return false;
-  const double limit = M >= TMEM_MAX_ROWS ? other / 1.2 : other;
+  const double limit = M < TMEM_MAX_ROWS ? other : other > 100.0 ? other / 1.35 : other / 1.2;
   double best = limit;
   const auto consider = [&](bool pair, int64_t row_tiles, int split) {
     const int64_t unit = pair ? 32 : 16, most = pair ? 256 : 128;

@@ -81,7 +81,8 @@ __device__ __forceinline__ void tile_coords(int tile, const I8Params& p, int& m_
 }
 
 // EPILOGUE 0: bf16(acc * sa[m] * sb[n]);  1: int32 acc + bias[n]
-template <int EPILOGUE, bool B_K_MAJOR, int CG>
+// SPLIT: lone tiles, each shared by a cluster (an instance of its own: the other ones keep their registers)
+template <int EPILOGUE, bool B_K_MAJOR, int CG, bool SPLIT = false>
 __global__ void __launch_bounds__(THREADS, 1)
 i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const I8Params p) {
@@ -105,7 +106,7 @@ i8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int warp = tid >> 5;
   const int lane = tid & 31;
   const int tiles = p.m_tiles * p.n_tiles;
-  const bool split = CG == 1 && p.split > 1;
+  constexpr bool split = CG == 1 && SPLIT;
   const int rank = CG == 2 ? int(cluster_rank()) : 0;
   const SplitShare share{split ? int(cluster_rank()) : 0, p.split};
   // split: a row of the grid is a cluster, and has one tile
@@ -345,12 +346,12 @@ int launch(const I8Operands& q, I8Params& p, int sms, cudaStream_t stream) {
                   : make_tensor_map_2d(&map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, q.b.p, uint64_t(q.K), uint64_t(q.N),
                                        uint64_t(q.N), BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)))
     return INTENT_B200_ERR_UNSUPPORTED;
-  auto kernel = i8_gemm_kernel<EPILOGUE, B_K_MAJOR, CG>;
+  const int tiles = p.m_tiles * p.n_tiles;
+  p.split = CG == 1 && tiles <= 65535 ? split_of(tiles, p.k_blocks, q.M, B_K_MAJOR ? 0.25 : 0.45, sms) : 1;
+  auto kernel = p.split > 1 ? i8_gemm_kernel<EPILOGUE, B_K_MAJOR, CG, CG == 1> : i8_gemm_kernel<EPILOGUE, B_K_MAJOR, CG, false>;
   constexpr int smem = Ring<CG>::SMEM_BYTES;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_status(e);
-  const int tiles = p.m_tiles * p.n_tiles;
-  p.split = CG == 1 && tiles <= 65535 ? split_of(tiles, p.k_blocks, q.M, B_K_MAJOR ? 0.25 : 0.45, sms) : 1;
   const int grid = p.split > 1 ? tiles * p.split : CG * std::min(tiles, sms / CG);
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel),
