@@ -7,6 +7,12 @@
 
 namespace ib200 {
 
+// How many CTAs of clusters of that size run side by side: larger clusters do not fill every part of the chip.  33 clusters of
+// four were seen at once; with 14 of eight a call took 6.4 us, with 16 it took two rounds (M18 K5760 N1752, and M12 K8192 N2048 13.7 us against 10.3 with clusters of four).
+inline int64_t clustered_ctas(int cluster, int64_t sms) {
+  return cluster <= 2 ? sms : cluster == 4 ? sms * 9 / 10 : sms * 77 / 100;
+}
+
 #ifdef __CUDACC__
 
 __device__ __forceinline__ uint32_t cluster_rank() {

@@ -22,14 +22,13 @@ constexpr int kPartRoom = 192 * 1024;           // shared memory for the sums th
 
 // How many CTAs share a tile of up to `rows` rows: the least by estimate, in microseconds, `block` for 128 k of a lone tile
 // (0.45; int8 rows of B in one box each 0.25) and 3 to 5 for the exchange, 1.5 more among eight.  What bounds the choice is
-// room: clusters do not fill every part of the chip - 33 of four and 16 of eight CTAs run side by side - and the sums have
-// kPartRoom.
+// room, for the clusters (clustered_ctas) and for the sums.
 inline int split_of(int64_t tiles, int64_t k_blocks, int64_t rows, double block, int64_t sms) {
   const int64_t warps = rows >= 128 ? 4 : (rows + 31) / 32;
   int best = 1;
   double least = block * double(k_blocks);
   for (int split = 2; split <= 8; split *= 2) {
-    if (tiles * split > (split == 2 ? sms : split == 4 ? sms * 9 / 10 : sms * 7 / 8) || k_blocks < 2 * split) break;
+    if (tiles * split > clustered_ctas(split, sms) || k_blocks < 2 * split) break;
     if (2 * (kPartChunks - kPartChunks / split) * warps * kPartBytes > kPartRoom) break;
     const double cost = block * double((k_blocks + split - 1) / split) + 3.0 + 0.5 * double(warps) + (split == 8 ? 1.5 : 0.0);
     if (cost < least) least = cost, best = split;

@@ -51,6 +51,7 @@
 //           the result does not depend on the order of the two additions: (0 + a) + b == (0 + b) + a.
 #include <type_traits>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "tma.cuh"
 #include "umma.cuh"
@@ -671,7 +672,7 @@ Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
 // times below, if that is less than what the forms above take.  Microseconds, bf16, group 128, replayed as a graph over
 // weights that do not stay in the L2; `blocks` are k blocks of 128 per CTA:
 //   lone CTA of r <= 128 rows x 128 columns   4.2 + 0.014 r + waves * blocks * (0.24 + 0.0014 r)
-//   the k blocks over a cluster of 2 or 4     + 2.0 or 2.5, one wave
+//   the k blocks over a cluster of 2, 4 or 8  + 2.0, 2.5 or 3.3 + 0.010 r, one wave
 //   CTA pair of r rows x 256 columns          5 + 0.012 r + waves * blocks * (0.405 at 128 rows, 0.52 at 192, 0.735 at 256)
 // Measured against the forms above: M17 K4096 N4096 27.2 -> 9.2 us, M77 K14336 N4096 81.1 -> 18.0, M256 K8192 N1024
 // 48.8 -> 13.1, M256 K4096 N14336 52.9 -> 30.4, M512 K2048 N4096 19.8 -> 13.5, M1024 K4096 N4096 50.9 -> 30.3.
@@ -690,7 +691,8 @@ Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
 // among all kernels) a row agrees with the same row of another call, and a column shard with the whole, to rounding only.
 // Up to K = 2048 nothing is split and the bits are the same.  The entry of the tensor-core kernels and the tiled layout
 // never split and take whole tiles however few there are: M77 K4096 N4096 14.2 us against 10.8 with a split, M77 K14336
-// N4096 37.1 against 17.0, M511 K8192 N1024 23.8 against 16.4 (27.1, 81.0 and 48.7 with the weights in shared memory).
+// N4096 37.1 against 17.0, M511 K8192 N1024 23.8 against 16.4 (27.1, 81.0 and 48.7 with the weights in shared memory).  Eight CTAs in place of four:
+// M35 K8064 N1024 9.0 -> 7.2, M24 K6144 N1536 7.8 -> 6.5.
 bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split_allowed, double other, TmemCall* call,
                  bool* pairs) {
   const int64_t sms = device_sms(), blocks = (K + 127) / 128;
@@ -706,9 +708,8 @@ bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split
     double cost;
     if (split > 1) {
       if (!split_allowed || M >= TMEM_MAX_ROWS) return;
-      // clusters of four do not fill every part of the chip: 33 of them were seen side by side
-      if (K <= 2048 || blocks < 4 * split || ctas > (split == 2 ? sms : sms * 9 / 10)) return;
-      cost = (split == 2 ? 6.2 : 6.7) + 0.014 * double(rows) +
+      if (K <= 2048 || blocks < 4 * split || ctas > clustered_ctas(split, sms)) return;
+      cost = (split == 2 ? 6.2 : split == 4 ? 6.7 : 7.5) + (split == 8 ? 0.024 : 0.014) * double(rows) +
              double((blocks + split - 1) / split) * (0.24 + 0.0014 * double(rows));
     } else {
       if (split_allowed && K >= 2048 && 2 * ctas < sms) return;
@@ -730,10 +731,10 @@ bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split
   const int64_t least_rows = M >= TMEM_MAX_ROWS ? 128 : K < 2048 ? 48 : 64, most_tiles = (M + 31) / 32;
   for (int64_t t = (M + 255) / 256; t <= (M + least_rows - 1) / least_rows && t <= most_tiles; ++t) {
     if (pairs_allowed) consider(true, t, 1);
-    for (const int split : {1, 2, 4}) consider(false, t, split);
+    for (const int split : {1, 2, 4, 8}) consider(false, t, split);
   }
   if (M < 64) {
-    for (const int split : {1, 2, 4}) consider(false, 1, split);
+    for (const int split : {1, 2, 4, 8}) consider(false, 1, split);
   }
   return best < limit;
 }
@@ -818,8 +819,8 @@ int grouped_tmem(int mode, View2 x, View1 tile_expert, View1 total, View3 w, Vie
 }
 
 // Calls of SKINNY_LEAST to 16 rows with the weights in tensor memory and the scales in f32 (kTableDeclined: not that kind
-// of call, or one that the bandwidth kernel refuses with its own status).  Tiles are spread over clusters of up to four CTAs
-// as long as every CTA keeps four k blocks.  Against the bandwidth kernel (bf16, group 128, cold weights): M16 K4096 N4096
+// of call, or one that the bandwidth kernel refuses with its own status).  Tiles are spread over clusters of up to eight CTAs
+// as long as every CTA keeps four k blocks (eight in place of four: M16 K8192 N1024 10.1 -> 7.3, M16 K4096 N1024 7.3 -> 5.9).  Against the bandwidth kernel (bf16, group 128, cold weights): M16 K4096 N4096
 // 21.9 -> 9.8 us, M9 18.0 -> 9.6, M16 K8192 N1024 25.4 -> 11.6, M16 K1024 N1024 16.2 -> 6.6, M16 K4096 N14336 47.0 -> 16.4;
 // error against 64 bits 2.08e-4 of 2.09e-4 (f16), 1.673e-3 of 1.673e-3 (bf16).  Against the ride-along kernel (bf16, group
 // 128): M6 K4096 N4096 9.5 -> 7.9 us, K1024 N1024 8.1 -> 6.2, K8192 N8192 18.7 -> 17.3, K8192 N1024 10.4 and 10.4; four rows
@@ -845,7 +846,7 @@ int skinny(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, c
   if (M <= 6 && 2 * tiles > sms) return kTableDeclined;
   if (M <= 8 && (!selection().table_single || !selection().table_ride)) return kTableDeclined;   // (asked not to take them)
   int split = 1;
-  while (split < 4 && tiles * split * 2 <= (split == 1 ? sms : sms * 9 / 10) && blocks >= 8 * split) split *= 2;
+  while (split < 8 && tiles * split * 2 <= clustered_ctas(2 * split, sms) && blocks >= 8 * split) split *= 2;
   TmemCall q{};
   q.x = x.p, q.rows = M, q.K = K;
   q.w = w.p, q.s = s.p, q.experts = 1, q.WN = N;

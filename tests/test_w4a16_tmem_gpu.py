@@ -26,6 +26,7 @@ LONE, PAIRS, SPLIT = ("w4a16_tmem_kernel " + s for s in ("single CTA", "CTA pair
     (torch.bfloat16, 8, 128, 511, 8192, 8200, PAIRS),                  # 256-row tiles, one accumulator
     (torch.float16, 8, 128, 1030, 4096, 4104, PAIRS),                  # 128-row tiles, eight columns in the last tile
     (torch.bfloat16, 8, 128, 35, 2048, 19208, LONE),                   # more tiles than SMs, three rows past a chunk of 32
+    (torch.float16, 8, 128, 33, 8192, 1032, SPLIT),                    # eight CTAs a tile
     (torch.float16, "twos_complement", 32, 36, 1184, 1000, LONE),      # the shortest K, a quarter of a block at its end
     (torch.bfloat16, 8, 128, 546, 1408, 1112, LONE),                   # twelve row tiles of 48
     (torch.bfloat16, 8, 64, 2180, 2112, 1224, PAIRS),                  # more than 2047 rows
@@ -57,6 +58,7 @@ def test_dense_tiles(cuda_device, dtype, zero_point, group, M, K, N, kernel):
     (torch.bfloat16, "twos_complement", 32, 9, 1056, 136),       # four groups a k block, a quarter block at the end
     (torch.float16, "twos_complement", 64, 13, 2112, 1000),
     (torch.bfloat16, 8, 128, 12, 2048, 19208),                   # more tiles than SMs
+    (torch.bfloat16, 8, 64, 13, 8256, 520),                      # eight CTAs a tile, four of which own no row
     (torch.float16, 8, 128, 5, 4096, 9472),                      # the fewest rows, on the most columns that they may have
     (torch.bfloat16, "twos_complement", 32, 8, 1056, 1032),
     (torch.bfloat16, 8, 64, 7, 2112, 9608),                      # more tiles than half the SMs
