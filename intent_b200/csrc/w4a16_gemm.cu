@@ -686,13 +686,14 @@ Form choose_form(int64_t M, int64_t K, int64_t N, bool pairs, double* time) {
 // From 2048 rows on it has to be faster by the estimate, which does not know the power cap, by a fifth, or by a third where
 // the other form takes 100 us: M2180 K7936 N1224 33.6 of 81.0, M2358 K1920 N7512 50.8 of 87.1, M3339 K6016 N8032 227 of 326,
 // but M2048 K4096 N4096 60.8 of 53.7, M4096 K4096 N4096 120.8 of 117.7, 8192 cubed 939 of 916 (a fifth by the estimate).
-// Where a split is allowed from K = 2048 on, unsplit calls with less than a tile for every second SM are left out.  A split changes the order of a row's sum: which split a call takes follows
-// from its rows, its columns, the number of SMs and the pairs switch, so where one is allowed (the entry that chooses
-// among all kernels) a row agrees with the same row of another call, and a column shard with the whole, to rounding only.
+// Where a split is allowed, from K = 2048 on, unsplit calls with less than a tile for every second SM are left out.
+// A split (of calls of fewer than 2048 rows) changes the order of a row's sum: which split a call takes follows from its rows,
+// its columns, the number of SMs and the pairs switch, so where one is allowed (the entry that chooses among all kernels) a row
+// agrees with the same row of another call, and a column shard with the whole, to rounding only.
 // Up to K = 2048 nothing is split and the bits are the same.  The entry of the tensor-core kernels and the tiled layout
 // never split and take whole tiles however few there are: M77 K4096 N4096 14.2 us against 10.8 with a split, M77 K14336
-// N4096 37.1 against 17.0, M511 K8192 N1024 23.8 against 16.4 (27.1, 81.0 and 48.7 with the weights in shared memory).  Eight CTAs in place of four:
-// M35 K8064 N1024 9.0 -> 7.2, M24 K6144 N1536 7.8 -> 6.5.
+// N4096 37.1 against 17.0, M511 K8192 N1024 23.8 against 16.4 (27.1, 81.0 and 48.7 with the weights in shared memory).  Eight CTAs
+// in place of four: M35 K8064 N1024 9.0 -> 7.2, M24 K6144 N1536 7.8 -> 6.5.
 bool choose_tmem(int64_t M, int64_t K, int64_t N, bool pairs_allowed, bool split_allowed, double other, TmemCall* call,
                  bool* pairs) {
   const int64_t sms = device_sms(), blocks = (K + 127) / 128;
