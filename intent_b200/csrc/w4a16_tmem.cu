@@ -173,13 +173,14 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   // in stage i % x_stages of shared memory, its expanded weights in stage i % A_STAGES of tensor memory.
   const uint32_t full = empty_w + 8 * p.w_stages;      // [x_stages] leader: activations landed, expanded weights stored
   const uint32_t empty = full + 8 * p.x_stages;        // [x_stages] MMAs done with them
-  const uint32_t tmem_full = empty + 8 * p.x_stages;   // [2; RING] accumulators complete
+  const uint32_t tmem_full = empty + 8 * p.x_stages;   // [2; RING] accumulators complete (but of the last tile)
   const uint32_t tmem_empty = tmem_full + 8 * RING;    // [2; RING] leader: accumulators drained
   const uint32_t tmem_slot = tmem_empty + 8 * RING;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
   const uint32_t parts_full = tmem_slot + 8;           // split: the partial sums of this CTA's rows have arrived
+  const uint32_t last_full = tmem_slot + 16;           // the accumulators of this CTA's last tile are complete
   // grouped: {expert, rows in use} of this CTA's items, or of every tile where those are fewer
-  int2* list = reinterpret_cast<int2*>(base_ptr + (tmem_slot - base) + 16);
+  int2* list = reinterpret_cast<int2*>(base_ptr + (tmem_slot - base) + 24);
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // known to be uniform
@@ -193,6 +194,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       prefetch_tensormap(&map_s);
       prefetch_tensormap(&map_x);
       mbar_init(parts_full, 1);
+      mbar_init(last_full, 1);
     }
     if (lane < p.w_stages) {
       mbar_init(full_w + 8 * lane, 1);
@@ -425,8 +427,9 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           __syncwarp();
         }
         if (MODE != MODE_SKINNY && ok && issue) {
-          if (CG == 2) umma_commit_pair(tmem_full + 8 * acc);
-          else umma_commit(tmem_full + 8 * acc);
+          const uint32_t complete = int(local) == my_items - 1 ? last_full : tmem_full + 8 * acc;
+          if (CG == 2) umma_commit_pair(complete);
+          else umma_commit(complete);
         }
         __syncwarp();
       }
@@ -600,7 +603,9 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // ------------------------------ epilogue -----------------------------------
     // The dequantisers, whose work is done by then, take four fifths of the last tile: nothing is left to overlap it with.
     // Bound by the stores: two bytes a lane and four warps took 4 of the 13 us of a call of M512 K2048 N4096 (a tile a
-    // CTA); eight bytes a lane and twenty warps, 13.06 -> 10.77 us.
+    // CTA); eight bytes a lane and twenty warps, 13.06 -> 10.77 us.  That tile has a barrier of its own:
+    // of tmem_full the dequantisers have seen no phase, and a wait by parity on a barrier that is two phases behind returns at
+    // once (with fewer than four k blocks a tile, eight with one accumulator set, nothing else has them wait for the tiles before).
     const int quadrant = warp & 3, last = my_items - 1;
     const int share = warp >= FIRST_DEQUANT ? 1 + ((warp - FIRST_DEQUANT) >> 2) : 0;
     uint16_t* y = reinterpret_cast<uint16_t*>(p.y);
@@ -627,7 +632,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = uint32_t(p.acc_sets == 2 ? local >> 1 : local);
       const int step = local == last ? (1 + SETS) * CHUNK : CHUNK;
       if (MODE == MODE_DOWN_SCATTER) next_route(t, share * CHUNK);
-      if (!mbar_wait_warp(tmem_full + 8 * acc, use & 1)) {
+      if (!mbar_wait_warp(local == last ? last_full : tmem_full + 8 * acc, local == last ? 0 : use & 1)) {
         if (lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
         break;
       }

@@ -111,6 +111,48 @@ def test_routed_rows(cuda_device, rows_of_expert, hidden, intermediate, block):
     assert max_abs_rel(y.cpu(), ref) <= 2e-2
 
 
+@pytest.mark.parametrize("tokens,hidden,intermediate", [
+    (1024, 4096, 128), (5120, 4096, 128),     # one k block in the down projection; 3.5 and 17.3 tiles a CTA or pair
+    (1024, 4096, 256), (5120, 4096, 256),
+    (1024, 4096, 384), (2048, 4096, 384),     # three; 3.5 and 6.9
+    (1024, 128, 2048), (1280, 128, 8192),     # the same for up|gate
+    (1024, 256, 2048), (1280, 256, 8192),
+    (1024, 384, 2048),
+])
+def test_several_tiles_of_few_k_blocks(cuda_device, tokens, hidden, intermediate):
+    """The dequantiser warps take rows of a CTA's last tile: only once it is complete, also where all of a set's blocks are
+    out before the tiles ahead have been multiplied."""
+    experts = 8                               # full blocks of 128 rows: every expert has tokens / 4 of them
+    first = torch.arange(tokens) % experts
+    ids = torch.stack([first, (first + 3) % experts], 1).to(torch.int32)
+    data = ib.workloads.moe_inputs(tokens, hidden, experts, intermediate, dtype=torch.bfloat16, seed=tokens + hidden)
+    dev = {k: v.to(cuda_device) for k, v in data.items()}
+    weights = torch.rand((tokens, 2), generator=torch.Generator().manual_seed(4)) + 0.1
+    sizes = dict(tokens=tokens, hidden=hidden, intermediate=intermediate, experts=experts, target=ib.B200Target(0))
+    args = (dev["x"], ids.to(cuda_device), weights.to(cuda_device), dev["up_gate_packed"], dev["up_gate_scales"],
+            dev["down_packed"], dev["down_scales"])
+    rows_args = args[:2] + args[3:]
+    plain, tiled = MoEW4A16FFN(**sizes), MoEW4A16FFN(prelayout=True, **sizes)
+    expected, rows = tiled(*args), tiled.experts_forward(*rows_args)[0]      # (no block has padding rows)
+    library = native.library()
+    try:
+        for pairs in (1, 0):
+            library.intent_b200_w4a16_gemm_pairs(pairs)
+            for _ in range(8):
+                y = plain(*args)
+                assert plain.down_scatter.observation.kernel.startswith(PAIRS if pairs else LONE)
+                assert torch.equal(y, expected)
+                assert torch.equal(plain.experts_forward(*rows_args)[0][:2 * tokens], rows[:2 * tokens])
+    finally:
+        library.intent_b200_w4a16_gemm_pairs(1)
+    torch.cuda.synchronize()
+    plain.down_scatter.check()
+    some = torch.arange(0, tokens, tokens // 64)
+    ref = oracle.moe_w4a16_swiglu_ffn(data["x"][some], ids[some], weights[some], data["up_gate_packed"],
+                                      data["up_gate_scales"], data["down_packed"], data["down_scales"])
+    assert max_abs_rel(expected[some.to(cuda_device)].cpu(), ref) <= 2e-2
+
+
 @pytest.mark.parametrize("sizes", [
     ((32, 2176, 512), (128, 2176, 512)),     # one instance of this kernel, 214528 and 224768 bytes of shared memory
     ((1, 1024, 512), (1, 4096, 4096)),       # the bandwidth kernel: rings of a few slots and of many
