@@ -171,8 +171,6 @@ struct Elem<__half> {
     return d;
   }
   static constexpr float kTinyScale = 512.f;
-  static constexpr uint32_t kTinyScale2 = 0x60006000u;
-  static constexpr bool kWideScale = false;        // a scale times that may leave the type's range
   __device__ static __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -216,8 +214,6 @@ struct Elem<__nv_bfloat16> {
     return d;
   }
   static constexpr float kTinyScale = 64.f;
-  static constexpr uint32_t kTinyScale2 = 0x42804280u;
-  static constexpr bool kWideScale = true;         // a scale times that stays in the type's range (up to 2^121)
   __device__ static __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));

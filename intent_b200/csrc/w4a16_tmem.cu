@@ -449,7 +449,6 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   } else if (warp >= FIRST_DEQUANT) {
     // ------------------------------ dequantisers --------------------------------
     const int set = (warp - FIRST_DEQUANT) >> 2, quadrant = warp & 3;
-    constexpr bool TINY = MODE == MODE_SKINNY || Elem<T>::kWideScale;
     const uint32_t magic = Elem<T>::kMagic2 ^ (p.twos_complement ? 0x00080008u : 0u);
     const uint32_t flip = p.twos_complement ? 0x08080808u : 0u;
     // where this thread's column lies in a stage.  up|gate: a quadrant of lanes is 16 gate columns and the 16 up
@@ -486,7 +485,6 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       for (int g = 0; g < 4; ++g) {
         const uint32_t v = MODE == MODE_SKINNY ? 0u : lds16(stage + s_of[g]);
         scale[g] = v | (v << 16);
-        if (TINY && MODE != MODE_SKINNY) scale[g] = Elem<T>::mul2(scale[g], Elem<T>::kTinyScale2);
       }
       // the words are in registers before the stage is handed back: the arrival waits for the loads it depends on
       asm volatile("" ::"r"(words[0]), "r"(words[W_ROWS - 1]), "r"(scale[3]) : "memory");
@@ -500,12 +498,12 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const uint32_t w = words[half * 8 + j], scale2 = scale[half * 2 + (j >> 2)];
-          if (TINY) {
+          if (MODE == MODE_SKINNY) {
             // A 16-bit integer q is the number q times the smallest subnormal, so that one multiply-add gives q - 8 exactly,
             // times a power of two.  The pairs come out of two masked words, a byte of zeros - the sign of a nibble - between.
-            // 11 or 15 instructions a word instead of 13 or 17, the same bits: M12 K4096 N14336 15.7 -> 15.3 us, M8 K8192
-            // N8192 17.3 -> 16.7, 300 tokens on 16 experts of 2048 x 1024 40.1 -> 39.6.  Halves with their scale keep the
-            // other way, as a scale times 512 would leave their range from 128 on (a bfloat16 times 64 does from 2^122).
+            // 11 instructions a word instead of 13: M12 K4096 N14336 15.7 -> 15.3 us, M8 K8192 N8192 17.3 -> 16.7.  Weights
+            // with their scale keep the other way: the scale times that power of two leaves the type's range (a half from 128
+            // on, a bfloat16 from 2^122), and the choice between two ways costs more than the instructions do.
             const uint32_t even = lop3_and_xor_u32(w, 0x0F0F0F0Fu, flip), odd = lop3_and_xor_u32(w >> 4, 0x0F0F0F0Fu, flip);
             o[4 * j + 0] = prmt(even, odd, 0xC480);  // (k0, k1)
             o[4 * j + 1] = prmt(even, odd, 0xD591);  // (k2, k3)
@@ -520,8 +518,8 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           }
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            o[4 * j + c] = TINY ? Elem<T>::tiny2(o[4 * j + c]) : Elem<T>::sub2(o[4 * j + c], Elem<T>::kBias2);
-            if (MODE != MODE_SKINNY) o[4 * j + c] = Elem<T>::mul2(o[4 * j + c], scale2);
+            if (MODE == MODE_SKINNY) o[4 * j + c] = Elem<T>::tiny2(o[4 * j + c]);
+            else o[4 * j + c] = Elem<T>::mul2(Elem<T>::sub2(o[4 * j + c], Elem<T>::kBias2), scale2);
           }
         }
         if (half == 0) {
@@ -567,7 +565,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         for (int g = 0; g < groups; ++g) {
           uint32_t v[SKINNY_ROWS];
           tmem_load_32x16(taddr + g * SKINNY_ROWS, v);
-          const float scale = Elem<T>::to_float(uint16_t(lds16(stage + g * (COLS * 2)))) * Elem<T>::kTinyScale;
+          const float scale = Elem<T>::to_float(uint16_t(lds16(stage + g * (COLS * 2))));
           tmem_load_wait();
 #pragma unroll
           for (int r = 0; r < SKINNY_ROWS; ++r) sum[r] = fmaf(__uint_as_float(v[r]), scale, sum[r]);
@@ -581,6 +579,9 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         if (++ring == RING) ring = 0, ring_phase ^= 1;
         if (++s == uint32_t(p.w_stages)) s = 0, phase ^= 1;
       }
+      // the weights' power of two, at the end: a scale times it may leave the range of f32
+#pragma unroll
+      for (int r = 0; r < SKINNY_ROWS; ++r) sum[r] *= Elem<T>::kTinyScale;
       const int col = t.n_tile * COLS + column;
       if (p.split > 1) {
         cluster_wait();

@@ -111,6 +111,48 @@ def test_routed_rows(cuda_device, rows_of_expert, hidden, intermediate, block):
     assert max_abs_rel(y.cpu(), ref) <= 2e-2
 
 
+@pytest.mark.parametrize("M,K,N,group", [(8, 1056, 1032, 32), (13, 2112, 520, 64), (300, 2048, 2056, 128)])
+def test_scales_at_the_end_of_the_range(cuda_device, M, K, N, group):
+    """bfloat16 scales up to 2^124 beside ordinary ones: times the weight they are finite, and so is the result.  An
+    infinite or NaN scale reaches its own column only."""
+    x, p, s = ib.workloads.w4a16_inputs(M, K, N, dtype=torch.bfloat16, group_size=group, seed=M)
+    x = (x.float() * 2.0 ** -40).to(torch.bfloat16)
+    picked = torch.rand(s.shape, generator=torch.Generator().manual_seed(1)) < 0.02
+    exponents = torch.randint(118, 125, s.shape, generator=torch.Generator().manual_seed(2))
+    s = torch.where(picked, 2.0 ** exponents.float(), s.float()).to(torch.bfloat16)
+    s[:, 7] = 2.0 ** 124
+    artifact = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0),
+                          constexprs={"GROUP_SIZE": group, "ZERO_POINT": 8, "ACT_DTYPE": "bf16"})
+    xd, pd = x.to(cuda_device), p.to(cuda_device)
+    out = artifact.run(xd, pd, s.to(cuda_device))
+    assert artifact.observation.kernel.startswith("w4a16_tmem_kernel"), artifact.observation.kernel
+    exact = x.double() @ ((oracle.unpack_int4(p).double() - 8) * s.double().repeat_interleave(group, dim=0))
+    assert torch.isfinite(out).all()
+    # (a sum's terms are rounded to 2^-9 of their size and so is the result, and terms are no larger than eight times x times s)
+    worst = x.double().abs() @ (8 * s.double().repeat_interleave(group, dim=0))
+    assert ((out.cpu().double() - exact).abs() <= 2 ** -8 * worst).all()
+    s[0, 3], s[1, 5] = float("inf"), float("nan")
+    broken = artifact.run(xd, pd, s.to(cuda_device))
+    good = torch.ones(N, dtype=torch.bool)
+    good[[3, 5]] = False
+    assert torch.equal(broken[:, good], out[:, good]) and not torch.isfinite(broken[:, ~good]).any()
+
+
+def test_grouped_scales_at_the_end_of_the_range(cuda_device):
+    tokens, hidden, intermediate, experts = 300, 512, 256, 4
+    data = ib.workloads.moe_inputs(tokens, hidden, experts, intermediate, dtype=torch.bfloat16, seed=6)
+    data["down_scales"][:, 0, ::3] = 2.0 ** 123
+    dev = {k: v.to(cuda_device) for k, v in data.items()}
+    sizes = dict(tokens=tokens, hidden=hidden, intermediate=intermediate, experts=experts, target=ib.B200Target(0))
+    plain, tiled = MoEW4A16FFN(**sizes), MoEW4A16FFN(prelayout=True, **sizes)
+    ids, weights = plain.route(dev["logits"])
+    # hidden rows small enough for sums of 2^126 times them to stay finite
+    args = ((dev["x"].float() * 2.0 ** -12).to(torch.bfloat16), ids, weights, dev["up_gate_packed"], dev["up_gate_scales"],
+            dev["down_packed"], dev["down_scales"])
+    y = plain(*args)
+    assert torch.isfinite(y).all() and torch.equal(y, tiled(*args))
+
+
 @pytest.mark.parametrize("tokens,hidden,intermediate", [
     (1024, 4096, 128), (5120, 4096, 128),     # one k block in the down projection; 3.5 and 17.3 tiles a CTA or pair
     (1024, 4096, 256), (5120, 4096, 256),
