@@ -245,6 +245,35 @@ def test_host_pipelined_ffn_gives_the_whole_batch_bits(cuda_device):
         HostPipelinedFFN(tokens=510, hidden=hidden, intermediate=intermediate, experts=experts, chunks=4)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_gate_over_its_range(cuda_device, dtype):
+    """silu(g) * u against 64 bits for gates from the smallest to the largest, where the exponential is zero or infinite
+    among them.  The result is rounded once (2^-11 of it in f16, 2^-8 in bf16) after f32 steps that are off by 2^-18 at most
+    (__expf by 2 + 1.2 |g| units of 2^-24 with |g| up to 24, four roundings; beyond, the result is below 1e-6)."""
+    ends = torch.tensor([0.0, 1e-6, 0.5, 16.0, 80.0, 87.0, 88.0, 88.5, 89.0, 104.0, 250.0])
+    if dtype == torch.bfloat16:
+        ends = torch.cat((ends, torch.tensor([1e4, 1e18])))
+    spread = torch.randn((128 - 2 * ends.numel(),), generator=torch.Generator().manual_seed(1)) * 6
+    values = torch.cat((ends, -ends, spread)).to(dtype)
+    hidden, intermediate, experts = 128, 128, 1
+    data = ib.workloads.moe_inputs(64, hidden, experts, intermediate, dtype=dtype, seed=1)
+    x = torch.zeros((128, hidden), dtype=dtype)
+    x[:, 0] = values                                                # times a weight of (9 - 8) * 1
+    layer = MoEW4A16FFN(tokens=64, hidden=hidden, intermediate=intermediate, experts=experts, target=ib.B200Target(0),
+                        act_dtype="f16" if dtype == torch.float16 else "bf16")
+    packed = torch.full_like(data["up_gate_packed"], int("99999999", 16) - 2 ** 32)
+    out = layer.up_gate.run(x.to(cuda_device), torch.zeros(1, dtype=torch.int32, device=cuda_device),
+                            torch.full((1,), 128, dtype=torch.int32, device=cuda_device), packed.to(cuda_device),
+                            torch.ones_like(data["up_gate_scales"]).to(cuda_device)).cpu().double()
+    g = values.double()
+    exact = (g * torch.sigmoid(g) * g)[:, None].expand_as(out)
+    largest = torch.finfo(dtype).max
+    fits = exact.abs() < largest
+    assert not torch.isnan(out).any() and torch.equal(out[~fits], exact[~fits].sign() * float("inf"))
+    relative = (2 ** -11 if dtype == torch.float16 else 2 ** -8) + 2 ** -18
+    assert ((out - exact).abs() <= relative * exact.abs() + 1e-6)[fits].all()
+
+
 @pytest.mark.parametrize("prelayout", [False, True])
 def test_a_layer_says_what_a_call_ran(cuda_device, prelayout):
     """``chain`` holds the programs of a call; ``gather`` and ``up_gate``, which take all rows, describe the call of the
