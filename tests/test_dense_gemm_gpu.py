@@ -76,3 +76,18 @@ def test_quantized_gemm_matches_oracle(cuda_device, M, K, N):
     assert difference.max().item() <= 2
     assert (difference > 0).float().mean().item() < 0.02
     assert out.min().item() >= -128 and out.max().item() <= 127 and (out == 127).any()   # saturation is reached
+
+
+def test_quantized_gemm_bytes_do_not_depend_on_the_call(cuda_device):
+    """A truncated sum keeps its value only if k is added in one order: few rows, whose tiles leave most SMs idle, give the
+    bytes that they have among more rows."""
+    M, K, N = 96, 4096, 8192
+    gen = torch.Generator().manual_seed(1)
+    a = (torch.randn((3 * M, K), generator=gen) / K ** 0.5).half().to(cuda_device)
+    b = torch.randn((K, N), generator=gen).half().to(cuda_device)
+    bias, scale = torch.randn((N,), generator=gen).to(cuda_device), torch.full((N,), 1.0 / 48.0, device=cuda_device)
+    residual = torch.randn((3 * M, N), generator=gen).half().to(cuda_device)
+    artifact = ib.compile(ib.programs.quantized_gemm, target=ib.B200Target(0))
+    whole = artifact.run(a, b, bias, residual, scale)
+    part = artifact.run(a[M:2 * M].contiguous(), b, bias, residual[M:2 * M].contiguous(), scale)
+    assert torch.equal(part, whole[M:2 * M])
