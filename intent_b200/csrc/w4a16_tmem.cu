@@ -18,6 +18,7 @@
 // wait for the kernel ahead ends 1.3 us after that kernel, first words 1 us later), its k blocks and the exchange between
 // the CTAs of a cluster (2 us).  Against the forms with the weights in shared memory: M77 K14336 N4096 81.1 -> 14.5 us,
 // M1024 K4096 N4096 50.9 -> 28, 64 tokens on 64 experts of 4096 x 1408 414 -> 155 (the whole layer).
+#include <algorithm>
 #include <type_traits>
 
 #include "cluster.cuh"
@@ -76,6 +77,7 @@ struct TmemParams {
   int routes, top_k;
   float4* clear;             // MODE_UPGATE_SILU: filled with zeros by a warp that has nothing else to do; may be null
   int64_t clear_vectors;
+  int clear_pause;           // nanoseconds after each piece of 2 KiB
 };
 
 // MODE_SKINNY: dense calls of at most SKINNY_ROWS rows, as precise as the bandwidth kernels that serve the others: the
@@ -437,14 +439,13 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
   } else if (MODE == MODE_UPGATE_SILU && warp == 3) {
     // ------------------------------ zeros for the kernel that adds to this buffer ----
-    // In pieces of 2 KiB with a pause between them, about 1 TB/s over all SMs: far from the operands' loads in the way, and
-    // done before them (16384 tokens of 4096: 268 MB beside 600 us of contraction; a fill of its own took 38).
+    // Beside 600 us of contraction (16384 tokens of 4096: 268 MB), where a fill of its own takes 38.
     const int64_t step = int64_t(gridDim.x) * 128;
     for (int64_t at = int64_t(blockIdx.x) * 128; at < p.clear_vectors; at += step) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         if (at + i * 32 + lane < p.clear_vectors) p.clear[at + i * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-      __nanosleep(200);
+      if (p.clear_pause > 0) __nanosleep(p.clear_pause);
     }
   } else if (warp >= FIRST_DEQUANT) {
     // ------------------------------ dequantisers --------------------------------
@@ -886,6 +887,25 @@ int launch(const TmemCall& q, cudaStream_t stream) {
                          : p.split > 1 ? "w4a16_tmem_kernel k split over a cluster, 128 columns"
                                        : "w4a16_tmem_kernel single CTA, 128 columns",
                          grid, THREADS, smem, cluster);
+  if (p.clear_vectors > 0) {
+    // The warp that clears writes a piece of 2 KiB in 60 ns, and pauses so that it is done in about half of the contraction, a
+    // k block of which takes 300 (`least`: tiles that the routes fill at least).  Where that is too short for it, because the
+    // experts are narrow or the tiles few, a fill ahead of the launch is faster.  Whole layer, us, pause 0 / 50 / 200 / fill ahead:
+    // 16384 tokens of 4096 on 64 experts of 128 columns 509 / 506 / 633 / 506, of 256 (one choice) 327 / 318 / 451 / 325, of
+    // 512 665 / 688 / 707 / 727; 16384 of 8192, 8 of 128 (one choice) 536 / 555 / 843 / 523; 1024 of 4096, 2 of 128 (one choice)
+    // 42 / 59 / 127 / 40; 256 on 8 of 128 32.9 / 32.0 / 41.4 / 35.9.  From 1024 columns on the pause makes no difference.
+    const int64_t at_a_time = int64_t(grid) * 128, pieces = (p.clear_vectors + at_a_time - 1) / at_a_time;
+    const int64_t least = std::min(items, (q.routes + 127) / 128 * p.n_tiles);
+    const double contraction = 300.0 * double(p.k_blocks) * double((least + at_once - 1) / at_once);
+    const double fill = 60.0 * double(pieces), ahead = 1000.0 + double(p.clear_vectors) * 16.0 / 7000.0;
+    if (fill > contraction + ahead) {
+      const cudaError_t filled = cudaMemsetAsync(p.clear, 0, size_t(p.clear_vectors) * 16, stream);
+      if (filled != cudaSuccess) return cuda_status(filled);
+      p.clear_vectors = 0;
+    } else {
+      p.clear_pause = int(std::min(50.0, std::max(0.0, (0.6 * contraction - fill) / double(pieces))));
+    }
+  }
   cudaLaunchConfig_t config = {};
   config.gridDim = p.split > 1 ? dim3(unsigned(p.split), unsigned(items), 1) : dim3(unsigned(grid), 1, 1);
   config.blockDim = dim3(THREADS, 1, 1);

@@ -316,3 +316,19 @@ def test_a_call_clears_its_result(cuda_device, tokens, hidden):
     assert layer(*args, y=onto) is onto and torch.equal(onto[-1], torch.ones_like(onto[-1]))
     with pytest.raises((TypeError, ValueError, RuntimeError)):     # one token more than there are weights
         layer(torch.cat((dev["x"], dev["x"][:1])), *args[1:])
+
+
+def test_a_call_clears_its_result_ahead(cuda_device):
+    """Few tiles and a large result: it is filled ahead of the up|gate contraction, not beside it."""
+    tokens, hidden, intermediate, experts = 1024, 4096, 128, 2
+    data, ids, weights = _ffn_case(tokens, hidden, intermediate, experts, torch.bfloat16, seed=9)
+    dev = {k: v.to(cuda_device) for k, v in data.items()}
+    layer = MoEW4A16FFN(tokens=tokens, hidden=hidden, intermediate=intermediate, experts=experts, top_k=1,
+                        target=ib.B200Target(0))
+    args = (dev["x"], ids[:, :1].contiguous().to(cuda_device), weights[:, :1].contiguous().to(cuda_device),
+            dev["up_gate_packed"], dev["up_gate_scales"], dev["down_packed"], dev["down_scales"])
+    expected = layer(*args, y=torch.zeros((tokens, hidden), dtype=torch.float32, device=cuda_device))
+    for _ in range(4):
+        stale = torch.full((tokens, hidden), float("nan"), dtype=torch.float32, device=cuda_device)
+        del stale                                                  # (the result comes from this block)
+        assert torch.equal(layer(*args), expected)
