@@ -15,8 +15,11 @@ namespace ib200 {
 // Process-wide count of kernels launched by this library.
 void note_launch(int count = 1);
 
+// The status of a CUDA call.  An error that is returned is not left for the next caller who asks for the last one.
 inline int cuda_status(cudaError_t error) {
-  return error == cudaSuccess ? INTENT_B200_OK : INTENT_B200_ERR_CUDA + static_cast<int>(error);
+  if (error == cudaSuccess) return INTENT_B200_OK;
+  cudaGetLastError();
+  return INTENT_B200_ERR_CUDA + static_cast<int>(error);
 }
 
 // Returns the status of the launch that was just issued (cudaPeekAtLastError
@@ -98,9 +101,7 @@ cudaError_t launch_programmatic(void (*kernel)(P...), dim3 grid, dim3 block, siz
   attribute[1].val.clusterDim.z = 1;
   config.attrs = attribute;
   config.numAttrs = cluster > 1 ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<P>(arguments)...);
-  if (e != cudaSuccess) cudaGetLastError();   // (returned here, and not left for the next one who asks)
-  return e;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<P>(arguments)...);
 }
 
 #define IB200_VIEW1_ARG(p) ib200::View1{p, p##_d0, p##_s0}

@@ -590,22 +590,12 @@ int launch_kernel(const CUtensorMap& map_w, const CUtensorMap& map_s, const CUte
   // (the limit belongs to the kernel: the same value from every thread, not each plan's own)
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   if (e != cudaSuccess) return cuda_status(e);
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(plan.grid, 1, 1);
-  config.blockDim = dim3(WARPS * 32, 1, 1);
-  config.dynamicSmemBytes = plan.smem_bytes;
-  config.stream = stream;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute[0].val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = attribute;
-  config.numAttrs = 1;
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel),
                          XSTAGED ? (RING ? "w4a16_stream_kernel staged activations, slot ring" : "w4a16_stream_kernel staged activations")
                                  : (RING ? "w4a16_stream_kernel activations per unit, slot ring" : "w4a16_stream_kernel activations per unit"),
                          plan.grid, WARPS * 32, int(plan.smem_bytes), 1);
-  e = cudaLaunchKernelEx(&config, kernel, map_w, map_s, map_x, p);
+  e = launch_programmatic(kernel, plan.grid, WARPS * 32, plan.smem_bytes, stream, 1, map_w, map_s, map_x, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();

@@ -1287,20 +1287,10 @@ int launch_table(const TableMaps& maps, const TableParams& p, int grid, size_t s
   auto kernel = w4a16_table_kernel<T, MB, STEPS, WARPS>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);   // as in w4a16_stream.cu
   if (e != cudaSuccess) return cuda_status(e);
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(grid, 1, 1);
-  config.blockDim = dim3(WARPS * 32, 1, 1);
-  config.dynamicSmemBytes = smem;
-  config.stream = stream;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute[0].val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = attribute;
-  config.numAttrs = 1;
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel), "w4a16_table_kernel staged activations", grid,
                          WARPS * 32, int(smem), 1);
-  e = cudaLaunchKernelEx(&config, kernel, maps, p);
+  e = launch_programmatic(kernel, grid, WARPS * 32, smem, stream, 1, maps, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();
@@ -1311,20 +1301,10 @@ int launch_ride(const TableMaps& maps, const TableParams& p, int grid, size_t sm
   auto kernel = w4a16_ride_kernel<T, STEPS, UR, CORR_MMA>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);   // as in w4a16_stream.cu
   if (e != cudaSuccess) return cuda_status(e);
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(grid, 1, 1);
-  config.blockDim = dim3(1024, 1, 1);
-  config.dynamicSmemBytes = smem;
-  config.stream = stream;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute[0].val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = attribute;
-  config.numAttrs = 1;
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel), "w4a16_ride_kernel activations ride with the units",
                          grid, 1024, int(smem), 1);
-  e = cudaLaunchKernelEx(&config, kernel, maps, p);
+  e = launch_programmatic(kernel, grid, 1024, smem, stream, 1, maps, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();

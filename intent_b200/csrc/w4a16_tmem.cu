@@ -161,7 +161,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   // Programmatic launch: a CTA of the next such launch may set itself up on an SM that this one has left, and this launch
   // touches no global memory before everything ahead of it in the stream has completed.  One call after another:
   // M16 K4096 N4096 10.3 -> 8.4 us, M77 K14336 N4096 19.1 -> 17.4, M512 K2048 N4096 14.4 -> 13.0 (each as it was then).
-  asm volatile("griddepcontrol.launch_dependents;");
+  programmatic_begin();
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - smem_u32(smem_raw));
   const int x_rows = p.row_tile / CG;                  // activation rows this CTA stages
@@ -223,7 +223,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
   // everything above is done while the kernel before is still at work, everything below may read what that one wrote
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  programmatic_wait();
   int m_tiles = p.m_tiles;
   if (!dense_mode(MODE)) m_tiles = min(m_tiles, (*p.total_rows + 127) / 128);
   const int items = m_tiles * p.n_tiles;
@@ -906,21 +906,8 @@ int launch(const TmemCall& q, cudaStream_t stream) {
       p.clear_pause = int(std::min(50.0, std::max(0.0, (0.6 * contraction - fill) / double(pieces))));
     }
   }
-  cudaLaunchConfig_t config = {};
-  config.gridDim = p.split > 1 ? dim3(unsigned(p.split), unsigned(items), 1) : dim3(unsigned(grid), 1, 1);
-  config.blockDim = dim3(THREADS, 1, 1);
-  config.dynamicSmemBytes = smem;
-  config.stream = stream;
-  cudaLaunchAttribute attribute[2];
-  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute[0].val.programmaticStreamSerializationAllowed = 1;
-  attribute[1].id = cudaLaunchAttributeClusterDimension;
-  attribute[1].val.clusterDim.x = unsigned(cluster);
-  attribute[1].val.clusterDim.y = 1;
-  attribute[1].val.clusterDim.z = 1;
-  config.attrs = attribute;
-  config.numAttrs = cluster > 1 ? 2 : 1;
-  e = cudaLaunchKernelEx(&config, kernel, map_x, map_w, map_s, p);
+  const dim3 ctas = p.split > 1 ? dim3(unsigned(p.split), unsigned(items), 1) : dim3(unsigned(grid), 1, 1);
+  e = launch_programmatic(kernel, ctas, THREADS, smem, stream, cluster, map_x, map_w, map_s, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();
