@@ -147,7 +147,8 @@ INTENT_B200_API int intent_b200_w4a16_gemm_pairs(int32_t enable);
  * while the kernel before it on the stream is still running; it waits for that
  * kernel before it reads the activations or writes the output.  Only enable it when the packed weights are not written by the kernel
  * launched immediately before, nor by one ahead of a row of W4A16 launches of this library that come before: those may
- * still be under way themselves (the weights are static model state in a decode loop).
+ * still be under way themselves (the weights are static model state in a decode loop).  Other kernels of this library that are
+ * launched while it is on start only when all work ahead of them has completed.
  * Process-global; off by default. */
 INTENT_B200_API int intent_b200_w4a16_gemv_overlap(int32_t enable);
 /* Number of CTAs of the bandwidth kernel (0 = one per SM).  For measurement

@@ -85,8 +85,8 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // (programmatic_wait) for everything ahead of it in the stream before it touches global memory.  What it does before that -
 // barriers, tensor memory, indexes - and the launch itself then cost nothing beside the kernel ahead.
 template <typename... P, typename... A>
-cudaError_t launch_programmatic(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
-                                const A&... arguments) {
+cudaError_t launch_early(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
+                         const A&... arguments) {
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
@@ -94,7 +94,7 @@ cudaError_t launch_programmatic(void (*kernel)(P...), dim3 grid, dim3 block, siz
   config.stream = stream;
   cudaLaunchAttribute attribute[2];
   attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  attribute[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
   attribute[1].id = cudaLaunchAttributeClusterDimension;
   attribute[1].val.clusterDim.x = unsigned(cluster);
   attribute[1].val.clusterDim.y = 1;
@@ -102,6 +102,25 @@ cudaError_t launch_programmatic(void (*kernel)(P...), dim3 grid, dim3 block, siz
   config.attrs = attribute;
   config.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&config, kernel, static_cast<P>(arguments)...);
+}
+
+// Whether a bandwidth or table launch asks for its weights before its own wait (w4a16_stream.cu, w4a16_table.cu).
+bool overlap_switched();
+
+// For the W4A16 kernels of few rows and those with the weights in tensor memory, a row of which such a launch may overtake.
+template <typename... P, typename... A>
+cudaError_t launch_w4a16(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
+                         const A&... arguments) {
+  return launch_early(true, kernel, grid, block, smem, stream, cluster, arguments...);
+}
+
+// For all others: with the switch on these start when all ahead of them has completed, so that the launch behind them cannot
+// overtake what wrote its weights.  (To let it start only after their own wait costs small chains 1 us: an MoE layer's call 25.3
+// -> 26.3 us.)
+template <typename... P, typename... A>
+cudaError_t launch_programmatic(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
+                                const A&... arguments) {
+  return launch_early(!overlap_switched(), kernel, grid, block, smem, stream, cluster, arguments...);
 }
 
 #define IB200_VIEW1_ARG(p) ib200::View1{p, p##_d0, p##_s0}

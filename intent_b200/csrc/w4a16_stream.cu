@@ -583,6 +583,11 @@ int device_sms() {
 
 int g_overlap = 0;
 
+}  // namespace
+extern int g_table_overlap;   // w4a16_table.cu
+bool overlap_switched() { return g_overlap != 0 || g_table_overlap != 0; }
+namespace {
+
 template <typename T, int MB, int STEPS, int WARPS, bool XSTAGED, int RING>
 int launch_kernel(const CUtensorMap& map_w, const CUtensorMap& map_s, const CUtensorMap& map_x, const StreamParams& p, const Plan& plan,
                   cudaStream_t stream) {
@@ -595,7 +600,7 @@ int launch_kernel(const CUtensorMap& map_w, const CUtensorMap& map_s, const CUte
                          XSTAGED ? (RING ? "w4a16_stream_kernel staged activations, slot ring" : "w4a16_stream_kernel staged activations")
                                  : (RING ? "w4a16_stream_kernel activations per unit, slot ring" : "w4a16_stream_kernel activations per unit"),
                          plan.grid, WARPS * 32, int(plan.smem_bytes), 1);
-  e = launch_programmatic(kernel, plan.grid, WARPS * 32, plan.smem_bytes, stream, 1, map_w, map_s, map_x, p);
+  e = launch_w4a16(kernel, plan.grid, WARPS * 32, plan.smem_bytes, stream, 1, map_w, map_s, map_x, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();

@@ -1267,7 +1267,9 @@ int table_sms() {
   return sms;
 }
 
+}  // namespace
 int g_table_overlap = 0;
+namespace {
 
 int validate(const HostProblem& h, int group_size) {
   if (h.M < 0 || h.K < 0 || h.N < 0) return INTENT_B200_ERR_SHAPE;
@@ -1290,7 +1292,7 @@ int launch_table(const TableMaps& maps, const TableParams& p, int grid, size_t s
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel), "w4a16_table_kernel staged activations", grid,
                          WARPS * 32, int(smem), 1);
-  e = launch_programmatic(kernel, grid, WARPS * 32, smem, stream, 1, maps, p);
+  e = launch_w4a16(kernel, grid, WARPS * 32, smem, stream, 1, maps, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();
@@ -1304,7 +1306,7 @@ int launch_ride(const TableMaps& maps, const TableParams& p, int grid, size_t sm
   if (LaunchFacts* sink = observe_sink())
     return record_launch(sink, reinterpret_cast<const void*>(kernel), "w4a16_ride_kernel activations ride with the units",
                          grid, 1024, int(smem), 1);
-  e = launch_programmatic(kernel, grid, 1024, smem, stream, 1, maps, p);
+  e = launch_w4a16(kernel, grid, 1024, smem, stream, 1, maps, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();

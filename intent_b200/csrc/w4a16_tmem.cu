@@ -907,7 +907,7 @@ int launch(const TmemCall& q, cudaStream_t stream) {
     }
   }
   const dim3 ctas = p.split > 1 ? dim3(unsigned(p.split), unsigned(items), 1) : dim3(unsigned(grid), 1, 1);
-  e = launch_programmatic(kernel, ctas, THREADS, smem, stream, cluster, map_x, map_w, map_s, p);
+  e = launch_w4a16(kernel, ctas, THREADS, smem, stream, cluster, map_x, map_w, map_s, p);
   if (e != cudaSuccess) return cuda_status(e);
   note_launch();
   return launch_status();

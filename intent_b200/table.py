@@ -148,7 +148,8 @@ class PreparedTable:
 def set_launch_overlap(enabled: bool) -> None:
     """Process-wide: a table launch may start requesting its packed weights while the kernel before it on
     the stream is still running (programmatic dependent launch).  Only valid when the weights are not
-    written by that kernel (static model weights in a decode loop)."""
+    written by that kernel, nor by one ahead of a row of W4A16 calls that come before (static model weights in a
+    decode loop)."""
     native.check(native.library().intent_b200_w4a16_gemv_table_overlap(1 if enabled else 0),
                  "intent_b200_w4a16_gemv_table_overlap")
 

@@ -6,6 +6,7 @@ import torch
 import intent_b200 as ib
 import oracle
 from intent_b200.moe import MoEW4A16FFN
+from intent_b200.runtime import native
 
 pytestmark = pytest.mark.gpu
 TARGET = ib.B200Target(0)
@@ -70,3 +71,30 @@ def test_layer_calls_in_a_row(cuda_device):
     torch.cuda.synchronize()
     for i, out in enumerate(outs):
         assert torch.equal(out, alone[i % 3]), i
+
+
+def test_the_overlap_switch_behind_other_kernels(cuda_device):
+    """With the switch on a bandwidth call may ask for its weights while the call before it is running.  That call, when it
+    is of another program, must not have started before the copy ahead of it wrote the weights."""
+    K, N = 4096, 4096
+    x, p, s = ib.workloads.w4a16_inputs(1, K, N, dtype=torch.bfloat16, seed=1)
+    other = ib.workloads.w4a16_inputs(1, K, N, dtype=torch.bfloat16, seed=2)[1].to(cuda_device)
+    xd, pd, sd = x.to(cuda_device), p.to(cuda_device), s.to(cuda_device)
+    gemv = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0), constexprs={
+        "GROUP_SIZE": 128, "ZERO_POINT": 8, "ACT_DTYPE": "bf16", "KERNEL": "gemv"})
+    between = ib.compile(ib.programs.bitnet_int2_matmul, target=ib.B200Target(0))
+    act = torch.ones((1, 256), dtype=torch.int8, device=cuda_device)
+    codes = torch.ones((16, 64), dtype=torch.uint8, device=cuda_device)
+    expected = gemv.run(xd, other, sd)
+    weights, busy = pd.clone(), torch.randn((4096, 4096), device=cuda_device)
+    library = native.library()
+    try:
+        assert library.intent_b200_w4a16_gemv_overlap(1) == 0
+        for _ in range(50):
+            weights.copy_(pd)
+            busy @ busy
+            weights.copy_(other)
+            between.run(act, codes)
+            assert torch.equal(gemv.run(xd, weights, sd), expected)
+    finally:
+        library.intent_b200_w4a16_gemv_overlap(0)
