@@ -85,6 +85,7 @@ struct TmemParams {
 // which the epilogue warps scale and add up in f32 while the next k blocks are multiplied.
 constexpr int MODE_DENSE = 0, MODE_UPGATE_SILU = 1, MODE_GROUPED_F32 = 2, MODE_DOWN_SCATTER = 3, MODE_SKINNY = 4;
 constexpr int SKINNY_ROWS = 16, RING = 4;    // accumulators of RING k blocks in flight, up to four groups each
+constexpr uint32_t LAST_TILE = 2;            // other modes: the barrier of tmem_full for a CTA's last tile
 __host__ __device__ constexpr bool dense_mode(int mode) { return mode == MODE_DENSE || mode == MODE_SKINNY; }
 
 // D[tmem] (+)= A[tmem] * B[smem]
@@ -175,14 +176,13 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
   // in stage i % x_stages of shared memory, its expanded weights in stage i % A_STAGES of tensor memory.
   const uint32_t full = empty_w + 8 * p.w_stages;      // [x_stages] leader: activations landed, expanded weights stored
   const uint32_t empty = full + 8 * p.x_stages;        // [x_stages] MMAs done with them
-  const uint32_t tmem_full = empty + 8 * p.x_stages;   // [2; RING] accumulators complete (but of the last tile)
+  const uint32_t tmem_full = empty + 8 * p.x_stages;   // [2 and the last tile's; RING] accumulators complete
   const uint32_t tmem_empty = tmem_full + 8 * RING;    // [2; RING] leader: accumulators drained
   const uint32_t tmem_slot = tmem_empty + 8 * RING;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
   const uint32_t parts_full = tmem_slot + 8;           // split: the partial sums of this CTA's rows have arrived
-  const uint32_t last_full = tmem_slot + 16;           // the accumulators of this CTA's last tile are complete
   // grouped: {expert, rows in use} of this CTA's items, or of every tile where those are fewer
-  int2* list = reinterpret_cast<int2*>(base_ptr + (tmem_slot - base) + 24);
+  int2* list = reinterpret_cast<int2*>(base_ptr + (tmem_slot - base) + 16);
 
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // known to be uniform
@@ -196,7 +196,6 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       prefetch_tensormap(&map_s);
       prefetch_tensormap(&map_x);
       mbar_init(parts_full, 1);
-      mbar_init(last_full, 1);
     }
     if (lane < p.w_stages) {
       mbar_init(full_w + 8 * lane, 1);
@@ -429,7 +428,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
           __syncwarp();
         }
         if (MODE != MODE_SKINNY && ok && issue) {
-          const uint32_t complete = int(local) == my_items - 1 ? last_full : tmem_full + 8 * acc;
+          const uint32_t complete = tmem_full + 8 * (int(local) == my_items - 1 ? LAST_TILE : acc);
           if (CG == 2) umma_commit_pair(complete);
           else umma_commit(complete);
         }
@@ -634,7 +633,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       const uint32_t acc = p.acc_sets == 2 ? local & 1 : 0, use = uint32_t(p.acc_sets == 2 ? local >> 1 : local);
       const int step = local == last ? (1 + SETS) * CHUNK : CHUNK;
       if (MODE == MODE_DOWN_SCATTER) next_route(t, share * CHUNK);
-      if (!mbar_wait_warp(local == last ? last_full : tmem_full + 8 * acc, local == last ? 0 : use & 1)) {
+      if (!mbar_wait_warp(tmem_full + 8 * (local == last ? LAST_TILE : acc), local == last ? 0 : use & 1)) {
         if (lane == 0) atomicExch(&g_w4a16_tmem_status, INTENT_B200_ERR_TIMEOUT);
         break;
       }
