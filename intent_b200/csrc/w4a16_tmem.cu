@@ -57,7 +57,7 @@ struct TmemParams {
   int row_tile;              // most rows of a tile, a multiple of 16 * CG
   int box_rows;              // rows of one activation box
   int x_stages;              // stages of activations, A_STAGES .. 8
-  int w_stages;              // stages of packed words, SETS .. 16
+  int w_stages;              // stages of packed words, 2 * SETS .. 16
   int acc_sets;              // accumulator sets that alternate between tiles
   int split;                 // CTAs of a cluster that share a tile's k blocks (1 = none)
   int kb_each, kb_extra;     // k blocks of a CTA: the first kb_extra ranks of a cluster take one more
@@ -86,6 +86,10 @@ struct TmemParams {
 constexpr int MODE_DENSE = 0, MODE_UPGATE_SILU = 1, MODE_GROUPED_F32 = 2, MODE_DOWN_SCATTER = 3, MODE_SKINNY = 4;
 constexpr int SKINNY_ROWS = 16, RING = 4;    // accumulators of RING k blocks in flight, up to four groups each
 constexpr uint32_t LAST_TILE = 2;            // other modes: the barrier of tmem_full for a CTA's last tile
+constexpr int GROUP_ACC = 4 * SKINNY_ROWS;   // columns of a k block's accumulators
+static_assert(RING * GROUP_ACC <= ACC_COLUMNS && ACC_COLUMNS <= A_COLUMN, "accumulators end where the expanded weights begin");
+static_assert(A_COLUMN + A_STAGES * 64 <= 512, "columns of tensor memory");
+static_assert(LAST_TILE >= 2 && LAST_TILE < RING, "a barrier that no accumulator set has");
 __host__ __device__ constexpr bool dense_mode(int mode) { return mode == MODE_DENSE || mode == MODE_SKINNY; }
 
 // D[tmem] (+)= A[tmem] * B[smem]
@@ -409,7 +413,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk) {
                 const uint32_t low = desc_low + (kk >= 4 ? (x_half >> 4) : 0u) + 2 * (kk & 3);
-                umma_f16_ts<CG>(tmem_base + ring * 64 + (kk >> (p.group_shift - 4)) * SKINNY_ROWS, tmem_a + kk * 8,
+                umma_f16_ts<CG>(tmem_base + ring * GROUP_ACC + (kk >> (p.group_shift - 4)) * SKINNY_ROWS, tmem_a + kk * 8,
                                 (uint64_t(desc_high) << 32) | low, idesc, (kk & (steps - 1)) != 0);
               }
               umma_commit(done);
@@ -561,7 +565,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         if (!ok) break;
         tcgen05_fence_after();
         const uint32_t stage = smem_w + s * W_STAGE + s_offset;
-        const uint32_t taddr = tmem_base + ring * 64 + (uint32_t(quadrant * 32) << 16);
+        const uint32_t taddr = tmem_base + ring * GROUP_ACC + (uint32_t(quadrant * 32) << 16);
         for (int g = 0; g < groups; ++g) {
           uint32_t v[SKINNY_ROWS];
           tmem_load_32x16(taddr + g * SKINNY_ROWS, v);
@@ -847,7 +851,9 @@ int launch(const TmemCall& q, cudaStream_t stream) {
   while (p.x_stages > A_STAGES && fixed + p.x_stages * x_stage + 9 * W_STAGE > SMEM_LIMIT) --p.x_stages;
   p.w_stages = (SMEM_LIMIT - fixed - p.x_stages * x_stage) / W_STAGE;
   if (p.w_stages > 16) p.w_stages = 16;
-  if (p.w_stages < SETS) return INTENT_B200_ERR_UNSUPPORTED;
+  // A set waits for the words of every SETS-th k block: that the stage's earlier words have landed follows for it from
+  // the block 2 * SETS before having been multiplied, with fewer stages it would not (a wait by parity, two phases behind)
+  if (p.w_stages < 2 * SETS) return INTENT_B200_ERR_UNSUPPORTED;
   const int smem = fixed + p.x_stages * x_stage + p.w_stages * W_STAGE, operands = p.x_stages * x_stage + p.w_stages * W_STAGE;
   if (sums > operands) return INTENT_B200_ERR_UNSUPPORTED;
   if (sums > 0 && fixed >= 1024 + 512 + sums) p.exchange = uint32_t(operands + 512);
