@@ -175,14 +175,15 @@ class MoEW4A16FFN:
         self._routed = self.fused_combine and not prelayout
         if self._routed:
             # (the up|gate contraction clears the result that the down projection adds to)
-            self._chain = (self._bind(programs.moe_gather_rows, dict(gathered, PADDING=False)),
-                           self._bind(programs.moe_grouped_upgate_silu, dict(grouped, ROUTED=True, CLEAR=True)))
+            self._clearing_up_gate = self._bind(programs.moe_grouped_upgate_silu, dict(grouped, ROUTED=True, CLEAR=True))
+            self._chain = (self._bind(programs.moe_gather_rows, dict(gathered, PADDING=False)), self._clearing_up_gate)
         else:
             self._chain = (self.gather, self.up_gate)
 
     @property
     def chain(self):
-        """The programs that a call runs after the alignment, in order."""
+        """The programs that a call runs after the alignment, in order: those of the latest one, as a call onto a ``y``
+        that is there already, or a prepared one, runs another up|gate program."""
         return (*self._chain, self.down_scatter) if self.fused_combine else (self.gather, self.up_gate, self.down, self.combine)
 
     # What only the other chains use is bound at its first use.
@@ -205,6 +206,18 @@ class MoEW4A16FFN:
     def _routed_up_gate(self):
         """The up|gate contraction of the routed rows for a ``y`` that is there already."""
         return self._bind(programs.moe_grouped_upgate_silu, dict(self._grouped, ROUTED=True))
+
+    def _up_gate_of(self, clears):
+        """The up|gate program of a call, from here on that of ``chain``."""
+        gather, up_gate = self._chain
+        if not self._routed:
+            return up_gate
+        runs = self._clearing_up_gate if clears else self._routed_up_gate
+        if runs is not up_gate:
+            self._chain = (gather, runs)
+            if "up_gate" in self.__dict__:
+                self._in_place_of(1, self.up_gate)
+        return runs
 
     def _in_place_of(self, step, artifact):
         if self._routed:
@@ -266,14 +279,14 @@ class MoEW4A16FFN:
         if self.fused_combine:
             up_gate_packed, down_packed = self._weights(up_gate_packed, down_packed)
             sorted_routes, expert_blocks, total = self.alignment.run(topk_ids)
-            gather, up_gate = self._chain
-            rows = gather.run(x, sorted_routes, total)
+            rows = self._chain[0].run(x, sorted_routes, total)
+            up_gate = self._up_gate_of(clears)
             inputs = self._up_gate_inputs(rows, expert_blocks, total, up_gate_packed, up_gate_scales, sorted_routes,
                                           topk_weights)
             if clears:
                 hidden, y = up_gate.run(*inputs)
             else:
-                hidden = (self._routed_up_gate if self._routed else up_gate).run(*inputs)
+                hidden = up_gate.run(*inputs)
             self.down_scatter(hidden, expert_blocks, total, down_packed, down_scales, sorted_routes, topk_weights, y)
             return y
         rows, positions = self.experts_forward(x, topk_ids, up_gate_packed, up_gate_scales, down_packed,
@@ -294,10 +307,8 @@ class MoEW4A16FFN:
         align = self.alignment.prepare(topk_ids)
         sorted_routes, expert_blocks, total = align.result()
         if self.fused_combine and not clear_positions:
-            gather, up_gate = self._chain
-            if self._routed:
-                up_gate = self._routed_up_gate
-            gather_call = gather.prepare(x, sorted_routes, total)
+            gather_call = self._chain[0].prepare(x, sorted_routes, total)
+            up_gate = self._up_gate_of(False)
             up_call = up_gate.prepare(*self._up_gate_inputs(gather_call.result(), expert_blocks, total, up_gate_packed,
                                                             up_gate_scales, sorted_routes, topk_weights))
             scatter_call = self.down_scatter.prepare(up_call.result(), expert_blocks, total, down_packed, down_scales,

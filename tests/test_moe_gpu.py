@@ -295,6 +295,22 @@ def test_a_layer_says_what_a_call_ran(cuda_device, prelayout):
     assert layer.gather.observation.entry == "intent_b200_moe_gather_rows"
 
 
+def test_a_layer_says_what_the_latest_call_ran(cuda_device):
+    """A call onto a ``y`` that is there, and a prepared one, run another up|gate program than a call that makes its own."""
+    tokens, hidden, intermediate, experts = 64, 256, 128, 4
+    data = ib.workloads.moe_inputs(tokens, hidden, experts, intermediate, dtype=torch.bfloat16, seed=6)
+    dev = {k: v.to(cuda_device) for k, v in data.items()}
+    layer = MoEW4A16FFN(tokens=tokens, hidden=hidden, intermediate=intermediate, experts=experts, target=ib.B200Target(0))
+    ids, weights = layer.route(dev["logits"])
+    args = (dev["x"], ids, weights, dev["up_gate_packed"], dev["up_gate_scales"], dev["down_packed"], dev["down_scales"])
+    y = torch.zeros((tokens, hidden), dtype=torch.float32, device=cuda_device)
+    for call, entry in ((lambda: layer(*args), "clear"), (lambda: layer(*args, y=y), "routed"), (lambda: layer(*args), "clear"),
+                        (lambda: layer.prepare(*args, y).launch(), "routed")):
+        call()
+        assert layer.chain[1].observation.entry == f"intent_b200_moe_grouped_w4a16_upgate_silu_{entry}_bf16"
+        assert layer.up_gate.observation.entry == layer.chain[1].observation.entry
+
+
 @pytest.mark.parametrize("tokens,hidden", [(1, 128), (33, 1152), (300, 256)])
 def test_a_call_clears_its_result(cuda_device, tokens, hidden):
     """The up|gate contraction zero-fills the result: whatever its memory held before, a call gives what adding to a zeroed
