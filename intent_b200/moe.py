@@ -273,7 +273,8 @@ class MoEW4A16FFN:
         """y[t] (+)= sum_c topk_weights[t, c] * FFN_{topk_ids[t, c]}(x[t]); y f32 [T, H]."""
         import torch
 
-        clears = y is None and self._routed and tuple(x.shape) == (topk_weights.shape[0], self.hidden)
+        clears = (y is None and self._routed and isinstance(topk_weights, torch.Tensor)
+                  and tuple(x.shape) == (*topk_weights.shape[:1], self.hidden))
         if y is None and not clears:
             y = torch.zeros((x.shape[0], self.hidden), dtype=torch.float32, device=x.device)
         if self.fused_combine:

@@ -332,6 +332,10 @@ def test_a_call_clears_its_result(cuda_device, tokens, hidden):
     assert layer(*args, y=onto) is onto and torch.equal(onto[-1], torch.ones_like(onto[-1]))
     with pytest.raises((TypeError, ValueError, RuntimeError)):     # one token more than there are weights
         layer(torch.cat((dev["x"], dev["x"][:1])), *args[1:])
+    with pytest.raises(TypeError, match="route_weights must be a torch.Tensor"):
+        layer(*args[:2], weights.tolist(), *args[3:])
+    with pytest.raises(ValueError, match="rank"):
+        layer(*args[:2], weights.sum(), *args[3:])
 
 
 def test_a_call_clears_its_result_ahead(cuda_device):
