@@ -210,14 +210,12 @@ class MoEW4A16FFN:
     def _up_gate_of(self, clears):
         """The up|gate program of a call, from here on that of ``chain``."""
         gather, up_gate = self._chain
-        if not self._routed:
+        if not self._routed or clears is (up_gate is self._clearing_up_gate):
             return up_gate
-        runs = self._clearing_up_gate if clears else self._routed_up_gate
-        if runs is not up_gate:
-            self._chain = (gather, runs)
-            if "up_gate" in self.__dict__:
-                self._in_place_of(1, self.up_gate)
-        return runs
+        self._chain = (gather, self._clearing_up_gate if clears else self._routed_up_gate)
+        if "up_gate" in self.__dict__:
+            self._in_place_of(1, self.up_gate)
+        return self._chain[1]
 
     def _in_place_of(self, step, artifact):
         if self._routed:
@@ -273,8 +271,12 @@ class MoEW4A16FFN:
         """y[t] (+)= sum_c topk_weights[t, c] * FFN_{topk_ids[t, c]}(x[t]); y f32 [T, H]."""
         import torch
 
-        clears = (y is None and self._routed and isinstance(topk_weights, torch.Tensor)
-                  and tuple(x.shape) == (*topk_weights.shape[:1], self.hidden))
+        clears = y is None and self._routed
+        if clears:
+            try:
+                clears = x.shape == (topk_weights.shape[0], self.hidden)
+            except (AttributeError, IndexError):     # refused below
+                clears = False
         if y is None and not clears:
             y = torch.zeros((x.shape[0], self.hidden), dtype=torch.float32, device=x.device)
         if self.fused_combine:
