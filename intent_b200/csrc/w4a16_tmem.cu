@@ -13,11 +13,11 @@
 // 16, instead of 128.
 //
 // What bounds it: per 128 k 600 cycles for a lone tile or a pair of up to 128 rows with all SMs at work - the issue loop (450 of
-// them) and the dequantisers, 290 issue slots of every scheduler (f16 320), hand their blocks to each other; with neither
+// them) and the dequantisers, 320 issue slots of every scheduler (290 with the scales in f32), hand their blocks to each other; with neither
 // conversion nor more than one MMA a block it is 560.  At 256 rows of a pair the MMAs' 1024 cycles count.  A small call is start-up (the
 // wait for the kernel ahead ends 1.3 us after that kernel, first words 1 us later), its k blocks and the exchange between
-// the CTAs of a cluster (2 us).  Against the forms with the weights in shared memory: M77 K14336 N4096 81.1 -> 14.5 us,
-// M1024 K4096 N4096 50.9 -> 28, 64 tokens on 64 experts of 4096 x 1408 414 -> 155 (the whole layer).
+// the CTAs of a cluster (2 us).  Against the forms with the weights in shared memory: M77 K14336 N4096 81.1 -> 14.7 us,
+// M1024 K4096 N4096 50.9 -> 25.3, 64 tokens on 64 experts of 4096 x 1408 414 -> 157 (the whole layer).
 #include <algorithm>
 #include <type_traits>
 
@@ -507,7 +507,9 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             // times a power of two.  The pairs come out of two masked words, a byte of zeros - the sign of a nibble - between.
             // 11 instructions a word instead of 13: M12 K4096 N14336 15.7 -> 15.3 us, M8 K8192 N8192 17.3 -> 16.7.  Weights
             // with their scale keep the other way: the scale times that power of two leaves the type's range (a half from 128
-            // on, a bfloat16 from 2^122), and the choice between two ways costs more than the instructions do.
+            // on, a bfloat16 from 2^122).  In bfloat16, with the factor in the scale / with a vote on the scales between the two
+            // ways / so: M512 K2048 N4096 9.7 / 10.3 / 9.9 us, M24 K4096 N4096 7.05 / 7.45 / 7.20, 64 tokens on 64 experts 155.6 /
+            // 160.0 / 156.8.
             const uint32_t even = lop3_and_xor_u32(w, 0x0F0F0F0Fu, flip), odd = lop3_and_xor_u32(w >> 4, 0x0F0F0F0Fu, flip);
             o[4 * j + 0] = prmt(even, odd, 0xC480);  // (k0, k1)
             o[4 * j + 1] = prmt(even, odd, 0xD591);  // (k2, k3)

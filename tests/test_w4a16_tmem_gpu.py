@@ -239,8 +239,8 @@ def test_threads_launch_one_instance(cuda_device, sizes):
 ])
 def test_rows_of_one_kernel_keep_their_bits(cuda_device, dtype, group, K, N):
     """KERNEL='gemm' adds the k blocks in one order whatever else a call holds: the bits of a row depend neither on the
-    number of rows, nor on the columns beside it, nor on the layout of the weights.  The default may cut K into two or four
-    parts for few rows; the same products are then added in f32 in another order, so that results agree to the rounding
+    number of rows, nor on the columns beside it, nor on the layout of the weights.  The default may cut K into two, four
+    or eight parts for few rows; the same products are then added in f32 in another order, so that results agree to the rounding
     of the output type (half a unit in the last place each: 2^-8 of the value in bf16, 2^-11 in f16; cancellation leaves
     sums that are small against their terms, hence the root mean square beside the value)."""
     M = 2100                                 # runs on another kernel
