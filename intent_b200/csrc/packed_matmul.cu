@@ -92,8 +92,10 @@ __global__ void expand_fp4_kernel(const uint32_t* __restrict__ packed, uint4* __
 template <int ROWS>
 __global__ void int2_gemv_kernel(const int8_t* __restrict__ activation, const uint32_t* __restrict__ packed,
                                  int32_t* __restrict__ out, int M, int N, int K) {
-  programmatic_begin();
   programmatic_wait();
+  // (no programmatic_begin: with several CTAs an SM those of the next launch would be dealt out over the gaps that this one
+  // leaves, some SMs getting more than others.  Begun early / at the end / plain launches, us: M1 K4096 N4096 4.87 / 4.51 / 6.20,
+  // M12 K3840 N9120 42.4 / 32.8 / 34.9, M5 K6656 N7568 30.5 / 23.2 / 24.7)
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
