@@ -823,11 +823,12 @@ int grouped_tmem(int mode, View2 x, View1 tile_expert, View1 total, View3 w, Vie
 // of call, or one that the bandwidth kernel refuses with its own status).  Tiles are spread over clusters of up to eight CTAs
 // as long as every CTA keeps four k blocks (eight in place of four: M16 K8192 N1024 10.1 -> 7.3, M16 K4096 N1024 7.3 -> 5.9).  Against the bandwidth kernel (bf16, group 128, cold weights): M16 K4096 N4096
 // 21.9 -> 9.8 us, M9 18.0 -> 9.6, M16 K8192 N1024 25.4 -> 11.6, M16 K1024 N1024 16.2 -> 6.6, M16 K4096 N14336 47.0 -> 16.4;
-// error against 64 bits 2.08e-4 of 2.09e-4 (f16), 1.673e-3 of 1.673e-3 (bf16).  Against the ride-along kernel (bf16, group
-// 128): M6 K4096 N4096 9.5 -> 7.9 us, K1024 N1024 8.1 -> 6.2, K8192 N8192 18.7 -> 17.3, K8192 N1024 10.4 and 10.4; four rows
-// and fewer are left to it (M4 K8192 N1024 8.2 of 10.4, K4096 N14336 14.9 of 15.7, but K4096 N4096 8.6 of 7.9), and so are
-// calls with more tiles than half the SMs, whose tiles cannot be cut, up to six rows (M6 K4096 N14336 15.6 of 15.7, M8
-// 16.1 of 15.7).
+// error against 64 bits 2.08e-4 of 2.09e-4 (f16), 1.673e-3 of 1.673e-3 (bf16).  Up to eight rows
+// by the lesser of two estimates, fitted to 300 drawn sizes of five to eight rows (K 1024 - 16384, N 128 - 16384): this kernel is
+// bound by the k blocks of a CTA, the ride-along kernel by the bytes of the weights.  M6 K4096 N4096 9.5 -> 7.7 us, K1024 N1024 8.1
+// -> 6.2, K10496 N160 33.3 -> 8.7; left to the other M7 K14592 N5144 18.5 of 25.0, K7040 N10640 19.1 of 26.0.  In those 300 sizes
+// 1.354 times as fast as the ride-along kernel alone on (geometric) average, the better of the two each time 1.358, and 4.8 % slower
+// at worst; in 110 others 1.177 of 1.178, none slower.  Four rows and fewer are left to it (M4 K8192 N1024 8.2 of 10.4, K4096 N14336 14.9 of 15.7, but K4096 N4096 8.6 of 7.9).
 template <typename T>
 int skinny(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, const void* workspace,
            int64_t workspace_bytes, cudaStream_t stream) {
@@ -844,10 +845,14 @@ int skinny(View2 x, View2 w, View2 s, View2 y, int group_size, int zero_point, c
   const int64_t asked = w4a16_stream_workspace_bytes(M, K, N);   // 0: the bandwidth kernel has no plan for the call
   if (asked <= 0 || !workspace || !aligned16(workspace) || workspace_bytes < asked) return kTableDeclined;
   const int64_t tiles = (N + 127) / 128, blocks = (K + 127) / 128, sms = device_sms();
-  if (M <= 6 && 2 * tiles > sms) return kTableDeclined;
   if (M <= 8 && (!selection().table_single || !selection().table_ride)) return kTableDeclined;   // (asked not to take them)
   int split = 1;
   while (split < 8 && tiles * split * 2 <= clustered_ctas(2 * split, sms) && blocks >= 8 * split) split *= 2;
+  if (M <= 8) {
+    const double here = 3.3 + (split > 1 ? 1.2 : 0.0) + 0.38 * double((tiles + sms - 1) / sms * ((blocks + split - 1) / split));
+    const double ride = 7.25 + 0.21e-6 * double(K * N / 2) + 0.2e-3 * double(K);
+    if (here >= ride) return kTableDeclined;
+  }
   TmemCall q{};
   q.x = x.p, q.rows = M, q.K = K;
   q.w = w.p, q.s = s.p, q.experts = 1, q.WN = N;

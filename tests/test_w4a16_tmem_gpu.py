@@ -82,6 +82,27 @@ def test_nine_to_sixteen_rows(cuda_device, dtype, zero_point, group, M, K, N):
     assert error <= before * 1.02       # both are the rounding of the result; 2 % for sums in another order
 
 
+@pytest.mark.parametrize("dtype,group,M,K,N,kernel", [
+    (torch.float16, 128, 7, 14592, 5144, "w4a16_ride_kernel"),      # 57 k blocks for each of 82 CTAs
+    (torch.bfloat16, 32, 8, 6656, 13448, "w4a16_ride_kernel"),      # tiles that cannot be cut
+    (torch.bfloat16, 64, 5, 10496, 160, "w4a16_tmem_kernel 16 rows"),
+    (torch.float16, 128, 8, 2048, 13448, "w4a16_tmem_kernel 16 rows"),
+    (torch.float16, 128, 4, 4096, 4096, "w4a16_ride_kernel"),
+])
+def test_four_to_eight_rows(cuda_device, dtype, group, M, K, N, kernel):
+    """On either side of the line between the two kernels the result is as far from 64 bits as the bandwidth kernel's."""
+    x, p, s = ib.workloads.w4a16_inputs(M, K, N, dtype=dtype, group_size=group, seed=M)
+    constants = {"GROUP_SIZE": group, "ZERO_POINT": 8, "ACT_DTYPE": "f16" if dtype == torch.float16 else "bf16"}
+    artifact = ib.compile(ib.programs.weight_only_int4_matmul, target=ib.B200Target(0), constexprs=constants)
+    out = artifact.run(x.to(cuda_device), p.to(cuda_device), s.to(cuda_device))
+    assert artifact.observation.kernel.startswith(kernel), artifact.observation.kernel
+    torch.cuda.synchronize()
+    artifact.check()
+    exact = x.double() @ ((oracle.unpack_int4(p).double() - 8) * s.double().repeat_interleave(group, dim=0))
+    rounded = exact.to(dtype).double()
+    assert (out.cpu().double() - exact).norm() <= 1.02 * (rounded - exact).norm()   # the rounding of the result; 2 % for the sums
+
+
 @pytest.mark.parametrize("rows_of_expert,hidden,intermediate,block", [
     ((1, 16, 17, 0, 32, 33, 15, 2), 512, 128, 128),            # few rows: lone CTAs
     ((127, 128, 129, 0, 256, 1, 300, 31), 1024, 384, 128),     # blocks full and nearly empty: CTA pairs
